@@ -80,7 +80,7 @@ struct MechContext {
     // linkers / motors
     DeviceBuffer lk_bead, lk_k, lk_l0, lk_s1, lk_s2, lk_sf, mt_bead, mt_k, mt_l0, mt_s1, mt_s2, mt_sf;
     // boundary
-    DeviceBuffer planes, plane_k, plane_slen, bb_k, bb_slen;
+    DeviceBuffer planes, planes_f, plane_k, plane_slen, bb_k, bb_slen;
     // excluded volume
     DeviceBuffer ev_bead, ev_k, ev_la, ev_lb, ev_list, ev_list_count, ev_energy, ev_energy2;
     // tiles, partials, state
@@ -91,8 +91,7 @@ struct MechContext {
     PairBuild pb;
     BndBuild bbuild;
     CsrBuild cb;
-    DeviceBuffer rep_cell, rep_dims, rep_rmax2, rep_rmin2, rep_margin, rep_q, rep_ncyl, rep_plane, rep_cyl, rep_bcut,
-        gather_idx, gather_out;
+    DeviceBuffer nl_rep, gather_out;
     DeviceBuffer perm_all, stage;   // caller -> internal bead map of all replicas; coordinate staging
     // Hessian-vector products, adjoint and Newton solves (FP64 engine)
     DeviceBuffer hv_a, hv_b, cg_x, cg_r, cg_p, cg_Ap, cg_scal, cg_part, cg_ticket;
@@ -288,9 +287,13 @@ __global__ void k_bb_build(const int* bb_plane, long long n, const double* pk, c
     bs[i] = (Real)ps[bb_plane[i]];
 }
 
-__global__ void k_gather_i32(const int* src, const long long* idx, int n, long long* out) {
+// Pair offsets at the replicas' first cylinders, the total, and the number of
+// listed boundary entries, for one read-back.
+__global__ void k_pair_offsets(const int* off, const NLReplica* rep, int R, int ncyl, const int* nbcyl, long long* out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = src[idx[i]];
+    if (i > R) return;
+    out[i] = off[i < R ? rep[i].cyl_begin : ncyl];
+    if (i == R) out[R + 1] = *nbcyl;
 }
 
 // caller order <-> internal order of one replica's coordinates / forces
@@ -333,7 +336,7 @@ struct LoadForceArgs {
     int ntypes, nfil, stride;
     const int* cyl_b1;         // internal first bead of each (global) cylinder
     int cyl_begin, ncyl;
-    const int* bcnt;           // boundary list entry counts of the last rebuild, replica's first entry
+    const uint8_t* bcnt;       // boundary list entry counts of the last rebuild, replica's first entry
     int nplanes;
     const double* planes;      // replica's planes (a, b, c, d)
     const double* plane_k;
@@ -641,7 +644,8 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
         return rc;
     CU(c->lk_sf.ensure(sizeof(double) * std::max(nlk, 1)));
     CU(c->mt_sf.ensure(sizeof(double) * std::max(nmt, 1)));
-    if ((rc = upload(c->planes, planes, s)) || (rc = upload(c->plane_k, pk, s)) || (rc = upload(c->plane_slen, ps, s)))
+    const std::vector<float> planes_f(planes.begin(), planes.end());
+    if ((rc = upload(c->planes, planes, s)) || (rc = upload(c->planes_f, planes_f, s)) || (rc = upload(c->plane_k, pk, s)) || (rc = upload(c->plane_slen, ps, s)))
         return rc;
     // filament tiles (static)
     std::vector<Tile> ft;
@@ -721,10 +725,8 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
     cudaStream_t s = c->stream;
     const int R = c->R;
     // per replica grid
-    std::vector<double> rcell(R), rmax2(R), rmin2(R), bcut(R);
-    std::vector<int4> dims(R);
-    std::vector<float> margin(R);
-    long long ncells = 0;
+    std::vector<NLReplica> rep(R);
+    long long ncells = 0, nq = 0;
     for (int r = 0; r < R; ++r) {
         ReplicaHost& h = c->reps[r];
         double cell = cell_req;
@@ -747,22 +749,35 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
         }
         h.cell = cell;
         h.cell_off = ncells;
+        NLReplica& R1 = rep[r];
+        R1.dims = make_int4(h.gx, h.gy, h.gz, (int)h.cell_off);
         ncells += (long long)h.gx * h.gy * h.gz;
-        rcell[r] = cell;
-        dims[r] = make_int4(h.gx, h.gy, h.gz, (int)h.cell_off);
-        rmax2[r] = (double)(float)(h.rmax * h.rmax);
-        rmin2[r] = 0.0;
-        bcut[r] = h.bcut;
-        // float-midpoint prefilter slack (coordinates up to a few boxes from the origin)
-        const double M = 4.0 * std::max(h.box[0], std::max(h.box[1], h.box[2])) + 1e4;
-        const double delta = (2.0 * M + h.rmax) * 6.0e-8;
-        margin[r] = (float)(2.0 * h.rmax * std::sqrt(3.0) * delta + 3.0 * delta * delta + 4e-7 * h.rmax * h.rmax + 1e-2);
+        R1.rmax2 = (double)(float)(h.rmax * h.rmax);
+        R1.rmin2 = 0.0;
+        const double box = std::max(h.box[0], std::max(h.box[1], h.box[2]));
+        // float-midpoint prefilter slack (coordinates up to a few boxes from the origin; 2 ulp per midpoint)
+        const double M = 4.0 * box + 1e4;
+        const double delta = (2.0 * M + h.rmax) * 1.2e-7;
+        const double slack = 2.0 * h.rmax * std::sqrt(3.0) * delta + 3.0 * delta * delta + 4e-7 * h.rmax * h.rmax + 1e-2;
+        R1.pre = (float)(R1.rmax2 + slack);
+        R1.sure = (float)(R1.rmax2 - slack);
+        // Bins of single-precision midpoints: the edge grows by the rounding of
+        // the two midpoints and of the products with its reciprocal.  Beyond
+        // the box every midpoint falls in the outer bins, so coordinates up to
+        // one edge outside bound that rounding.
+        R1.inv = (float)(1.0 / (cell + 2e-6 * (box + 2.0 * cell)));
+        R1.bnd_cutoff = h.bcut;
+        R1.bnd_begin = h.bq_begin = nq;
+        nq += (long long)h.nplanes * h.ncyl;
+        R1.ncyl = h.ncyl;
+        R1.cyl_begin = h.cyl_begin;
+        R1.plane_begin = h.plane_begin;
+        R1.bnd_cutoff_f = (float)h.bcut;
+        R1.pad = 0;
     }
     if (ncells > 2000000000LL) return set_err(MECH_ERR_CAPACITY, "bin grid too large");
     int rc;
-    if ((rc = upload(c->rep_cell, rcell, s)) || (rc = upload(c->rep_dims, dims, s)) || (rc = upload(c->rep_rmax2, rmax2, s)) ||
-        (rc = upload(c->rep_rmin2, rmin2, s)) || (rc = upload(c->rep_margin, margin, s)) || (rc = upload(c->rep_bcut, bcut, s)))
-        return rc;
+    if ((rc = upload(c->nl_rep, rep, s))) return rc;
     NLInput in{};
     in.ncyl = c->ncyl;
     in.cyl_b1 = c->cyl_b1.as<int>();
@@ -770,12 +785,7 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
     in.cyl_fil = c->cyl_fil.as<int>();
     in.cyl_pos = c->cyl_pos.as<int>();
     in.cyl_rep = c->cyl_rep.as<int>();
-    // current coordinates: replica buffers may differ; gather them into x[0] first
-    in.x = nullptr;
-    in.rep_cell = c->rep_cell.as<double>();
-    in.rep_dims = c->rep_dims.as<int4>();
-    in.rep_rmax2 = c->rep_rmax2.as<double>();
-    in.rep_rmin2 = c->rep_rmin2.as<double>();
+    in.rep = c->nl_rep.as<NLReplica>();
     in.R = R;
     in.ncells = ncells;
     // Current coordinates live in x[xbuf] per replica; canonicalize them to
@@ -783,26 +793,41 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
     if ((rc = canonicalize_x(c))) return rc;
     in.x = c->x[0].p;
     in.mixed = c->precision == MECH_PREC_MIXED;
-    long long P = 0;
-    CU(build_pairs(in, c->pb, c->rep_margin.as<float>(), &P, s));
-    c->nev = P;
-    // per replica pair ranges: pair offsets at the replicas' first cylinders
-    {
-        std::vector<long long> idx(R + 1);
-        for (int r = 0; r < R; ++r) idx[r] = c->reps[r].cyl_begin;
-        idx[R] = c->ncyl;
-        if ((rc = upload(c->gather_idx, idx, s))) return rc;
-        CU(c->gather_out.ensure(sizeof(long long) * (R + 1)));
-        k_gather_i32<<<(R + 1 + 127) / 128, 128, 0, s>>>(c->pb.off.as<int>(), c->gather_idx.as<long long>(), R + 1,
-                                                      c->gather_out.as<long long>());
-        std::vector<long long> o(R + 1);
-        CU(cudaMemcpyAsync(o.data(), c->gather_out.p, sizeof(long long) * (R + 1), cudaMemcpyDeviceToHost, s));
-        CU(cudaStreamSynchronize(s));
-        for (int r = 0; r < R; ++r) {
-            c->reps[r].ev_begin = o[r];
-            c->reps[r].nev = o[r + 1] - o[r];
-        }
+    CU(count_pairs(in, c->pb, s));
+    BndInput bi{};
+    bi.nq = nq;
+    bi.R = R;
+    bi.rep = in.rep;
+    bi.planes = c->planes.as<double>();
+    bi.planes_f = c->planes_f.as<float4>();
+    bi.midf = c->pb.midf.as<float4>();
+    bi.x = in.x;
+    bi.mixed = in.mixed;
+    bi.cyl_b1 = in.cyl_b1;
+    bi.cyl_minus = c->cyl_minus.as<uint8_t>();
+    // list offsets of every replica: boundary beads, then pairs, then the
+    // number of listed boundary entries, in one read-back
+    CU(c->gather_out.ensure(sizeof(long long) * (2 * (size_t)R + 3)));
+    long long* offs = c->gather_out.as<long long>();
+    CU(count_boundary(bi, c->bbuild, offs, s));
+    k_pair_offsets<<<(R + 1 + 127) / 128, 128, 0, s>>>(c->pb.off.as<int>(), in.rep, R, c->ncyl, c->bbuild.ncyl.as<int>(),
+                                                    offs + R + 1);
+    CU(cudaGetLastError());
+    std::vector<long long> o(2 * (size_t)R + 3);
+    CU(cudaMemcpyAsync(o.data(), offs, sizeof(long long) * o.size(), cudaMemcpyDeviceToHost, s));
+    CU(cudaStreamSynchronize(s));
+    for (int r = 0; r < R; ++r) {
+        c->reps[r].bb_begin = o[r];
+        c->reps[r].nbb = o[r + 1] - o[r];
+        c->reps[r].ev_begin = o[R + 1 + r];
+        c->reps[r].nev = o[R + 2 + r] - o[R + 1 + r];
     }
+    const long long P = o[2 * (size_t)R + 1], nbb = o[R];
+    c->nev = P;
+    c->nbb = nbb;
+    c->nbcyl = o[2 * (size_t)R + 2];
+    CU(write_pairs(in, c->pb, P, s));
+    CU(write_boundary(bi, c->bbuild, nbb, s));
     const size_t rs = real_size(c);
     CU(c->ev_bead.ensure(sizeof(int4) * std::max<long long>(P, 1)));
     CU(c->ev_k.ensure(rs * std::max<long long>(P, 1)));
@@ -825,50 +850,8 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
                                                   c->cyl_type.as<int>(), c->cyl_l0.as<double>(), c->ev_bead.as<int4>(),
                                                   c->ev_k.as<float>(), c->ev_la.as<float>(), c->ev_lb.as<float>());
     }
-    // boundary lists
+    // boundary constants
     {
-        std::vector<long long> rq(R);
-        std::vector<int> rnc(R), rpl(R), rcy(R);
-        long long nq = 0;
-        for (int r = 0; r < R; ++r) {
-            rq[r] = nq;
-            rnc[r] = c->reps[r].ncyl;
-            rpl[r] = c->reps[r].plane_begin;
-            rcy[r] = c->reps[r].cyl_begin;
-            nq += (long long)c->reps[r].nplanes * c->reps[r].ncyl;
-        }
-        if ((rc = upload(c->rep_q, rq, s)) || (rc = upload(c->rep_ncyl, rnc, s)) || (rc = upload(c->rep_plane, rpl, s)) ||
-            (rc = upload(c->rep_cyl, rcy, s)))
-            return rc;
-        BndInput bi{};
-        bi.nq = nq;
-        bi.R = R;
-        bi.rep_q = c->rep_q.as<long long>();
-        bi.rep_ncyl = c->rep_ncyl.as<int>();
-        bi.rep_plane = c->rep_plane.as<int>();
-        bi.rep_cyl = c->rep_cyl.as<int>();
-        bi.cutoff = c->rep_bcut.as<double>();
-        bi.planes = c->planes.as<double>();
-        bi.cyl_b1 = c->cyl_b1.as<int>();
-        bi.cyl_minus = c->cyl_minus.as<uint8_t>();
-        long long nbb = 0, nbcyl = 0;
-        CU(build_boundary(bi, c->pb.mid.as<double>(), c->bbuild, &nbb, &nbcyl, s));
-        c->nbb = nbb;
-        c->nbcyl = nbcyl;
-        for (int r = 0; r < R; ++r) c->reps[r].bq_begin = rq[r];
-        std::vector<long long> idx(R + 1);
-        for (int r = 0; r < R; ++r) idx[r] = rq[r];
-        idx[R] = nq;
-        if ((rc = upload(c->gather_idx, idx, s))) return rc;
-        k_gather_i32<<<(R + 1 + 127) / 128, 128, 0, s>>>(c->bbuild.off.as<int>(), c->gather_idx.as<long long>(), R + 1,
-                                                      c->gather_out.as<long long>());
-        std::vector<long long> o(R + 1);
-        CU(cudaMemcpyAsync(o.data(), c->gather_out.p, sizeof(long long) * (R + 1), cudaMemcpyDeviceToHost, s));
-        CU(cudaStreamSynchronize(s));
-        for (int r = 0; r < R; ++r) {
-            c->reps[r].bb_begin = o[r];
-            c->reps[r].nbb = o[r + 1] - o[r];
-        }
         CU(c->bb_k.ensure(rs * std::max<long long>(nbb, 1)));
         CU(c->bb_slen.ensure(rs * std::max<long long>(nbb, 1)));
         if (nbb > 0) {
@@ -1533,9 +1516,9 @@ int32_t mech_get_boundary_list(MechContext* ctx, int32_t r, int32_t* entries, in
     if (!ctx->have_lists) return set_err(MECH_ERR_STATE, "no lists");
     const ReplicaHost& h = ctx->reps[r];
     const long long nq = (long long)h.nplanes * h.ncyl;
-    std::vector<int> cnt((size_t)std::max(nq, 1LL));
+    std::vector<uint8_t> cnt((size_t)std::max(nq, 1LL));
     if (nq > 0)
-        CU(cudaMemcpy(cnt.data(), ctx->bbuild.cnt.as<int>() + h.bq_begin, sizeof(int) * nq, cudaMemcpyDeviceToHost));
+        CU(cudaMemcpy(cnt.data(), ctx->bbuild.cnt.as<uint8_t>() + h.bq_begin, (size_t)nq, cudaMemcpyDeviceToHost));
     long long k = 0;
     for (long long q = 0; q < nq; ++q) {
         if (!cnt[q]) continue;
@@ -1578,7 +1561,7 @@ int32_t mech_load_forces(MechContext* ctx, int32_t r, int32_t n_types, const dou
     a.cyl_b1 = ctx->cyl_b1.as<int>();
     a.cyl_begin = h.cyl_begin;
     a.ncyl = h.ncyl;
-    a.bcnt = ctx->bbuild.cnt.as<int>() + h.bq_begin;
+    a.bcnt = ctx->bbuild.cnt.as<uint8_t>() + h.bq_begin;
     a.nplanes = h.nplanes;
     a.planes = ctx->planes.as<double>() + 4 * (size_t)h.plane_begin;
     a.plane_k = ctx->plane_k.as<double>() + h.plane_begin;
