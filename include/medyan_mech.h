@@ -250,7 +250,7 @@ int32_t mech_get_forces(MechContext* ctx, int32_t replica, double* f_out);
 
 /*
  * How mech_minimize drives the device.  MECH_GRAPH_UNROLLED (default): a graph
- * of 8 unrolled iteration blocks (line search: 2 single-trial passes, FP64,
+ * of 2, in longer runs 8, unrolled iteration blocks (line search: 2 single-trial passes, FP64,
  * or one two-trial pass, mixed; forces, direction,
  * reset) relaunched by the host, every kernel reading its replica's phase and
  * exiting when it has nothing to do.  MECH_GRAPH_CONDITIONAL: one CUDA graph

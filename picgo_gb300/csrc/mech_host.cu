@@ -84,7 +84,7 @@ struct MechContext {
     // excluded volume
     DeviceBuffer ev_bead, ev_k, ev_la, ev_lb, ev_list, ev_list_count, ev_energy, ev_energy2;
     // tiles, partials, state
-    DeviceBuffer ftile, stile, stile_kind, rt, part_fil, part_sp, part_sp2, st, ticket, gticket, err, cond_counter;
+    DeviceBuffer ftile, stile, stile_kind, rt, part_fil, part_sp, part_sp2, st, ticket, gticket, cond_counter;
     int graph_mode = MECH_GRAPH_UNROLLED;
     DeviceBuffer contrib, ev_fb_count, ev_fb_list, ev_fb_energy, fb_moments, fb_tickets;
     // rebuild scratch
@@ -95,6 +95,7 @@ struct MechContext {
     DeviceBuffer perm_all, stage;   // caller -> internal bead map of all replicas; coordinate staging
     // Hessian-vector products, adjoint and Newton solves (FP64 engine)
     DeviceBuffer hv_a, hv_b, cg_x, cg_r, cg_p, cg_Ap, cg_scal, cg_part, cg_ticket;
+    DeviceBuffer lf_ends, lf_types, lf_ms, lf_nm, lf_out;   // load forces
     DeviceBuffer gbar;   // grid barrier of the cooperative iteration tail (2 unsigned)
     int n_ftiles = 0, n_stiles = 0;
     int sp_tiles[K_NUM_SPARSE] = {0, 0, 0, 0};
@@ -123,15 +124,33 @@ struct MechContext {
     int sp_tiles_c[K_NUM_SPARSE] = {0, 0, 0, 0};
     int slot_base[K_NUM_SPARSE + 1] = {0, 0, 0, 0, 0};
     std::vector<RepTiles> h_rt;
-    CGState* h_st = nullptr;   // pinned mirror of the states
+    // pinned mirror of the states, followed by the error word as on the device
+    // (one copy brings both); `h_fresh` while no launch has changed the device's
+    // since, so that a call which needs a replica's buffer index need not ask for it
+    CGState* h_st = nullptr;
     unsigned* h_err = nullptr;
-    // pinned snapshots taken after each minimizer graph launch: states, error
-    // word and the conditional graph's body counters, double-buffered
+    bool h_fresh = false;
+    int h_cap = 0;             // replicas the pinned buffers hold
+    unsigned* d_err() const { return reinterpret_cast<unsigned*>(st.as<CGState>() + R); }
+    // pinned snapshots taken after each minimizer graph launch (k_snapshot):
+    // error word, the conditional graph's body counters, then every replica's
+    // phase; double-buffered
     struct Snapshot {
-        CGState* st = nullptr;
-        unsigned* err = nullptr;   // [0] error word, [1..8] body counters
+        int* word = nullptr;       // [0] error word, [1..8] body counters, [9 + r] phases
         cudaEvent_t done = nullptr;
+        int launches = 0;          // kernels of the unrolled graph it follows
+        unsigned err() const { return (unsigned)word[0]; }
+        const int* phase() const { return word + 9; }
     } snap[2];
+    cudaEvent_t t0 = nullptr, t1 = nullptr;   // device time of a minimization
+    // The unrolled iteration graphs (short and long, kGraphBlocks) of the last
+    // minimizations and the launch arguments they were built for: equal
+    // arguments reuse a graph, others update it in place where its shape allows.
+    struct IterGraph {
+        cudaGraphExec_t exec = nullptr;
+        std::vector<unsigned char> key;
+        int launches = 0;
+    } iter[2];
     MechTiming timing{};
 #ifdef MECH_TRACE
     DeviceBuffer trace;   // kernel timeline of the diagnostic build (MECH_TRACE_FILE names the dump)
@@ -139,13 +158,15 @@ struct MechContext {
     std::vector<int32_t> cyl_local_first;   // replica-local cylinder -> internal global first bead
 
     ~MechContext() {
+        for (auto& g : iter)
+            if (g.exec) cudaGraphExecDestroy(g.exec);
         if (h_st) cudaFreeHost(h_st);
-        if (h_err) cudaFreeHost(h_err);
         for (auto& k : snap) {
-            if (k.st) cudaFreeHost(k.st);
-            if (k.err) cudaFreeHost(k.err);
+            if (k.word) cudaFreeHost(k.word);
             if (k.done) cudaEventDestroy(k.done);
         }
+        if (t0) cudaEventDestroy(t0);
+        if (t1) cudaEventDestroy(t1);
         if (fork) cudaEventDestroy(fork);
         if (join) cudaEventDestroy(join);
         if (join2) cudaEventDestroy(join2);
@@ -166,7 +187,8 @@ int upload(DeviceBuffer& b, const std::vector<T>& v, cudaStream_t s) {
 
 template <typename Real>
 DevNet<Real> make_devnet(MechContext* c) {
-    DevNet<Real> n{};
+    DevNet<Real> n;
+    std::memset(&n, 0, sizeof(n));   // padding too: the bytes are compared (iteration_graph)
     n.nb = c->nb;
     n.R = c->R;
     n.x[0] = c->x[0].as<Real>();
@@ -246,7 +268,7 @@ DevNet<Real> make_devnet(MechContext* c) {
     n.rt = (c->compact ? c->rt_c : c->rt).as<RepTiles>();
     n.ticket = c->ticket.as<int>();
     n.gticket = c->gticket.as<int>();
-    n.err = c->err.as<unsigned>();
+    n.err = c->d_err();
 #ifdef MECH_TRACE
     n.trace = c->trace.as<unsigned long long>();
 #endif
@@ -411,6 +433,29 @@ __global__ void k_gather_coords(const Real* in, const int* perm, int nb, int bas
     out[3 * (size_t)i + 2] = (double)in[3 * (size_t)j + 2];
 }
 
+// A minimization's initial states: everything but the buffer indices afresh.
+__global__ void k_cg_reset(CGState* st, const RepTiles* rt, int R, MechCGParams p) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= R) return;
+    CGState S;
+    memset(&S, 0, sizeof(S));
+    S.xbuf = st[r].xbuf;
+    S.fbuf = st[r].fbuf;
+    S.method = p.method;
+    S.maxDist = p.max_dist;
+    S.lambdaMax = p.lambda_max;
+    S.gradTol = p.grad_tol;
+    S.energyRelTol = p.energy_rel_tol;
+    S.energyCallLimit = p.energy_call_limit;
+    S.forceCallLimit = max(p.force_call_limit, 3 * rt[r].n_beads);
+    S.tryToRecover = p.try_to_recover;
+    S.minimumE = S.maxF = S.energyRelChange = 1.0 / 0.0;
+    S.active = 1;
+    S.phase = PH_IDLE;
+    st[r] = S;
+}
+
+// After the first energies and forces: energiesBefore, then the loop head.
 __global__ void k_cg_init(CGState* st, int R) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= R) return;
@@ -418,6 +463,7 @@ __global__ void k_cg_init(CGState* st, int R) {
     if (!S.active) return;
     S.numEnergyCall = 1;
     S.numForceCall = 1;
+    for (int k = 0; k <= MECH_NUM_FF; ++k) S.before[k] = S.eval[k];
     S.prevEnergy = S.eval[MECH_NUM_FF];   // energiesBefore.total
     if (!isfinite(S.maxF)) {
         S.status = MECH_ERR_NONFINITE;
@@ -425,6 +471,23 @@ __global__ void k_cg_init(CGState* st, int R) {
         return;
     }
     S.phase = PH_RESET;                   // resetCGParams, then the loop head
+}
+
+// A call-limit exit restores the minimum-energy backup (CGMethod.hpp:1589-1610).
+__global__ void k_cg_finish(CGState* st, int R, int report_on_call_limit) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= R) return;
+    CGState& S = st[r];
+    S.restore = report_on_call_limit && call_limit(S) && S.backupValid;
+    S.active = 1;
+}
+
+// What the host looks at after each graph launch, written to pinned memory:
+// the error word, the conditional graph's body counters and every phase.
+__global__ void k_snapshot(const CGState* st, int R, const unsigned* err, const int* counters, int* out) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < 9) out[r] = r == 0 ? (int)*err : counters[r - 1];
+    if (r < R) out[9 + r] = st[r].phase;
 }
 
 // the replica's slice of the caller -> internal map (replica-local indices)
@@ -444,7 +507,7 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
     c->reps.assign(R, ReplicaHost());
     c->R = R;
     int nb = 0, ncyl = 0, nlk = 0, nmt = 0, npl = 0;
-    std::vector<double> x, kstr, l0b, kbend, t0, cyl_kex, cyl_l0, lkk, lkl, lks1, lks2, mtk, mtl, mts1, mts2, planes,
+    std::vector<double> kstr, l0b, kbend, t0, cyl_kex, cyl_l0, lkk, lkl, lks1, lks2, mtk, mtl, mts1, mts2, planes,
         pk, ps;
     std::vector<uint8_t> flags, minus;
     std::vector<int> cyl_b1, cyl_fil, cyl_pos, cyl_rep, cyl_type;
@@ -502,15 +565,11 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
         }
         if (li != N.n_beads) return set_err(MECH_ERR_TOPOLOGY, "beads outside filaments");
         // bead arrays in internal order
-        const size_t xoff = x.size();
-        x.resize(xoff + 3 * (size_t)N.n_beads);
         flags.resize(nb + N.n_beads, 0);
         kstr.resize(nb + N.n_beads, 0.0);
         l0b.resize(nb + N.n_beads, 0.0);
         kbend.resize(nb + N.n_beads, 0.0);
         t0.resize(nb + N.n_beads, 0.0);
-        for (int b = 0; b < N.n_beads; ++b)
-            for (int k = 0; k < 3; ++k) x[xoff + 3 * (size_t)h.perm[b] + k] = N.coord[3 * (size_t)b + k];
         for (int f = 0; f < N.n_filaments; ++f) {
             const int cs = N.fil_cyl_start[f], ce = N.fil_cyl_start[f + 1];
             for (int cc = cs; cc < ce; ++cc) {
@@ -591,35 +650,34 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
     const size_t rs = real_size(c);
     int rc;
     // positions in the engine's format (24 bytes per bead either way)
-    {
-        DeviceBuffer xd, ident;
-        if ((rc = upload(xd, x, s))) return rc;
-        std::vector<int> id(nb);
-        for (int i = 0; i < nb; ++i) id[i] = i;
-        if ((rc = upload(ident, id, s))) return rc;
-        CU(c->x[0].ensure(sizeof(double) * x.size() + kBulkPad));
+    const size_t nx = 3 * (size_t)nb;
+    CU(c->x[0].ensure(sizeof(double) * nx + kBulkPad));
+    for (int r = 0; r < R; ++r) {
+        const ReplicaHost& h = c->reps[r];
+        double* in = c->stage.as<double>() + 3 * (size_t)h.bead_begin;
+        CU(cudaMemcpyAsync(in, nets[r].coord, sizeof(double) * 3 * h.nb, cudaMemcpyHostToDevice, s));
+        const unsigned nblk = (unsigned)((h.nb + 255) / 256);
         if (c->precision == MECH_PREC_FP64)
-            k_scatter_coords<double><<<(nb + 255) / 256, 256, 0, s>>>(xd.as<double>(), ident.as<int>(), nb, 0, c->x[0].as<double>());
+            k_scatter_coords<double><<<nblk, 256, 0, s>>>(in, perm_of(c, r), h.nb, h.bead_begin, c->x[0].as<double>());
         else
-            k_scatter_coords<float><<<(nb + 255) / 256, 256, 0, s>>>(xd.as<double>(), ident.as<int>(), nb, 0, c->x[0].as<float>());
-        CU(cudaGetLastError());
-        CU(cudaStreamSynchronize(s));
+            k_scatter_coords<float><<<nblk, 256, 0, s>>>(in, perm_of(c, r), h.nb, h.bead_begin, c->x[0].as<float>());
     }
-    CU(c->x[1].ensure(sizeof(double) * x.size() + kBulkPad));
-    CU(cudaMemcpyAsync(c->x[1].p, c->x[0].p, sizeof(double) * x.size(), cudaMemcpyDeviceToDevice, s));
+    CU(cudaGetLastError());
+    CU(c->x[1].ensure(sizeof(double) * nx + kBulkPad));
+    CU(cudaMemcpyAsync(c->x[1].p, c->x[0].p, sizeof(double) * nx, cudaMemcpyDeviceToDevice, s));
     if (c->precision == MECH_PREC_MIXED) {   // the second trial buffer of the two-trial line-search passes
-        CU(c->x[2].ensure(sizeof(double) * x.size() + kBulkPad));
-        CU(cudaMemcpyAsync(c->x[2].p, c->x[0].p, sizeof(double) * x.size(), cudaMemcpyDeviceToDevice, s));
+        CU(c->x[2].ensure(sizeof(double) * nx + kBulkPad));
+        CU(cudaMemcpyAsync(c->x[2].p, c->x[0].p, sizeof(double) * nx, cudaMemcpyDeviceToDevice, s));
     }
-    CU(c->xbest.ensure(sizeof(double) * x.size()));
-    CU(c->xinit.ensure(sizeof(double) * x.size()));
-    CU(cudaMemcpyAsync(c->xinit.p, c->x[0].p, sizeof(double) * x.size(), cudaMemcpyDeviceToDevice, s));
-    CU(c->f[0].ensure(rs * x.size() + kBulkPad));
-    CU(c->f[1].ensure(rs * x.size() + kBulkPad));
-    CU(c->d.ensure(rs * x.size() + kBulkPad));
-    CU(cudaMemsetAsync(c->f[0].p, 0, rs * x.size(), s));
-    CU(cudaMemsetAsync(c->f[1].p, 0, rs * x.size(), s));
-    CU(cudaMemsetAsync(c->d.p, 0, rs * x.size(), s));
+    CU(c->xbest.ensure(sizeof(double) * nx));
+    CU(c->xinit.ensure(sizeof(double) * nx));
+    CU(cudaMemcpyAsync(c->xinit.p, c->x[0].p, sizeof(double) * nx, cudaMemcpyDeviceToDevice, s));
+    CU(c->f[0].ensure(rs * nx + kBulkPad));
+    CU(c->f[1].ensure(rs * nx + kBulkPad));
+    CU(c->d.ensure(rs * nx + kBulkPad));
+    CU(cudaMemsetAsync(c->f[0].p, 0, rs * nx, s));
+    CU(cudaMemsetAsync(c->f[1].p, 0, rs * nx, s));
+    CU(cudaMemsetAsync(c->d.p, 0, rs * nx, s));
     flags.resize((size_t)nb + 32, 0);   // tail padding read by 16-byte-rounded bulk copies
     if ((rc = upload(c->bflag, flags, s))) return rc;
     {
@@ -656,6 +714,7 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
         for (int b = 0; b < h.nb; b += kFilTile)
             ft.push_back(Tile{r, h.bead_begin + b, h.bead_begin + std::min(h.nb, b + kFilTile), 0});
         c->h_rt[r].fil_end = (int)ft.size();
+        c->h_rt[r].n_beads = h.nb;
     }
     c->n_ftiles = (int)ft.size();
     c->h_ftiles = ft;
@@ -663,16 +722,14 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
     if ((rc = upload(c->ftile, ft, s))) return rc;
     CU(c->part_fil.ensure(sizeof(double) * 4 * ft.size()));
     // states
-    CU(c->st.ensure(sizeof(CGState) * R));
-    CU(cudaMemsetAsync(c->st.p, 0, sizeof(CGState) * R, s));
+    CU(c->st.ensure(sizeof(CGState) * R + 16));
+    CU(cudaMemsetAsync(c->st.p, 0, sizeof(CGState) * R + 16, s));
     CU(c->ticket.ensure(sizeof(int) * R));
     CU(cudaMemsetAsync(c->ticket.p, 0, sizeof(int) * R, s));
     CU(c->gticket.ensure(sizeof(int) * 4));
     CU(cudaMemsetAsync(c->gticket.p, 0, sizeof(int) * 4, s));
     CU(c->cond_counter.ensure(sizeof(int) * 8));
     CU(cudaMemsetAsync(c->cond_counter.p, 0, sizeof(int) * 8, s));
-    CU(c->err.ensure(sizeof(unsigned) * 4));
-    CU(cudaMemsetAsync(c->err.p, 0, sizeof(unsigned) * 4, s));
     CU(c->ev_fb_count.ensure(sizeof(int) * 4));
     CU(cudaMemsetAsync(c->ev_fb_count.p, 0, sizeof(int) * 4, s));
     CU(c->ev_fb_list.ensure(sizeof(int) * 2 * kExvolFallbackCap));
@@ -680,17 +737,26 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
     CU(c->fb_moments.ensure(sizeof(double) * 6 * kFbChunks * (size_t)kExvolFallbackCap));
     CU(c->fb_tickets.ensure(sizeof(int) * kExvolFallbackCap));
     CU(cudaMemsetAsync(c->fb_tickets.p, 0, sizeof(int) * kExvolFallbackCap, s));
-    if (c->h_st) cudaFreeHost(c->h_st);
-    CU(cudaMallocHost(&c->h_st, sizeof(CGState) * R));
-    if (!c->h_err) CU(cudaMallocHost(&c->h_err, sizeof(unsigned) * 4));
-    for (auto& k : c->snap) {
-        if (k.st) cudaFreeHost(k.st);
-        k.st = nullptr;
-        CU(cudaMallocHost(&k.st, sizeof(CGState) * R));
-        if (!k.err) CU(cudaMallocHost(&k.err, sizeof(unsigned) * 9));
-        if (!k.done) CU(cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming));
+    if (c->h_cap < R) {   // pinned allocations take ~100 us each: kept while they hold the replicas
+        c->h_cap = 0;
+        if (c->h_st) cudaFreeHost(c->h_st);
+        c->h_st = nullptr;
+        CU(cudaMallocHost(&c->h_st, sizeof(CGState) * R + 16));
+        for (auto& k : c->snap) {
+            if (k.word) cudaFreeHost(k.word);
+            k.word = nullptr;
+            CU(cudaMallocHost(&k.word, sizeof(int) * (9 + (size_t)R)));
+        }
+        c->h_cap = R;
     }
+    for (auto& k : c->snap)
+        if (!k.done) CU(cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming));
+    if (!c->t0) CU(cudaEventCreate(&c->t0));
+    if (!c->t1) CU(cudaEventCreate(&c->t1));
     CU(cudaStreamSynchronize(s));
+    std::memset(c->h_st, 0, sizeof(CGState) * R + 16);   // as on the device
+    c->h_err = reinterpret_cast<unsigned*>(c->h_st + R);
+    c->h_fresh = true;
     c->have_net = true;
     c->have_lists = false;
     return MECH_OK;
@@ -699,12 +765,45 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
 // ===========================================================================
 // neighbor lists
 // ===========================================================================
+// The states and the error word to the pinned mirror.
+static int pull_states(MechContext* c) {
+    CU(cudaMemcpyAsync(c->h_st, c->st.p, sizeof(CGState) * c->R + sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    CU(cudaStreamSynchronize(c->stream));
+    c->h_fresh = true;
+    return MECH_OK;
+}
+// The mirror, up to date.
+static int states(MechContext* c) { return c->h_fresh ? MECH_OK : pull_states(c); }
+// The mirror's states to the device; the mirror is not written again before the stream is waited for.
+static int push_states(MechContext* c) {
+    CU(cudaMemcpyAsync(c->st.p, c->h_st, sizeof(CGState) * c->R, cudaMemcpyHostToDevice, c->stream));
+    return MECH_OK;
+}
+// Replicas an evaluation works on: all (replica < 0) or one.
+static int select_replicas(MechContext* c, int replica) {
+    int rc;
+    if ((rc = states(c))) return rc;
+    bool same = true;
+    for (int r = 0; r < c->R; ++r) {
+        const int a = replica < 0 || r == replica;
+        same = same && c->h_st[r].active == a;
+        c->h_st[r].active = a;
+    }
+    return same ? MECH_OK : push_states(c);
+}
+// Zero the device's error word, unless it is known to be zero.
+static int clear_error(MechContext* c) {
+    if (c->h_fresh && *c->h_err == 0) return MECH_OK;
+    CU(cudaMemsetAsync(c->d_err(), 0, sizeof(unsigned), c->stream));
+    return MECH_OK;
+}
+
 // Bring every replica's current coordinates to x[0] (a replica whose last
 // accepted step left them in a trial buffer is copied back) and reset its xbuf.
 static int canonicalize_x(MechContext* c) {
     cudaStream_t s = c->stream;
-    CU(cudaMemcpyAsync(c->h_st, c->st.p, sizeof(CGState) * c->R, cudaMemcpyDeviceToHost, s));
-    CU(cudaStreamSynchronize(s));
+    int rc;
+    if ((rc = states(c))) return rc;
     bool moved = false;
     for (int r = 0; r < c->R; ++r) {
         if (c->h_st[r].xbuf) {
@@ -716,7 +815,9 @@ static int canonicalize_x(MechContext* c) {
             moved = true;
         }
     }
-    if (moved) CU(cudaMemcpyAsync(c->st.p, c->h_st, sizeof(CGState) * c->R, cudaMemcpyHostToDevice, s));
+    if (!moved) return MECH_OK;
+    if ((rc = push_states(c))) return rc;
+    CU(cudaStreamSynchronize(s));
     return MECH_OK;
 }
 
@@ -929,12 +1030,6 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
 // ===========================================================================
 // evaluation and minimization
 // ===========================================================================
-static int pull_states(MechContext* c) {
-    CU(cudaMemcpyAsync(c->h_st, c->st.p, sizeof(CGState) * c->R, cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaMemcpyAsync(c->h_err, c->err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaStreamSynchronize(c->stream));
-    return MECH_OK;
-}
 // Status of the device error word's bits (kernels set them with atomicOr).
 static int err_status(unsigned bits) {
     if (bits & 64u) return set_err(MECH_ERR_ITER_LIMIT, "a grid barrier of the cooperative iteration tail timed out");
@@ -945,38 +1040,48 @@ static int err_status(unsigned bits) {
     return set_err(MECH_ERR_CAPACITY, "excluded-volume work list overflow");
 }
 
-static int push_states(MechContext* c) {
-    CU(cudaMemcpyAsync(c->st.p, c->h_st, sizeof(CGState) * c->R, cudaMemcpyHostToDevice, c->stream));
-    return MECH_OK;
-}
-
 template <typename Real>
 static int eval_energy(MechContext* c, int replica) {
     int rc;
-    if ((rc = pull_states(c))) return rc;
-    for (int r = 0; r < c->R; ++r) c->h_st[r].active = (replica < 0 || r == replica);
-    if ((rc = push_states(c))) return rc;
-    CU(cudaMemsetAsync(c->err.p, 0, sizeof(unsigned), c->stream));
+    if ((rc = select_replicas(c, replica)) || (rc = clear_error(c))) return rc;
     const DevNet<Real> n = make_devnet<Real>(c);
+    c->h_fresh = false;
     c->timing.launches += launch_energy<Real>(n, -1, 0, c->lanes());
     CU(cudaGetLastError());
     return pull_states(c);
 }
 
+// One replica's forces with f_out: they are gathered from the buffer the
+// evaluation is about to make current, so that one synchronization serves the
+// evaluation and the read-back.
 template <typename Real>
-static int eval_forces(MechContext* c, int replica) {
+static int eval_forces(MechContext* c, int replica, double* f_out = nullptr) {
     int rc;
-    if ((rc = pull_states(c))) return rc;
-    for (int r = 0; r < c->R; ++r) c->h_st[r].active = (replica < 0 || r == replica);
-    if ((rc = push_states(c))) return rc;
-    CU(cudaMemsetAsync(c->err.p, 0, sizeof(unsigned), c->stream));
+    if ((rc = select_replicas(c, replica)) || (rc = clear_error(c))) return rc;
     const DevNet<Real> n = make_devnet<Real>(c);
+    c->h_fresh = false;
     c->timing.launches += launch_forces<Real>(n, -1, c->lanes());
+    if (f_out) {
+        const ReplicaHost& h = c->reps[replica];
+        const Real* f = c->f[c->h_st[replica].fbuf ^ 1].as<Real>();
+        k_gather_coords<Real><<<(h.nb + 255) / 256, 256, 0, c->stream>>>(f, perm_of(c, replica), h.nb, h.bead_begin,
+                                                                       c->stage.as<double>());
+        CU(cudaGetLastError());
+        CU(cudaMemcpyAsync(f_out, c->stage.p, sizeof(double) * 3 * h.nb, cudaMemcpyDeviceToHost, c->stream));
+    }
     CU(cudaGetLastError());
     return pull_states(c);
 }
 
-static constexpr int kBlocksPerGraph = 8;
+// Iteration blocks per graph.  The host looks at the states after each graph
+// and has launched the next one by then, so a minimization that ends runs on
+// average 1.5 graphs of kernels that find nothing to do (25 us a block: 0.3 ms
+// with 8 blocks), while each graph's start and snapshot cost ~8 us (151 us
+// per iteration of the 1M-cylinder network with 2 blocks, 147 with 8).  So a
+// minimization starts on the short graph and goes to the long one when it has
+// run long enough for that one's construction (0.2 ms) to pay.
+static constexpr int kGraphBlocks[2] = {2, 8};
+static constexpr int kShortGraphs = 64;
 // Line-search launches per iteration block: FP64, two single-trial passes;
 // mixed, one two-trial pass (lambda and lambda / 2).
 template <typename Real>
@@ -985,8 +1090,13 @@ static int trial_launches(const DevNet<Real>& n, const Lanes& L) {
     return launch_energy<Real>(n, PH_LS_TRIAL, 1, L) + launch_energy<Real>(n, PH_LS_TRIAL, 1, L);
 }
 
+// The unrolled iteration graph of kGraphBlocks[which] blocks for the context's
+// present networks, lists and tuning, in c->iter[which]: as it is when its
+// launch arguments are unchanged, updated in place when only they changed,
+// else instantiated.
 template <typename Real>
-static int capture_iteration_graph(MechContext* c, cudaGraphExec_t* exec, int* nlaunch) {
+static int iteration_graph(MechContext* c, int which) {
+    auto& ig = c->iter[which];
     DevNet<Real> n = make_devnet<Real>(c);
     n.pdl = c->graph_mode == MECH_GRAPH_UNROLLED_PDL ? 1 : 0;
     // the cooperative tail: mixed engine, one replica (its blocks reduce for replica 0)
@@ -998,10 +1108,16 @@ static int capture_iteration_graph(MechContext* c, cudaGraphExec_t* exec, int* n
         CU(cudaMemsetAsync(c->gbar.p, 0, 2 * sizeof(unsigned), c->stream));
         n.gbar = c->gbar.as<unsigned>();
     }
+    std::vector<unsigned char> key(sizeof(n) + 2 * sizeof(int));
+    const int form[2] = {c->graph_mode, coop_grid};
+    std::memcpy(key.data(), &n, sizeof(n));
+    std::memcpy(key.data() + sizeof(n), form, sizeof(form));
+    if (ig.exec && key == ig.key) return MECH_OK;
+    ig.key.clear();
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int k = 0;
-    for (int b = 0; b < kBlocksPerGraph; ++b) {
+    for (int b = 0; b < kGraphBlocks[which]; ++b) {
         k += trial_launches<Real>(n, c->lanes());
         if (coop_grid > 0) {
             k += launch_forces<Real>(n, PH_FORCE, c->lanes(), coop_grid);
@@ -1013,10 +1129,22 @@ static int capture_iteration_graph(MechContext* c, cudaGraphExec_t* exec, int* n
     }
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (e != cudaSuccess) return set_err(MECH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiate(exec, g, cudaGraphInstantiateFlagUseNodePriority);
+    if (ig.exec) {
+        cudaGraphExecUpdateResultInfo info;
+        if (cudaGraphExecUpdate(ig.exec, g, &info) != cudaSuccess) {
+            cudaGetLastError();   // another shape: a new graph below
+            cudaGraphExecDestroy(ig.exec);
+            ig.exec = nullptr;
+        }
+    }
+    if (!ig.exec) e = cudaGraphInstantiate(&ig.exec, g, cudaGraphInstantiateFlagUseNodePriority);
     cudaGraphDestroy(g);
-    if (e != cudaSuccess) return set_err(MECH_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    *nlaunch = k;
+    if (e != cudaSuccess) {
+        ig.exec = nullptr;
+        return set_err(MECH_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+    }
+    ig.key = std::move(key);
+    ig.launches = k;
     return MECH_OK;
 }
 
@@ -1127,6 +1255,7 @@ static int compact_tiles(MechContext* c, const std::vector<char>& active) {
         rt[r].fil_begin = (int)ft.size();
         ft.insert(ft.end(), c->h_ftiles.begin() + full.fil_begin, c->h_ftiles.begin() + full.fil_end);
         rt[r].fil_end = (int)ft.size();
+        rt[r].n_beads = full.n_beads;
     }
     for (int k = 0; k < K_NUM_SPARSE; ++k) {
         const int t0 = (int)st.size();
@@ -1163,58 +1292,36 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
     auto t_start = std::chrono::steady_clock::now();
     cudaStream_t s = c->stream;
     int rc;
-    if ((rc = pull_states(c))) return rc;
-    for (int r = 0; r < c->R; ++r) {
-        CGState& S = c->h_st[r];
-        const int xb = S.xbuf, fb = S.fbuf;
-        std::memset(&S, 0, sizeof(S));
-        S.xbuf = xb;
-        S.fbuf = fb;
-        S.method = p->method;
-        S.maxDist = p->max_dist;
-        S.lambdaMax = p->lambda_max;
-        S.gradTol = p->grad_tol;
-        S.energyRelTol = p->energy_rel_tol;
-        S.energyCallLimit = p->energy_call_limit;
-        S.forceCallLimit = std::max(p->force_call_limit, 3 * c->reps[r].nb);
-        S.tryToRecover = p->try_to_recover;
-        S.minimumE = std::numeric_limits<double>::infinity();
-        S.maxF = std::numeric_limits<double>::infinity();
-        S.energyRelChange = std::numeric_limits<double>::infinity();
-        S.active = 1;
-        S.phase = PH_IDLE;
-    }
-    if ((rc = push_states(c))) return rc;
-    CU(cudaMemsetAsync(c->err.p, 0, sizeof(unsigned), s));
+    if ((rc = clear_error(c))) return rc;
+    c->h_fresh = false;
     c->compact = false;
     DevNet<Real> n = make_devnet<Real>(c);
-    cudaEvent_t e0, e1;
-    CU(cudaEventCreate(&e0));
-    CU(cudaEventCreate(&e1));
-    CU(cudaEventRecord(e0, s));
+    CU(cudaEventRecord(c->t0, s));
     // energiesBefore, initial forces, resetCGParams, loop head
-    long long launches = 0;
+    long long launches = 3;
+    k_cg_reset<<<(c->R + 127) / 128, 128, 0, s>>>(n.st, n.rt, c->R, *p);
     launches += launch_energy<Real>(n, -1, 0, c->lanes());
     launches += launch_forces<Real>(n, -1, c->lanes());
     k_cg_init<<<(c->R + 127) / 128, 128, 0, s>>>(n.st, c->R);
-    launches += 1 + launch_reset<Real>(n, s);
+    launches += launch_reset<Real>(n, s);
     CU(cudaGetLastError());
-    if ((rc = pull_states(c))) return rc;
-    std::vector<std::vector<double>> before(c->R);
-    for (int r = 0; r < c->R; ++r) before[r].assign(c->h_st[r].eval, c->h_st[r].eval + MECH_NUM_FF + 1);
-    cudaGraphExec_t exec = nullptr;
-    int per_graph = 0;
+    // the conditional graph belongs to this call, the unrolled one to the context
+    struct CallGraph {
+        cudaGraphExec_t exec = nullptr;
+        ~CallGraph() { if (exec) cudaGraphExecDestroy(exec); }
+    } cond;
     CondGraphCounts cc{};
     const bool conditional = c->graph_mode == MECH_GRAPH_CONDITIONAL;
+    int which = 0;   // the unrolled graph in use
     auto build_graph = [&]() {
-        return conditional ? capture_conditional_graph<Real>(c, &exec, &cc)
-                           : capture_iteration_graph<Real>(c, &exec, &per_graph);
+        return conditional ? capture_conditional_graph<Real>(c, &cond.exec, &cc) : iteration_graph<Real>(c, which);
     };
     if ((rc = build_graph())) return rc;
     long long graphs = 0;
     long long max_graphs = 0;
     for (int r = 0; r < c->R; ++r)
-        max_graphs = std::max<long long>(max_graphs, 4LL * c->h_st[r].forceCallLimit / kBlocksPerGraph + 1000);
+        max_graphs = std::max<long long>(
+            max_graphs, 4LL * std::max(p->force_call_limit, 3 * c->reps[r].nb) / kGraphBlocks[0] + 1000);
     int status = MECH_OK;
     // The next graph is launched before the host reads the snapshot of the
     // previous one, so the device does not idle while the host checks the
@@ -1223,28 +1330,32 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
     // on a finished, failed or compactable state the host drains the launch
     // in flight and acts on the newest snapshot.
     auto launch = [&](int k) -> int {
-        CU(cudaGraphLaunch(exec, s));
+        if (!conditional && which == 0 && graphs >= kShortGraphs) {
+            which = 1;
+            int rl;
+            if ((rl = build_graph())) return rl;
+        }
+        CU(cudaGraphLaunch(conditional ? cond.exec : c->iter[which].exec, s));
         ++graphs;
         auto& sn = c->snap[k];
-        CU(cudaMemcpyAsync(sn.st, c->st.p, sizeof(CGState) * c->R, cudaMemcpyDeviceToHost, s));
-        CU(cudaMemcpyAsync(sn.err, c->err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-        if (conditional)   // bodies and phases this launch ran
-            CU(cudaMemcpyAsync(sn.err + 1, c->cond_counter.p, 8 * sizeof(int), cudaMemcpyDeviceToHost, s));
+        sn.launches = c->iter[which].launches;
+        k_snapshot<<<(std::max(c->R, 9) + 127) / 128, 128, 0, s>>>(n.st, c->R, n.err, c->cond_counter.as<int>(), sn.word);
+        CU(cudaGetLastError());
         CU(cudaEventRecord(sn.done, s));
         return MECH_OK;
     };
     // launches of snapshot k's graph (the conditional graph counts what its bodies ran)
     auto account = [&](int k) {
-        const int* bc = reinterpret_cast<const int*>(c->snap[k].err + 1);
-        launches += conditional ? (long long)bc[0] * cc.head + (long long)bc[2] * cc.trial +
+        const int* bc = c->snap[k].word + 1;
+        launches += 1 + (conditional ? (long long)bc[0] * cc.head + (long long)bc[2] * cc.trial +
                                       (long long)bc[3] * cc.force + (long long)bc[4] * cc.dir + (long long)bc[5] * cc.misc
-                                : per_graph;
+                                : c->snap[k].launches);
     };
-    auto wants_host = [&](const CGState* st, unsigned err, bool* all_done) {
+    auto wants_host = [&](const MechContext::Snapshot& sn, bool* all_done) {
         bool done = true, host = false;
         long long live = 0;
         for (int r = 0; r < c->R; ++r) {
-            const int ph = st[r].phase;
+            const int ph = sn.phase()[r];
             const bool act = ph != PH_DONE && ph != PH_ERROR;
             if (act) {
                 done = false;
@@ -1255,27 +1366,26 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
         *all_done = done;
         // batched runs: relaunch over the live replicas once they hold at most half of the tiles
         const bool compactable = c->R > 1 && !done && 2 * live <= (long long)n.n_ftiles;
-        return err != 0 || done || host || compactable || graphs > max_graphs;
+        return sn.err() != 0 || done || host || compactable || graphs > max_graphs;
     };
     int cur = 0;
-    if ((rc = launch(cur))) { cudaGraphExecDestroy(exec); return rc; }
+    if ((rc = launch(cur))) return rc;
     for (;;) {
         const int nxt = cur ^ 1;
-        if ((rc = launch(nxt))) { cudaGraphExecDestroy(exec); return rc; }
+        if ((rc = launch(nxt))) return rc;
         CU(cudaEventSynchronize(c->snap[cur].done));
         account(cur);
         bool all_done = false;
-        if (!wants_host(c->snap[cur].st, *c->snap[cur].err, &all_done)) {
+        if (!wants_host(c->snap[cur], &all_done)) {
             cur = nxt;
             continue;
         }
         // drain the launch in flight and act on its (newest) snapshot
         CU(cudaEventSynchronize(c->snap[nxt].done));
         account(nxt);
-        std::memcpy(c->h_st, c->snap[nxt].st, sizeof(CGState) * c->R);
-        *c->h_err = *c->snap[nxt].err;
-        if (*c->h_err) {
-            status = err_status(*c->h_err);
+        const auto& sn = c->snap[nxt];
+        if (sn.err()) {
+            status = err_status(sn.err());
             break;
         }
         bool recover = false;
@@ -1283,7 +1393,7 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
         long long live = 0;
         all_done = true;
         for (int r = 0; r < c->R; ++r) {
-            const int ph = c->h_st[r].phase;
+            const int ph = sn.phase()[r];
             act[r] = ph != PH_DONE && ph != PH_ERROR;
             if (act[r]) {
                 all_done = false;
@@ -1301,38 +1411,27 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
             CU(cudaGetLastError());
         }
         if (c->R > 1 && 2 * live <= (long long)n.n_ftiles) {
-            cudaGraphExecDestroy(exec);
-            exec = nullptr;
+            if (cond.exec) {
+                cudaGraphExecDestroy(cond.exec);
+                cond.exec = nullptr;
+            }
             if ((rc = compact_tiles(c, act))) { c->compact = false; return rc; }
             n = make_devnet<Real>(c);
             if ((rc = build_graph())) { c->compact = false; return rc; }
         }
         cur = nxt ^ 1;
-        if ((rc = launch(cur))) { cudaGraphExecDestroy(exec); return rc; }
+        if ((rc = launch(cur))) return rc;
     }
-    CU(cudaStreamSynchronize(s));
-    if (exec) cudaGraphExecDestroy(exec);
     c->compact = false;   // the full lists again for energiesAfter and later calls
     n = make_devnet<Real>(c);
-    // call-limit exit restores the minimum-energy backup (CGMethod.hpp:1589-1610)
-    bool restore = false;
-    for (int r = 0; r < c->R; ++r) {
-        CGState& S = c->h_st[r];
-        const bool limit = (S.energyCallLimit != 0 && S.numEnergyCall > S.energyCallLimit) ||
-                           (S.forceCallLimit != 0 && S.numForceCall > S.forceCallLimit);
-        S.restore = (p->report_on_call_limit && limit && S.backupValid) ? 1 : 0;
-        restore = restore || S.restore;
-        S.active = 1;
-    }
-    if ((rc = push_states(c))) return rc;
-    if (restore) launches += launch_backup_restore<Real>(n, s);
+    k_cg_finish<<<(c->R + 127) / 128, 128, 0, s>>>(n.st, c->R, p->report_on_call_limit);
+    launches += 1 + launch_backup_restore<Real>(n, s);
     launches += launch_energy<Real>(n, -1, 0, c->lanes());   // energiesAfter
-    CU(cudaEventRecord(e1, s));
+    CU(cudaGetLastError());
+    CU(cudaEventRecord(c->t1, s));
     if ((rc = pull_states(c))) return rc;
     float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    cudaEventElapsedTime(&ms, c->t0, c->t1);
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
     c->timing.ms_total = ms;
     c->timing.launches = launches;
@@ -1358,7 +1457,7 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
         o.energy_rel_change = S.energyRelChange;
         o.energy_rel_tol = S.energyRelTol;
         for (int k = 0; k <= MECH_NUM_FF; ++k) {
-            o.energies_before[k] = before[r][k];
+            o.energies_before[k] = S.before[k];
             o.energies_after[k] = S.eval[k];
         }
         o.seconds = secs;
@@ -1432,12 +1531,14 @@ static int check_replica(MechContext* ctx, int32_t r) {
     return MECH_OK;
 }
 
-int32_t mech_set_coords(MechContext* ctx, int32_t r, const double* coord) {
-    int rc = check_replica(ctx, r);
-    if (rc) return rc;
-    if (!coord) return set_err(MECH_ERR_ARG, "null coord");
+}  // extern "C"
+
+// The caller's coordinates of replica r to its current buffer, in stream order:
+// the caller of this waits for the stream before it returns.
+static int put_coords(MechContext* ctx, int r, const double* coord) {
     CU(cudaSetDevice(ctx->device));
-    if ((rc = pull_states(ctx))) return rc;
+    int rc;
+    if ((rc = states(ctx))) return rc;
     const ReplicaHost& h = ctx->reps[r];
     CU(cudaMemcpyAsync(ctx->stage.p, coord, sizeof(double) * 3 * h.nb, cudaMemcpyHostToDevice, ctx->stream));
     void* X = ctx->x[ctx->h_st[r].xbuf].p;
@@ -1448,6 +1549,16 @@ int32_t mech_set_coords(MechContext* ctx, int32_t r, const double* coord) {
         k_scatter_coords<float><<<(h.nb + 255) / 256, 256, 0, ctx->stream>>>(ctx->stage.as<double>(), perm_of(ctx, r),
                                                                              h.nb, h.bead_begin, (float*)X);
     CU(cudaGetLastError());
+    return MECH_OK;
+}
+
+extern "C" {
+
+int32_t mech_set_coords(MechContext* ctx, int32_t r, const double* coord) {
+    int rc = check_replica(ctx, r);
+    if (rc) return rc;
+    if (!coord) return set_err(MECH_ERR_ARG, "null coord");
+    if ((rc = put_coords(ctx, r, coord))) return rc;
     CU(cudaStreamSynchronize(ctx->stream));
     return MECH_OK;
 }
@@ -1457,7 +1568,7 @@ int32_t mech_get_coords(MechContext* ctx, int32_t r, double* coord) {
     if (rc) return rc;
     if (!coord) return set_err(MECH_ERR_ARG, "null coord");
     CU(cudaSetDevice(ctx->device));
-    if ((rc = pull_states(ctx))) return rc;
+    if ((rc = states(ctx))) return rc;
     const ReplicaHost& h = ctx->reps[r];
     const void* X = ctx->x[ctx->h_st[r].xbuf].p;
     if (ctx->precision == MECH_PREC_FP64)
@@ -1476,7 +1587,7 @@ int32_t mech_get_forces(MechContext* ctx, int32_t r, double* f_out) {
     if (rc) return rc;
     if (!f_out) return set_err(MECH_ERR_ARG, "null output");
     CU(cudaSetDevice(ctx->device));
-    if ((rc = pull_states(ctx))) return rc;
+    if ((rc = states(ctx))) return rc;
     const ReplicaHost& h = ctx->reps[r];
     const int fb = ctx->h_st[r].fbuf;
     if (ctx->precision == MECH_PREC_FP64)
@@ -1540,10 +1651,10 @@ int32_t mech_load_forces(MechContext* ctx, int32_t r, int32_t n_types, const dou
         return set_err(MECH_ERR_ARG, "mech_load_forces: bad argument");
     if (!ctx->have_lists) return set_err(MECH_ERR_STATE, "no lists");
     CU(cudaSetDevice(ctx->device));
-    if ((rc = pull_states(ctx))) return rc;
+    if ((rc = states(ctx))) return rc;
     const ReplicaHost& h = ctx->reps[r];
     const size_t nout = 2 * (size_t)h.nfil * (size_t)stride;
-    DeviceBuffer ends, types, ms, nm, out;
+    DeviceBuffer &ends = ctx->lf_ends, &types = ctx->lf_types, &ms = ctx->lf_ms, &nm = ctx->lf_nm, &out = ctx->lf_out;
     cudaStream_t s = ctx->stream;
     if ((rc = upload(ends, h.fil_end_cyl, s)) || (rc = upload(types, h.fil_type, s))) return rc;
     if ((rc = upload(ms, std::vector<double>(mon_size, mon_size + n_types), s)) ||
@@ -1589,9 +1700,8 @@ int32_t mech_energy_terms(MechContext* ctx, int32_t r, double* stretch, double* 
     if (!stretch || !bend) return set_err(MECH_ERR_ARG, "null output");
     if (!ctx->have_lists && (rc = rebuild(ctx, 0.0, nullptr))) return rc;
     CU(cudaSetDevice(ctx->device));
-    if ((rc = pull_states(ctx))) return rc;
-    for (int q = 0; q < ctx->R; ++q) ctx->h_st[q].active = (q == r);
-    if ((rc = push_states(ctx))) return rc;
+    if ((rc = select_replicas(ctx, r))) return rc;
+    ctx->h_fresh = false;
     const ReplicaHost& h = ctx->reps[r];
     DeviceBuffer terms, out;
     const size_t rs = real_size(ctx);
@@ -1625,7 +1735,8 @@ int32_t mech_energy_terms(MechContext* ctx, int32_t r, double* stretch, double* 
 int32_t mech_energy(MechContext* ctx, int32_t r, const double* coord, double* per_ff, double* total, double* energy) {
     int rc = check_replica(ctx, r);
     if (rc) return rc;
-    if (coord && (rc = mech_set_coords(ctx, r, coord))) return rc;
+    if (coord && (rc = put_coords(ctx, r, coord))) return rc;
+    CU(cudaSetDevice(ctx->device));
     if (!ctx->have_lists && (rc = rebuild(ctx, 0.0, nullptr))) return rc;
     rc = ctx->precision == MECH_PREC_FP64 ? eval_energy<double>(ctx, r) : eval_energy<float>(ctx, r);
     if (rc) return rc;
@@ -1641,12 +1752,12 @@ int32_t mech_energy(MechContext* ctx, int32_t r, const double* coord, double* pe
 int32_t mech_forces(MechContext* ctx, int32_t r, const double* coord, double* f_out) {
     int rc = check_replica(ctx, r);
     if (rc) return rc;
-    if (coord && (rc = mech_set_coords(ctx, r, coord))) return rc;
+    if (coord && (rc = put_coords(ctx, r, coord))) return rc;
+    CU(cudaSetDevice(ctx->device));
     if (!ctx->have_lists && (rc = rebuild(ctx, 0.0, nullptr))) return rc;
-    rc = ctx->precision == MECH_PREC_FP64 ? eval_forces<double>(ctx, r) : eval_forces<float>(ctx, r);
+    rc = ctx->precision == MECH_PREC_FP64 ? eval_forces<double>(ctx, r, f_out) : eval_forces<float>(ctx, r, f_out);
     if (rc) return rc;
-    if (*ctx->h_err) return err_status(*ctx->h_err);
-    return f_out ? mech_get_forces(ctx, r, f_out) : MECH_OK;
+    return *ctx->h_err ? err_status(*ctx->h_err) : MECH_OK;
 }
 
 int32_t mech_minimize(MechContext* ctx, const MechCGParams* params, MechResult* results) {
@@ -1712,7 +1823,7 @@ int32_t mech_reset_coords(MechContext* ctx) {
     if (!ctx->have_net) return set_err(MECH_ERR_STATE, "no network");
     CU(cudaSetDevice(ctx->device));
     int rc;
-    if ((rc = pull_states(ctx))) return rc;
+    if ((rc = states(ctx))) return rc;
     for (int r = 0; r < ctx->R; ++r) ctx->h_st[r].xbuf = 0;
     if ((rc = push_states(ctx))) return rc;
     CU(cudaMemcpyAsync(ctx->x[0].p, ctx->xinit.p, 24 * (size_t)ctx->nb, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -1726,9 +1837,8 @@ template <typename Real>
 static int profile_impl(MechContext* c, int iters, MechProfile* o) {
     int rc;
     if (!c->have_lists && (rc = rebuild(c, 0.0, nullptr))) return rc;
-    if ((rc = pull_states(c))) return rc;
-    for (int r = 0; r < c->R; ++r) c->h_st[r].active = 1;
-    if ((rc = push_states(c))) return rc;
+    if ((rc = select_replicas(c, -1))) return rc;
+    c->h_fresh = false;
     const DevNet<Real> n = make_devnet<Real>(c);
     cudaStream_t s = c->stream;
     cudaEvent_t e0, e1;
@@ -1858,9 +1968,8 @@ static int autotune_impl(MechContext* c, int flags, MechTuning* out) {
     t.force_blocks_per_sm = c->blocks_per_sm[1];
     t.cell_scale = c->cell_scale;
     cudaStream_t s = c->stream;
-    if ((rc = pull_states(c))) return rc;
-    for (int r = 0; r < c->R; ++r) c->h_st[r].active = 1;
-    if ((rc = push_states(c))) return rc;
+    if ((rc = select_replicas(c, -1))) return rc;
+    c->h_fresh = false;
     if ((flags & MECH_TUNE_KERNELS) && c->precision == MECH_PREC_MIXED) {
         cudaEvent_t e0, e1;
         CU(cudaEventCreate(&e0));
@@ -2018,7 +2127,8 @@ int32_t mech_hvp(MechContext* ctx, int32_t r, int32_t mode, const double* v, dou
     HvpCgWork w{};
     if ((rc = hvp_buffers(ctx, &w))) return rc;
     if ((rc = put_replica_vec(ctx, r, v, ctx->hv_a))) return rc;
-    CU(cudaMemsetAsync(ctx->err.p, 0, sizeof(unsigned), ctx->stream));
+    if ((rc = clear_error(ctx))) return rc;
+    ctx->h_fresh = false;
     const DevNet<double> n = make_devnet<double>(ctx);
     ctx->timing.launches += launch_hvp(n, ctx->hv_a.as<double>(), ctx->hv_b.as<double>(), 0.0,
                                        mode == MECH_HVP_FORCE_JACOBIAN, ctx->stream);
@@ -2064,7 +2174,8 @@ int32_t mech_adjoint(MechContext* ctx, int32_t r, const double* dL_dx, double dL
     HvpCgWork w{};
     if ((rc = hvp_buffers(ctx, &w))) return rc;
     if ((rc = put_replica_vec(ctx, r, dL_dx, ctx->hv_a))) return rc;
-    CU(cudaMemsetAsync(ctx->err.p, 0, sizeof(unsigned), ctx->stream));
+    if ((rc = clear_error(ctx))) return rc;
+    ctx->h_fresh = false;
     const DevNet<double> n = make_devnet<double>(ctx);
     HvpCgResult cr{};
     CU(hvp_cg_solve(n, ctx->hv_a.as<double>(), ctx->cg_x.as<double>(), w, sp->rel_tol, sp->max_iter, sp->shift,

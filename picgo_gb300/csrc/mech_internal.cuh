@@ -83,6 +83,7 @@ struct CGState {
     int method, energyCallLimit, forceCallLimit, tryToRecover;
     // energies of the last evaluation: per FF, then the plain total
     double eval[MECH_NUM_FF + 1];
+    double before[MECH_NUM_FF + 1];   // energiesBefore of the current minimization
     int evalFailed;        // an FF reported failure in the last evaluation
     int phase;
     int safeMode;
@@ -106,6 +107,7 @@ struct Tile {
 struct RepTiles {
     int fil_begin, fil_end;          // filament (bead) tiles
     int sp_begin[K_NUM_SPARSE], sp_end[K_NUM_SPARSE];
+    int n_beads;
 };
 
 // Conditions of the minimizer's conditional graph: a while loop whose body

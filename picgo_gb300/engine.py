@@ -212,7 +212,7 @@ class Engine:
         check(self._L.mech_reset_coords(self._ctx))
 
     def set_graph_mode(self, mode: str) -> None:
-        """'unrolled' (default): relaunched graphs of 8 unrolled iteration blocks;
+        """'unrolled' (default): relaunched graphs of 2 (longer runs: 8) unrolled iteration blocks;
         'unrolled_pdl': the same with programmatic dependent launch around the reductions;
         'conditional': one graph whose device while loop runs only the phases in use;
         'unrolled_coop': the unrolled graph with each iteration's tail (gather, reductions, direction, reset) as one
