@@ -94,7 +94,7 @@ struct MechContext {
     DeviceBuffer nl_rep, gather_out;
     DeviceBuffer perm_all, stage;   // caller -> internal bead map of all replicas; coordinate staging
     // Hessian-vector products, adjoint and Newton solves (FP64 engine)
-    DeviceBuffer hv_a, hv_b, cg_x, cg_r, cg_p, cg_Ap, cg_scal, cg_part, cg_ticket;
+    DeviceBuffer hv_a, hv_b, cg_x, cg_r, cg_p, cg_Ap, cg_scal, cg_part, cg_ticket, hess_fil, hess_lm, hess_ev, hess_bb;
     DeviceBuffer lf_ends, lf_types, lf_ms, lf_nm, lf_out;   // load forces
     DeviceBuffer gbar;   // grid barrier of the cooperative iteration tail (2 unsigned)
     int n_ftiles = 0, n_stiles = 0;
@@ -2055,18 +2055,32 @@ __global__ void k_axpy_from(double* x, const double* x0, double alpha, const dou
 
 }  // namespace
 
-// the solver's work vectors (3 * nb doubles each) and scalars
-static int hvp_buffers(MechContext* c, HvpCgWork* w) {
+// the two vectors of a Hessian-vector product
+static int hvp_vectors(MechContext* c) {
     const size_t v = sizeof(double) * 3 * (size_t)std::max(c->nb, 1);
     CU(c->hv_a.ensure(v));
     CU(c->hv_b.ensure(std::max(v, sizeof(double) * 2 * (size_t)std::max(c->nlk, 1))));
+    return MECH_OK;
+}
+
+// the solver's vectors (3 * nb doubles each), scalars and Hessian blocks
+static int hvp_buffers(MechContext* c, HvpCgWork* w) {
+    int rc;
+    if ((rc = hvp_vectors(c))) return rc;
+    const size_t v = sizeof(double) * 3 * (size_t)std::max(c->nb, 1);
     CU(c->cg_x.ensure(v));
     CU(c->cg_r.ensure(v));
     CU(c->cg_p.ensure(v));
     CU(c->cg_Ap.ensure(v));
     CU(c->cg_scal.ensure(sizeof(double) * 8));
-    CU(c->cg_part.ensure(sizeof(double) * 512));
+    CU(c->cg_part.ensure(sizeof(double) * std::max<size_t>(512, (size_t)c->nb / 256 + 1)));
     CU(c->cg_ticket.ensure(sizeof(unsigned) * 4));
+    CU(c->hess_fil.ensure(12 * v));
+    CU(c->hess_lm.ensure(sizeof(double) * 5 * (size_t)std::max(c->nlk + c->nmt, 1)));
+    CU(c->hess_ev.ensure(sizeof(double) * 81 * (size_t)std::max<long long>(c->nev, 1)));
+    CU(c->hess_bb.ensure(sizeof(double) * (size_t)std::max<long long>(c->nbb, 1)));
+    w->blocks = HvpBlocks{c->hess_fil.as<double>(), c->hess_lm.as<double>(), c->hess_ev.as<double>(),
+                          c->hess_bb.as<double>()};
     w->r = c->cg_r.as<double>();
     w->p = c->cg_p.as<double>();
     w->Ap = c->cg_Ap.as<double>();
@@ -2124,8 +2138,7 @@ int32_t mech_hvp(MechContext* ctx, int32_t r, int32_t mode, const double* v, dou
     if (mode != MECH_HVP_ENERGY && mode != MECH_HVP_FORCE_JACOBIAN) return set_err(MECH_ERR_ARG, "bad mode");
     CU(cudaSetDevice(ctx->device));
     if ((rc = hvp_ready(ctx))) return rc;
-    HvpCgWork w{};
-    if ((rc = hvp_buffers(ctx, &w))) return rc;
+    if ((rc = hvp_vectors(ctx))) return rc;
     if ((rc = put_replica_vec(ctx, r, v, ctx->hv_a))) return rc;
     if ((rc = clear_error(ctx))) return rc;
     ctx->h_fresh = false;

@@ -1,4 +1,5 @@
-// Hessian-vector products of the full energy and the solves built on them
+// Hessian-vector products of the full energy (one product: dual numbers; a
+// solve: the Hessian's blocks, set up once) and the solves built on them
 // (FP64 engine): the conjugate-gradient solve of (H + shift I) y = b used by
 // the implicit adjoint and by Newton refinement of an equilibrium, and the
 // per-linker parameter gradient of the adjoint.
@@ -206,12 +207,251 @@ __global__ void __launch_bounds__(kHvpBlock) k_hvp_fil(DevNet<double> n, const d
     for (int q = 0; q < 3; ++q) HV[3 * (size_t)b + q] = h[q] + shift * V[3 * (size_t)b + q];
 }
 
-// ---- CG vector kernels: deterministic dots (fixed grid, per-block slots, the
-// last block sums the slots in order) and fused updates -----------------------
+// ---- The Hessian of a solve, held as blocks ------------------------------------
+// A solve applies one H to many vectors, and an application by duals costs
+// 119 + 85 us on 60,000 cylinders (FP64 pipe: ~1,500 instructions per excluded-
+// volume pair and ~250 per bead, most of them the same for every vector).  So a
+// solve first evaluates the duals along the unit vectors of each interaction's
+// difference vectors and keeps the derivatives:
+//   filaments  with u_c = v_{c+1} - v_c of the cylinder (c, c+1), the derivative of
+//              the force between the beads is G_c = D_c u_c + M_c u_{c-1} + P_c u_{c+1}
+//              (3x3 each: stretching, and the bending triples on c and c+1), and
+//              (H v)_c = G_{c-1} - G_c; arrays of [nb] per entry, D, M, P and the
+//              part of D that the triple on c+1 adds
+//   linkers    H dl = f0 dl + beta (l . dl) l along the linker's vector l: 5 values
+//   exvol      the 9x9 matrix over (v12, v34, v31), 81 arrays of [pairs]
+//   boundary   (H v) = c (n . v) n: one value
+// An application is then ~45 FP64 instructions per bead and ~60 per 8 pairs, and
+// reads the blocks once, coalesced (the 216 bytes per cylinder bound it from
+// about 100,000 cylinders on, when they leave L2).  Setting them up costs about
+// two applications by duals.
+__device__ __forceinline__ Dual unit(double v, bool on) { return Dual(v, on ? 1.0 : 0.0); }
+
+__global__ void __launch_bounds__(kHvpBlock) k_hess_fil(DevNet<double> n, double* __restrict__ A) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= n.nb) return;
+    const size_t N = n.nb;
+    double *D = A + c, *M = A + 9 * N + c, *P = A + 18 * N + c, *T = A + 27 * N + c;
+    const int fl = n.bflag[c];
+    if (!(fl & 1)) {   // no cylinder starts here
+        for (int k = 0; k < 9; ++k) D[k * N] = M[k * N] = P[k * N] = T[k * N] = 0.0;
+        return;
+    }
+    const double* X = n.x[0] + 3 * (size_t)c;
+    double ks, l0, kb, th;
+    load_par(n.bpar, c, ks, l0, kb, th);
+    const double r2[3] = {X[3] - X[0], X[4] - X[1], X[5] - X[2]};
+    double d[9];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        Dual F[3];
+        stretch_force<Dual>(unit(r2[0], j == 0), unit(r2[1], j == 1), unit(r2[2], j == 2), Dual(ks), Dual(l0), F);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) d[3 * q + j] = -F[q].d;
+    }
+    if (fl & 2) {   // the triple on c: (c-1, c, c+1)
+        const double r1[3] = {X[0] - X[-3], X[1] - X[-2], X[2] - X[-1]};
+#pragma unroll 1
+        for (int j = 0; j < 3; ++j) {
+            const Dual a[3] = {unit(r1[0], j == 0), unit(r1[1], j == 1), unit(r1[2], j == 2)};
+            const Dual b[3] = {Dual(r2[0]), Dual(r2[1]), Dual(r2[2])};
+            Dual F1[3], F2[3];
+            bend_force<Dual>(a, b, Dual(kb), Dual(th), F1, F2);
+            for (int q = 0; q < 3; ++q) {
+                T[(3 * q + j) * N - 1] = -F1[q].d;   // on u_{c-1}, of the force across cylinder c-1
+                M[(3 * q + j) * N] = -F2[q].d;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const Dual a[3] = {Dual(r1[0]), Dual(r1[1]), Dual(r1[2])};
+            const Dual b[3] = {unit(r2[0], j == 0), unit(r2[1], j == 1), unit(r2[2], j == 2)};
+            Dual F1[3], F2[3];
+            bend_force<Dual>(a, b, Dual(kb), Dual(th), F1, F2);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                P[(3 * q + j) * N - 1] = -F1[q].d;
+                d[3 * q + j] -= F2[q].d;
+            }
+        }
+    } else {
+        for (int k = 0; k < 9; ++k) M[k * N] = 0.0;
+    }
+    for (int k = 0; k < 9; ++k) D[k * N] = d[k];
+    if (!(n.bflag[c + 1] & 1)) {   // the filament's last cylinder: no triple on c+1
+        for (int k = 0; k < 9; ++k) P[k * N] = T[k * N] = 0.0;
+    }
+}
+__global__ void __launch_bounds__(kHvpBlock) k_hess_fil_sum(long long n9, double* __restrict__ D,
+                                                           const double* __restrict__ T) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i < n9) D[i] += T[i];
+}
+
+__global__ void __launch_bounds__(kHvpBlock) k_hess_bonds(DevNet<double> n, double* __restrict__ lm,
+                                                         double* __restrict__ bb) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const double* X = n.x[0];
+    const int nlm = n.n_lk + n.n_mt;
+    if (i < nlm) {
+        const bool lk = i < n.n_lk;
+        const int j = lk ? i : i - n.n_lk;
+        const int4 bs = lk ? n.lk_bead[j] : n.mt_bead[j];
+        const double k = lk ? n.lk_k[j] : n.mt_k[j], l0 = lk ? n.lk_l0[j] : n.mt_l0[j];
+        const double s1 = lk ? n.lk_s1[j] : n.mt_s1[j], s2 = lk ? n.lk_s2[j] : n.mt_s2[j];
+        double l[3];
+        for (int q = 0; q < 3; ++q) {
+            const double c1 = X[3 * (size_t)bs.x + q], c2 = X[3 * (size_t)bs.y + q], c3 = X[3 * (size_t)bs.z + q],
+                         c4 = X[3 * (size_t)bs.w + q];
+            l[q] = (c3 + (c4 - c3) * s2) - (c1 + (c2 - c1) * s1);
+        }
+        const double d = sqrt(l[0] * l[0] + l[1] * l[1] + l[2] * l[2]);
+        const size_t N = nlm;
+        lm[i] = k * (d - l0) / d;             // f0
+        lm[N + i] = k * l0 / (d * d * d);     // beta
+        for (int q = 0; q < 3; ++q) lm[(2 + q) * N + i] = l[q];
+        return;
+    }
+    const int m = i - nlm;
+    if (m < n.n_bb) {
+        const double* pl = n.planes + 4 * n.bb_plane[m];
+        const double* x = X + 3 * (size_t)n.bb_bead[m];
+        const double nrm = sqrt(pl[0] * pl[0] + pl[1] * pl[1] + pl[2] * pl[2]);
+        const double r = (x[0] * pl[0] + x[1] * pl[1] + x[2] * pl[2] + pl[3]) / nrm;
+        const double sl = n.bb_slen[m];
+        bb[m] = n.bb_k[m] * exp(-r / sl) / sl / (sl * nrm);
+    }
+}
+
+// One thread per pair and column; the columns of a pair are one grid row apart,
+// so that a warp's loads and stores stay coalesced over pairs.
+__global__ void __launch_bounds__(128) k_hess_exvol(DevNet<double> n, double* __restrict__ H) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = blockIdx.y;
+    if (e >= n.n_ev) return;
+    const double* X = n.x[0];
+    const int4 bs = n.ev_bead[e];
+    const double* c[4] = {X + 3 * (size_t)bs.x, X + 3 * (size_t)bs.y, X + 3 * (size_t)bs.z, X + 3 * (size_t)bs.w};
+    Dual v12[3], v34[3], v31[3], v14[3], v32[3], v24[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double da = j == q ? 1.0 : 0.0, db = j == 3 + q ? 1.0 : 0.0, dc = j == 6 + q ? 1.0 : 0.0;
+        v12[q] = Dual(c[1][q] - c[0][q], da);
+        v34[q] = Dual(c[3][q] - c[2][q], db);
+        v31[q] = Dual(c[0][q] - c[2][q], dc);
+        v14[q] = Dual(c[3][q] - c[0][q], db - dc);
+        v32[q] = Dual(c[1][q] - c[2][q], da + dc);
+        v24[q] = Dual(c[3][q] - c[1][q], db - dc - da);
+    }
+    PairInv<Dual> p;
+    pair_inv(v12, v34, v31, v14, v32, v24, p, true);
+    Dual out[4][3];
+    if (!forces_from<true>(p, v12, v34, v31, Dual(n.ev_k[e] * n.ev_la[e] * n.ev_lb[e]), out)) atomicOr(n.err, 8u);
+    const size_t N = n.n_ev;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        H[(9 * q + j) * N + e] = -out[1][q].d;
+        H[(9 * (3 + q) + j) * N + e] = -out[3][q].d;
+        H[(9 * (6 + q) + j) * N + e] = -out[0][q].d - out[1][q].d;
+    }
+}
+
+// The sparse interactions' part of H v to the contribution slots: blocks
+// [0, lm_blocks) linkers and motors, then excluded-volume pairs (four lanes a
+// pair: lane k < 3 the gradient along the k-th difference vector, lane a bead
+// a's share), then boundary beads.
+__global__ void __launch_bounds__(kHvpBlock) k_hess_apply_sparse(DevNet<double> n, const double* __restrict__ V,
+                                                                HvpBlocks h, int lm_blocks, int ev_blocks) {
+    const int blk = blockIdx.x;
+    if (blk < lm_blocks) {
+        const int i = blk * blockDim.x + threadIdx.x, nlm = n.n_lk + n.n_mt;
+        if (i >= nlm) return;
+        const bool lk = i < n.n_lk;
+        const int j = lk ? i : i - n.n_lk;
+        const int4 bs = lk ? n.lk_bead[j] : n.mt_bead[j];
+        const double s1 = lk ? n.lk_s1[j] : n.mt_s1[j], s2 = lk ? n.lk_s2[j] : n.mt_s2[j];
+        double dl[3], l[3], dot = 0.0;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const double v1 = V[3 * (size_t)bs.x + q], v2 = V[3 * (size_t)bs.y + q], v3 = V[3 * (size_t)bs.z + q],
+                         v4 = V[3 * (size_t)bs.w + q];
+            dl[q] = (v3 + (v4 - v3) * s2) - (v1 + (v2 - v1) * s1);
+            l[q] = h.lm[(2 + q) * (size_t)nlm + i];
+            dot += l[q] * dl[q];
+        }
+        const double f0 = h.lm[i], bd = h.lm[(size_t)nlm + i] * dot;
+        const int sb = n.slot_base[lk ? K_LINKER : K_MOTOR] + 4 * j;
+        const double w[4] = {s1 - 1.0, -s1, 1.0 - s2, s2};
+        double g[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) g[q] = f0 * dl[q] + bd * l[q];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            double* c = slot_ptr(n, sb + a);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) c[q] = w[a] * g[q];
+        }
+        return;
+    }
+    if (blk < lm_blocks + ev_blocks) {
+        const int t = (blk - lm_blocks) * blockDim.x + threadIdx.x;
+        const int e = t >> 2, a = t & 3, k = a < 3 ? a : 2;
+        const bool valid = e < n.n_ev;
+        double g[3] = {0, 0, 0};
+        if (valid) {
+            const int4 bs = n.ev_bead[e];
+            double w[9];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const double v1 = V[3 * (size_t)bs.x + q], v2 = V[3 * (size_t)bs.y + q], v3 = V[3 * (size_t)bs.z + q],
+                             v4 = V[3 * (size_t)bs.w + q];
+                w[q] = v2 - v1;
+                w[3 + q] = v4 - v3;
+                w[6 + q] = v1 - v3;
+            }
+            const size_t N = n.n_ev;
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+#pragma unroll
+                for (int j = 0; j < 9; ++j) g[q] += h.ev[(9 * (3 * k + q) + j) * N + e] * w[j];
+        }
+        const int base = threadIdx.x & 28;
+        double o[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const double g12 = __shfl_sync(0xffffffffu, g[q], base), g34 = __shfl_sync(0xffffffffu, g[q], base + 1),
+                         g31 = __shfl_sync(0xffffffffu, g[q], base + 2);
+            o[q] = a == 0 ? g31 - g12 : a == 1 ? g12 : a == 2 ? -g34 - g31 : g34;
+        }
+        if (valid) {
+            double* c = slot_ptr(n, n.slot_base[K_EXVOL] + 4 * e + a);
+            c[0] = o[0];
+            c[1] = o[1];
+            c[2] = o[2];
+        }
+        return;
+    }
+    const int m = (blk - lm_blocks - ev_blocks) * blockDim.x + threadIdx.x;
+    if (m < n.n_bb) {
+        const double* pl = n.planes + 4 * n.bb_plane[m];
+        const double* v = V + 3 * (size_t)n.bb_bead[m];
+        const double f = h.bb[m] * (v[0] * pl[0] + v[1] * pl[1] + v[2] * pl[2]);
+        double* c = slot_ptr(n, n.slot_base[K_BOUNDARY] + m);
+        c[0] = f * pl[0];
+        c[1] = f * pl[1];
+        c[2] = f * pl[2];
+    }
+}
+
+// ---- CG kernels: deterministic dots (per-block slots, the last block sums the
+// slots in order and forms the step) and fused updates --------------------------
 constexpr int kCgBlocks = 304;
 
-// scal: [0] rr, [1] pAp, [2] rr_new, [3] bb
-__device__ __forceinline__ void finish_dot(double v, double* part, unsigned* ticket, double* out, double* sh) {
+// scal: [0], [1] r.r of the even and odd iterations, [2] alpha, [3] b.b,
+// [4] curvature flag, [5] beta
+// Sum over the grid's blocks; `finish` gets it in one thread of the last block.
+template <typename F>
+__device__ __forceinline__ void grid_dot(double v, double* part, unsigned* ticket, double* sh, F&& finish) {
     v = block_sum(v, sh);
     __shared__ bool last;
     if (threadIdx.x == 0) {
@@ -226,30 +466,96 @@ __device__ __forceinline__ void finish_dot(double v, double* part, unsigned* tic
     for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) a += __ldcg(part + k);
     a = block_sum(a, sh);
     if (threadIdx.x == 0) {
-        *out = a;
         *ticket = 0u;
+        finish(a);
     }
 }
 
-__global__ void __launch_bounds__(kHvpBlock) k_dot(const double* __restrict__ a, const double* __restrict__ b, long long n,
-                                                   double* part, unsigned* ticket, double* out) {
+__global__ void __launch_bounds__(kHvpBlock) k_cg_start(const double* __restrict__ b, double* __restrict__ x,
+                                                        double* __restrict__ r, double* __restrict__ p, long long n,
+                                                        double* scal, double* part, unsigned* ticket) {
     __shared__ double sh[32];
     double v = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        v += a[i] * b[i];
-    finish_dot(v, part, ticket, out, sh);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const double bi = b[i];
+        x[i] = 0.0;
+        r[i] = bi;
+        p[i] = bi;
+        v += bi * bi;
+    }
+    grid_dot(v, part, ticket, sh, [&](double bb) { scal[0] = scal[3] = bb; });
 }
 
-// x += alpha p, r -= alpha Ap, alpha = rr / pAp; rr_new = r . r
+// hv = H v + shift v at the beads (the filaments' blocks and the gathered sparse
+// contributions), v . hv, and the CG step alpha = r.r / v.hv.  scal[4] latches
+// non-positive curvature: the iterate is frozen there (alpha = 0; the truncated
+// solution is what the caller gets).
+__global__ void __launch_bounds__(kHvpBlock) k_hess_apply_fil(DevNet<double> n, const double* __restrict__ V,
+                                                             const double* __restrict__ A, double shift,
+                                                             double* __restrict__ HV, double* scal, int odd,
+                                                             double* part, unsigned* ticket) {
+    __shared__ double sh[32];
+    __shared__ double su[kHvpBlock + 3][3];   // u of cylinders first - 2 .. first + kHvpBlock
+    __shared__ double sg[kHvpBlock + 1][3];   // G of cylinders first - 1 .. first + kHvpBlock - 1
+    const int first = blockIdx.x * kHvpBlock, nb = n.nb;
+    const size_t N = nb;
+    for (int i = threadIdx.x; i < kHvpBlock + 3; i += kHvpBlock) {
+        const int c = first - 2 + i;
+        const bool ok = c >= 0 && c + 1 < nb;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) su[i][q] = ok ? V[3 * (size_t)(c + 1) + q] - V[3 * (size_t)c + q] : 0.0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kHvpBlock + 1; i += kHvpBlock) {
+        const int c = first - 1 + i;
+        double g[3] = {0, 0, 0};
+        if (c >= 0 && c < nb) {
+            const double* a = A + c;
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    g[q] += a[(3 * q + j) * N] * su[i + 1][j];
+                    g[q] += a[(9 + 3 * q + j) * N] * su[i][j];
+                    g[q] += a[(18 + 3 * q + j) * N] * su[i + 2][j];
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) sg[i][q] = g[q];
+    }
+    __syncthreads();
+    const int b = first + threadIdx.x;
+    double v = 0.0;
+    if (b < nb) {
+        double h[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) h[q] = sg[threadIdx.x][q] - sg[threadIdx.x + 1][q];
+        const int c0 = n.csr_off[b], c1 = n.csr_off[b + 1];
+        for (int c = c0; c < c1; ++c)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) h[q] += n.contrib[3 * (size_t)c + q];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const double vq = V[3 * (size_t)b + q];
+            h[q] += shift * vq;
+            HV[3 * (size_t)b + q] = h[q];
+            v += vq * h[q];
+        }
+    }
+    grid_dot(v, part, ticket, sh, [&](double pAp) {
+        const bool stop = scal[4] != 0.0 || !(pAp > 0.0);
+        if (stop) scal[4] = 1.0;
+        scal[2] = stop ? 0.0 : scal[odd] / pAp;
+    });
+}
+
+// x += alpha p, r -= alpha Ap; the new r . r and beta
 __global__ void __launch_bounds__(kHvpBlock) k_cg_step(double* __restrict__ x, double* __restrict__ r,
                                                        const double* __restrict__ p, const double* __restrict__ Ap,
-                                                       long long n, double* scal, double* part, unsigned* ticket) {
+                                                       long long n, double* scal, int odd, double* part,
+                                                       unsigned* ticket) {
     __shared__ double sh[32];
-    // scal[4] latches non-positive curvature p.Ap <= 0: the iterate is frozen
-    // there (the truncated solution is what the caller gets)
-    const bool stop = scal[4] != 0.0 || !(scal[1] > 0.0);
-    if (stop && blockIdx.x == 0 && threadIdx.x == 0) scal[4] = 1.0;
-    const double alpha = stop ? 0.0 : scal[0] / scal[1];
+    const double alpha = scal[2];
     double v = 0.0;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         x[i] += alpha * p[i];
@@ -257,19 +563,18 @@ __global__ void __launch_bounds__(kHvpBlock) k_cg_step(double* __restrict__ x, d
         r[i] = ri;
         v += ri * ri;
     }
-    finish_dot(v, part, ticket, scal + 2, sh);
+    grid_dot(v, part, ticket, sh, [&](double rr) {
+        scal[5] = rr / scal[odd];
+        scal[odd ^ 1] = rr;
+    });
 }
 
-// p = r + (rr_new / rr) p; rr = rr_new
+// p = r + beta p
 __global__ void __launch_bounds__(kHvpBlock) k_cg_dir(double* __restrict__ p, const double* __restrict__ r, long long n,
-                                                      double* scal) {
-    const double beta = scal[2] / scal[0];
+                                                      const double* scal) {
+    const double beta = scal[5];
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         p[i] = r[i] + beta * p[i];
-}
-
-__global__ void k_cg_roll(double* scal) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) scal[0] = scal[2];
 }
 
 // Linker parameter gradient of the implicit adjoint, per linker j:
@@ -312,24 +617,34 @@ int launch_hvp(const DevNet<double>& n, const double* v, double* hv, double shif
     return k + 1;
 }
 
+// Blocks of the Hessian at x[0] into h; returns the kernels launched.
+static int assemble_hessian(const DevNet<double>& n, const HvpBlocks& h, cudaStream_t s) {
+    const int B = kHvpBlock, nbnd = n.n_lk + n.n_mt + n.n_bb;
+    int k = 2;
+    k_hess_fil<<<(n.nb + B - 1) / B, B, 0, s>>>(n, h.fil);
+    const long long n9 = 9LL * n.nb;
+    k_hess_fil_sum<<<(unsigned)((n9 + B - 1) / B), B, 0, s>>>(n9, h.fil, h.fil + 27 * (size_t)n.nb);
+    if (nbnd > 0) {
+        k_hess_bonds<<<(nbnd + B - 1) / B, B, 0, s>>>(n, h.lm, h.bb);
+        ++k;
+    }
+    if (n.n_ev > 0) {
+        k_hess_exvol<<<dim3((unsigned)((n.n_ev + 127) / 128), 9), 128, 0, s>>>(n, h.ev);
+        ++k;
+    }
+    return k;
+}
+
 cudaError_t hvp_cg_solve(const DevNet<double>& n, const double* b, double* x, const HvpCgWork& w, double rel_tol,
                          int max_iter, double shift, cudaStream_t s, HvpCgResult* res) {
     const long long N = 3LL * n.nb;
     const int G = kCgBlocks, B = kHvpBlock;
     cudaError_t e;
-    res->iterations = 0;
-    res->launches = 0;
-    res->rel_residual = 0.0;
-    res->converged = 0;
-    res->negative_curvature = 0;
+    *res = HvpCgResult{};
     // x = 0, r = b, p = b; rr = bb = b . b; no curvature flag
-    if ((e = cudaMemsetAsync(x, 0, sizeof(double) * N, s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(w.scal, 0, sizeof(double) * 8, s)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(w.r, b, sizeof(double) * N, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(w.p, b, sizeof(double) * N, cudaMemcpyDeviceToDevice, s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(w.ticket, 0, sizeof(unsigned), s)) != cudaSuccess) return e;
-    k_dot<<<G, B, 0, s>>>(b, b, N, w.part, w.ticket, w.scal + 0);
-    k_dot<<<G, B, 0, s>>>(b, b, N, w.part, w.ticket, w.scal + 3);
+    k_cg_start<<<G, B, 0, s>>>(b, x, w.r, w.p, N, w.scal, w.part, w.ticket);
     double h[5];
     if ((e = cudaMemcpyAsync(h, w.scal, sizeof(h), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
@@ -339,21 +654,27 @@ cudaError_t hvp_cg_solve(const DevNet<double>& n, const double* b, double* x, co
         return cudaSuccess;
     }
     const double tol2 = rel_tol * rel_tol * bb;
+    res->launches = assemble_hessian(n, w.blocks, s);
     // kCheck iterations per CUDA graph launch; the host reads the residual between launches
-    constexpr int kCheck = 16;
+    constexpr int kCheck = 16;   // even: a graph starts on an even iteration
+    const int lm_blocks = (n.n_lk + n.n_mt + B - 1) / B, ev_blocks = (int)((4LL * n.n_ev + B - 1) / B),
+              sp_blocks = lm_blocks + ev_blocks + (n.n_bb + B - 1) / B;
     int per_iter = 0;
-    auto iteration = [&]() {
-        per_iter = launch_hvp(n, w.p, w.Ap, shift, false, s);
-        k_dot<<<G, B, 0, s>>>(w.p, w.Ap, N, w.part, w.ticket, w.scal + 1);
-        k_cg_step<<<G, B, 0, s>>>(x, w.r, w.p, w.Ap, N, w.scal, w.part, w.ticket);
+    auto iteration = [&](int it) {
+        const int odd = it & 1;
+        per_iter = 3;
+        if (sp_blocks > 0) {
+            k_hess_apply_sparse<<<sp_blocks, B, 0, s>>>(n, w.p, w.blocks, lm_blocks, ev_blocks);
+            ++per_iter;
+        }
+        k_hess_apply_fil<<<(n.nb + B - 1) / B, B, 0, s>>>(n, w.p, w.blocks.fil, shift, w.Ap, w.scal, odd, w.part, w.ticket);
+        k_cg_step<<<G, B, 0, s>>>(x, w.r, w.p, w.Ap, N, w.scal, odd, w.part, w.ticket);
         k_cg_dir<<<G, B, 0, s>>>(w.p, w.r, N, w.scal);
-        k_cg_roll<<<1, 32, 0, s>>>(w.scal);
-        per_iter += 4;
     };
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return e;
-    for (int j = 0; j < kCheck; ++j) iteration();
+    for (int j = 0; j < kCheck; ++j) iteration(j);
     e = cudaStreamEndCapture(s, &graph);
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
@@ -365,7 +686,7 @@ cudaError_t hvp_cg_solve(const DevNet<double>& n, const double* b, double* x, co
             res->launches += (long long)kCheck * per_iter;
         } else {
             for (; it < max_iter; ++it) {
-                iteration();
+                iteration(it);
                 res->launches += per_iter;
             }
             e = cudaGetLastError();
@@ -373,13 +694,14 @@ cudaError_t hvp_cg_solve(const DevNet<double>& n, const double* b, double* x, co
         if (e != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(h, w.scal, sizeof(h), cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) break;
+        const double rr = h[it & 1];
         res->iterations = it;
-        res->rel_residual = sqrt(h[0] / bb);
+        res->rel_residual = sqrt(rr / bb);
         if (h[4] != 0.0) {   // non-positive curvature met: the iterate stopped there
             res->negative_curvature = 1;
             break;
         }
-        if (h[0] <= tol2) {
+        if (rr <= tol2) {
             res->converged = 1;
             break;
         }

@@ -337,11 +337,19 @@ template <typename Real> int launch_exvol_forces(const DevNet<Real>& n, int want
 // order; H is the energy's Hessian, or with `jacobian` minus the Jacobian of
 // the force routine (which moves nearly coplanar excluded-volume pairs)
 int launch_hvp(const DevNet<double>& n, const double* v, double* hv, double shift, bool jacobian, cudaStream_t s);
+// blocks of the Hessian that a solve applies (mech_hvp.cu)
+struct HvpBlocks {
+    double* fil;   // [36 * nb]
+    double* lm;    // [5 * (linkers + motors)]
+    double* ev;    // [81 * pairs]
+    double* bb;    // [boundary beads]
+};
 struct HvpCgWork {
     double* r; double* p; double* Ap;   // [3 * nb] each
-    double* scal;                        // [8]: r.r, p.Ap, new r.r, b.b, curvature flag
-    double* part;                        // [304] per-block partial sums
+    double* scal;                        // [8] (see mech_hvp.cu)
+    double* part;                        // per-block partial sums: [max(304, blocks of 256 beads)]
     unsigned* ticket;
+    HvpBlocks blocks;
 };
 struct HvpCgResult {
     int iterations, converged, negative_curvature;
