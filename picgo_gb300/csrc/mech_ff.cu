@@ -10,10 +10,9 @@
 //
 // Filament forces are computed owner-side: a block loads its 256 beads plus a
 // two-bead halo into shared memory, evaluates every cylinder and bending
-// triple touching its beads once, and each bead sums its own terms in the
-// reference's order (stretching, then bending, then the sparse force fields
-// through the CSR gather), so no floating-point atomics are used and FP64
-// forces follow the reference's per-bead summation order.
+// triple touching its beads once, and each bead sums its own terms in a fixed
+// order (the filament's, then the sparse force fields' through the CSR gather),
+// so no floating-point atomics are used.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -138,157 +137,278 @@ __global__ void __launch_bounds__(kBlock) k_body_head(DevNet<Real> n) {
 }
 
 // ---------------------------------------------------------------------------
-// filament energy: stretching + bending of the tile's own cylinders/triples
+// FP64 engine: filament energy and forces.  Bound by the FP64 pipe (a warp's
+// FP64 instruction holds its sub-partition's pipe for ~70 cycles), so what
+// counts is FP64 instructions per bead: every cylinder's vector, length and
+// reciprocal length is formed once and read by the bending terms on both of its
+// ends, comparisons are made on the bits of the numbers, and the sums of a warp
+// share the additions of their trees.
 // ---------------------------------------------------------------------------
-template <typename Real>
-__global__ void __launch_bounds__(kBlock) k_fil_energy(DevNet<Real> n, int want, int trial) {
-    pdl_wait();      // the previous kernel of the main lane has finished
-    MECH_TRACE_KERNEL(n, TK_FIL_ENERGY);
-    __shared__ Pos<Real> xs[kFilTile + 4];
-    __shared__ double sh[32 * MECH_NUM_FF];
-    __shared__ int s_go, s_xb;
-    __shared__ double s_lam;
-    const Tile t = n.ftile[blockIdx.x];
-    const int r = t.replica;
-    if (threadIdx.x == 0) {
-        const CGState& S = n.st[r];
-        s_go = replica_selected(S, want);
-        s_xb = S.xbuf;
-        s_lam = S.lambda;
+// Sums of N values (a power of two) over each warp and then the block: the
+// first steps of the trees halve the number of values a lane carries, so N
+// trees take N + 3 additions (N = 4: 6) where one after another they take 5 N.
+// Thread t < N gets value t.  A value's tree has the same shape whatever its
+// place among the N, so a tile's sums do not depend on the tiles it shares a
+// block with.  `sh` holds N * kBlock / 32 doubles.
+template <int N>
+__device__ __forceinline__ double block_sums(double (&v)[N], double* sh) {
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int idx = 0, o = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (l & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const double keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+        if (up) idx += h;
     }
+#pragma unroll
+    for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
     __syncthreads();
-    if (s_go) {
-        const int T = t.end - t.begin;
-        const Real* X = n.x[s_xb];
-        const bool tr = trial != 0;
-        for (int i = threadIdx.x; i < T + 4; i += blockDim.x) {
-            const int b = t.begin - 2 + i;
-            if (b >= 0 && b < n.nb) xs[i] = bead_at(X, n.d, b, tr, s_lam);
-        }
-        __syncthreads();
-        Real es = 0, eb = 0;
-        const int i = threadIdx.x;
-        if (i < T) {
-            const int j = t.begin + i;
-            const int fl = n.bflag[j];
-            if (tr) store_pos(n.x[s_xb ^ 1], j, xs[i + 2]);   // materialize the owned trial position
-            if (fl & 1) {
-                Real ks, l0, kb, t0;
-                load_par(n.bpar, j, ks, l0, kb, t0);
-                Real r2[3];
-                pdiff(xs[i + 3], xs[i + 2], r2);
-                es = stretch_energy<Real>(r2[0], r2[1], r2[2], ks, l0);
-                if (fl & 2) {
-                    Real r1[3];
-                    pdiff(xs[i + 2], xs[i + 1], r1);
-                    eb = bend_energy<Real>(r1, r2, kb, t0);
-                }
-                if (n.terms) {
-                    n.terms[j] = es;
-                    n.terms[(size_t)n.nb + j] = eb;
-                }
-            }
-        }
-        double red[2] = {warp_sum_r(es), warp_sum_r(eb)};
-        const int ops[2] = {0, 0};
-        block_combine<2>(red, ops, sh);
-        if (threadIdx.x == 0) {
-            n.part_fil[4 * (size_t)blockIdx.x + 0] = red[0];
-            n.part_fil[4 * (size_t)blockIdx.x + 1] = red[1];
-        }
+    if ((l & (32 / N - 1)) == 0) sh[w * N + idx] = v[0];
+    __syncthreads();
+    double a = 0.0;
+    if (threadIdx.x < N) {
+        a = sh[threadIdx.x];
+#pragma unroll
+        for (int k = 1; k < kBlock / 32; ++k) a += sh[k * N + threadIdx.x];
     }
+    return a;
+}
+// the same for maxima of N unsigned values
+template <int N>
+__device__ __forceinline__ unsigned long long block_maxima(unsigned long long (&v)[N], unsigned long long* sh) {
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int idx = 0, o = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (l & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const unsigned long long keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
+            v[k] = max(keep, __shfl_xor_sync(0xffffffffu, send, o));
+        }
+        if (up) idx += h;
+    }
+#pragma unroll
+    for (; o >= 1; o >>= 1) v[0] = max(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
+    __syncthreads();
+    if ((l & (32 / N - 1)) == 0) sh[w * N + idx] = v[0];
+    __syncthreads();
+    unsigned long long a = 0;
+    if (threadIdx.x < N)
+        for (int k = 0; k < kBlock / 32; ++k) a = max(a, sh[k * N + threadIdx.x]);
+    return a;
 }
 
-// ---------------------------------------------------------------------------
-// filament forces of the tile's own beads (the sparse force fields' shares are
-// added by k_force_gather once they are written)
-// ---------------------------------------------------------------------------
-template <typename Real>
-__global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<Real> n, int want) {
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+    return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+}
+// areEqual(theta0, 0) on bits: the order of finite magnitudes is that of their
+// bits, and a NaN lies above every threshold
+__device__ __forceinline__ bool theta_is_zero(double t) {
+    return abs_bits(t) < (unsigned long long)__double_as_longlong(1e-6);
+}
+// x clamped to [-1, 1], a NaN kept
+__device__ __forceinline__ double clamp_unit(double x) {
+    const unsigned long long a = abs_bits(x);
+    return a > 0x3ff0000000000000ULL && a <= 0x7ff0000000000000ULL ? copysign(1.0, x) : x;
+}
+
+// What a block of the FP64 filament kernels needs of its tile's replica.
+struct FilTile {
+    int begin, end, go, xb, fb;
+    double lam;
+};
+__device__ __forceinline__ void load_fil_tile(const DevNet<double>& n, int want, FilTile* s) {
+    if (threadIdx.x == 0) {
+        const Tile t = n.ftile[blockIdx.x];
+        const CGState& S = n.st[t.replica];
+        *s = FilTile{t.begin, t.end, replica_selected(S, want), S.xbuf, S.fbuf, S.lambda};
+    }
+    __syncthreads();
+}
+
+// Stretching + bending energy of the tile's own cylinders and triples.  1M
+// beads: 86 us, against 121 us (66 FP64 instructions per bead) with each length
+// formed two or three times and a tree per sum.
+__global__ void __launch_bounds__(kBlock) k_fil_energy(DevNet<double> n, int want, int trial) {
+    pdl_wait();      // the previous kernel of the main lane has finished
+    MECH_TRACE_KERNEL(n, TK_FIL_ENERGY);
+    __shared__ double xs[3][kFilTile + 2];    // beads begin - 1 .. end
+    __shared__ double rs[4][kFilTile + 1];    // cylinders begin - 1 .. end - 1: vector, length
+    __shared__ double sh[2 * kBlock / 32];
+    __shared__ FilTile t;
+    const bool tr = trial != 0;
+    load_fil_tile(n, want, &t);
+    if (!t.go) return;
+    const int T = t.end - t.begin;
+    const double* X = n.x[t.xb];
+    for (int i = threadIdx.x; i < T + 2; i += blockDim.x) {
+        const int b = t.begin - 1 + i;
+        if (b < 0 || b >= n.nb) continue;
+        const Pos<double> p = bead_at(X, n.d, b, tr, t.lam);
+        xs[0][i] = p.x[0];
+        xs[1][i] = p.x[1];
+        xs[2][i] = p.x[2];
+        if (tr && i >= 1 && i <= T) store_pos(n.x[t.xb ^ 1], b, p);   // materialize the owned trial position
+    }
+    __syncthreads();
+    const int i = threadIdx.x, j = t.begin + i;
+    const int fl = i < T ? n.bflag[j] : 0;
+    double r2[3] = {0, 0, 0}, L2 = 0.0, ks = 0.0, l0 = 0.0, kb = 0.0, th = 0.0;
+    double e[2] = {0.0, 0.0};   // stretching, bending
+    if (fl & 1) {
+        load_par(n.bpar, j, ks, l0, kb, th);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) r2[q] = xs[q][i + 2] - xs[q][i + 1];
+        L2 = sqrt(r2[0] * r2[0] + r2[1] * r2[1] + r2[2] * r2[2]);
+        const double dl = L2 - l0;
+        e[0] = 0.5 * ks * dl * dl;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) rs[q][i + 1] = r2[q];
+        rs[3][i + 1] = L2;
+    }
+    if (i == kFilTile - 32 && (n.bflag[t.begin] & 2)) {   // the cylinder that ends at the first bead
+        double r[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) rs[q][0] = r[q] = xs[q][1] - xs[q][0];
+        rs[3][0] = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+    }
+    __syncthreads();
+    if ((fl & 3) == 3) {
+        const double l1l2 = rs[0][i] * r2[0] + rs[1][i] * r2[1] + rs[2][i] * r2[2];
+        const double x = clamp_unit(l1l2 / (rs[3][i] * L2));
+        if (theta_is_zero(th)) {
+            e[1] = kb * (1.0 - x);
+        } else {
+            const double sinA = fmax(sqrt(1.0 - x * x), 0.0);
+            e[1] = kb * (1.0 - (x * cos(th) + sinA * sin(th)));
+        }
+    }
+    if (n.terms && (fl & 1)) {
+        n.terms[j] = e[0];
+        n.terms[(size_t)n.nb + j] = e[1];
+    }
+    const double a = block_sums<2>(e, sh);
+    if (threadIdx.x < 2) n.part_fil[4 * (size_t)blockIdx.x + threadIdx.x] = a;
+}
+
+// Filament forces of the tile's own beads (the sparse force fields' shares are
+// added by k_force_gather once they are written).  With r_c the vector and L_c
+// the length of cylinder (c, c+1), the derivative of the energy by r_c is
+//   G_c = (f0_c + C_c + B_{c+1}) r_c - A_c r_{c-1} - A_{c+1} r_{c+1},
+// f0 = k (L - l0) / L, and for the triple on bead c, with x its cosine and k
+// its (theta0-dependent) constant, A = k / (L_{c-1} L_c), B = k x / L_{c-1}^2,
+// C = k x / L_c^2 (FilamentBendingCosine.cpp:285-345); the force on bead b is
+// G_b - G_{b-1}.  1M beads: 109 us, against 233 us (121 FP64 instructions per
+// bead) with three divisions and two roots per triple and the six bead shares
+// summed one by one.
+__global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want) {
     pdl_wait();      // the previous kernel of the main lane has finished
     MECH_TRACE_KERNEL(n, TK_FIL_FORCE);
-    __shared__ Pos<Real> xs[kFilTile + 4];
-    __shared__ Real fs[(kFilTile + 2) * 3];    // stretch force on the second bead
-    __shared__ Real f1[(kFilTile + 2) * 3];    // bending Fr1
-    __shared__ Real f2[(kFilTile + 2) * 3];    // bending Fr2
-    __shared__ int s_go, s_xb, s_fb;
-    const Tile t = n.ftile[blockIdx.x];
-    const int r = t.replica;
-    if (threadIdx.x == 0) {
-        const CGState& S = n.st[r];
-        s_go = replica_selected(S, want);
-        s_xb = S.xbuf;
-        s_fb = S.fbuf;
-    }
-    __syncthreads();
-    if (!s_go) return;
+    __shared__ double xs[3][kFilTile + 4];                       // beads begin - 2 .. end + 1; then G of begin - 1 .. end - 1
+    __shared__ double rs[3][kFilTile + 3], iL[kFilTile + 3], f0[kFilTile + 3];   // cylinders begin - 2 .. end
+    __shared__ double cA[kFilTile + 2], cB[kFilTile + 2], cC[kFilTile + 2];      // triples on begin - 1 .. end
+    __shared__ bool tri[kFilTile + 2];   // such a triple exists (where not, the next filament is not to be read: it may be non-finite)
+    __shared__ FilTile t;
+    load_fil_tile(n, want, &t);
+    if (!t.go) return;
     const int T = t.end - t.begin;
-    const Real* X = n.x[s_xb];
+    const double* X = n.x[t.xb];
     for (int i = threadIdx.x; i < T + 4; i += blockDim.x) {
         const int b = t.begin - 2 + i;
-        if (b >= 0 && b < n.nb) xs[i] = load_pos(X, b);
+        if (b < 0 || b >= n.nb) continue;
+        const Pos<double> p = load_pos(X, b);
+        xs[0][i] = p.x[0];
+        xs[1][i] = p.x[1];
+        xs[2][i] = p.x[2];
     }
     __syncthreads();
-    // interaction slots s in [0, T + 2): bead j = begin - 1 + s, shared index s + 1
-    for (int s = threadIdx.x; s < T + 2; s += blockDim.x) {
-        const int j = t.begin - 1 + s;
-        Real a[3] = {0, 0, 0}, b1[3] = {0, 0, 0}, b2[3] = {0, 0, 0};
-        if (j >= 0 && j < n.nb) {
-            const int fl = n.bflag[j];
-            if (fl & 1) {
-                Real ks, l0, kb, t0;
-                load_par(n.bpar, j, ks, l0, kb, t0);
-                Real r2[3];
-                pdiff(xs[s + 2], xs[s + 1], r2);
-                stretch_force<Real>(r2[0], r2[1], r2[2], ks, l0, a);
-                if (fl & 2) {
-                    Real r1[3];
-                    pdiff(xs[s + 1], xs[s], r1);
-                    bend_force<Real>(r1, r2, kb, t0, b1, b2);
-                }
+    for (int i = threadIdx.x; i < T + 3; i += blockDim.x) {
+        const int c = t.begin - 2 + i;
+        double r[3] = {0, 0, 0}, inv = 0.0, f = 0.0;
+        if (c >= 0 && c < n.nb && (n.bflag[c] & 1)) {
+            const double2 kl = reinterpret_cast<const double2*>(n.bpar)[2 * (size_t)c];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) r[q] = xs[q][i + 1] - xs[q][i];
+            const double L = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+            inv = 1.0 / L;
+            f = kl.x * (L - kl.y) * inv;
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) rs[q][i] = r[q];
+        iL[i] = inv;
+        f0[i] = f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < T + 2; i += blockDim.x) {
+        const int c = t.begin - 1 + i;   // cylinders c - 1, c at i, i + 1
+        double a = 0.0, bb = 0.0, cc = 0.0;
+        const bool has = c >= 0 && c < n.nb && (n.bflag[c] & 3) == 3;
+        if (has) {
+            const double2 kt = reinterpret_cast<const double2*>(n.bpar)[2 * (size_t)c + 1];
+            const double A = iL[i] * iL[i + 1];
+            double x = (rs[0][i] * rs[0][i + 1] + rs[1][i] * rs[1][i + 1] + rs[2][i] * rs[2][i + 1]) * A;
+            const double x0 = x;
+            double kk = kt.x;
+            if (!theta_is_zero(kt.y)) {
+                if (fabs(fabs(x) - 1.0) < 0.001) x = 0.999 * x;
+                x = clamp_unit(x);
+                const double sinp = sqrt(fmax(1.0 - x * x, 0.0));
+                kk = kk * (sinp * cos(kt.y) - x * sin(kt.y)) / sinp;
             }
+            a = kk * A;
+            const double kx = kk * x0;
+            bb = kx * iL[i] * iL[i];
+            cc = kx * iL[i + 1] * iL[i + 1];
         }
+        cA[i] = a;
+        cB[i] = bb;
+        cC[i] = cc;
+        tri[i] = has;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < T + 1; i += blockDim.x) {   // cylinder begin - 1 + i, at i + 1
+        const double w = f0[i + 1] + cC[i] + cB[i + 1], a0 = cA[i], a1 = cA[i + 1];
+        const bool before = tri[i], after = tri[i + 1];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            fs[3 * s + q] = a[q];
-            f1[3 * s + q] = b1[q];
-            f2[3 * s + q] = b2[q];
+            double g = w * rs[q][i + 1];
+            if (before) g -= a0 * rs[q][i];
+            if (after) g -= a1 * rs[q][i + 2];
+            xs[q][i] = g;
         }
     }
     __syncthreads();
-    const int i = threadIdx.x;
-    if (i < T) {
-        const int b = t.begin + i;
-        Real* Fo = n.f[s_fb ^ 1] + 3 * (size_t)b;
+    if (threadIdx.x < T) {
+        double* Fo = n.f[t.fb ^ 1] + 3 * (size_t)(t.begin + threadIdx.x);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            // stretching: cylinder (b-1, b) then (b, b+1); bending: triples
-            // centred on b-1, b, b+1 (the reference's interaction order)
-            Real v = fs[3 * i + q];
-            v += -fs[3 * (i + 1) + q];
-            v += f2[3 * i + q];
-            v += f1[3 * (i + 1) + q] - f2[3 * (i + 1) + q];
-            v += -f1[3 * (i + 2) + q];
-            Fo[q] = v;
-        }
+        for (int q = 0; q < 3; ++q) Fo[q] = xs[q][threadIdx.x + 1] - xs[q][threadIdx.x];
     }
 }
 
 // ---------------------------------------------------------------------------
 // Every bead adds its sparse contributions (contiguous, in the CSR order) to
 // its filament force, then the CG partials: max |F|, F.F, F.Fprev per tile,
-// reduced by k_finalize_force (a per-tile completion ticket on one address
-// per replica would serialize thousands of atomics).  FP64 engine: each block
-// takes kGatherTiles consecutive tiles and issues the loads of all of them
-// before the per-tile reductions, so a thread keeps several beads' loads in
-// flight; the mixed engine's version is k_force_gather_mx below.
+// reduced by k_finalize_force (a per-tile completion ticket on one address per
+// replica would serialize thousands of atomics).  Each block takes
+// kGatherTiles consecutive tiles and issues the loads of all of them before
+// the reduction.  FP64 engine: FP64-pipe bound (53 us on 1M beads, 94 us with a
+// tree per sum, and the maximum and the finiteness tests in FP64); the maximum
+// is formed on the bits.  The mixed engine's
+// version is k_force_gather_mx below.
 // ---------------------------------------------------------------------------
-
 template <typename Real>
-__device__ __forceinline__ void gather_bead(const DevNet<Real>& n, int b, int fb, Real& mx, Real& ff, Real& ffp) {
+__device__ __forceinline__ void gather_force(const DevNet<Real>& n, int b, int fb, Real F[3], Real& ff, Real& ffp) {
     Real* Fo = n.f[fb ^ 1] + 3 * (size_t)b;
     const Real* Fp = n.f[fb] + 3 * (size_t)b;
-    Real F[3] = {Fo[0], Fo[1], Fo[2]};
+    F[0] = Fo[0];
+    F[1] = Fo[1];
+    F[2] = Fo[2];
+    const Real p0 = Fp[0], p1 = Fp[1], p2 = Fp[2];
     const int c0 = n.csr_off[b], c1 = n.csr_off[b + 1];
     for (int c = c0; c < c1; ++c) {
         F[0] += n.contrib[3 * (size_t)c];
@@ -298,54 +418,75 @@ __device__ __forceinline__ void gather_bead(const DevNet<Real>& n, int b, int fb
     Fo[0] = F[0];
     Fo[1] = F[1];
     Fo[2] = F[2];
-    // a non-finite component makes the bead's max infinite (fmax would drop a NaN)
-    const bool fin = F[0] - F[0] == 0 && F[1] - F[1] == 0 && F[2] - F[2] == 0;
-    mx = fin ? fmax(fmax(fabs(F[0]), fabs(F[1])), fabs(F[2])) : Real(1.0 / 0.0);
     ff = bead_dot(F[0], F[1], F[2], F[0], F[1], F[2]);
-    ffp = bead_dot(F[0], F[1], F[2], Fp[0], Fp[1], Fp[2]);
+    ffp = bead_dot(F[0], F[1], F[2], p0, p1, p2);
+}
+// a non-finite component makes the bead's max infinite (fmax would drop a NaN)
+__device__ __forceinline__ void gather_bead(const DevNet<float>& n, int b, int fb, float& mx, float& ff, float& ffp) {
+    float F[3];
+    gather_force(n, b, fb, F, ff, ffp);
+    const bool fin = F[0] - F[0] == 0 && F[1] - F[1] == 0 && F[2] - F[2] == 0;
+    mx = fin ? fmaxf(fmaxf(fabsf(F[0]), fabsf(F[1])), fabsf(F[2])) : INFINITY;
+}
+// the same on bits: infinity and NaN have the largest, cut to infinity's
+__device__ __forceinline__ void gather_bead(const DevNet<double>& n, int b, int fb, unsigned long long& mx, double& ff,
+                                            double& ffp) {
+    double F[3];
+    gather_force(n, b, fb, F, ff, ffp);
+    mx = min(max(max(abs_bits(F[0]), abs_bits(F[1])), abs_bits(F[2])), 0x7ff0000000000000ULL);
 }
 
-template <typename Real>
-__global__ void __launch_bounds__(kBlock) k_force_gather(DevNet<Real> n, int want) {
-    pdl_trigger();   // the next kernel of the main lane may be scheduled now
-    MECH_TRACE_KERNEL(n, TK_GATHER);
-    __shared__ double sh[32 * 3];
-    __shared__ int s_go[kGatherTiles], s_fb[kGatherTiles];
-    const int t0 = blockIdx.x * kGatherTiles;
+// What a block of kGatherTiles tiles needs of them.
+struct GatherTiles {
+    int go[kGatherTiles], fb[kGatherTiles], rep[kGatherTiles];
+};
+__device__ __forceinline__ void load_gather_tiles(const DevNet<double>& n, int t0, int want, GatherTiles& g) {
     if (threadIdx.x < kGatherTiles) {
         const int ti = t0 + threadIdx.x;
-        int go = 0, fb = 0;
+        int go = 0, fb = 0, rep = -1;
         if (ti < n.n_ftiles) {
-            const CGState& S = n.st[n.ftile[ti].replica];
+            rep = n.ftile[ti].replica;
+            const CGState& S = n.st[rep];
             go = replica_selected(S, want);
             fb = S.fbuf;
         }
-        s_go[threadIdx.x] = go;
-        s_fb[threadIdx.x] = fb;
+        g.go[threadIdx.x] = go;
+        g.fb[threadIdx.x] = fb;
+        g.rep[threadIdx.x] = rep;
     }
     __syncthreads();
-    Real mx[kGatherTiles], ff[kGatherTiles], ffp[kGatherTiles];
+}
+
+__global__ void __launch_bounds__(kBlock) k_force_gather(DevNet<double> n, int want) {
+    pdl_trigger();   // the next kernel of the main lane may be scheduled now
+    MECH_TRACE_KERNEL(n, TK_GATHER);
+    __shared__ double sh[2 * kGatherTiles * kBlock / 32];
+    __shared__ unsigned long long s_mx[kGatherTiles * kBlock / 32];
+    __shared__ GatherTiles g;
+    const int t0 = blockIdx.x * kGatherTiles;
+    load_gather_tiles(n, t0, want, g);
+    unsigned long long mx[kGatherTiles];
+    double v[2 * kGatherTiles];   // F.F of each tile, then F.Fprev
+    int any = 0;
 #pragma unroll
     for (int j = 0; j < kGatherTiles; ++j) {
         mx[j] = 0;
-        ff[j] = 0;
-        ffp[j] = 0;
-        if (!s_go[j]) continue;
+        v[j] = v[kGatherTiles + j] = 0.0;
+        if (!g.go[j]) continue;
+        any = 1;
         const Tile t = n.ftile[t0 + j];
         const int b = t.begin + threadIdx.x;
-        if (b < t.end) gather_bead(n, b, s_fb[j], mx[j], ff[j], ffp[j]);
+        if (b < t.end) gather_bead(n, b, g.fb[j], mx[j], v[j], v[kGatherTiles + j]);
     }
-#pragma unroll
-    for (int j = 0; j < kGatherTiles; ++j) {
-        if (!s_go[j]) continue;   // block-uniform
-        const size_t slot = 4 * (size_t)(t0 + j);
-        double red[3] = {warp_max_r(mx[j]), warp_sum_r(ff[j]), warp_sum_r(ffp[j])};
-        const int ops[3] = {1, 0, 0};
-        block_combine<3>(red, ops, sh);
-        if (threadIdx.x == 0) {
-            n.part_fil[slot + 0] = red[0];
-            n.part_fil[slot + 1] = red[1];
-            n.part_fil[slot + 2] = red[2];
+    if (!any) return;   // block-uniform
+    const unsigned long long m = block_maxima<kGatherTiles>(mx, s_mx);
+    const double a = block_sums<2 * kGatherTiles>(v, sh);
+    if (threadIdx.x < 2 * kGatherTiles) {
+        const int j = threadIdx.x % kGatherTiles;
+        if (g.go[j]) {
+            double* slot = n.part_fil + 4 * (size_t)(t0 + j);
+            if (threadIdx.x < kGatherTiles) slot[0] = __longlong_as_double((long long)m);
+            slot[1 + threadIdx.x / kGatherTiles] = a;
         }
     }
 }
@@ -1297,43 +1438,41 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
 }
 
 // ---------------------------------------------------------------------------
-// direction update d = F + beta d, conjugacy check, backup copy
+// FP64 engine: direction update d = F + beta d, backup copy; kGatherTiles tiles
+// per block as the gather, d.F per tile (26 us on 1M beads with one tile and
+// tree per block)
 // ---------------------------------------------------------------------------
-template <typename Real>
-__global__ void __launch_bounds__(kBlock) k_direction(DevNet<Real> n) {
+__global__ void __launch_bounds__(kBlock) k_direction(DevNet<double> n) {
     pdl_wait();      // the previous kernel of the main lane has finished
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_DIRECTION);
-    __shared__ double sh[32];
-    __shared__ int s_go, s_fb, s_xb, s_bk;
-    __shared__ double s_beta;
-    const Tile t = n.ftile[blockIdx.x];
-    const int r = t.replica;
-    if (threadIdx.x == 0) {
-        const CGState& S = n.st[r];
-        s_go = S.phase == PH_DIR;
-        s_fb = S.fbuf;
-        s_xb = S.xbuf;
-        s_bk = S.backupPending;
-        s_beta = S.beta;
-    }
-    __syncthreads();
-    if (!s_go) return;
-    const int b = t.begin + threadIdx.x;
-    Real dF = 0;
-    if (b < t.end) {
-        const Real* F = n.f[s_fb] + 3 * (size_t)b;
-        Real* D = n.d + 3 * (size_t)b;
-        const Real beta = (Real)s_beta;
-        const Real d0 = F[0] + beta * D[0], d1 = F[1] + beta * D[1], d2 = F[2] + beta * D[2];
+    __shared__ double sh[kGatherTiles * kBlock / 32];
+    __shared__ GatherTiles g;
+    const int t0 = blockIdx.x * kGatherTiles;
+    load_gather_tiles(n, t0, PH_DIR, g);
+    if (!(g.go[0] | g.go[1] | g.go[2] | g.go[3])) return;
+    double dF[kGatherTiles];
+#pragma unroll
+    for (int j = 0; j < kGatherTiles; ++j) {
+        dF[j] = 0.0;
+        if (!g.go[j]) continue;
+        const Tile t = n.ftile[t0 + j];
+        const int b = t.begin + threadIdx.x;
+        if (b >= t.end) continue;
+        const CGState& S = n.st[g.rep[j]];
+        const double beta = S.beta;
+        const double* F = n.f[g.fb[j]] + 3 * (size_t)b;
+        double* D = n.d + 3 * (size_t)b;
+        const double f0 = F[0], f1 = F[1], f2 = F[2];
+        const double d0 = f0 + beta * D[0], d1 = f1 + beta * D[1], d2 = f2 + beta * D[2];
         D[0] = d0;
         D[1] = d1;
         D[2] = d2;
-        dF = bead_dot(d0, d1, d2, F[0], F[1], F[2]);
-        if (s_bk) store_pos(n.xbest, b, load_pos(n.x[s_xb], b));
+        dF[j] = bead_dot(d0, d1, d2, f0, f1, f2);
+        if (S.backupPending) store_pos(n.xbest, b, load_pos(n.x[S.xbuf], b));
     }
-    const double sdF = block_sum_r(dF, sh);
-    if (threadIdx.x == 0) n.part_fil[4 * (size_t)blockIdx.x + 3] = sdF;
+    const double a = block_sums<kGatherTiles>(dF, sh);
+    if (threadIdx.x < kGatherTiles && g.go[threadIdx.x]) n.part_fil[4 * (size_t)(t0 + threadIdx.x) + 3] = a;
 }
 
 template <typename Real>
@@ -1500,7 +1639,7 @@ int launch_energy(const DevNet<Real>& n, int want, int trial, const Lanes& L) {
     cudaStreamWaitEvent(L.side2, L.fork, 0);
     auto fil = [&] {
         if constexpr (sizeof(Real) == 4) launch_k(n.pdl, k_fil_energy_bulk, n.pgrid[0], kBlock, L.main, n, want, trial);
-        else launch_k(n.pdl, k_fil_energy<Real>, n.n_ftiles, kBlock, L.main, n, want, trial);
+        else launch_k(n.pdl, k_fil_energy, n.n_ftiles, kBlock, L.main, n, want, trial);
     };
     if (n.fil_first[0]) fil();
     launched += launch_exvol_energy<Real>(n, want, trial, L.side, false);
@@ -1527,7 +1666,7 @@ int launch_forces(const DevNet<Real>& n, int want, const Lanes& L, int coop_grid
     cudaStreamWaitEvent(L.side2, L.fork, 0);
     auto fil = [&] {
         if constexpr (sizeof(Real) == 4) launch_k(n.pdl, k_fil_force_bulk, n.pgrid[1], kBlock, L.main, n, want);
-        else launch_k(n.pdl, k_fil_force<Real>, n.n_ftiles, kBlock, L.main, n, want);
+        else launch_k(n.pdl, k_fil_force, n.n_ftiles, kBlock, L.main, n, want);
     };
     if (n.fil_first[1]) fil();
     launched += launch_exvol_forces<Real>(n, want, L.side, false);
@@ -1547,7 +1686,7 @@ int launch_forces(const DevNet<Real>& n, int want, const Lanes& L, int coop_grid
         }
     }
     if constexpr (sizeof(Real) == 4) k_force_gather_mx<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, L.main>>>(n, want);
-    else k_force_gather<Real><<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, L.main>>>(n, want);
+    else k_force_gather<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, L.main>>>(n, want);
     launch_k(n.pdl, k_finalize_force<Real>, n.R, kBlock, L.main, n, want);
     return launched + 3;
 }
@@ -1555,7 +1694,7 @@ int launch_forces(const DevNet<Real>& n, int want, const Lanes& L, int coop_grid
 template <typename Real>
 int launch_direction(const DevNet<Real>& n, cudaStream_t s) {
     if constexpr (sizeof(Real) == 4) launch_k(n.pdl, k_direction_mx, n.pgrid[2], kBlock, s, n);
-    else launch_k(n.pdl, k_direction<Real>, n.n_ftiles, kBlock, s, n);
+    else launch_k(n.pdl, k_direction, (n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, s, n);
     launch_k(n.pdl, k_finalize_direction<Real>, n.R, kBlock, s, n);
     return 2;
 }
@@ -1598,13 +1737,13 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
     switch (which) {
         case 0:
             if constexpr (sizeof(Real) == 4) k_fil_energy_bulk<<<n.pgrid[0], kBlock, 0, s>>>(n, -1, 0);
-            else k_fil_energy<Real><<<n.n_ftiles, kBlock, 0, s>>>(n, -1, 0);
+            else k_fil_energy<<<n.n_ftiles, kBlock, 0, s>>>(n, -1, 0);
             return 1;
         case 1:
             if constexpr (sizeof(Real) == 4) k_fil_force_bulk<<<n.pgrid[1], kBlock, 0, s>>>(n, -1);
-            else k_fil_force<Real><<<n.n_ftiles, kBlock, 0, s>>>(n, -1);
+            else k_fil_force<<<n.n_ftiles, kBlock, 0, s>>>(n, -1);
             if constexpr (sizeof(Real) == 4) k_force_gather_mx<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
-            else k_force_gather<Real><<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
+            else k_force_gather<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
             k_finalize_force<Real><<<n.R, kBlock, 0, s>>>(n, -1);
             return 3;
         case 2: if (lm + bb_t > 0) { k_bond_bnd<Real><<<lm + bb_t, kBlock, 0, s>>>(n, -1, 0, 0, lm, ev_t); return 1; } return 0;
@@ -1612,15 +1751,15 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
         case 4:   // filament energy of a line-search pass (positions x + lambda d formed and written;
                   // mixed: the two-trial pass, lambda and lambda / 2)
             if constexpr (sizeof(Real) == 4) k_fil_energy_bulk<<<n.pgrid[0], kBlock, 0, s>>>(n, -1, kTrialDual);
-            else k_fil_energy<Real><<<n.n_ftiles, kBlock, 0, s>>>(n, -1, 1);
+            else k_fil_energy<<<n.n_ftiles, kBlock, 0, s>>>(n, -1, 1);
             return 1;
         case 5:   // filament forces alone
             if constexpr (sizeof(Real) == 4) k_fil_force_bulk<<<n.pgrid[1], kBlock, 0, s>>>(n, -1);
-            else k_fil_force<Real><<<n.n_ftiles, kBlock, 0, s>>>(n, -1);
+            else k_fil_force<<<n.n_ftiles, kBlock, 0, s>>>(n, -1);
             return 1;
         case 6:   // the sparse gather with the CG partials alone
             if constexpr (sizeof(Real) == 4) k_force_gather_mx<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
-            else k_force_gather<Real><<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
+            else k_force_gather<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
             return 1;
     }
     return 0;
