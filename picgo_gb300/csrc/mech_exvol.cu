@@ -41,13 +41,33 @@ static __device__ double pair_energy_d(const double* c1, const double* c2, const
 }
 
 
+// The reference's coplanarity decision |n . v3| / (|n| |v3|) < 0.1: on the
+// squares, without its two roots and six divisions (~75 FP64 instructions),
+// unless they lie so near the threshold that its rounding decides (or compare
+// with nothing).
+static __device__ __forceinline__ bool nearly_coplanar(const double* c1, const double* c2, const double* c3,
+                                                       const double* c4) {
+    double a[3], b[3], v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        a[k] = c2[k] - c1[k];
+        b[k] = c3[k] - c1[k];
+        v[k] = c4[k] - c1[k];
+    }
+    const double n[3] = {a[1] * b[2] - a[2] * b[1], a[2] * b[0] - a[0] * b[2], a[0] * b[1] - a[1] * b[0]};
+    const double nv = dot3(n, v), lhs = nv * nv, rhs = 0.01 * (dot3(n, n) * dot3(v, v)), gap = 1e-10 * rhs;
+    if (lhs < rhs - gap) return true;
+    if (lhs > rhs + gap) return false;
+    return coplanarity<double>(c1, c2, c3, c4) < 0.1;
+}
+
 // FP64 forces of a pair at double positions, with the reference's coplanar
 // move of c2 (:610-626, force path only).
 static __device__ bool pair_forces_d(const double* c1, const double* c2in, const double* c3, const double* c4, double kRep,
                                      double out[4][3]) {
     double moved2[3];
     const double* c2 = c2in;
-    if (coplanarity<double>(c1, c2in, c3, c4) < 0.1) {
+    if (nearly_coplanar(c1, c2in, c3, c4)) {
         push_c2(c1, c2in, c3, moved2);
         c2 = moved2;
     }
@@ -195,7 +215,7 @@ __global__ void __launch_bounds__(kBlock) k_exvol_fb_force(DevNet<Real> n, doubl
 }
 
 // ---------------------------------------------------------------------------
-// main pair kernel (energy partials or force contributions)
+// mixed engine: main pair kernel (per-pair energies or force contributions)
 // ---------------------------------------------------------------------------
 template <typename Real>
 __device__ __forceinline__ void flag_fallback(const DevNet<Real>& n, int r, int pr, double lam) {
@@ -260,12 +280,274 @@ __device__ __forceinline__ float mixed_pair_energy(const Pos<float>& p1, const P
     return u;
 }
 
+// ---------------------------------------------------------------------------
+// FP64 engine: the reference's formulas for every pair, bound by the FP64 pipe
+// (a warp's FP64 instruction holds its SM sub-partition's pipe for ~70 cycles
+// whatever the number of active lanes).  A pair per lane takes ~800 FP64
+// instructions for the energy and ~1,650 for the forces in one warp, so a few
+// pairs take as long as 608 warps of them (28 and 59 us).  Split over the four
+// warps of a block (32 pairs on the lanes, warp w the w-th arctangent term, the
+// invariants formed by every warp), the longest warp has about a third of that.
+// Full rounds of 608 warps (76 tiles of 256 pairs) go unsplit; the rest goes
+// split where that beats another round: three split blocks on every SM, 57
+// tiles.  Both forms make the same operations in the same order: same bits.
+// 78 pairs: energy 35 -> 19 us, forces 62 -> 29 us (with the chain's other
+// launches); 59,737 pairs, where a fourth round held 3% of the pairs: 131 ->
+// 111 and 234 -> 189 us.
+// ---------------------------------------------------------------------------
+constexpr int kExvolRoundTiles = 152 * 4 * 32 / kSparseTile;
+constexpr int kExvolSplitTiles = 3 * 152 * 32 / kSparseTile;
+inline int exvol_split_tiles(int nt) {
+    const int rest = nt % kExvolRoundTiles;
+    return rest <= kExvolSplitTiles ? rest : 0;
+}
+
+// One pair's term w of the four: operands shared through shared memory.
+struct SplitTerm {
+    double tC, tX, te, ta;    // partials of the term (forces)
+    double S;                 // N / Y * ATG
+};
+struct SplitShared {
+    double c[4][3][32];       // bead positions; c2 moved off the plane for forces
+    double N[4][32];          // CC, GG, DD (HH = CC + GG - DD)
+    SplitTerm t[4][32];
+    double Y[4][32];
+    double G[6][32];          // G00, G01, G02, G11, G12, G22
+    int bad[32];
+};
+
+// The invariants that every warp forms (pair_inv, cross = false).
+struct SplitInv {
+    double v12[3], v34[3], v31[3];
+    double a, b, c, d, e, F, JJ;
+};
+__device__ __forceinline__ void split_invariants(const SplitShared& s, int l, SplitInv& p) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        p.v12[k] = s.c[1][k][l] - s.c[0][k][l];
+        p.v34[k] = s.c[3][k][l] - s.c[2][k][l];
+        p.v31[k] = s.c[0][k][l] - s.c[2][k][l];
+    }
+    p.a = dot3(p.v12, p.v12);
+    p.b = dot3(p.v34, p.v34);
+    p.c = dot3(p.v31, p.v31);
+    p.d = dot3(p.v12, p.v34);
+    p.e = dot3(p.v12, p.v31);
+    p.F = dot3(p.v34, p.v31);
+    const double* v12 = p.v12;
+    const double* v34 = p.v34;
+    const double* v31 = p.v31;
+    const double x21[3] = {v34[1] * v12[2] - v34[2] * v12[1], v34[2] * v12[0] - v34[0] * v12[2],
+                           v34[0] * v12[1] - v34[1] * v12[0]};
+    const double trip = -(x21[0] * v31[0] + x21[1] * v31[1] + x21[2] * v31[2]);
+    p.JJ = -trip * trip;
+}
+
+// 32 pairs [i0, min(i0 + 32, end)) of replica r in a block of four warps.
+template <typename Real>
+__device__ void exvol_split(const DevNet<Real>& n, int r, const Real* X, bool tr, double lam, int force, int i0, int end,
+                            SplitShared& s) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, i = i0 + l;
+    const bool valid = i < end;
+    if (valid) {
+        const int4 bs = n.ev_bead[i];
+        const int bead = w == 0 ? bs.x : w == 1 ? bs.y : w == 2 ? bs.z : bs.w;
+        double c[3];
+        to_double(bead_at(X, n.d, bead, tr, lam), c);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s.c[w][k][l] = c[k];
+    }
+    if (w == 0) s.bad[l] = 0;
+    __syncthreads();
+    if (force) {   // the reference's move of c2, decided and applied by one warp
+        if (w == 1 && valid) {
+            double c[4][3], m[3];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) c[a][k] = s.c[a][k][l];
+            if (nearly_coplanar(c[0], c[1], c[2], c[3])) {
+                push_c2(c[0], c[1], c[2], m);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) s.c[1][k][l] = m[k];
+            }
+        }
+        __syncthreads();
+    }
+    SplitInv p;
+    double Y = 1, N = 0, ATG = 0, al = 0, be = 0;
+    if (valid) {
+        split_invariants(s, l, p);
+        // term w: Y, N and the two abscissae (A, E, B, F of the reference)
+        double u = p.a, v = p.c, x = p.e;   // Y = sqrt((sqrt(u v) + x) (sqrt(u v) - x))
+        al = p.a + p.e;
+        be = p.e;
+        if (w == 0) {
+            N = p.d * p.e - p.a * p.F;
+        } else if (w == 1) {
+            double v14[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v14[k] = s.c[3][k][l] - s.c[0][k][l];
+            v = dot3(v14, v14);
+            x = dot3(p.v12, v14);
+            N = p.d * x - p.a * dot3(p.v34, v14);
+            al = p.a + p.e - p.d;
+            be = p.e - p.d;
+        } else if (w == 2) {
+            u = p.b;
+            x = p.F;
+            N = p.b * p.e - p.d * p.F;
+            al = p.F;
+            be = p.F - p.b;
+        } else {
+            double v32[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v32[k] = s.c[1][k][l] - s.c[2][k][l];
+            u = p.b;
+            v = dot3(v32, v32);
+            x = dot3(p.v34, v32);
+            al = p.d + p.F;
+            be = p.d + p.F - p.b;
+        }
+        const double uv = sqrt(u * v);
+        Y = sqrt(fmax(0.0, (uv + x) * (uv - x)));
+        if (w < 3) s.N[w][l] = N;
+        ATG = atan_of(al / Y) - atan_of(be / Y);
+    }
+    __syncthreads();
+    if (valid) {
+        if (w == 3) N = s.N[0][l] + s.N[1][l] - s.N[2][l];
+        SplitTerm t;
+        t.S = N / Y * ATG;
+        t.tC = t.tX = t.te = t.ta = 0.0;
+        if (force) {
+            const double T1 = Y * Y / (Y * Y + al * al), T2 = Y * Y / (Y * Y + be * be);
+            t.tC = ATG / Y;
+            t.tX = -(ATG * N) / (Y * Y) + (-T1 * al + T2 * be) * N / (Y * Y * Y);
+            t.te = (T1 - T2) * N / (Y * Y);
+            t.ta = T1 * N / (Y * Y);
+        }
+        s.t[w][l] = t;
+        s.Y[w][l] = Y;
+    }
+    __syncthreads();
+    const double kRep = valid ? (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i] : 0.0;
+    if (!force) {
+        if (w == 0 && valid) {
+            const double U = 0.5 * kRep / p.JJ * (s.t[0][l].S + s.t[1][l].S + s.t[2][l].S + s.t[3][l].S);
+            const bool ok = !(bad_value(U) || U < -1.0);
+            n.ev_energy[i] = ok ? U : 0.0;
+            if (!ok) flag_fallback(n, r, i, tr ? lam : 0.0);
+        }
+        return;
+    }
+    if (valid) {   // entries of G, split over the warps
+        const SplitTerm A = s.t[0][l], E = s.t[1][l], B = s.t[2][l], T = s.t[3][l];
+        const double AA = s.Y[0][l], EE = s.Y[1][l], BB = s.Y[2][l], FF = s.Y[3][l];
+        const double a = p.a, b = p.b, c = p.c, d = p.d, e = p.e, F = p.F;
+        if (w == 0) {
+            s.G[0][l] = A.tC * (-2 * F) + A.tX * (c / AA) + A.ta * 2 + E.tC * (2 * (F - b)) + E.tX * ((b + c - 2 * F) / EE) +
+                        E.ta * 2 + T.tC * (-2 * b) + T.tX * (b / FF);
+            s.G[5][l] = A.tX * (a / AA) + E.tX * (a / EE) + B.tX * (b / BB) + T.tX * (b / FF);
+        } else if (w == 1) {
+            s.G[1][l] = A.tC * e + E.tC * (2 * d - e) + E.tX * ((e - d) / EE) + E.te * (-1) + B.tC * (-F) +
+                        T.tC * (2 * d + F) + T.tX * (-(d + F) / FF) + T.te;
+            s.G[2][l] = A.tC * d + A.tX * (-e / AA) + A.te + E.tC * (-d) + E.tX * (-(e - d) / EE) + E.te + B.tC * b +
+                        T.tC * (-b) + T.tX * (b / FF);
+        } else if (w == 2) {
+            s.G[3][l] = E.tC * (-2 * a) + E.tX * (a / EE) + B.tC * (2 * e) + B.tX * (c / BB) + B.te * (-2) + B.ta * 2 +
+                        T.tC * (-2 * (a + e)) + T.tX * ((a + c + 2 * e) / FF) + T.te * (-2) + T.ta * 2;
+        } else {
+            s.G[4][l] = A.tC * (-a) + E.tC * a + E.tX * (-a / EE) + B.tC * (-d) + B.tX * (-F / BB) + B.te + T.tC * d +
+                        T.tX * (-(d + F) / FF) + T.te;
+        }
+    }
+    __syncthreads();
+    if (valid) {   // warp w: the force on bead w
+        const double a = p.a, b = p.b, c = p.c, d = p.d, e = p.e, F = p.F;
+        const double G[3][3] = {{s.G[0][l], s.G[1][l], s.G[2][l]}, {s.G[1][l], s.G[3][l], s.G[4][l]}, {s.G[2][l], s.G[4][l], s.G[5][l]}};
+        const double J00 = 2 * (-b * c + F * F), J01 = 2 * (c * d - e * F), J02 = 2 * (b * e - d * F),
+                     J11 = 2 * (-a * c + e * e), J12 = 2 * (-d * e + a * F), J22 = 2 * (d * d - a * b);
+        const double J[3][3] = {{J00, J01, J02}, {J01, J11, J12}, {J02, J12, J22}};
+        const double invJJ = 1.0 / p.JJ;
+        const double S = s.t[0][l].S + s.t[1][l].S + s.t[2][l].S + s.t[3][l].S;
+        const double pref = kRep * invJJ / 2.0;
+        double dv[3];
+#pragma unroll
+        for (int y = 0; y < 3; ++y) {
+            const double Jw = w == 0 ? J[2][y] - J[0][y] : w == 1 ? J[0][y] : w == 2 ? -J[2][y] - J[1][y] : J[1][y];
+            const double Gw = w == 0 ? G[2][y] - G[0][y] : w == 1 ? G[0][y] : w == 2 ? -G[2][y] - G[1][y] : G[1][y];
+            dv[y] = pref * (-invJJ * S * Jw + Gw);
+        }
+        Real* dst = slot_ptr(n, n.slot_base[K_EXVOL] + 4 * i + w);
+        bool bad = false;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double o = -(dv[0] * p.v12[k] + dv[1] * p.v34[k] + dv[2] * p.v31[k]);
+            if (bad_value(o)) bad = true;
+            dst[k] = (Real)o;
+        }
+        if (bad) atomicOr(&s.bad[l], 1);
+    }
+    __syncthreads();
+    if (w == 0 && valid && s.bad[l]) flag_fallback(n, r, i, 0.0);
+}
+
+// Blocks [0, 2 unsplit): half a tile each, a pair per thread; then eight blocks
+// per split tile.
+template <typename Real>
+__global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, int trial, int force, int tile_off,
+                                                    int unsplit) {
+    MECH_TRACE_KERNEL(n, TK_EXVOL);
+    __shared__ int s_go, s_xb;
+    __shared__ double s_lam;
+    __shared__ SplitShared s;
+    const int sb = (int)blockIdx.x - 2 * unsplit;
+    const Tile t = n.stile[tile_off + (sb < 0 ? (int)blockIdx.x >> 1 : unsplit + (sb >> 3))];
+    const int begin = t.begin + (sb < 0 ? 128 * ((int)blockIdx.x & 1) : 32 * (sb & 7));
+    if (begin >= t.end) return;
+    if (threadIdx.x == 0) {
+        const CGState& S = n.st[t.replica];
+        s_go = want < 0 ? (S.active != 0) : (S.phase == want);
+        s_xb = S.xbuf;
+        s_lam = S.lambda;
+    }
+    __syncthreads();
+    if (!s_go) return;
+    const Real* X = n.x[s_xb];
+    const bool tr = trial != 0;
+    if (sb >= 0) {
+        exvol_split(n, t.replica, X, tr, s_lam, force, begin, t.end, s);
+        return;
+    }
+    const int i = begin + threadIdx.x;
+    if (i >= t.end) return;
+    const int4 bs = n.ev_bead[i];
+    const double kRep = (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i];
+    double c1[3], c2[3], c3[3], c4[3];
+    to_double(bead_at(X, n.d, bs.x, tr, s_lam), c1);
+    to_double(bead_at(X, n.d, bs.y, tr, s_lam), c2);
+    to_double(bead_at(X, n.d, bs.z, tr, s_lam), c3);
+    to_double(bead_at(X, n.d, bs.w, tr, s_lam), c4);
+    if (!force) {
+        const double u = pair_energy_d(c1, c2, c3, c4, kRep);
+        n.ev_energy[i] = u == u ? u : 0.0;
+        if (u != u) flag_fallback(n, t.replica, i, tr ? s_lam : 0.0);
+    } else {
+        double out[4][3];
+        const bool ok = pair_forces_d(c1, c2, c3, c4, kRep, out);
+        for (int a = 0; a < 4; ++a) {
+            Real* cdst = slot_ptr(n, n.slot_base[K_EXVOL] + 4 * i + a);
+            for (int k = 0; k < 3; ++k) cdst[k] = (Real)out[a][k];
+        }
+        if (!ok) flag_fallback(n, t.replica, i, 0.0);
+    }
+}
+
 template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int trial, int force, int tile_off) {
     MECH_TRACE_KERNEL(n, TK_EXVOL);
-    __shared__ double sh[32];
     __shared__ int s_go, s_xb;
-    __shared__ double s_lam;
     __shared__ float s_lf;   // the step rounded once (mixed engine)
     const int ti = tile_off + blockIdx.x;
     const Tile t = n.stile[ti];
@@ -274,7 +556,6 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
         const CGState& S = n.st[r];
         s_go = want < 0 ? (S.active != 0) : (S.phase == want);
         s_xb = S.xbuf;
-        s_lam = S.lambda;
         s_lf = (float)S.lambda;
     }
     __syncthreads();
@@ -283,44 +564,18 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
     const bool tr = trial != 0;
     const int i = t.begin + threadIdx.x;
     const bool valid = i < t.end;
-    double e = 0.0;   // FP64 engine
-    float ef = 0.f;   // mixed engine
+    float ef = 0.f;
     bool need64 = false, need64b = false;
     // a two-trial pass also evaluates the energy at lambda / 2 (mixed engine)
-    const bool dual = sizeof(Real) == 4 && trial == kTrialDual && !force;
+    const bool dual = trial == kTrialDual && !force;
     if (valid) {
         const int4 bs = n.ev_bead[i];
-        auto pos = [&](int b) -> Pos<Real> {
-            if constexpr (sizeof(Real) == 4) {
-                const Pos<float> p = load_pos(X, b);
-                return tr ? moved_f(p, n.d, b, s_lf) : p;
-            } else {
-                return bead_at(X, n.d, b, tr, s_lam);
-            }
+        auto pos = [&](int b) -> Pos<float> {
+            const Pos<float> p = load_pos(X, b);
+            return tr ? moved_f(p, n.d, b, s_lf) : p;
         };
         const Pos<Real> p1 = pos(bs.x), p2 = pos(bs.y), p3 = pos(bs.z), p4 = pos(bs.w);
-        if constexpr (sizeof(Real) == 8) {
-            const double kRepD = (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i];
-            // FP64 engine: the reference's formulas, every pair
-            double c1[3], c2[3], c3[3], c4[3];
-            to_double(p1, c1);
-            to_double(p2, c2);
-            to_double(p3, c3);
-            to_double(p4, c4);
-            if (!force) {
-                const double u = pair_energy_d(c1, c2, c3, c4, kRepD);
-                if (u != u) flag_fallback(n, r, i, tr ? s_lam : 0.0);
-                else e = u;
-            } else {
-                double out[4][3];
-                const bool ok = pair_forces_d(c1, c2, c3, c4, kRepD, out);
-                for (int a = 0; a < 4; ++a) {
-                    Real* cdst = slot_ptr(n, n.slot_base[K_EXVOL] + 4 * i + a);
-                    for (int k = 0; k < 3; ++k) cdst[k] = (Real)out[a][k];
-                }
-                if (!ok) flag_fallback(n, r, i, 0.0);
-            }
-        } else if (!force) {
+        if (!force) {
             // mixed engine: single precision unless the pair is ill-conditioned
             const float kRep = n.ev_k[i] * n.ev_la[i] * n.ev_lb[i];
             ef = mixed_pair_energy(p1, p2, p3, p4, kRep, need64);
@@ -383,14 +638,8 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
             }
         }
     }
-    if constexpr (sizeof(Real) == 4) {
-        append_fp64(n, need64, r, i);
-        if (dual) append_fp64(n, need64b, r, i | kExtSecond);   // block-uniform
-    }
-    if (!force && sizeof(Real) == 8) {
-        e = block_sum(e, sh);
-        if (threadIdx.x == 0) n.part_sp[ti] = e;
-    }
+    append_fp64(n, need64, r, i);
+    if (dual) append_fp64(n, need64b, r, i | kExtSecond);   // block-uniform
 }
 
 // Mixed engine's extended pass: the listed (ill-conditioned) pairs in FP64,
@@ -618,8 +867,8 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
 
 // The end of an energy evaluation's excluded-volume chain, one launch:
 // blocks [0, kFbEnergyBlocks) compute the Simpson energies of flagged pairs;
-// in the mixed engine the following blocks form the deterministic per-tile
-// sums of the per-pair energies (one block per exvol tile).
+// the following blocks form the deterministic per-tile sums of the per-pair
+// energies (one block per exvol tile).
 constexpr int kFbEnergyBlocks = 64;
 template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_exvol_energy_tail(DevNet<Real> n, int want, int trial, int tile_off) {
@@ -654,6 +903,10 @@ __global__ void __launch_bounds__(kBlock) k_exvol_energy_tail(DevNet<Real> n, in
                     if (threadIdx.x == 0) store_pair(n.part_sp + ti, a[0].h, a[0].l);
                 }
             }
+        } else if (go) {
+            const int i = t.begin + threadIdx.x;
+            const double e = block_sum(i < t.end ? n.ev_energy[i] : 0.0, sh);
+            if (threadIdx.x == 0) n.part_sp[ti] = e;
         }
     }
 }
@@ -686,13 +939,16 @@ int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t
     const int nt = ev_tiles_of(n, &off);
     if (nt == 0) return 0;
     if (standalone) reset_counts(n, s);
-    k_exvol<Real><<<nt, kBlock, 0, s>>>(n, want, trial, 0, off);
     int k = 1;
-    if constexpr (sizeof(Real) == 4) {
+    if constexpr (sizeof(Real) == 8) {
+        const int split = exvol_split_tiles(nt);
+        k_exvol_fp64<Real><<<2 * (nt - split) + 8 * split, 128, 0, s>>>(n, want, trial, 0, off, nt - split);
+    } else {
+        k_exvol<Real><<<nt, kBlock, 0, s>>>(n, want, trial, 0, off);
         k_exvol_ext<Real><<<kExtBlocks, 128, 0, s>>>(n, trial, 0);
         ++k;
     }
-    k_exvol_energy_tail<Real><<<kFbEnergyBlocks + (sizeof(Real) == 4 ? nt : 0), kBlock, 0, s>>>(n, want, trial, off);
+    k_exvol_energy_tail<Real><<<kFbEnergyBlocks + nt, kBlock, 0, s>>>(n, want, trial, off);
     return k + 1;
 }
 
@@ -702,9 +958,12 @@ int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool st
     const int nt = ev_tiles_of(n, &off);
     if (nt == 0) return 0;
     if (standalone) reset_counts(n, s);
-    k_exvol<Real><<<nt, kBlock, 0, s>>>(n, want, 0, 1, off);
     int k = 1;
-    if constexpr (sizeof(Real) == 4) {
+    if constexpr (sizeof(Real) == 8) {
+        const int split = exvol_split_tiles(nt);
+        k_exvol_fp64<Real><<<2 * (nt - split) + 8 * split, 128, 0, s>>>(n, want, 0, 1, off, nt - split);
+    } else {
+        k_exvol<Real><<<nt, kBlock, 0, s>>>(n, want, 0, 1, off);
         k_exvol_ext<Real><<<kExtBlocks, 128, 0, s>>>(n, 0, 1);
         ++k;
     }
