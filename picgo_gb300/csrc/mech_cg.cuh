@@ -10,6 +10,11 @@
 
 namespace mech {
 
+// whether a pass of mode `trial` evaluates a second trial for a replica in state S
+__device__ __forceinline__ bool second_trial(int trial, int dual) {
+    return trial == kTrialBoth || (trial == kTrialDual && dual);
+}
+
 __device__ __forceinline__ bool replica_selected(const CGState& S, int want) {
     return want < 0 ? (S.active != 0) : (S.phase == want);
 }
@@ -89,7 +94,7 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
     const int nslot = run_slots(rt.fil_begin, rt.fil_end, stride);
     const int ffk[K_NUM_SPARSE] = {MECH_FF_LINKER, MECH_FF_MOTOR, MECH_FF_EXVOL, MECH_FF_BOUNDARY};
     double e[MECH_NUM_FF], e2[MECH_NUM_FF];
-    const bool dual = sizeof(Real) == 4 && trial == kTrialDual;
+    const bool dual = sizeof(Real) == 4 && second_trial(trial, n.st[r].dual);
     // the fallback list's length, loaded now so that thread 0's step logic does
     // not wait on it at the end
     const int fb_count = threadIdx.x == 0 ? __ldcg(n.ev_fb_count) : 0;

@@ -12,6 +12,7 @@
 namespace mech {
 
 constexpr int kBlock = 256;
+constexpr int kDualSearches = 4;         // see CGState::dual
 constexpr double kLambdaTol = 1e-8;      // CGMethod::LAMBDATOL (CGMethod.hpp:98)
 constexpr double kLambdaReduce = 0.5;    // CGMethod::LAMBDAREDUCE
 constexpr double kBacktrackSlope = 0.4;  // CGMethod::BACKTRACKSLOPE
@@ -161,6 +162,9 @@ __device__ __forceinline__ void begin_iteration(CGState& S) {
     S.numEnergyCall++;       // the reference evaluates E0 here
     const double armijo = S.safeMode ? 0.0 : kBacktrackSlope;
     S.reducedSlope = armijo * S.slope;
+    if (S.searchTrials > 1) S.dual = kDualSearches;
+    else if (S.dual > 0) --S.dual;
+    S.searchTrials = 0;
     S.phase = PH_LS_TRIAL;
 }
 
@@ -169,6 +173,7 @@ __device__ __forceinline__ void begin_iteration(CGState& S) {
 __device__ __forceinline__ void line_search_step(CGState& S, double E, int trial_buf) {
     S.numEnergyCall++;
     S.numTrials++;
+    S.searchTrials++;
     double lambda = S.lambda;
     double Elam = E;
     const double ideal = -S.reducedSlope * lambda;
@@ -186,7 +191,10 @@ __device__ __forceinline__ void line_search_step(CGState& S, double E, int trial
         Elam = S.E0;
     }
     S.lambda = lambda;
-    if (!done) return;                 // next trial at the halved lambda
+    if (!done) {                       // next trial at the halved lambda
+        S.dual = kDualSearches;
+        return;
+    }
     S.totalEnergy = Elam;
     if (lambda == 0.0) {
         S.phase = PH_FAILED;

@@ -18,6 +18,7 @@
 // rounding of its threshold, which go to the extended pass.
 #include <cuda_runtime.h>
 
+#include "mech_cg.cuh"
 #include "mech_device.cuh"
 #include "mech_exvol_math.cuh"
 
@@ -547,7 +548,7 @@ __global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, in
 template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int trial, int force, int tile_off) {
     MECH_TRACE_KERNEL(n, TK_EXVOL);
-    __shared__ int s_go, s_xb;
+    __shared__ int s_go, s_xb, s_dual;
     __shared__ float s_lf;   // the step rounded once (mixed engine)
     const int ti = tile_off + blockIdx.x;
     const Tile t = n.stile[ti];
@@ -557,6 +558,7 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
         s_go = want < 0 ? (S.active != 0) : (S.phase == want);
         s_xb = S.xbuf;
         s_lf = (float)S.lambda;
+        s_dual = S.dual;
     }
     __syncthreads();
     if (!s_go) return;
@@ -566,8 +568,8 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
     const bool valid = i < t.end;
     float ef = 0.f;
     bool need64 = false, need64b = false;
-    // a two-trial pass also evaluates the energy at lambda / 2 (mixed engine)
-    const bool dual = trial == kTrialDual && !force;
+    // a pass with a second trial also evaluates the energy at lambda / 2
+    const bool dual = !force && second_trial(trial, s_dual);
     if (valid) {
         const int4 bs = n.ev_bead[i];
         auto pos = [&](int b) -> Pos<float> {
@@ -885,7 +887,7 @@ __global__ void __launch_bounds__(kBlock) k_exvol_energy_tail(DevNet<Real> n, in
             if (go) {   // block-uniform
                 // per-pair energies as (hi, lo) pairs, summed compensated in single precision
                 const int i = t.begin + threadIdx.x;
-                if (trial == kTrialDual) {   // both trials of a two-trial pass
+                if (second_trial(trial, S.dual)) {   // both trials of the pass
                     FF a[2];
                     if (i < t.end) {
                         add_pair(a[0], load_pair(n.ev_energy + i));

@@ -723,7 +723,8 @@ __device__ __forceinline__ StageRange stage_range(int tb, int te, int nb, int ha
 // A block's tile descriptors, read once at kernel start (one thread per tile)
 // so the producing thread issues copies without chasing global pointers:
 // (begin, end, replica, bits) with bit 0 = selected by this launch, bits 1-2 =
-// xbuf, bit 3 = fbuf of the tile's replica, plus that replica's lambda.  A
+// xbuf, bit 3 = fbuf of the tile's replica, bit 4 = its pass has a second trial,
+// plus that replica's lambda.  A
 // replica's state cannot change while this block still holds unprocessed
 // tiles of it (its finalizer waits for every tile), so the copies stay valid.
 constexpr int kBulkMaxTiles = kFilBulkMaxTiles;
@@ -734,7 +735,7 @@ __device__ __forceinline__ void load_descriptors(const DevNet<float>& n, int t0,
         const Tile t = n.ftile[t0 + k];
         const CGState& S = n.st[t.replica];
         desc[k] = make_int4(t.begin, t.end, t.replica,
-                            (replica_selected(S, want) ? 1 : 0) | (S.xbuf << 1) | (S.fbuf << 3));
+                            (replica_selected(S, want) ? 1 : 0) | (S.xbuf << 1) | (S.fbuf << 3) | (S.dual ? 16 : 0));
         lf[k] = (float)S.lambda;
     }
 }
@@ -818,10 +819,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
                 ++issued;
             }
     }
-    // a two-trial pass (trial == kTrialDual): energies at lambda into slots 0, 1
-    // of the run and at lambda / 2 into slots 2, 3; trial positions into the
-    // two buffers after the current one
-    const bool dual = trial == kTrialDual;
+    // a pass with a second trial: energies at lambda into slots 0, 1 of the run
+    // and at lambda / 2 into slots 2, 3; trial positions into the two buffers
+    // after the current one
+    bool dual = false;
     int cur = -1, first = 0, cnt = 0, xb = 0, j = 0;
     bool go = false;
     float lf = 0.f;
@@ -848,6 +849,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
             eb2 = FF();
             go = t.w & 1;
             xb = (t.w >> 1) & 3;
+            dual = second_trial(trial, t.w & 16);
             lf = s_lf[k];
         }
         if (!go) continue;
@@ -1318,7 +1320,7 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
                                                      int ev_tiles) {
     MECH_TRACE_KERNEL(n, TK_BOND);
     __shared__ double sh[64];   // block_reduce_ff<2>: 32 * 4 floats
-    __shared__ int s_go, s_xb;
+    __shared__ int s_go, s_xb, s_dual;
     __shared__ double s_lam;
     __shared__ float s_lf;   // the step rounded once (mixed engine)
     const int ti = blockIdx.x < n_lm_tiles ? blockIdx.x : blockIdx.x + ev_tiles;
@@ -1331,13 +1333,14 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
         s_xb = S.xbuf;
         s_lam = S.lambda;
         s_lf = (float)S.lambda;
+        s_dual = S.dual;
     }
     __syncthreads();
     if (!s_go) return;
     const Real* X = n.x[s_xb];
     const bool tr = trial != 0;
-    // a two-trial pass also evaluates the energy at lambda / 2 (mixed engine)
-    const bool dual = sizeof(Real) == 4 && trial == kTrialDual && !force;
+    // a pass with a second trial also evaluates the energy at lambda / 2 (mixed engine)
+    const bool dual = sizeof(Real) == 4 && !force && second_trial(trial, s_dual);
     auto pos_at = [&](int b, float lfs) -> Pos<Real> {
         if constexpr (sizeof(Real) == 4) {
             const Pos<float> p = load_pos(X, b);
@@ -1750,7 +1753,7 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
         case 3: if (lm + bb_t > 0) { k_bond_bnd<Real><<<lm + bb_t, kBlock, 0, s>>>(n, -1, 0, 1, lm, ev_t); return 1; } return 0;
         case 4:   // filament energy of a line-search pass (positions x + lambda d formed and written;
                   // mixed: the two-trial pass, lambda and lambda / 2)
-            if constexpr (sizeof(Real) == 4) k_fil_energy_bulk<<<n.pgrid[0], kBlock, 0, s>>>(n, -1, kTrialDual);
+            if constexpr (sizeof(Real) == 4) k_fil_energy_bulk<<<n.pgrid[0], kBlock, 0, s>>>(n, -1, kTrialBoth);
             else k_fil_energy<<<n.n_ftiles, kBlock, 0, s>>>(n, -1, 1);
             return 1;
         case 5:   // filament forces alone

@@ -1896,7 +1896,7 @@ static int profile_impl(MechContext* c, int iters, MechProfile* o) {
     if (c->ev_list_count.p) CU(cudaMemsetAsync(c->ev_list_count.p, 0, 4 * sizeof(int), s));
     CU(cudaMemsetAsync(n.ev_fb_count, 0, sizeof(int), s));
     // a line-search trial: positions x + lambda d formed and materialized on the fly
-    o->ms_trial_energy_eval = timeit([&] { launch_energy<Real>(n, -1, sizeof(Real) == 4 ? kTrialDual : 1, c->lanes()); });
+    o->ms_trial_energy_eval = timeit([&] { launch_energy<Real>(n, -1, sizeof(Real) == 4 ? kTrialBoth : 1, c->lanes()); });
     // every replica finished: each launch of an iteration block reads its phase and exits
     const std::vector<CGState> saved(c->h_st, c->h_st + c->R);
     for (int r = 0; r < c->R; ++r) c->h_st[r].phase = PH_DONE;

@@ -36,10 +36,12 @@ constexpr int kFilBulkMaxTiles = 64;   // filament tiles per block of the bulk-s
 constexpr int kExvolFallbackCap = 4096;
 constexpr int kFbChunks = 64;       // work split of one numeric force fallback
 // `trial` argument of the evaluation kernels: 0 plain evaluation at x, 1 one
-// line-search trial at x + lambda d, 2 (mixed engine) two trials in one pass,
-// at x + lambda d and at x + (lambda / 2) d, the next step of the backtracking
-// search, with the second trial's energies in their own partial slots
+// line-search trial at x + lambda d, 2 (mixed engine) the same and, for replicas
+// whose state asks for it (CGState::dual), a second trial in the same pass at
+// x + (lambda / 2) d, the next step of the backtracking search, with its
+// energies in their own partial slots
 constexpr int kTrialDual = 2;
+constexpr int kTrialBoth = 3;   // (profiling) as kTrialDual with a second trial for every replica
 // the ext-pass list marks entries of the second trial with this bit of the pair index
 constexpr int kExtSecond = 1 << 30;
 
@@ -87,6 +89,14 @@ struct CGState {
     int evalFailed;        // an FF reported failure in the last evaluation
     int phase;
     int safeMode;
+    // Searches left whose passes also evaluate lambda / 2 (mixed engine).  A
+    // second trial costs 12 of 41 us of a pass on 1M cylinders and 1 us on
+    // 4,000; a rejected trial without it costs a block of idle launches (20-25
+    // us).  It is wanted in 3% of the searches near the start of a minimization
+    // and in up to half of them later, in runs: a rejected trial brings it for
+    // the rest of that search and the kDualSearches after it.
+    int dual;
+    int searchTrials;      // trials of the current line search
     int xbuf, fbuf;
     int numIter, numEnergyCall, numForceCall, numEnergyEval, numTrials, numSafeMode, numRecover;
     int backupValid, backupPending;
