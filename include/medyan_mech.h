@@ -251,8 +251,7 @@ int32_t mech_get_forces(MechContext* ctx, int32_t replica, double* f_out);
 /*
  * How mech_minimize drives the device.  MECH_GRAPH_UNROLLED (default): a graph
  * of 2, in longer runs 8, unrolled iteration blocks (line search: 2 single-trial passes, FP64,
- * or one two-trial pass, mixed; forces, direction,
- * reset) relaunched by the host, every kernel reading its replica's phase and
+ * or one pass, mixed; forces) relaunched by the host, every kernel reading its replica's phase and
  * exiting when it has nothing to do.  MECH_GRAPH_CONDITIONAL: one CUDA graph
  * whose device while loop runs, per body, only the phases some replica is in
  * (line-search pass, forces, direction, reset to steepest descent); the host is
@@ -269,13 +268,10 @@ int32_t mech_get_forces(MechContext* ctx, int32_t replica, double* f_out);
  * kernels around each single-block reduction are scheduled while their
  * predecessor runs and wait for it on the device (same results) */
 #define MECH_GRAPH_UNROLLED_PDL 2
-/* the unrolled graph with each iteration's tail after the force lanes (force
- * gather, force reduction, direction update, its reduction, reset) run as one
- * cooperative launch whose blocks meet at grid barriers instead of five
- * launches (mixed contexts with one replica; other contexts use
- * MECH_GRAPH_UNROLLED).  Same work units, partial slots and reduction order:
- * bitwise the same results.  A grid barrier that waits too long ends the
- * minimization with MECH_ERR_ITER_LIMIT. */
+/* accepted and run as MECH_GRAPH_UNROLLED: the mode's cooperative tail (gather,
+ * reductions, direction update, reset in one launch) was slower than the
+ * launches it replaced, and the direction update and the reset are part of the
+ * line-search pass now */
 #define MECH_GRAPH_UNROLLED_COOP 3
 int32_t mech_set_graph_mode(MechContext* ctx, int32_t mode);
 

@@ -93,17 +93,18 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
     const int stride = sizeof(Real) == 4 ? n.ptiles[0] : 1;
     const int nslot = run_slots(rt.fil_begin, rt.fil_end, stride);
     const int ffk[K_NUM_SPARSE] = {MECH_FF_LINKER, MECH_FF_MOTOR, MECH_FF_EXVOL, MECH_FF_BOUNDARY};
-    double e[MECH_NUM_FF], e2[MECH_NUM_FF];
+    double e[MECH_NUM_FF], e2[MECH_NUM_FF], slope;
     const bool dual = sizeof(Real) == 4 && second_trial(trial, n.st[r].dual);
+    const bool pend = trial && n.st[r].dPending;   // the pass formed a new direction
     // the fallback list's length, loaded now so that thread 0's step logic does
     // not wait on it at the end
     const int fb_count = threadIdx.x == 0 ? __ldcg(n.ev_fb_count) : 0;
     MECH_TRACE_STAMP(ts_load);
     if constexpr (sizeof(Real) == 4) {
         // mixed: (hi, lo) pair slots summed compensated in single precision;
-        // the doubles are formed in thread 0 only.  acc[0, 6): the (first)
-        // trial, acc[6, 12): the second trial of a two-trial pass.
-        FF acc[2 * MECH_NUM_FF];
+        // the doubles are formed in warp 0 only.  acc[0, 6): the (first) trial,
+        // acc[6, 12): the second trial, acc[12]: d . F of a new direction.
+        FF acc[2 * MECH_NUM_FF + 1];
         // each sparse kind's first slot of this thread, loaded with the first filament slots
         float2 sp0[K_NUM_SPARSE], sp1[K_NUM_SPARSE];
 #pragma unroll
@@ -124,6 +125,7 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
                 add_pair(acc[MECH_NUM_FF + MECH_FF_STRETCHING], load_pair(slot + 2));
                 add_pair(acc[MECH_NUM_FF + MECH_FF_BENDING], load_pair(slot + 3));
             }
+            if (pend) add_pair(acc[2 * MECH_NUM_FF], load_pair(n.part_df + run_slot(rt.fil_begin, stride, k)));
         }
 #pragma unroll
         for (int k = 0; k < K_NUM_SPARSE; ++k) {
@@ -140,12 +142,7 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
         }
         MECH_TRACE_SECTION(n, TK_SEC_FE_LOAD, ts_load);
         MECH_TRACE_STAMP(ts_red);
-        if (dual) {
-            block_reduce_ff<2 * MECH_NUM_FF, 0>(acc, nullptr, reinterpret_cast<float*>(sh));
-        } else {
-            FF (&a6)[MECH_NUM_FF] = *reinterpret_cast<FF(*)[MECH_NUM_FF]>(acc);
-            block_reduce_ff<MECH_NUM_FF, 0>(a6, nullptr, reinterpret_cast<float*>(sh));
-        }
+        block_reduce_ff<2 * MECH_NUM_FF + 1, 0>(acc, nullptr, reinterpret_cast<float*>(sh));
         MECH_TRACE_SECTION(n, TK_SEC_FE_REDUCE, ts_red);
         if (threadIdx.x >= 32) return;
         // hi + lo in double, one pair per lane of warp 0: an FP64 warp
@@ -154,7 +151,7 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
         const int lane = threadIdx.x;
         float ph = 0.f, pl = 0.f;
 #pragma unroll
-        for (int k = 0; k < 2 * MECH_NUM_FF; ++k) {
+        for (int k = 0; k < 2 * MECH_NUM_FF + 1; ++k) {
             const float h = __shfl_sync(0xffffffffu, acc[k].h, 0), l = __shfl_sync(0xffffffffu, acc[k].l, 0);
             if (lane == k) {
                 ph = h;
@@ -167,16 +164,18 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
             e[k] = __shfl_sync(0xffffffffu, v, k);
             e2[k] = __shfl_sync(0xffffffffu, v, MECH_NUM_FF + k);
         }
+        slope = __shfl_sync(0xffffffffu, v, 2 * MECH_NUM_FF);
         if (threadIdx.x != 0) return;
     } else {
         // every thread issues its loads back to back, then sums in a fixed order
-        double acc[MECH_NUM_FF] = {0, 0, 0, 0, 0, 0};
+        double acc[MECH_NUM_FF + 1] = {0, 0, 0, 0, 0, 0, 0};   // last: d . F of a new direction
 #pragma unroll 8
         for (int k = threadIdx.x; k < nslot; k += blockDim.x) {
             const int i = run_slot(rt.fil_begin, stride, k);
             const double2 v = __ldcg(reinterpret_cast<const double2*>(n.part_fil + 4 * (size_t)i));
             acc[MECH_FF_STRETCHING] += v.x;
             acc[MECH_FF_BENDING] += v.y;
+            if (pend) acc[MECH_NUM_FF] += __ldcg(n.part_df + i);
         }
 #pragma unroll
         for (int k = 0; k < K_NUM_SPARSE; ++k) {
@@ -185,16 +184,42 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
                 acc[ffk[k]] += __ldcg(n.part_sp + i);
         }
 #pragma unroll
-        for (int k = 0; k < MECH_NUM_FF; ++k) e[k] = warp_sum(acc[k]);
-        const int ops[MECH_NUM_FF] = {0, 0, 0, 0, 0, 0};
-        block_combine<MECH_NUM_FF>(e, ops, sh);
+        for (int k = 0; k <= MECH_NUM_FF; ++k) acc[k] = warp_sum(acc[k]);
+        const int ops[MECH_NUM_FF + 1] = {0, 0, 0, 0, 0, 0, 0};
+        block_combine<MECH_NUM_FF + 1>(acc, ops, sh);
         if (threadIdx.x != 0) return;
+        for (int k = 0; k < MECH_NUM_FF; ++k) e[k] = acc[k];
+        slope = acc[MECH_NUM_FF];
     }
     MECH_TRACE_STAMP(ts_tail);
     const double lam = S.lambda;   // the (first) trial's step, before the line search moves it
     const int xb = S.xbuf;
     add_fallback_energies(n, r, fb_count, dual, lam, e);
     const double E = record_energies(S, e);
+    if (trial && S.phase == PH_LS_TRIAL && S.dPending) {
+        if (S.backupPending) {
+            S.backupValid = 1;
+            S.backupPending = 0;
+        }
+        S.dPending = 0;
+        if (slope <= 0) {
+            // conjugacy lost (CGMethod.hpp:1553-1560): the search starts over
+            // along F, at the same step; this pass's energies are not used
+            S.dIsF = 1;
+            S.slope = S.FdotF;
+            S.lastFdotF = S.FdotF;
+        } else {
+            S.slope = slope;
+            S.dIsF = 0;
+            S.dbuf ^= 1;
+            if (S.method >= 1) S.lastFdotF = S.newGrad;
+        }
+        S.reducedSlope = (S.safeMode ? 0.0 : kBacktrackSlope) * S.slope;
+        if (S.dIsF) {
+            n.st[r] = S;
+            return;
+        }
+    }
     if (trial && S.phase == PH_LS_TRIAL) {
         S.Etrial = E;
         // the trial positions: the other buffer (FP64), or the next of three (mixed)
@@ -215,6 +240,7 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
     } else {
         S.E0 = E;
     }
+    settle(S);
     n.st[r] = S;
     MECH_TRACE_SECTION(n, TK_SEC_FE_TAIL, ts_tail);
 }
@@ -249,17 +275,17 @@ __device__ __forceinline__ void force_step(CGState& S, double mx, double ff, dou
             S.minimumE = S.totalEnergy;
             S.backupPending = 1;
         }
-        S.phase = PH_DIR;
+        // the new direction F + beta d is formed by the first pass of the search
+        S.dPending = 1;
+        begin_iteration(S);
+        settle(S);
     } else if (ph == PH_RECOVER_FORCE) {
         S.phase = PH_RECOVER_ENERGY;
     }
 }
 
-// `store`: write the state back (k_tail_coop runs this in every block on the
-// block's own copy and stores it from one block).
 template <typename Real>
-__device__ void finalize_force(const DevNet<Real>& n, int r, const RepTiles& rt, CGState& S, double* sh,
-                               bool store = true) {
+__device__ void finalize_force(const DevNet<Real>& n, int r, const RepTiles& rt, CGState& S, double* sh) {
     // k_force_gather writes one slot per tile, k_force_gather_mx one per run of
     // a replica's tiles in a block
     const int stride = sizeof(Real) == 4 ? kGatherTiles : 1;
@@ -311,41 +337,8 @@ __device__ void finalize_force(const DevNet<Real>& n, int r, const RepTiles& rt,
     }
     MECH_TRACE_STAMP(ts_tail);
     force_step(S, mx, ff, ffp);
-    if (store) n.st[r] = S;
+    n.st[r] = S;
     MECH_TRACE_SECTION(n, TK_SEC_FF_TAIL, ts_tail);
-}
-
-// One block per replica after the direction update: the slope d.F, the
-// conjugacy test and the next iteration's start (CGMethod.hpp:1553-1560).
-template <typename Real>
-__device__ void finalize_direction(const DevNet<Real>& n, int r, const RepTiles& rt, CGState& S, double* sh,
-                                   bool store = true) {
-    double slope;
-    if constexpr (sizeof(Real) == 8) {
-        slope = sum_slots(n.part_fil, 4, 3, rt.fil_begin, rt.fil_end, sh);
-    } else {
-        FF a[1];
-        const int nslot = run_slots(rt.fil_begin, rt.fil_end, n.ptiles[2]);
-#pragma unroll 8
-        for (int k = threadIdx.x; k < nslot; k += blockDim.x)
-            add_pair(a[0], load_pair(n.part_fil + 4 * (size_t)run_slot(rt.fil_begin, n.ptiles[2], k) + 3));
-        block_reduce_ff<1, 0>(a, nullptr, reinterpret_cast<float*>(sh));
-        slope = threadIdx.x == 0 ? (double)a[0].h + (double)a[0].l : 0.0;
-    }
-    if (threadIdx.x == 0) {
-        if (S.backupPending) {
-            S.backupValid = 1;
-            S.backupPending = 0;
-        }
-        if (slope <= 0) {          // conjugacy lost: reset to steepest descent
-            S.phase = PH_RESET;
-        } else {
-            S.slope = slope;
-            if (S.method >= 1) S.lastFdotF = S.newGrad;
-            begin_iteration(S);
-        }
-        if (store) n.st[r] = S;
-    }
 }
 
 }  // namespace mech

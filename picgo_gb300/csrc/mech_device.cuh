@@ -142,6 +142,19 @@ __device__ __forceinline__ void dispatch_failed(CGState& S) {
     }
 }
 
+__device__ __forceinline__ void begin_iteration(CGState& S);
+// d = F (resetCGParams, CGMethod.hpp:963-972), as long as the step logic asks
+// for it: a search that cannot begin asks once more, in safe mode.
+__device__ __forceinline__ void settle(CGState& S) {
+    for (int k = 0; k < 2 && S.phase == PH_RESET; ++k) {
+        S.dIsF = 1;
+        S.dPending = 0;
+        S.slope = S.FdotF;
+        S.lastFdotF = S.FdotF;
+        begin_iteration(S);
+    }
+}
+
 // Loop head and the start of backtrackingLineSearch (CGMethod.hpp:238-296, :1279-1320).
 // The energy at the current coordinates is the cached E0: it is the accepted
 // trial's energy, bit for bit, because the trial coordinates x + lambda d are
@@ -252,20 +265,51 @@ __device__ __forceinline__ void store_pos(float* X, int b, const Pos<float>& p) 
     q[2] = make_float2(p.l[1], p.l[2]);
 }
 
+// The search direction as a line-search pass reads it (CGState::dPending): the
+// vector at `d`, or F + beta d (CGMethod.hpp:1553-1556) when `F` is set, rounded
+// alike in every kernel.
+template <typename Real>
+struct Direction {
+    const Real* d;
+    const Real* F;
+    Real* out;      // where the filament kernel stores a new direction
+    Real beta;
+};
+template <typename Real>
+__device__ __forceinline__ Direction<Real> direction_of(const DevNet<Real>& n, const CGState& S) {
+    Direction<Real> D;
+    const int fd = S.dPending ? S.fbuf ^ 1 : S.fbuf;   // the forces that are the direction
+    D.d = S.dIsF ? n.f[fd] : n.d[S.dbuf];
+    D.F = S.dPending ? n.f[S.fbuf] : nullptr;
+    D.out = n.d[S.dbuf ^ 1];
+    D.beta = (Real)S.beta;
+    return D;
+}
+__device__ __forceinline__ float new_direction(float F, float beta, float d) { return fmaf(beta, d, F); }
+__device__ __forceinline__ double new_direction(double F, double beta, double d) { return fma(beta, d, F); }
+template <typename Real>
+__device__ __forceinline__ void direction_at(const Direction<Real>& D, int b, Real v[3]) {
+    const Real* d = D.d + 3 * (size_t)b;
+    v[0] = d[0]; v[1] = d[1]; v[2] = d[2];
+    if (D.F) {
+        const Real* F = D.F + 3 * (size_t)b;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) v[k] = new_direction(F[k], D.beta, v[k]);
+    }
+}
+
 // x + lambda d (CGMethod.cpp:43-46).  Every kernel that needs the trial
 // position uses these, so the materialized trial coordinates and the ones
-// formed on the fly are identical.
-__device__ __forceinline__ Pos<double> moved(const Pos<double>& p, const double* D, int b, double lam) {
+// formed on the fly are identical.  Mixed engine: the step rounded to single
+// precision.
+__device__ __forceinline__ Pos<double> moved(const Pos<double>& p, const double d[3], double lam) {
     Pos<double> o;
-    const double* d = D + 3 * (size_t)b;
 #pragma unroll
     for (int k = 0; k < 3; ++k) o.x[k] = fma(lam, d[k], p.x[k]);
     return o;
 }
-__device__ __forceinline__ Pos<float> moved(const Pos<float>& p, const float* D, int b, double lam) {
+__device__ __forceinline__ Pos<float> moved(const Pos<float>& p, const float d[3], float lf) {
     Pos<float> o;
-    const float* d = D + 3 * (size_t)b;
-    const float lf = (float)lam;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         float s, e, lo;
@@ -276,23 +320,14 @@ __device__ __forceinline__ Pos<float> moved(const Pos<float>& p, const float* D,
     return o;
 }
 
+// bead b at x (trial = false) or x + lambda d
 template <typename Real>
-__device__ __forceinline__ Pos<Real> bead_at(const Real* X, const Real* D, int b, bool trial, double lam) {
+__device__ __forceinline__ Pos<Real> bead_at(const Real* X, const Direction<Real>& D, int b, bool trial, Real lam) {
     const Pos<Real> p = load_pos(X, b);
-    return trial ? moved(p, D, b, lam) : p;
-}
-// single-precision step already rounded by the caller (same result as the double-lambda form)
-__device__ __forceinline__ Pos<float> moved_f(const Pos<float>& p, const float* D, int b, float lf) {
-    Pos<float> o;
-    const float* d = D + 3 * (size_t)b;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        float s, e, lo;
-        two_sum(p.h[k], __fmul_rn(lf, d[k]), s, e);
-        lo = __fadd_rn(p.l[k], e);
-        fast_two_sum(s, lo, o.h[k], o.l[k]);
-    }
-    return o;
+    if (!trial) return p;
+    Real d[3];
+    direction_at(D, b, d);
+    return moved(p, d, lam);
 }
 
 // compensated single-precision accumulator

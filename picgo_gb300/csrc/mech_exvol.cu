@@ -113,11 +113,12 @@ __device__ void fb_energy_blocks(const DevNet<Real>& n, int blk, int nblk, doubl
         // positions of this evaluation: the entry records the trial lambda (0: plain evaluation)
         const double lam = __longlong_as_double(((const long long*)n.ev_fb_energy)[kExvolFallbackCap + k]);
         const bool tr = lam != 0.0;
+        const Direction<Real> dir = direction_of(n, S);
         double c1[3], c2[3], c3[3], c4[3];
-        to_double(bead_at(n.x[S.xbuf], n.d, bs.x, tr, lam), c1);
-        to_double(bead_at(n.x[S.xbuf], n.d, bs.y, tr, lam), c2);
-        to_double(bead_at(n.x[S.xbuf], n.d, bs.z, tr, lam), c3);
-        to_double(bead_at(n.x[S.xbuf], n.d, bs.w, tr, lam), c4);
+        to_double(bead_at(n.x[S.xbuf], dir, bs.x, tr, (Real)lam), c1);
+        to_double(bead_at(n.x[S.xbuf], dir, bs.y, tr, (Real)lam), c2);
+        to_double(bead_at(n.x[S.xbuf], dir, bs.z, tr, (Real)lam), c3);
+        to_double(bead_at(n.x[S.xbuf], dir, bs.w, tr, (Real)lam), c4);
         const Quad q = quad_of(c1, c2, c3, c4);
         const int N = kFbNodesEnergy;
         double acc = 0.0;
@@ -346,15 +347,15 @@ __device__ __forceinline__ void split_invariants(const SplitShared& s, int l, Sp
 
 // 32 pairs [i0, min(i0 + 32, end)) of replica r in a block of four warps.
 template <typename Real>
-__device__ void exvol_split(const DevNet<Real>& n, int r, const Real* X, bool tr, double lam, int force, int i0, int end,
-                            SplitShared& s) {
+__device__ void exvol_split(const DevNet<Real>& n, int r, const Real* X, const Direction<Real>& dir, bool tr, double lam,
+                            int force, int i0, int end, SplitShared& s) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, i = i0 + l;
     const bool valid = i < end;
     if (valid) {
         const int4 bs = n.ev_bead[i];
         const int bead = w == 0 ? bs.x : w == 1 ? bs.y : w == 2 ? bs.z : bs.w;
         double c[3];
-        to_double(bead_at(X, n.d, bead, tr, lam), c);
+        to_double(bead_at(X, dir, bead, tr, (Real)lam), c);
 #pragma unroll
         for (int k = 0; k < 3; ++k) s.c[w][k][l] = c[k];
     }
@@ -502,6 +503,7 @@ __global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, in
     MECH_TRACE_KERNEL(n, TK_EXVOL);
     __shared__ int s_go, s_xb;
     __shared__ double s_lam;
+    __shared__ Direction<Real> s_dir;
     __shared__ SplitShared s;
     const int sb = (int)blockIdx.x - 2 * unsplit;
     const Tile t = n.stile[tile_off + (sb < 0 ? (int)blockIdx.x >> 1 : unsplit + (sb >> 3))];
@@ -512,13 +514,14 @@ __global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, in
         s_go = want < 0 ? (S.active != 0) : (S.phase == want);
         s_xb = S.xbuf;
         s_lam = S.lambda;
+        s_dir = direction_of(n, S);
     }
     __syncthreads();
     if (!s_go) return;
     const Real* X = n.x[s_xb];
     const bool tr = trial != 0;
     if (sb >= 0) {
-        exvol_split(n, t.replica, X, tr, s_lam, force, begin, t.end, s);
+        exvol_split(n, t.replica, X, s_dir, tr, s_lam, force, begin, t.end, s);
         return;
     }
     const int i = begin + threadIdx.x;
@@ -526,10 +529,10 @@ __global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, in
     const int4 bs = n.ev_bead[i];
     const double kRep = (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i];
     double c1[3], c2[3], c3[3], c4[3];
-    to_double(bead_at(X, n.d, bs.x, tr, s_lam), c1);
-    to_double(bead_at(X, n.d, bs.y, tr, s_lam), c2);
-    to_double(bead_at(X, n.d, bs.z, tr, s_lam), c3);
-    to_double(bead_at(X, n.d, bs.w, tr, s_lam), c4);
+    to_double(bead_at(X, s_dir, bs.x, tr, (Real)s_lam), c1);
+    to_double(bead_at(X, s_dir, bs.y, tr, (Real)s_lam), c2);
+    to_double(bead_at(X, s_dir, bs.z, tr, (Real)s_lam), c3);
+    to_double(bead_at(X, s_dir, bs.w, tr, (Real)s_lam), c4);
     if (!force) {
         const double u = pair_energy_d(c1, c2, c3, c4, kRep);
         n.ev_energy[i] = u == u ? u : 0.0;
@@ -549,7 +552,8 @@ template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int trial, int force, int tile_off) {
     MECH_TRACE_KERNEL(n, TK_EXVOL);
     __shared__ int s_go, s_xb, s_dual;
-    __shared__ float s_lf;   // the step rounded once (mixed engine)
+    __shared__ float s_lf;   // the step rounded once
+    __shared__ Direction<Real> s_dir;
     const int ti = tile_off + blockIdx.x;
     const Tile t = n.stile[ti];
     const int r = t.replica;
@@ -558,6 +562,7 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
         s_go = want < 0 ? (S.active != 0) : (S.phase == want);
         s_xb = S.xbuf;
         s_lf = (float)S.lambda;
+        s_dir = direction_of(n, S);
         s_dual = S.dual;
     }
     __syncthreads();
@@ -572,10 +577,7 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
     const bool dual = !force && second_trial(trial, s_dual);
     if (valid) {
         const int4 bs = n.ev_bead[i];
-        auto pos = [&](int b) -> Pos<float> {
-            const Pos<float> p = load_pos(X, b);
-            return tr ? moved_f(p, n.d, b, s_lf) : p;
-        };
+        auto pos = [&](int b) -> Pos<float> { return bead_at(X, s_dir, b, tr, s_lf); };
         const Pos<Real> p1 = pos(bs.x), p2 = pos(bs.y), p3 = pos(bs.z), p4 = pos(bs.w);
         if (!force) {
             // mixed engine: single precision unless the pair is ill-conditioned
@@ -584,10 +586,9 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
             store_pair(n.ev_energy + i, ef, 0.f);
             if (dual) {
                 const float lh = 0.5f * s_lf;
-                const float ef2 = mixed_pair_energy(moved_f(load_pos(X, bs.x), n.d, bs.x, lh),
-                                                    moved_f(load_pos(X, bs.y), n.d, bs.y, lh),
-                                                    moved_f(load_pos(X, bs.z), n.d, bs.z, lh),
-                                                    moved_f(load_pos(X, bs.w), n.d, bs.w, lh), kRep, need64b);
+                const float ef2 = mixed_pair_energy(bead_at(X, s_dir, bs.x, true, lh), bead_at(X, s_dir, bs.y, true, lh),
+                                                    bead_at(X, s_dir, bs.z, true, lh), bead_at(X, s_dir, bs.w, true, lh),
+                                                    kRep, need64b);
                 store_pair(n.ev_energy2 + i, ef2, 0.f);
             }
         } else {
@@ -698,7 +699,7 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
             const int4 bs = n.ev_bead[i];
             const int bead = w == 0 ? bs.x : w == 1 ? bs.y : w == 2 ? bs.z : bs.w;
             double c[3];
-            to_double(bead_at(n.x[S.xbuf], n.d, bead, trial != 0, lam), c);
+            to_double(bead_at(n.x[S.xbuf], direction_of(n, S), bead, trial != 0, (Real)lam), c);
             s_c[w][l][0] = c[0];
             s_c[w][l][1] = c[1];
             s_c[w][l][2] = c[2];

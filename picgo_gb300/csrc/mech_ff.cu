@@ -26,13 +26,21 @@ namespace mech {
 // ---------------------------------------------------------------------------
 // helpers
 // ---------------------------------------------------------------------------
-// the three products of one bead, in the engine's precision; the sum over
-// beads is carried by block_sum_r (compensated within a warp, then double)
+// The three products of one bead, in the engine's precision.  The fused forms
+// are written out so that a product rounds alike in whatever kernel it is
+// formed: beta, and with it the trajectory, hangs on the last bits of F.F and
+// F.Fprev (which round their first two products in different orders).
 __device__ __forceinline__ double bead_dot(double a0, double a1, double a2, double b0, double b1, double b2) {
-    return a0 * b0 + a1 * b1 + a2 * b2;
+    return fma(a2, b2, fma(a1, b1, a0 * b0));
 }
 __device__ __forceinline__ float bead_dot(float a0, float a1, float a2, float b0, float b1, float b2) {
     return fmaf(a2, b2, fmaf(a1, b1, a0 * b0));
+}
+__device__ __forceinline__ double bead_dot_prev(const double F[3], double p0, double p1, double p2) {
+    return fma(F[2], p2, fma(F[0], p0, F[1] * p1));
+}
+__device__ __forceinline__ float bead_dot_prev(const float F[3], float p0, float p1, float p2) {
+    return bead_dot(F[0], F[1], F[2], p0, p1, p2);
 }
 
 // plane distance of a position (BoundaryElementImpl.h:49-53)
@@ -70,7 +78,7 @@ __device__ __forceinline__ void bond_vector(const Pos<float>& c1, const Pos<floa
 // ---------------------------------------------------------------------------
 // Conditions of the minimizer's conditional graph (GraphConds).
 // ---------------------------------------------------------------------------
-constexpr int kCondTrial = 2, kCondForce = 3, kCondDir = 4, kCondMisc = 5;   // counter slots
+constexpr int kCondTrial = 2, kCondForce = 3;   // counter slots
 
 // Which phases the replicas are in, read past L1 (other blocks wrote the
 // states); every thread of one block calls it, thread 0 sets the handles.
@@ -78,41 +86,27 @@ constexpr int kCondTrial = 2, kCondForce = 3, kCondDir = 4, kCondMisc = 5;   // 
 // decides whether the loop runs another one after this body.
 template <typename Real>
 __device__ void set_conditions(const DevNet<Real>& n, bool head, int phase_slot) {
-    int tr = 0, fo = 0, di = 0, mi = 0, host = 0;
+    int tr = 0, fo = 0, host = 0;
     for (int r = threadIdx.x; r < n.R; r += blockDim.x) {
         const int ph = __ldcg(&n.st[r].phase);
         tr |= ph == PH_LS_TRIAL;
         fo |= ph == PH_FORCE;
-        di |= ph == PH_DIR;
-        mi |= ph == PH_RESET || ph == PH_FAILED;
         host |= ph >= PH_RECOVER;   // the recovery move is sequenced by the host
     }
     tr = __syncthreads_or(tr);
     fo = __syncthreads_or(fo);
-    di = __syncthreads_or(di);
-    mi = __syncthreads_or(mi);
     host = __syncthreads_or(host);
     if (threadIdx.x != 0) return;
     cudaGraphSetConditional(n.cond.trial, tr ? 1u : 0u);
     cudaGraphSetConditional(n.cond.force, fo ? 1u : 0u);
-    cudaGraphSetConditional(n.cond.dir, di ? 1u : 0u);
-    cudaGraphSetConditional(n.cond.misc, mi ? 1u : 0u);
     if (phase_slot >= 0) n.cond.counter[phase_slot]++;
     if (head) {
         // the loop ends after this body when nothing is left to do on the
         // device, an error is latched or the body budget of the launch is spent
         const int bodies = ++n.cond.counter[0];
-        const bool more = (tr | fo | di | mi) && !host && __ldcg(n.err) == 0 && bodies < n.cond.cap;
+        const bool more = (tr | fo) && !host && __ldcg(n.err) == 0 && bodies < n.cond.cap;
         cudaGraphSetConditional(n.cond.loop, more ? 1u : 0u);
     }
-}
-
-// After a phase's per-replica reduction (one block per replica): the last
-// block to finish sets the conditions of the phases that follow in the body.
-template <typename Real>
-__device__ void after_phase(const DevNet<Real>& n, int phase_slot, int* s_flag) {
-    if (!n.cond.on) return;
-    if (last_tile(n.cond.counter + 1, 0, gridDim.x, s_flag)) set_conditions(n, false, phase_slot);
 }
 
 // After an evaluation's per-replica reduction: the last block zeroes the
@@ -128,6 +122,9 @@ __device__ void after_evaluation(const DevNet<Real>& n, int phase_slot, int* s_f
     }
     if (n.cond.on) set_conditions(n, false, phase_slot);
 }
+
+// The head of an unrolled graph (launch_graph_head).
+__global__ void k_graph_head() {}
 
 // The kernel at the head of every body of the minimizer's while loop.
 template <typename Real>
@@ -147,9 +144,9 @@ __global__ void __launch_bounds__(kBlock) k_body_head(DevNet<Real> n) {
 // Sums of N values (a power of two) over each warp and then the block: the
 // first steps of the trees halve the number of values a lane carries, so N
 // trees take N + 3 additions (N = 4: 6) where one after another they take 5 N.
-// Thread t < N gets value t.  A value's tree has the same shape whatever its
-// place among the N, so a tile's sums do not depend on the tiles it shares a
-// block with.  `sh` holds N * kBlock / 32 doubles.
+// Thread t < N gets value t.  A value's tree has the shape of block_sum's
+// whatever its place among the N: same bits, and a tile's sums do not depend on
+// the tiles it shares a block with.  `sh` holds N * kBlock / 32 doubles.
 template <int N>
 __device__ __forceinline__ double block_sums(double (&v)[N], double* sh) {
     const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -169,13 +166,16 @@ __device__ __forceinline__ double block_sums(double (&v)[N], double* sh) {
     __syncthreads();
     if ((l & (32 / N - 1)) == 0) sh[w * N + idx] = v[0];
     __syncthreads();
-    double a = 0.0;
+    double a[kBlock / 32] = {};
     if (threadIdx.x < N) {
-        a = sh[threadIdx.x];
 #pragma unroll
-        for (int k = 1; k < kBlock / 32; ++k) a += sh[k * N + threadIdx.x];
+        for (int k = 0; k < kBlock / 32; ++k) a[k] = sh[k * N + threadIdx.x];
+#pragma unroll
+        for (int h = kBlock / 64; h >= 1; h >>= 1)
+#pragma unroll
+            for (int k = 0; k < h; ++k) a[k] += a[k + h];
     }
-    return a;
+    return a[0];
 }
 // the same for maxima of N unsigned values
 template <int N>
@@ -219,14 +219,16 @@ __device__ __forceinline__ double clamp_unit(double x) {
 
 // What a block of the FP64 filament kernels needs of its tile's replica.
 struct FilTile {
-    int begin, end, go, xb, fb;
+    int begin, end, go, xb, fb, backup;
     double lam;
+    Direction<double> dir;
 };
 __device__ __forceinline__ void load_fil_tile(const DevNet<double>& n, int want, FilTile* s) {
     if (threadIdx.x == 0) {
         const Tile t = n.ftile[blockIdx.x];
         const CGState& S = n.st[t.replica];
-        *s = FilTile{t.begin, t.end, replica_selected(S, want), S.xbuf, S.fbuf, S.lambda};
+        *s = FilTile{t.begin, t.end, replica_selected(S, want), S.xbuf, S.fbuf, S.backupPending, S.lambda,
+                     direction_of(n, S)};
     }
     __syncthreads();
 }
@@ -239,27 +241,45 @@ __global__ void __launch_bounds__(kBlock) k_fil_energy(DevNet<double> n, int wan
     MECH_TRACE_KERNEL(n, TK_FIL_ENERGY);
     __shared__ double xs[3][kFilTile + 2];    // beads begin - 1 .. end
     __shared__ double rs[4][kFilTile + 1];    // cylinders begin - 1 .. end - 1: vector, length
-    __shared__ double sh[2 * kBlock / 32];
+    __shared__ double dF[kFilTile];           // d . F of each bead (a new direction)
+    __shared__ double sh[4 * kBlock / 32];
     __shared__ FilTile t;
     const bool tr = trial != 0;
     load_fil_tile(n, want, &t);
     if (!t.go) return;
     const int T = t.end - t.begin;
     const double* X = n.x[t.xb];
+    const bool pend = tr && t.dir.F;     // this pass forms the direction
+    double e[4] = {0.0, 0.0, 0.0, 0.0};   // stretching, bending, d . F
     for (int i = threadIdx.x; i < T + 2; i += blockDim.x) {
         const int b = t.begin - 1 + i;
         if (b < 0 || b >= n.nb) continue;
-        const Pos<double> p = bead_at(X, n.d, b, tr, t.lam);
+        Pos<double> p = load_pos(X, b);
+        if (tr) {
+            const bool own = i >= 1 && i <= T;
+            double d[3];
+            direction_at(t.dir, b, d);
+            if (pend && own) {
+                double* o = t.dir.out + 3 * (size_t)b;
+                const double* F = t.dir.F + 3 * (size_t)b;
+                o[0] = d[0];
+                o[1] = d[1];
+                o[2] = d[2];
+                dF[i - 1] = bead_dot(d[0], d[1], d[2], F[0], F[1], F[2]);
+                if (t.backup) store_pos(n.xbest, b, p);
+            }
+            p = moved(p, d, t.lam);
+            if (own) store_pos(n.x[t.xb ^ 1], b, p);   // materialize the owned trial position
+        }
         xs[0][i] = p.x[0];
         xs[1][i] = p.x[1];
         xs[2][i] = p.x[2];
-        if (tr && i >= 1 && i <= T) store_pos(n.x[t.xb ^ 1], b, p);   // materialize the owned trial position
     }
     __syncthreads();
     const int i = threadIdx.x, j = t.begin + i;
     const int fl = i < T ? n.bflag[j] : 0;
+    if (pend && i < T) e[2] = dF[i];
     double r2[3] = {0, 0, 0}, L2 = 0.0, ks = 0.0, l0 = 0.0, kb = 0.0, th = 0.0;
-    double e[2] = {0.0, 0.0};   // stretching, bending
     if (fl & 1) {
         load_par(n.bpar, j, ks, l0, kb, th);
 #pragma unroll
@@ -292,27 +312,25 @@ __global__ void __launch_bounds__(kBlock) k_fil_energy(DevNet<double> n, int wan
         n.terms[j] = e[0];
         n.terms[(size_t)n.nb + j] = e[1];
     }
-    const double a = block_sums<2>(e, sh);
+    const double a = block_sums<4>(e, sh);
     if (threadIdx.x < 2) n.part_fil[4 * (size_t)blockIdx.x + threadIdx.x] = a;
+    if (threadIdx.x == 2) n.part_df[blockIdx.x] = a;
 }
 
 // Filament forces of the tile's own beads (the sparse force fields' shares are
-// added by k_force_gather once they are written).  With r_c the vector and L_c
-// the length of cylinder (c, c+1), the derivative of the energy by r_c is
-//   G_c = (f0_c + C_c + B_{c+1}) r_c - A_c r_{c-1} - A_{c+1} r_{c+1},
-// f0 = k (L - l0) / L, and for the triple on bead c, with x its cosine and k
-// its (theta0-dependent) constant, A = k / (L_{c-1} L_c), B = k x / L_{c-1}^2,
-// C = k x / L_c^2 (FilamentBendingCosine.cpp:285-345); the force on bead b is
-// G_b - G_{b-1}.  1M beads: 109 us, against 233 us (121 FP64 instructions per
-// bead) with three divisions and two roots per triple and the six bead shares
-// summed one by one.
+// added by k_force_gather once they are written), each cylinder's and triple's
+// terms formed once, and each bead's sum in the reference's order (stretching
+// of its two cylinders, bending of the three triples it is in): the FP64
+// engine's minimizations amplify a changed rounding by up to ~1e8 over a hundred
+// iterations, so the forces keep every operation.  A triple reads its
+// cylinders' vectors and squared lengths instead of forming them again.
 __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want) {
     pdl_wait();      // the previous kernel of the main lane has finished
     MECH_TRACE_KERNEL(n, TK_FIL_FORCE);
-    __shared__ double xs[3][kFilTile + 4];                       // beads begin - 2 .. end + 1; then G of begin - 1 .. end - 1
-    __shared__ double rs[3][kFilTile + 3], iL[kFilTile + 3], f0[kFilTile + 3];   // cylinders begin - 2 .. end
-    __shared__ double cA[kFilTile + 2], cB[kFilTile + 2], cC[kFilTile + 2];      // triples on begin - 1 .. end
-    __shared__ bool tri[kFilTile + 2];   // such a triple exists (where not, the next filament is not to be read: it may be non-finite)
+    __shared__ double xs[3][kFilTile + 4];                          // beads begin - 2 .. end + 1
+    __shared__ double rs[3][kFilTile + 3], Ls[kFilTile + 3];        // cylinders begin - 2 .. end: vector, L^2
+    __shared__ double fs[3][kFilTile + 3];                          // their stretching forces on the second bead
+    __shared__ double f1[3][kFilTile + 2], f2[3][kFilTile + 2];     // triples on begin - 1 .. end
     __shared__ FilTile t;
     load_fil_tile(n, want, &t);
     if (!t.go) return;
@@ -329,64 +347,66 @@ __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want
     __syncthreads();
     for (int i = threadIdx.x; i < T + 3; i += blockDim.x) {
         const int c = t.begin - 2 + i;
-        double r[3] = {0, 0, 0}, inv = 0.0, f = 0.0;
+        double F[3] = {0, 0, 0};
         if (c >= 0 && c < n.nb && (n.bflag[c] & 1)) {
             const double2 kl = reinterpret_cast<const double2*>(n.bpar)[2 * (size_t)c];
+            double r[3];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) r[q] = xs[q][i + 1] - xs[q][i];
-            const double L = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-            inv = 1.0 / L;
-            f = kl.x * (L - kl.y) * inv;
+            for (int q = 0; q < 3; ++q) rs[q][i] = r[q] = xs[q][i + 1] - xs[q][i];
+            const double L2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+            Ls[i] = L2;
+            const double L = sqrt(L2), invL = 1.0 / L, f0 = kl.x * (L - kl.y) * invL;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) F[q] = -f0 * r[q];
         }
 #pragma unroll
-        for (int q = 0; q < 3; ++q) rs[q][i] = r[q];
-        iL[i] = inv;
-        f0[i] = f;
+        for (int q = 0; q < 3; ++q) fs[q][i] = F[q];
     }
     __syncthreads();
     for (int i = threadIdx.x; i < T + 2; i += blockDim.x) {
         const int c = t.begin - 1 + i;   // cylinders c - 1, c at i, i + 1
-        double a = 0.0, bb = 0.0, cc = 0.0;
-        const bool has = c >= 0 && c < n.nb && (n.bflag[c] & 3) == 3;
-        if (has) {
+        double a[3] = {0, 0, 0}, b[3] = {0, 0, 0};
+        if (c >= 0 && c < n.nb && (n.bflag[c] & 3) == 3) {
             const double2 kt = reinterpret_cast<const double2*>(n.bpar)[2 * (size_t)c + 1];
-            const double A = iL[i] * iL[i + 1];
-            double x = (rs[0][i] * rs[0][i + 1] + rs[1][i] * rs[1][i + 1] + rs[2][i] * rs[2][i + 1]) * A;
-            const double x0 = x;
+            const double r1[3] = {rs[0][i], rs[1][i], rs[2][i]}, r2[3] = {rs[0][i + 1], rs[1][i + 1], rs[2][i + 1]};
+            const double L1 = Ls[i], L2 = Ls[i + 1];
+            const double l1l2 = r1[0] * r2[0] + r1[1] * r2[1] + r1[2] * r2[2];
+            const double A = 1.0 / sqrt(L1 * L2);
+            double x = l1l2 * A;
+            const double B = x / L1, C = x / L2;
             double kk = kt.x;
             if (!theta_is_zero(kt.y)) {
                 if (fabs(fabs(x) - 1.0) < 0.001) x = 0.999 * x;
                 x = clamp_unit(x);
                 const double sinp = sqrt(fmax(1.0 - x * x, 0.0));
-                kk = kk * (sinp * cos(kt.y) - x * sin(kt.y)) / sinp;
+                const double sinpmq = sinp * cos(kt.y) - x * sin(kt.y);
+                kk = kt.x * sinpmq / sinp;
             }
-            a = kk * A;
-            const double kx = kk * x0;
-            bb = kx * iL[i] * iL[i];
-            cc = kx * iL[i + 1] * iL[i + 1];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                a[q] = kk * (r2[q] * A - r1[q] * B);
+                b[q] = kk * (r1[q] * A - r2[q] * C);
+            }
         }
-        cA[i] = a;
-        cB[i] = bb;
-        cC[i] = cc;
-        tri[i] = has;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < T + 1; i += blockDim.x) {   // cylinder begin - 1 + i, at i + 1
-        const double w = f0[i + 1] + cC[i] + cB[i + 1], a0 = cA[i], a1 = cA[i + 1];
-        const bool before = tri[i], after = tri[i + 1];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            double g = w * rs[q][i + 1];
-            if (before) g -= a0 * rs[q][i];
-            if (after) g -= a1 * rs[q][i + 2];
-            xs[q][i] = g;
+            f1[q][i] = a[q];
+            f2[q][i] = b[q];
         }
     }
     __syncthreads();
-    if (threadIdx.x < T) {
-        double* Fo = n.f[t.fb ^ 1] + 3 * (size_t)(t.begin + threadIdx.x);
+    const int i = threadIdx.x;
+    if (i < T) {
+        double* Fo = n.f[t.fb ^ 1] + 3 * (size_t)(t.begin + i);
 #pragma unroll
-        for (int q = 0; q < 3; ++q) Fo[q] = xs[q][threadIdx.x + 1] - xs[q][threadIdx.x];
+        for (int q = 0; q < 3; ++q) {
+            double v = fs[q][i + 1];
+            v += -fs[q][i + 2];
+            v += f2[q][i];
+            v += f1[q][i + 1] - f2[q][i + 1];
+            v += -f1[q][i + 2];
+            Fo[q] = v;
+        }
     }
 }
 
@@ -419,7 +439,7 @@ __device__ __forceinline__ void gather_force(const DevNet<Real>& n, int b, int f
     Fo[1] = F[1];
     Fo[2] = F[2];
     ff = bead_dot(F[0], F[1], F[2], F[0], F[1], F[2]);
-    ffp = bead_dot(F[0], F[1], F[2], p0, p1, p2);
+    ffp = bead_dot_prev(F, p0, p1, p2);
 }
 // a non-finite component makes the bead's max infinite (fmax would drop a NaN)
 __device__ __forceinline__ void gather_bead(const DevNet<float>& n, int b, int fb, float& mx, float& ff, float& ffp) {
@@ -505,7 +525,7 @@ struct GatherMxShared {
 };
 
 // One gather unit (kGatherTiles consecutive tiles): the body of a
-// k_force_gather_mx block, also run unit after unit by k_tail_coop.
+// k_force_gather_mx block.
 __device__ void gather_mx_unit(const DevNet<float>& n, int want, int unit, GatherMxShared& g) {
     static_assert(kFilTile == 256 && kBlock == 64 * kGatherTiles, "64 threads x 4 beads per tile");
     float (&sh)[8][5] = g.sh;
@@ -633,6 +653,13 @@ __global__ void __launch_bounds__(kBlock) k_finalize_force(DevNet<Real> n, int w
     if (threadIdx.x == 0) S = n.st[r];   // issued together with the loads below
     const RepTiles rt = n.rt[r];
     if (replica_selected(n.st[r], want)) finalize_force(n, r, rt, S, sh);
+    if (n.snap && threadIdx.x == 0) {   // what the host looks at after each graph
+        if (S.phase == PH_DONE || S.phase >= PH_ERROR) n.snap[9 + r] = S.phase;
+        if (r == 0) {
+            const unsigned err = __ldcg(n.err);
+            if (err) n.snap[0] = (int)err;
+        }
+    }
     after_evaluation(n, kCondForce, &s_flag);
 }
 
@@ -642,7 +669,7 @@ template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_finalize_energy(DevNet<Real> n, int want, int trial) {
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_FIN_ENERGY);
-    __shared__ double sh[32 * 2 * MECH_NUM_FF];   // block_reduce_ff<12> of a two-trial pass: 32 * 24 floats
+    __shared__ double sh[32 * (2 * MECH_NUM_FF + 1)];   // block_reduce_ff<13>: 32 * 26 floats
     __shared__ int s_flag;
     const int r = blockIdx.x;
     CGState S;
@@ -664,20 +691,16 @@ __global__ void __launch_bounds__(kBlock) k_finalize_energy(DevNet<Real> n, int 
 
 // Store a run's compensated partial sums as (hi, lo) pairs in the slot of its
 // first tile; the reduction kernel that follows the evaluation reads them.
+// a: stretching, bending, d . F and, with a second trial, its stretching and bending.
 template <int N>
 __device__ __forceinline__ void write_run(const DevNet<float>& n, int first, FF (&a)[N], double* sh) {
     block_reduce_ff<N, 0>(a, nullptr, reinterpret_cast<float*>(sh));
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int k = 0; k < N; ++k) store_pair(n.part_fil + 4 * (size_t)first + k, a[k].h, a[k].l);
+        for (int k = 0; k < N; ++k)
+            store_pair(k == 2 ? n.part_df + first : n.part_fil + 4 * (size_t)first + (k < 2 ? k : k - 1), a[k].h, a[k].l);
     }
 }
-
-__device__ __forceinline__ Pos<float> pos_at(const DevNet<float>& n, const float* X, int b, bool tr, float lf) {
-    const Pos<float> p = load_pos(X, b);
-    return tr ? moved_f(p, n.d, b, lf) : p;
-}
-
 
 // ---------------------------------------------------------------------------
 // Mixed engine, bulk-staged filament energy: a persistent walk over runs of
@@ -724,20 +747,28 @@ __device__ __forceinline__ StageRange stage_range(int tb, int te, int nb, int ha
 // so the producing thread issues copies without chasing global pointers:
 // (begin, end, replica, bits) with bit 0 = selected by this launch, bits 1-2 =
 // xbuf, bit 3 = fbuf of the tile's replica, bit 4 = its pass has a second trial,
-// plus that replica's lambda.  A
+// bit 5 = dPending, 6 = dIsF, 7 = dbuf, 8 = backupPending, plus that replica's
+// lambda and beta.  A
 // replica's state cannot change while this block still holds unprocessed
 // tiles of it (its finalizer waits for every tile), so the copies stay valid.
 constexpr int kBulkMaxTiles = kFilBulkMaxTiles;
 
 __device__ __forceinline__ void load_descriptors(const DevNet<float>& n, int t0, int nt, int want, int4* desc,
-                                                 float* lf) {
+                                                 float2* step) {
     for (int k = threadIdx.x; k < nt; k += blockDim.x) {
         const Tile t = n.ftile[t0 + k];
         const CGState& S = n.st[t.replica];
         desc[k] = make_int4(t.begin, t.end, t.replica,
-                            (replica_selected(S, want) ? 1 : 0) | (S.xbuf << 1) | (S.fbuf << 3) | (S.dual ? 16 : 0));
-        lf[k] = (float)S.lambda;
+                            (replica_selected(S, want) ? 1 : 0) | (S.xbuf << 1) | (S.fbuf << 3) | (S.dual ? 16 : 0) |
+                                (S.dPending << 5) | (S.dIsF << 6) | (S.dbuf << 7) | (S.backupPending << 8));
+        step[k] = make_float2((float)S.lambda, (float)S.beta);
     }
+}
+
+// The direction that a tile's pass starts from (direction_of on descriptor bits).
+__device__ __forceinline__ const float* staged_direction(const DevNet<float>& n, int bits) {
+    const int fb = (bits >> 3) & 1;
+    return bits & 64 ? n.f[bits & 32 ? fb ^ 1 : fb] : n.d[(bits >> 7) & 1];
 }
 
 // Issue the copies of a tile into stage `st` (thread 0).  A range that fails
@@ -746,7 +777,8 @@ __device__ __forceinline__ void load_descriptors(const DevNet<float>& n, int t0,
 __device__ void issue_energy_stage(const DevNet<float>& n, int4 t, bool tr, EnergyStage* st, uint64_t* bar) {
     const float* X = n.x[(t.w >> 1) & 3];
     const StageRange rg = stage_range(t.x, t.y, n.nb, 1);
-    const void* src[4] = {X + 6 * (size_t)rg.xs, n.bpar + 4 * (size_t)t.x, n.d + 3 * (size_t)rg.ds, n.bflag + rg.fs};
+    const void* src[4] = {X + 6 * (size_t)rg.xs, n.bpar + 4 * (size_t)t.x, staged_direction(n, t.w) + 3 * (size_t)rg.ds,
+                          n.bflag + rg.fs};
     void* dst[4] = {st->x, st->par, st->d, st->flag};
     const unsigned bytes[4] = {24u * (unsigned)(rg.xe - rg.xs), 16u * (unsigned)(t.y - t.x),
                                tr ? 12u * (unsigned)(rg.de - rg.ds) : 0u, (unsigned)(rg.fe - rg.fs)};
@@ -791,8 +823,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
     __shared__ EnergyStage stage[kBulkStages];
     __shared__ __align__(8) uint64_t bar[kBulkStages];
     __shared__ int4 s_desc[kBulkMaxTiles];
-    __shared__ float s_lf[kBulkMaxTiles];
-    __shared__ double sh[32 * 4];   // write_run<4>: 32 * 8 floats
+    __shared__ float2 s_step[kBulkMaxTiles];
+    __shared__ double sh[32 * 5];   // block_reduce_ff<5>: 32 * 10 floats
     __shared__ __align__(16) float s_mv[6 * kBulkXBeads];   // the staged beads moved to a trial
     __shared__ int s_abort;
     const int t0 = blockIdx.x * n.ptiles[0], t1 = min(t0 + n.ptiles[0], n.n_ftiles);
@@ -808,7 +840,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
         if (threadIdx.x == 0) atomicOr(n.err, 16u);
         return;
     }
-    load_descriptors(n, t0, nt, want, s_desc, s_lf);
+    load_descriptors(n, t0, nt, want, s_desc, s_step);
     __syncthreads();
     // producer state (thread 0): next tile to consider, copies issued
     int pi = 0, issued = 0;
@@ -825,15 +857,16 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
     bool dual = false;
     int cur = -1, first = 0, cnt = 0, xb = 0, j = 0;
     bool go = false;
-    float lf = 0.f;
-    FF es, eb, es2, eb2;
+    bool pend = false;   // the pass forms the direction F + beta d
+    float lf = 0.f, beta = 0.f;
+    FF es, eb, es2, eb2, df;
     auto flush = [&]() {
         if (dual) {
-            FF a[4] = {es, eb, es2, eb2};
-            write_run<4>(n, first, a, sh);
+            FF a[5] = {es, eb, df, es2, eb2};
+            write_run(n, first, a, sh);
         } else {
-            FF a[2] = {es, eb};
-            write_run<2>(n, first, a, sh);
+            FF a[3] = {es, eb, df};
+            write_run(n, first, a, sh);
         }
     };
     for (int k = 0; k < nt; ++k) {
@@ -847,22 +880,35 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
             eb = FF();
             es2 = FF();
             eb2 = FF();
+            df = FF();
             go = t.w & 1;
             xb = (t.w >> 1) & 3;
             dual = second_trial(trial, t.w & 16);
-            lf = s_lf[k];
+            pend = tr && (t.w & 32);
+            lf = s_step[k].x;
+            beta = s_step[k].y;
         }
         if (!go) continue;
         ++cnt;
         const int sidx = j % kBulkStages;
+        const int b = t.x + threadIdx.x;
+        const StageRange rg = stage_range(t.x, t.y, n.nb, 1);
+        const bool own = b < t.y;
+        // the forces of a new direction are read directly (a fourth staged
+        // array would cost a resident block), ahead of the wait for the stage
+        const float* Fn = n.f[(t.w >> 3) & 1];
+        float Fq[3] = {0.f, 0.f, 0.f};
+        if (pend && rg.xs + (int)threadIdx.x < min(rg.xe, n.nb)) {
+            const float* F = Fn + 3 * (size_t)(rg.xs + threadIdx.x);
+            Fq[0] = F[0];
+            Fq[1] = F[1];
+            Fq[2] = F[2];
+        }
         if (!mbar_wait_bounded(&bar[sidx], (unsigned)((j / kBulkStages) & 1), kBulkWaitLimit)) {
             atomicOr(n.err, 32u);
             s_abort = 1;
         }
         const EnergyStage& S = stage[sidx];
-        const int b = t.x + threadIdx.x;
-        const StageRange rg = stage_range(t.x, t.y, n.nb, 1);
-        const bool own = b < t.y;
         int fl = 0;
         float4 pr = make_float4(0.f, 0.f, 0.f, 0.f);
         if (own) {
@@ -879,8 +925,31 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
             const float* P = S.x;
             if (tr) {
                 const float lch = ch ? 0.5f * lf : lf;
-                for (int q = threadIdx.x; q < rg.xe - rg.xs; q += blockDim.x)
-                    store_pos(s_mv, q, moved_f(load_pos(S.x, q), S.d, q + rg.xs - rg.ds, lch));
+                for (int q = threadIdx.x; q < rg.xe - rg.xs; q += blockDim.x) {
+                    const Pos<float> p = load_pos(S.x, q);
+                    const float* ds = S.d + 3 * (q + rg.xs - rg.ds);
+                    float d[3] = {ds[0], ds[1], ds[2]};
+                    if (pend) {
+                        const int bq = rg.xs + q;
+                        float F[3] = {Fq[0], Fq[1], Fq[2]};
+                        if (q >= kBlock && bq < n.nb) {   // the few beads past one per thread
+                            F[0] = Fn[3 * (size_t)bq];
+                            F[1] = Fn[3 * (size_t)bq + 1];
+                            F[2] = Fn[3 * (size_t)bq + 2];
+                        }
+#pragma unroll
+                        for (int m = 0; m < 3; ++m) d[m] = new_direction(F[m], beta, d[m]);
+                        if (!ch && bq >= t.x && bq < t.y) {   // the tile's own bead: the direction, d . F, the backup
+                            float* o = n.d[((t.w >> 7) & 1) ^ 1] + 3 * (size_t)bq;
+                            o[0] = d[0];
+                            o[1] = d[1];
+                            o[2] = d[2];
+                            df.add(bead_dot(d[0], d[1], d[2], F[0], F[1], F[2]));
+                            if (t.w & 256) store_pos(n.xbest, bq, p);
+                        }
+                    }
+                    store_pos(s_mv, q, moved(p, d, lch));
+                }
                 __syncthreads();
                 P = s_mv;
             }
@@ -1002,7 +1071,7 @@ __global__ void __launch_bounds__(kBlock) k_fil_force_bulk(DevNet<float> n, int 
     __shared__ ForceStage stage[kBulkStages];
     __shared__ __align__(8) uint64_t bar[kBulkStages];
     __shared__ int4 s_desc[kBulkMaxTiles];
-    __shared__ float s_lf[kBulkMaxTiles];
+    __shared__ float2 s_step[kBulkMaxTiles];
     __shared__ int s_abort;
     // per tile: stretching force of each cylinder (q, q + 1) and the two bending
     // terms of each triple centred on q, for q = tile begin - 1 .. tile end
@@ -1019,7 +1088,7 @@ __global__ void __launch_bounds__(kBlock) k_fil_force_bulk(DevNet<float> n, int 
         if (threadIdx.x == 0) atomicOr(n.err, 16u);
         return;
     }
-    load_descriptors(n, t0, nt, want, s_desc, s_lf);
+    load_descriptors(n, t0, nt, want, s_desc, s_step);
     __syncthreads();
     int pi = 0, issued = 0;
     if (threadIdx.x == 0) {
@@ -1105,213 +1174,6 @@ __global__ void __launch_bounds__(kBlock) k_fil_force_bulk(DevNet<float> n, int 
             mbar_wait_bounded(&bar[q % kBulkStages], (unsigned)((q / kBulkStages) & 1), kBulkWaitLimit);
 }
 
-// What the direction update needs of a replica's state.
-struct DirState {
-    int go, fb, xb, bk;
-    float beta;
-};
-
-// One direction unit (n.ptiles[2] consecutive tiles): the body of a
-// k_direction_mx block, also run unit after unit by k_tail_coop, which passes
-// the state its blocks hold instead of the one in memory.
-template <typename StateOf>
-__device__ void direction_mx_unit(const DevNet<float>& n, int unit, double* sh, StateOf state_of) {
-    const int t0 = unit * n.ptiles[2], t1 = min(t0 + n.ptiles[2], n.n_ftiles);
-    int cur = -1, first = 0, cnt = 0, fb = 0, xb = 0, bk = 0;
-    bool go = false;
-    float beta = 0.f;
-    FF dF;
-    // the run's partial goes to slot 3 of its first tile, as a (hi, lo) pair
-    auto finish = [&](int) {
-        FF a[1] = {dF};
-        block_reduce_ff<1, 0>(a, nullptr, reinterpret_cast<float*>(sh));
-        if (threadIdx.x == 0) store_pair(n.part_fil + 4 * (size_t)first + 3, a[0].h, a[0].l);
-    };
-    for (int ti = t0; ti < t1; ++ti) {
-        const Tile t = n.ftile[ti];
-        if (t.replica != cur) {
-            if (cnt) finish(cur);
-            cur = t.replica;
-            first = ti;
-            cnt = 0;
-            dF = FF();
-            const DirState ds = state_of(cur);
-            go = ds.go;
-            fb = ds.fb;
-            xb = ds.xb;
-            bk = ds.bk;
-            beta = ds.beta;
-        }
-        if (!go) continue;
-        ++cnt;
-        const int b = t.begin + threadIdx.x;
-        if (b < t.end) {
-            const float* F = n.f[fb] + 3 * (size_t)b;
-            float* D = n.d + 3 * (size_t)b;
-            const float d0 = F[0] + beta * D[0], d1 = F[1] + beta * D[1], d2 = F[2] + beta * D[2];
-            D[0] = d0;
-            D[1] = d1;
-            D[2] = d2;
-            dF.add(bead_dot(d0, d1, d2, F[0], F[1], F[2]));
-            if (bk) store_pos(n.xbest, b, load_pos(n.x[xb], b));
-        }
-    }
-    if (cnt) finish(cur);
-}
-
-// Mixed engine: persistent direction update d = F + beta d with the d.F partials.
-__global__ void __launch_bounds__(kBlock) k_direction_mx(DevNet<float> n) {
-    pdl_wait();      // the previous kernel of the main lane has finished
-    pdl_trigger();   // the next kernel of the main lane may be scheduled now
-    MECH_TRACE_KERNEL(n, TK_DIRECTION_MX);
-    __shared__ double sh[32];
-    direction_mx_unit(n, blockIdx.x, sh, [&](int r) {
-        const CGState& S = n.st[r];
-        return DirState{S.phase == PH_DIR, S.fbuf, S.xbuf, S.backupPending, (float)S.beta};
-    });
-}
-
-// ---------------------------------------------------------------------------
-// Mixed engine, one replica: the tail of an iteration after the force lanes
-// as one cooperatively launched grid (every block resident at once): the
-// force gather, the force finalizer, the direction update, the direction
-// finalizer and the reset, with grid barriers where the separate launches
-// had a launch boundary.  The finalizers' reductions run in every block over
-// the same partial slots in the same order, so every block holds the same new
-// state, and block 0 stores it.  Work units, partial slots and reduction
-// order are those of k_force_gather_mx, k_finalize_force, k_direction_mx,
-// k_finalize_direction and k_reset, so the minimization is bitwise the one
-// the separate launches give.
-// ---------------------------------------------------------------------------
-constexpr unsigned kGridWaitLimit = 1u << 22;   // polls before a grid barrier counts as lost
-
-// Barrier over the blocks of a co-resident grid: gbar[0] counts arrivals,
-// gbar[1] is the generation that the last arrival advances.  A wait gives up
-// after kGridWaitLimit polls, sets error bit 64 and returns false in every
-// thread of its block.
-__device__ bool grid_sync(unsigned* gbar, unsigned* err) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned* gen = gbar + 1;
-        const unsigned g0 = *gen;
-        __threadfence();
-        const unsigned arrived = atomicAdd(gbar, 1u);
-        int ok = 1;
-        if (arrived == gridDim.x - 1) {
-            atomicExch(gbar, 0u);
-            __threadfence();
-            atomicAdd(gbar + 1, 1u);
-        } else {
-            unsigned polls = 0;
-            while (*gen == g0) {
-                if (++polls > kGridWaitLimit) {
-                    atomicOr(err, 64u);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
-__global__ void __launch_bounds__(kBlock) k_tail_coop(DevNet<float> n) {
-    MECH_TRACE_KERNEL(n, TK_TAIL_COOP);
-    __shared__ GatherMxShared g;
-    __shared__ double sh[32 * 3];
-    __shared__ int s_phase, s_fb, s_xb, s_bk;
-    __shared__ float s_beta;
-    __shared__ CGState S;   // the block's copy of the replica's state (thread 0 works on it)
-    if (threadIdx.x == 0) {
-        S = n.st[0];
-        s_phase = S.phase;
-        s_fb = S.fbuf;
-        if (blockIdx.x == 0) {   // as after every force evaluation: the exvol work lists restart empty
-            if (n.ev_list_count) *n.ev_list_count = 0;
-            if (n.ev_fb_count) *n.ev_fb_count = 0;
-        }
-    }
-    __syncthreads();
-    const int start = s_phase;
-    if (start != PH_FORCE && start != PH_RESET) return;   // the same decision in every block
-    const RepTiles rt = n.rt[0];
-    int phase = start;
-    if (phase == PH_FORCE) {
-        const int units = (n.n_ftiles + kGatherTiles - 1) / kGatherTiles;
-        for (int u = blockIdx.x; u < units; u += gridDim.x) {
-            gather_mx_unit(n, PH_FORCE, u, g);
-            __syncthreads();
-        }
-        if (!grid_sync(n.gbar, n.err)) return;
-        finalize_force(n, 0, rt, S, sh, false);
-        if (threadIdx.x == 0) {
-            s_phase = S.phase;
-            s_fb = S.fbuf;
-            s_xb = S.xbuf;
-            s_bk = S.backupPending;
-            s_beta = (float)S.beta;
-        }
-        __syncthreads();
-        phase = s_phase;
-        if (phase == PH_DIR) {
-            const DirState ds{1, s_fb, s_xb, s_bk, s_beta};
-            for (int u = blockIdx.x; u < n.pgrid[2]; u += gridDim.x) {
-                direction_mx_unit(n, u, sh, [&](int) { return ds; });
-                __syncthreads();
-            }
-            if (!grid_sync(n.gbar, n.err)) return;
-            finalize_direction(n, 0, rt, S, sh, false);
-            if (threadIdx.x == 0) {
-                s_phase = S.phase;
-                s_fb = S.fbuf;
-            }
-            __syncthreads();
-            phase = s_phase;
-        }
-    }
-    if (phase == PH_RESET) {   // d = F, then the new slope and the next iteration's start
-        const float* F = n.f[s_fb];
-        const size_t nv = 3 * (size_t)n.nb;
-        for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nv; i += (size_t)gridDim.x * blockDim.x)
-            n.d[i] = F[i];
-        if (threadIdx.x == 0) {
-            S.slope = S.FdotF;
-            S.lastFdotF = S.FdotF;
-            begin_iteration(S);
-        }
-        // every block has read the state before block 0 replaces it (on the
-        // force path the barriers above already ensure that)
-        if (start == PH_RESET && !grid_sync(n.gbar, n.err)) return;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) n.st[0] = S;
-}
-
-int coop_tail_grid(int device) {
-    int sms = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tail_coop, kBlock, 0) != cudaSuccess) return 0;
-    return sms * per_sm;
-}
-
-static void launch_tail_coop(const DevNet<float>& n, int grid, cudaStream_t s) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kBlock);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_tail_coop, n);
-}
-
 // ---------------------------------------------------------------------------
 // linker, motor and boundary interactions (energy or force contributions)
 // ---------------------------------------------------------------------------
@@ -1321,8 +1183,8 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
     MECH_TRACE_KERNEL(n, TK_BOND);
     __shared__ double sh[64];   // block_reduce_ff<2>: 32 * 4 floats
     __shared__ int s_go, s_xb, s_dual;
-    __shared__ double s_lam;
-    __shared__ float s_lf;   // the step rounded once (mixed engine)
+    __shared__ Real s_lam;                 // (mixed engine: the step rounded once)
+    __shared__ Direction<Real> s_dir;
     const int ti = blockIdx.x < n_lm_tiles ? blockIdx.x : blockIdx.x + ev_tiles;
     const Tile t = n.stile[ti];
     const int kind = n.stile_kind[ti];
@@ -1331,8 +1193,8 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
         const CGState& S = n.st[r];
         s_go = replica_selected(S, want);
         s_xb = S.xbuf;
-        s_lam = S.lambda;
-        s_lf = (float)S.lambda;
+        s_lam = (Real)S.lambda;
+        s_dir = direction_of(n, S);
         s_dual = S.dual;
     }
     __syncthreads();
@@ -1341,15 +1203,9 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
     const bool tr = trial != 0;
     // a pass with a second trial also evaluates the energy at lambda / 2 (mixed engine)
     const bool dual = sizeof(Real) == 4 && !force && second_trial(trial, s_dual);
-    auto pos_at = [&](int b, float lfs) -> Pos<Real> {
-        if constexpr (sizeof(Real) == 4) {
-            const Pos<float> p = load_pos(X, b);
-            return tr ? moved_f(p, n.d, b, lfs) : p;
-        } else {
-            return bead_at(X, n.d, b, tr, s_lam);
-        }
-    };
-    auto pos = [&](int b) -> Pos<Real> { return pos_at(b, s_lf); };
+    auto pos = [&](int b) -> Pos<Real> { return bead_at(X, s_dir, b, tr, s_lam); };
+    const Real lh = (Real)0.5 * s_lam;
+    auto pos2 = [&](int b) -> Pos<Real> { return bead_at(X, s_dir, b, true, lh); };   // the second trial
     const int i = t.begin + threadIdx.x;
     Real e = 0, e2 = 0;
     if (i < t.end) {
@@ -1364,7 +1220,7 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
             if (!force) {
                 e = K * ex;
                 if (dual) {
-                    const Real rr2 = plane_dist_p(pl, pos_at(b, 0.5f * s_lf));
+                    const Real rr2 = plane_dist_p(pl, pos2(b));
                     e2 = K * exp(-rr2 / sl);
                 }
             } else {
@@ -1390,9 +1246,8 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
                 const Real dd = dist - l0;
                 e = (Real)0.5 * k * dd * dd;
                 if (dual) {
-                    const float lh = 0.5f * s_lf;
                     Real w[3];
-                    bond_vector(pos_at(bs.x, lh), pos_at(bs.y, lh), pos_at(bs.z, lh), pos_at(bs.w, lh), s1, s2, w);
+                    bond_vector(pos2(bs.x), pos2(bs.y), pos2(bs.z), pos2(bs.w), s1, s2, w);
                     const Real d2 = sqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]) - l0;
                     e2 = (Real)0.5 * k * d2 * d2;
                 }
@@ -1440,124 +1295,26 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
     }
 }
 
-// ---------------------------------------------------------------------------
-// FP64 engine: direction update d = F + beta d, backup copy; kGatherTiles tiles
-// per block as the gather, d.F per tile (26 us on 1M beads with one tile and
-// tree per block)
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) k_direction(DevNet<double> n) {
-    pdl_wait();      // the previous kernel of the main lane has finished
-    pdl_trigger();   // the next kernel of the main lane may be scheduled now
-    MECH_TRACE_KERNEL(n, TK_DIRECTION);
-    __shared__ double sh[kGatherTiles * kBlock / 32];
-    __shared__ GatherTiles g;
-    const int t0 = blockIdx.x * kGatherTiles;
-    load_gather_tiles(n, t0, PH_DIR, g);
-    if (!(g.go[0] | g.go[1] | g.go[2] | g.go[3])) return;
-    double dF[kGatherTiles];
-#pragma unroll
-    for (int j = 0; j < kGatherTiles; ++j) {
-        dF[j] = 0.0;
-        if (!g.go[j]) continue;
-        const Tile t = n.ftile[t0 + j];
-        const int b = t.begin + threadIdx.x;
-        if (b >= t.end) continue;
-        const CGState& S = n.st[g.rep[j]];
-        const double beta = S.beta;
-        const double* F = n.f[g.fb[j]] + 3 * (size_t)b;
-        double* D = n.d + 3 * (size_t)b;
-        const double f0 = F[0], f1 = F[1], f2 = F[2];
-        const double d0 = f0 + beta * D[0], d1 = f1 + beta * D[1], d2 = f2 + beta * D[2];
-        D[0] = d0;
-        D[1] = d1;
-        D[2] = d2;
-        dF[j] = bead_dot(d0, d1, d2, f0, f1, f2);
-        if (S.backupPending) store_pos(n.xbest, b, load_pos(n.x[S.xbuf], b));
-    }
-    const double a = block_sums<kGatherTiles>(dF, sh);
-    if (threadIdx.x < kGatherTiles && g.go[threadIdx.x]) n.part_fil[4 * (size_t)(t0 + threadIdx.x) + 3] = a;
-}
-
-template <typename Real>
-__global__ void __launch_bounds__(kBlock) k_finalize_direction(DevNet<Real> n) {
-    pdl_wait();      // the previous kernel of the main lane has finished
-    pdl_trigger();   // the next kernel of the main lane may be scheduled now
-    MECH_TRACE_KERNEL(n, TK_FIN_DIRECTION);
-    __shared__ double sh[32];
-    __shared__ int s_flag;
-    const int r = blockIdx.x;
-    CGState S;
-    if (threadIdx.x == 0) S = n.st[r];   // issued together with the loads below
-    const RepTiles rt = n.rt[r];
-    if (n.st[r].phase == PH_DIR) finalize_direction(n, r, rt, S, sh);
-    after_phase(n, kCondDir, &s_flag);
-}
-
-// d = F (resetCGParams, CGMethod.hpp:963-972); the new slope d.F is F.F.
-// kGatherTiles tiles per block, so that the launch costs little when no
-// replica is resetting (it is in every iteration of the graph).
-template <typename Real>
-__global__ void __launch_bounds__(kBlock) k_reset(DevNet<Real> n) {
-    pdl_wait();      // the previous kernel of the main lane has finished
-    pdl_trigger();   // the next kernel of the main lane may be scheduled now
-    MECH_TRACE_KERNEL(n, TK_RESET);
-    // the misc body of the conditional graph (failure dispatch is applied where a
-    // line search fails) counts its launches here
-    if (n.cond.on && blockIdx.x == 0 && threadIdx.x == 0) ++n.cond.counter[kCondMisc];
-    __shared__ int s_go[kGatherTiles], s_fb[kGatherTiles], s_flag;
-    const int t0 = blockIdx.x * kGatherTiles;
-    if (threadIdx.x < kGatherTiles) {
-        const int ti = t0 + threadIdx.x;
-        int go = 0, fb = 0;
-        if (ti < n.n_ftiles) {
-            const CGState& S = n.st[n.ftile[ti].replica];
-            go = S.phase == PH_RESET;
-            fb = S.fbuf;
-        }
-        s_go[threadIdx.x] = go;
-        s_fb[threadIdx.x] = fb;
-    }
-    __syncthreads();
-    for (int j = 0; j < kGatherTiles; ++j) {
-        if (!s_go[j]) continue;   // block-uniform
-        const Tile t = n.ftile[t0 + j];
-        const int r = t.replica;
-        const int b = t.begin + threadIdx.x;
-        if (b < t.end) {
-            const Real* F = n.f[s_fb[j]] + 3 * (size_t)b;
-            Real* D = n.d + 3 * (size_t)b;
-            D[0] = F[0];
-            D[1] = F[1];
-            D[2] = F[2];
-        }
-        const RepTiles rt = n.rt[r];
-        if (last_tile(n.ticket, r, rt.fil_end - rt.fil_begin, &s_flag)) {
-            if (threadIdx.x == 0) {
-                CGState& S = n.st[r];
-                S.slope = S.FdotF;
-                S.lastFdotF = S.FdotF;
-                begin_iteration(S);
-            }
-        }
-    }
-}
-
-
 // Recovery move: step = maxDist / max_i |d_i|, x += step d (MController.h:273-339).
 template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_recover_maxabs(DevNet<Real> n) {
     MECH_TRACE_KERNEL(n, TK_RECOVER_MAXABS);
     __shared__ double sh[32];
     __shared__ int s_go, s_flag;
+    __shared__ Direction<Real> s_dir;
     const Tile t = n.ftile[blockIdx.x];
     const int r = t.replica;
-    if (threadIdx.x == 0) s_go = n.st[r].phase == PH_RECOVER;
+    if (threadIdx.x == 0) {
+        s_go = n.st[r].phase == PH_RECOVER;
+        s_dir = direction_of(n, n.st[r]);
+    }
     __syncthreads();
     if (!s_go) return;
     const int b = t.begin + threadIdx.x;
     Real m = 0;
     if (b < t.end) {
-        const Real* D = n.d + 3 * (size_t)b;
+        Real D[3];
+        direction_at(s_dir, b, D);
         m = fmax(fmax(fabs(D[0]), fabs(D[1])), fabs(D[2]));
     }
     const double sm = block_max_r(m, sh);
@@ -1583,21 +1340,23 @@ template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_recover_move(DevNet<Real> n) {
     MECH_TRACE_KERNEL(n, TK_RECOVER_MOVE);
     __shared__ int s_go, s_xb, s_flag;
-    __shared__ double s_step;
+    __shared__ Real s_step;
+    __shared__ Direction<Real> s_dir;
     const Tile t = n.ftile[blockIdx.x];
     const int r = t.replica;
     if (threadIdx.x == 0) {
         const CGState& S = n.st[r];
         s_go = S.phase == PH_RECOVER_MOVE;
         s_xb = S.xbuf;
-        s_step = S.lambda;
+        s_step = (Real)S.lambda;
+        s_dir = direction_of(n, S);
     }
     __syncthreads();
     if (!s_go) return;
     const int b = t.begin + threadIdx.x;
     if (b < t.end) {   // coord += step * d (MController.h:321-323)
         Real* X = n.x[s_xb];
-        store_pos(X, b, moved(load_pos(X, b), n.d, b, s_step));
+        store_pos(X, b, bead_at(X, s_dir, b, true, s_step));
     }
     const RepTiles rt = n.rt[r];
     if (last_tile(n.ticket, r, rt.fil_end - rt.fil_begin, &s_flag)) {
@@ -1610,7 +1369,7 @@ __global__ void __launch_bounds__(kBlock) k_backup_restore(DevNet<Real> n) {
     MECH_TRACE_KERNEL(n, TK_BACKUP);
     const Tile t = n.ftile[blockIdx.x];
     const CGState& S = n.st[t.replica];
-    if (!S.restore) return;
+    if (!S.restore || S.backupPending) return;   // pending: the current positions are the backup
     const int b = t.begin + threadIdx.x;
     if (b < t.end) store_pos(n.x[S.xbuf], b, load_pos(n.xbest, b));
 }
@@ -1660,7 +1419,7 @@ int launch_energy(const DevNet<Real>& n, int want, int trial, const Lanes& L) {
 }
 
 template <typename Real>
-int launch_forces(const DevNet<Real>& n, int want, const Lanes& L, int coop_grid) {
+int launch_forces(const DevNet<Real>& n, int want, const Lanes& L) {
     int ev_t = 0, bb_t = 0;
     const int lm = n_lm_tiles(n, &ev_t, &bb_t);
     int launched = 0;
@@ -1682,29 +1441,14 @@ int launch_forces(const DevNet<Real>& n, int want, const Lanes& L, int coop_grid
     if (!n.fil_first[1]) fil();
     cudaStreamWaitEvent(L.main, L.join, 0);
     cudaStreamWaitEvent(L.main, L.join2, 0);
-    if constexpr (sizeof(Real) == 4) {
-        if (coop_grid > 0) {
-            launch_tail_coop(n, coop_grid, L.main);
-            return launched + 2;
-        }
-    }
     if constexpr (sizeof(Real) == 4) k_force_gather_mx<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, L.main>>>(n, want);
     else k_force_gather<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, L.main>>>(n, want);
     launch_k(n.pdl, k_finalize_force<Real>, n.R, kBlock, L.main, n, want);
     return launched + 3;
 }
 
-template <typename Real>
-int launch_direction(const DevNet<Real>& n, cudaStream_t s) {
-    if constexpr (sizeof(Real) == 4) launch_k(n.pdl, k_direction_mx, n.pgrid[2], kBlock, s, n);
-    else launch_k(n.pdl, k_direction, (n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, s, n);
-    launch_k(n.pdl, k_finalize_direction<Real>, n.R, kBlock, s, n);
-    return 2;
-}
-
-template <typename Real>
-int launch_reset(const DevNet<Real>& n, cudaStream_t s) {
-    launch_k(n.pdl, k_reset<Real>, (n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, s, n);
+int launch_graph_head(cudaStream_t s) {
+    k_graph_head<<<1, 32, 0, s>>>();
     return 1;
 }
 
@@ -1723,7 +1467,6 @@ int launch_recover(const DevNet<Real>& n, const Lanes& L) {
     k += 2;
     k += launch_forces<Real>(n, PH_RECOVER_FORCE, L);
     k += launch_energy<Real>(n, PH_RECOVER_ENERGY, 0, L);
-    k += launch_reset<Real>(n, L.main);
     return k;
 }
 
@@ -1772,14 +1515,13 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
 // many blocks as fit, or at most `per_sm` of them (leaving room on each SM for
 // the kernels of the other lanes).
 int persistent_blocks(int device, int which, int per_sm) {
-    static int cached_dev = -1, sms = 0, occ[3] = {0, 0, 0};
+    static int cached_dev = -1, sms = 0, occ[2] = {0, 0};
     if (cached_dev != device) {
-        int b[3] = {0, 0, 0};
+        int b[2] = {0, 0};
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[0], k_fil_energy_bulk, kBlock, 0);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[1], k_fil_force_bulk, kBlock, 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b[2], k_direction_mx, kBlock, 0);
-        for (int k = 0; k < 3; ++k) occ[k] = std::max(1, b[k]);
+        for (int k = 0; k < 2; ++k) occ[k] = std::max(1, b[k]);
         sms = std::max(1, sms);
         cached_dev = device;
     }
@@ -1790,9 +1532,7 @@ int persistent_blocks(int device, int which, int per_sm) {
 #define MECH_INSTANTIATE(R)                                                             \
     template int launch_part<R>(const DevNet<R>&, int, cudaStream_t);                   \
     template int launch_energy<R>(const DevNet<R>&, int, int, const Lanes&);            \
-    template int launch_forces<R>(const DevNet<R>&, int, const Lanes&, int);            \
-    template int launch_direction<R>(const DevNet<R>&, cudaStream_t);                   \
-    template int launch_reset<R>(const DevNet<R>&, cudaStream_t);                       \
+    template int launch_forces<R>(const DevNet<R>&, int, const Lanes&);                 \
     template int launch_body_head<R>(const DevNet<R>&, cudaStream_t);                   \
     template int launch_recover<R>(const DevNet<R>&, const Lanes&);                     \
     template int launch_backup_restore<R>(const DevNet<R>&, cudaStream_t);

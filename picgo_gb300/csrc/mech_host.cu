@@ -74,7 +74,7 @@ struct MechContext {
     std::vector<ReplicaHost> reps;
     bool have_net = false, have_lists = false;
     // beads
-    DeviceBuffer x[3], f[2], d, xbest, xinit, bflag, bpar;   // x[2]: mixed engine's second trial buffer
+    DeviceBuffer x[3], f[2], d[2], xbest, xinit, bflag, bpar;   // x[2]: mixed engine's second trial buffer
     // cylinders
     DeviceBuffer cyl_b1, cyl_id, cyl_fil, cyl_pos, cyl_rep, cyl_minus, cyl_kex, cyl_type, cyl_l0;
     // linkers / motors
@@ -84,7 +84,7 @@ struct MechContext {
     // excluded volume
     DeviceBuffer ev_bead, ev_k, ev_la, ev_lb, ev_list, ev_list_count, ev_energy, ev_energy2;
     // tiles, partials, state
-    DeviceBuffer ftile, stile, stile_kind, rt, part_fil, part_sp, part_sp2, st, ticket, gticket, cond_counter;
+    DeviceBuffer ftile, stile, stile_kind, rt, part_fil, part_df, part_sp, part_sp2, st, ticket, gticket, cond_counter;
     int graph_mode = MECH_GRAPH_UNROLLED;
     DeviceBuffer contrib, ev_fb_count, ev_fb_list, ev_fb_energy, fb_moments, fb_tickets;
     // rebuild scratch
@@ -96,7 +96,6 @@ struct MechContext {
     // Hessian-vector products, adjoint and Newton solves (FP64 engine)
     DeviceBuffer hv_a, hv_b, cg_x, cg_r, cg_p, cg_Ap, cg_scal, cg_part, cg_ticket, hess_fil, hess_lm, hess_ev, hess_bb;
     DeviceBuffer lf_ends, lf_types, lf_ms, lf_nm, lf_out;   // load forces
-    DeviceBuffer gbar;   // grid barrier of the cooperative iteration tail (2 unsigned)
     int n_ftiles = 0, n_stiles = 0;
     int sp_tiles[K_NUM_SPARSE] = {0, 0, 0, 0};
     // host copies of the full tile lists, and the compacted view that a
@@ -132,15 +131,17 @@ struct MechContext {
     bool h_fresh = false;
     int h_cap = 0;             // replicas the pinned buffers hold
     unsigned* d_err() const { return reinterpret_cast<unsigned*>(st.as<CGState>() + R); }
-    // pinned snapshots taken after each minimizer graph launch (k_snapshot):
+    // What the host looks at after a minimizer graph launch, in pinned memory:
     // error word, the conditional graph's body counters, then every replica's
-    // phase; double-buffered
+    // phase.  Conditional graph: written by k_snapshot after each launch, double-
+    // buffered.  Unrolled graph: the force finalizer writes to the first buffer
+    // when a replica has finished or waits for the host (DevNet::snap); the
+    // host sets the words before it launches, and a newer value than the launch
+    // it waited for gives does no harm.
     struct Snapshot {
         int* word = nullptr;       // [0] error word, [1..8] body counters, [9 + r] phases
         cudaEvent_t done = nullptr;
         int launches = 0;          // kernels of the unrolled graph it follows
-        unsigned err() const { return (unsigned)word[0]; }
-        const int* phase() const { return word + 9; }
     } snap[2];
     cudaEvent_t t0 = nullptr, t1 = nullptr;   // device time of a minimization
     // The unrolled iteration graphs (short and long, kGraphBlocks) of the last
@@ -196,7 +197,8 @@ DevNet<Real> make_devnet(MechContext* c) {
     n.x[2] = c->x[2].as<Real>();
     n.f[0] = c->f[0].as<Real>();
     n.f[1] = c->f[1].as<Real>();
-    n.d = c->d.as<Real>();
+    n.d[0] = c->d[0].as<Real>();
+    n.d[1] = c->d[1].as<Real>();
     n.xbest = c->xbest.as<Real>();
     n.ev_list = c->ev_list.as<int>();
     n.ev_list_count = c->ev_list_count.as<int>();
@@ -206,20 +208,18 @@ DevNet<Real> make_devnet(MechContext* c) {
     n.bpar = c->bpar.as<Real>();
     n.n_ftiles = c->compact ? c->n_ftiles_c : c->n_ftiles;
     n.ftile = (c->compact ? c->ftile_c : c->ftile).as<Tile>();
-    for (int k = 0; k < 3; ++k) {
-        const int per_sm = k < 2 ? c->blocks_per_sm[k] : 0;
-        if (k < 2) n.fil_first[k] = (c->precision == MECH_PREC_MIXED && per_sm > 0) ? 1 : 0;
+    for (int k = 0; k < 2; ++k) {
+        const int per_sm = c->blocks_per_sm[k];
+        n.fil_first[k] = (c->precision == MECH_PREC_MIXED && per_sm > 0) ? 1 : 0;
         const int resident = persistent_blocks(c->device, k, per_sm);
         n.pgrid[k] = std::max(1, std::min(n.n_ftiles, resident));
         n.ptiles[k] = (n.n_ftiles + n.pgrid[k] - 1) / n.pgrid[k];
-        if (k < 2) {
-            // the bulk-staged energy/force kernels keep a block's tile descriptors in
-            // shared memory (at most kFilBulkMaxTiles); a tuned smaller run length adds
-            // waves, unless a residency cap is set, which the grid then keeps to
-            n.ptiles[k] = std::max(1, std::min(n.ptiles[k], c->tile_cap[k]));
-            if (per_sm > 0) n.ptiles[k] = std::max(n.ptiles[k], (n.n_ftiles + resident - 1) / resident);
-            n.ptiles[k] = std::min(n.ptiles[k], kFilBulkMaxTiles);
-        }
+        // the bulk-staged energy/force kernels keep a block's tile descriptors in
+        // shared memory (at most kFilBulkMaxTiles); a tuned smaller run length adds
+        // waves, unless a residency cap is set, which the grid then keeps to
+        n.ptiles[k] = std::max(1, std::min(n.ptiles[k], c->tile_cap[k]));
+        if (per_sm > 0) n.ptiles[k] = std::max(n.ptiles[k], (n.n_ftiles + resident - 1) / resident);
+        n.ptiles[k] = std::min(n.ptiles[k], kFilBulkMaxTiles);
         n.pgrid[k] = (n.n_ftiles + n.ptiles[k] - 1) / n.ptiles[k];
     }
     n.n_lk = c->nlk;
@@ -262,6 +262,7 @@ DevNet<Real> make_devnet(MechContext* c) {
     n.fb_moments = c->fb_moments.as<double>();
     n.fb_tickets = c->fb_tickets.as<int>();
     n.part_fil = c->part_fil.as<double>();
+    n.part_df = c->part_df.as<double>();
     n.part_sp = c->part_sp.as<double>();
     n.part_sp2 = c->part_sp2.as<double>();
     n.st = c->st.as<CGState>();
@@ -471,6 +472,7 @@ __global__ void k_cg_init(CGState* st, int R) {
         return;
     }
     S.phase = PH_RESET;                   // resetCGParams, then the loop head
+    settle(S);
 }
 
 // A call-limit exit restores the minimum-energy backup (CGMethod.hpp:1589-1610).
@@ -478,7 +480,7 @@ __global__ void k_cg_finish(CGState* st, int R, int report_on_call_limit) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= R) return;
     CGState& S = st[r];
-    S.restore = report_on_call_limit && call_limit(S) && S.backupValid;
+    S.restore = report_on_call_limit && call_limit(S) && (S.backupValid || S.backupPending);
     S.active = 1;
 }
 
@@ -674,10 +676,10 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
     CU(cudaMemcpyAsync(c->xinit.p, c->x[0].p, sizeof(double) * nx, cudaMemcpyDeviceToDevice, s));
     CU(c->f[0].ensure(rs * nx + kBulkPad));
     CU(c->f[1].ensure(rs * nx + kBulkPad));
-    CU(c->d.ensure(rs * nx + kBulkPad));
+    for (auto& d : c->d) CU(d.ensure(rs * nx + kBulkPad));
     CU(cudaMemsetAsync(c->f[0].p, 0, rs * nx, s));
     CU(cudaMemsetAsync(c->f[1].p, 0, rs * nx, s));
-    CU(cudaMemsetAsync(c->d.p, 0, rs * nx, s));
+    for (auto& d : c->d) CU(cudaMemsetAsync(d.p, 0, rs * nx, s));
     flags.resize((size_t)nb + 32, 0);   // tail padding read by 16-byte-rounded bulk copies
     if ((rc = upload(c->bflag, flags, s))) return rc;
     {
@@ -721,6 +723,7 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
     c->compact = false;
     if ((rc = upload(c->ftile, ft, s))) return rc;
     CU(c->part_fil.ensure(sizeof(double) * 4 * ft.size()));
+    CU(c->part_df.ensure(sizeof(double) * ft.size()));
     // states
     CU(c->st.ensure(sizeof(CGState) * R + 16));
     CU(cudaMemsetAsync(c->st.p, 0, sizeof(CGState) * R + 16, s));
@@ -1032,7 +1035,6 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
 // ===========================================================================
 // Status of the device error word's bits (kernels set them with atomicOr).
 static int err_status(unsigned bits) {
-    if (bits & 64u) return set_err(MECH_ERR_ITER_LIMIT, "a grid barrier of the cooperative iteration tail timed out");
     if (bits & 32u) return set_err(MECH_ERR_ITER_LIMIT, "a bulk shared-memory copy did not complete in time");
     if (bits & 16u) return set_err(MECH_ERR_CUDA, "a bulk shared-memory copy range was misaligned");
     if (bits & 1u) return set_err(MECH_ERR_NONFINITE, "excluded-volume numeric fallback failed");
@@ -1099,33 +1101,18 @@ static int iteration_graph(MechContext* c, int which) {
     auto& ig = c->iter[which];
     DevNet<Real> n = make_devnet<Real>(c);
     n.pdl = c->graph_mode == MECH_GRAPH_UNROLLED_PDL ? 1 : 0;
-    // the cooperative tail: mixed engine, one replica (its blocks reduce for replica 0)
-    int coop_grid = 0;
-    if (c->graph_mode == MECH_GRAPH_UNROLLED_COOP && sizeof(Real) == 4 && c->R == 1) {
-        coop_grid = coop_tail_grid(c->device);
-        if (coop_grid <= 0) return set_err(MECH_ERR_CUDA, "cooperative tail: no resident blocks");
-        CU(c->gbar.ensure(2 * sizeof(unsigned)));
-        CU(cudaMemsetAsync(c->gbar.p, 0, 2 * sizeof(unsigned), c->stream));
-        n.gbar = c->gbar.as<unsigned>();
-    }
-    std::vector<unsigned char> key(sizeof(n) + 2 * sizeof(int));
-    const int form[2] = {c->graph_mode, coop_grid};
+    n.snap = c->snap[0].word;
+    std::vector<unsigned char> key(sizeof(n) + sizeof(int));
     std::memcpy(key.data(), &n, sizeof(n));
-    std::memcpy(key.data() + sizeof(n), form, sizeof(form));
+    std::memcpy(key.data() + sizeof(n), &c->graph_mode, sizeof(int));
     if (ig.exec && key == ig.key) return MECH_OK;
     ig.key.clear();
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    int k = 0;
+    int k = launch_graph_head(c->stream);
     for (int b = 0; b < kGraphBlocks[which]; ++b) {
         k += trial_launches<Real>(n, c->lanes());
-        if (coop_grid > 0) {
-            k += launch_forces<Real>(n, PH_FORCE, c->lanes(), coop_grid);
-            continue;
-        }
         k += launch_forces<Real>(n, PH_FORCE, c->lanes());
-        k += launch_direction<Real>(n, c->stream);
-        k += launch_reset<Real>(n, c->stream);
     }
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (e != cudaSuccess) return set_err(MECH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -1150,14 +1137,13 @@ static int iteration_graph(MechContext* c, int which) {
 
 // Kernels per body part of the conditional graph (for the launch count).
 struct CondGraphCounts {
-    int head, trial, force, dir, misc;
+    int head, trial, force;
 };
 static constexpr int kBodiesPerLaunch = 512;
 
 // The minimizer as one conditional graph: a while loop whose body is
-//   head -> if (trial) energy at x + lambda d -> if (force) forces
-//        -> if (direction) d = F + beta d -> if (misc) reset (d = F).
-// The head sets the four conditions from the replicas' phases and whether the
+//   head -> if (trial) energy at x + lambda d -> if (force) forces.
+// The head sets the two conditions from the replicas' phases and whether the
 // loop runs another body; each phase's reduction sets them again for the
 // phases after it in the same body.  Only phases some replica is in run, and
 // control returns to the host when no replica has device work left, a
@@ -1191,11 +1177,11 @@ static int capture_conditional_graph(MechContext* c, cudaGraphExec_t* exec, Cond
     cudaGraphNode_t loop_node = nullptr;
     if ((e = cudaGraphAddNode(&loop_node, g, &reset_node, nullptr, 1, &wp)) != cudaSuccess) return fail(e, "loop node");
     cudaGraph_t body = wp.conditional.phGraph_out[0];
-    cudaGraphConditionalHandle h[4] = {0, 0, 0, 0};
-    for (int k = 0; k < 4; ++k)
+    cudaGraphConditionalHandle h[2] = {0, 0};
+    for (int k = 0; k < 2; ++k)
         if ((e = cudaGraphConditionalHandleCreate(&h[k], body, 0, 0)) != cudaSuccess) return fail(e, "phase handle");
     DevNet<Real> n = make_devnet<Real>(c);
-    n.cond = GraphConds{h[0], h[1], h[2], h[3], h_loop, c->cond_counter.as<int>(), kBodiesPerLaunch, 1};
+    n.cond = GraphConds{h[0], h[1], h_loop, c->cond_counter.as<int>(), kBodiesPerLaunch, 1};
     // capture `fn` into `graph` after `dep` (none when null)
     auto capture_into = [&](cudaGraph_t graph, const cudaGraphNode_t* dep, auto&& fn) -> cudaError_t {
         cudaError_t err = cudaStreamBeginCaptureToGraph(c->stream, graph, dep, nullptr, dep ? 1 : 0,
@@ -1228,12 +1214,6 @@ static int capture_conditional_graph(MechContext* c, cudaGraphExec_t* exec, Cond
         return fail(e, "trial body");
     if ((e = add_if(h[1], [&] { counts->force = launch_forces<Real>(n, PH_FORCE, c->lanes()); })) != cudaSuccess)
         return fail(e, "force body");
-    if ((e = add_if(h[2], [&] { counts->dir = launch_direction<Real>(n, c->stream); })) != cudaSuccess)
-        return fail(e, "direction body");
-    if ((e = add_if(h[3], [&] {
-             counts->misc = launch_reset<Real>(n, c->stream);
-         })) != cudaSuccess)
-        return fail(e, "reset body");
     e = cudaGraphInstantiate(exec, g, cudaGraphInstantiateFlagUseNodePriority);
     cudaGraphDestroy(g);
     g = nullptr;
@@ -1298,12 +1278,11 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
     DevNet<Real> n = make_devnet<Real>(c);
     CU(cudaEventRecord(c->t0, s));
     // energiesBefore, initial forces, resetCGParams, loop head
-    long long launches = 3;
+    long long launches = 2;
     k_cg_reset<<<(c->R + 127) / 128, 128, 0, s>>>(n.st, n.rt, c->R, *p);
     launches += launch_energy<Real>(n, -1, 0, c->lanes());
     launches += launch_forces<Real>(n, -1, c->lanes());
     k_cg_init<<<(c->R + 127) / 128, 128, 0, s>>>(n.st, c->R);
-    launches += launch_reset<Real>(n, s);
     CU(cudaGetLastError());
     // the conditional graph belongs to this call, the unrolled one to the context
     struct CallGraph {
@@ -1339,7 +1318,8 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
         ++graphs;
         auto& sn = c->snap[k];
         sn.launches = c->iter[which].launches;
-        k_snapshot<<<(std::max(c->R, 9) + 127) / 128, 128, 0, s>>>(n.st, c->R, n.err, c->cond_counter.as<int>(), sn.word);
+        if (conditional)
+            k_snapshot<<<(std::max(c->R, 9) + 127) / 128, 128, 0, s>>>(n.st, c->R, n.err, c->cond_counter.as<int>(), sn.word);
         CU(cudaGetLastError());
         CU(cudaEventRecord(sn.done, s));
         return MECH_OK;
@@ -1347,15 +1327,17 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
     // launches of snapshot k's graph (the conditional graph counts what its bodies ran)
     auto account = [&](int k) {
         const int* bc = c->snap[k].word + 1;
-        launches += 1 + (conditional ? (long long)bc[0] * cc.head + (long long)bc[2] * cc.trial +
-                                      (long long)bc[3] * cc.force + (long long)bc[4] * cc.dir + (long long)bc[5] * cc.misc
+        launches += (conditional ? (long long)bc[0] * cc.head + (long long)bc[2] * cc.trial +
+                                      (long long)bc[3] * cc.force + 1
                                 : c->snap[k].launches);
     };
-    auto wants_host = [&](const MechContext::Snapshot& sn, bool* all_done) {
+    auto words = [&](int k) { return (const volatile int*)c->snap[conditional ? k : 0].word; };
+    auto wants_host = [&](int k, bool* all_done) {
+        const volatile int* w = words(k);
         bool done = true, host = false;
         long long live = 0;
         for (int r = 0; r < c->R; ++r) {
-            const int ph = sn.phase()[r];
+            const int ph = w[9 + r];
             const bool act = ph != PH_DONE && ph != PH_ERROR;
             if (act) {
                 done = false;
@@ -1366,9 +1348,13 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
         *all_done = done;
         // batched runs: relaunch over the live replicas once they hold at most half of the tiles
         const bool compactable = c->R > 1 && !done && 2 * live <= (long long)n.n_ftiles;
-        return sn.err() != 0 || done || host || compactable || graphs > max_graphs;
+        return w[0] != 0 || done || host || compactable || graphs > max_graphs;
     };
     int cur = 0;
+    if (!conditional) {
+        c->snap[0].word[0] = 0;
+        for (int r = 0; r < c->R; ++r) c->snap[0].word[9 + r] = PH_LS_TRIAL;
+    }
     if ((rc = launch(cur))) return rc;
     for (;;) {
         const int nxt = cur ^ 1;
@@ -1376,16 +1362,16 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
         CU(cudaEventSynchronize(c->snap[cur].done));
         account(cur);
         bool all_done = false;
-        if (!wants_host(c->snap[cur], &all_done)) {
+        if (!wants_host(cur, &all_done)) {
             cur = nxt;
             continue;
         }
         // drain the launch in flight and act on its (newest) snapshot
         CU(cudaEventSynchronize(c->snap[nxt].done));
         account(nxt);
-        const auto& sn = c->snap[nxt];
-        if (sn.err()) {
-            status = err_status(sn.err());
+        const volatile int* w = words(nxt);
+        if (w[0]) {
+            status = err_status((unsigned)w[0]);
             break;
         }
         bool recover = false;
@@ -1393,7 +1379,7 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
         long long live = 0;
         all_done = true;
         for (int r = 0; r < c->R; ++r) {
-            const int ph = sn.phase()[r];
+            const int ph = w[9 + r];
             act[r] = ph != PH_DONE && ph != PH_ERROR;
             if (act[r]) {
                 all_done = false;
@@ -1407,6 +1393,8 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
             break;
         }
         if (recover) {
+            for (int r = 0; r < c->R && !conditional; ++r)
+                if (c->snap[0].word[9 + r] >= PH_RECOVER) c->snap[0].word[9 + r] = PH_LS_TRIAL;
             launches += launch_recover<Real>(n, c->lanes());
             CU(cudaGetLastError());
         }
@@ -1814,7 +1802,7 @@ int32_t mech_set_graph_mode(MechContext* ctx, int32_t mode) {
     if (mode != MECH_GRAPH_CONDITIONAL && mode != MECH_GRAPH_UNROLLED && mode != MECH_GRAPH_UNROLLED_PDL &&
         mode != MECH_GRAPH_UNROLLED_COOP)
         return set_err(MECH_ERR_ARG, "bad graph mode");
-    ctx->graph_mode = mode;
+    ctx->graph_mode = mode == MECH_GRAPH_UNROLLED_COOP ? MECH_GRAPH_UNROLLED : mode;
     return MECH_OK;
 }
 
@@ -1904,8 +1892,6 @@ static int profile_impl(MechContext* c, int iters, MechProfile* o) {
     o->ms_iteration_idle = timeit([&] {
         trial_launches<Real>(n, c->lanes());
         launch_forces<Real>(n, PH_FORCE, c->lanes());
-        launch_direction<Real>(n, s);
-        launch_reset<Real>(n, s);
     });
     std::copy(saved.begin(), saved.end(), c->h_st);
     if ((rc = push_states(c))) return rc;

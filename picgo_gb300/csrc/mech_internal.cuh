@@ -4,7 +4,7 @@
 //   beads     internal order = filament by filament, minus end first, replica
 //             after replica; coordinates x[2][3*nb] double (AoS, current and
 //             trial buffer), forces f[2][3*nb] Real (current and previous),
-//             search direction d[3*nb] Real.
+//             search direction d[2][3*nb] Real (current and next).
 //   per bead  flag byte (bit0: cylinder to the next bead, bit1: cylinder from
 //             the previous bead); the cylinder (i, i+1) keeps its k_str, l0 at
 //             slot i; the bending triple centred on i keeps the constants of
@@ -51,9 +51,8 @@ enum Phase : int {
     PH_IDLE = 0,
     PH_LS_TRIAL = 1,   // a line-search trial energy is pending
     PH_FORCE = 2,      // trial accepted: forces at the new coordinates pending
-    PH_DIR = 3,        // forces, beta ready: direction update pending
-    PH_RESET = 4,      // conjugacy lost: d = F pending
-    PH_FAILED = 5,     // line search returned lambda = 0: host decides
+    PH_RESET = 4,      // conjugacy lost: d = F (never left in a stored state: settle)
+    PH_FAILED = 5,     // line search returned lambda = 0 (never left in a stored state: dispatch_failed)
     PH_DONE = 6,       // converged or call limit
     PH_ERROR = 7,      // non-finite max force or other fatal condition
     PH_RECOVER = 8,         // safe-mode failure: recovery move pending (MController.h:273-339)
@@ -98,6 +97,12 @@ struct CGState {
     int dual;
     int searchTrials;      // trials of the current line search
     int xbuf, fbuf;
+    // The search direction is d[dbuf], or (dIsF) the current forces themselves:
+    // a reset to steepest descent copies nothing.  dPending: the direction
+    // F + beta d of the search that begins is formed by its first line-search
+    // pass, every kernel for the beads it reads; the filament kernel stores it
+    // in d[dbuf ^ 1] with the d . F partials.
+    int dbuf, dIsF, dPending;
     int numIter, numEnergyCall, numForceCall, numEnergyEval, numTrials, numSafeMode, numRecover;
     int backupValid, backupPending;
     int errorFlags, status;
@@ -121,14 +126,13 @@ struct RepTiles {
 };
 
 // Conditions of the minimizer's conditional graph: a while loop whose body
-// runs one guarded phase after another (line-search trial, forces, direction,
-// failure dispatch + reset).  The kernel at the head of a body and the last
+// runs one guarded phase after another (line-search trial, forces).  The kernel at the head of a body and the last
 // block of each phase's reduction set them from the replicas' phases; outside
 // that graph `on` is 0 and no kernel touches them.
 struct GraphConds {
-    unsigned long long trial, force, dir, misc, loop;   // cudaGraphConditionalHandle values
-    int* counter;   // [0] bodies run in this graph launch, [1] reduction ticket,
-                    // [2..5] trial, force, direction, failure-dispatch bodies run (for the launch count)
+    unsigned long long trial, force, loop;   // cudaGraphConditionalHandle values
+    int* counter;   // [0] bodies run in this graph launch, [2], [3] trial and force
+                    // bodies run (for the launch count)
     int cap;        // bodies per graph launch before control returns to the host
     int on;
 };
@@ -143,7 +147,7 @@ struct DevNet {
     // positions (FP64: one trial buffer; mixed: two, for lambda and lambda / 2)
     Real* x[3];
     Real* f[2];
-    Real* d;
+    Real* d[2];
     Real* xbest;
     const uint8_t* bflag;
     const Real* bpar;       // per bead slot: k_str, l0 of cylinder (i, i+1); k_bend, theta0 of the triple on i
@@ -151,7 +155,7 @@ struct DevNet {
     // block `ptiles` consecutive tiles on a grid of `pgrid` blocks
     int n_ftiles;
     const Tile* ftile;
-    int pgrid[3], ptiles[3];   // [0] energy, [1] force, [2] direction kernels
+    int pgrid[2], ptiles[2];   // [0] energy, [1] force kernels
     int fil_first[2];          // energy / force: filament kernel launched before the side lanes (capped residency)
     // sparse interactions (internal bead indices)
     int n_lk, n_mt, n_ev, n_bb;
@@ -185,6 +189,7 @@ struct DevNet {
     double* ev_energy2; double* part_sp2;
     // partial sums
     double* part_fil;       // [n_ftiles * 4]
+    double* part_df;        // [n_ftiles]: d . F of a pass that forms the direction
     double* part_sp;        // [n_stiles]
     // per replica
     CGState* st;
@@ -202,8 +207,10 @@ struct DevNet {
     // in the engine's precision (a conversion to double in the mixed kernels
     // would be scheduled whether or not the store happens)
     Real* terms;
-    // grid barrier of the cooperative iteration tail: [0] arrivals, [1] generation
-    unsigned* gbar;
+    // pinned host words of the unrolled graph (null otherwise): [0] error word,
+    // [9 + r] the phase of a replica that is finished or waits for the host,
+    // written by the force finalizer, the last kernel of an iteration block
+    int* snap;
     // kernel timeline (builds with MECH_TRACE only; null otherwise):
     // [0] records written, [1] capacity, then (start ns, end ns, kernel << 32 | block) per block
     unsigned long long* trace;
@@ -212,12 +219,10 @@ struct DevNet {
 // Kernel ids of the timeline records.
 enum TraceKernel : unsigned {
     TK_FIL_ENERGY = 1, TK_FIL_FORCE, TK_GATHER, TK_FIN_FORCE, TK_FIN_ENERGY, TK_FIL_ENERGY_BULK, TK_FIL_FORCE_BULK,
-    TK_DIRECTION_MX, TK_BOND, TK_DIRECTION, TK_FIN_DIRECTION, TK_RESET, TK_RECOVER_MAXABS, TK_RECOVER_MOVE,
-    TK_BACKUP, TK_EXVOL_FB_FORCE, TK_EXVOL, TK_EXVOL_EXT, TK_EXVOL_TAIL, TK_BODY_HEAD, TK_GATHER_MX,
+    TK_BOND = 9, TK_RECOVER_MAXABS = 13, TK_RECOVER_MOVE, TK_BACKUP, TK_EXVOL_FB_FORCE, TK_EXVOL, TK_EXVOL_EXT, TK_EXVOL_TAIL, TK_BODY_HEAD, TK_GATHER_MX,
     // sections of the energy / force finalizers (thread 0's view): partial
     // loads, block reduction, the CG step logic and the state store
     TK_SEC_FE_LOAD, TK_SEC_FE_REDUCE, TK_SEC_FE_TAIL, TK_SEC_FF_LOAD, TK_SEC_FF_REDUCE, TK_SEC_FF_TAIL,
-    TK_TAIL_COOP,
 };
 
 #if defined(__CUDACC__) && defined(MECH_TRACE)
@@ -312,15 +317,12 @@ struct Lanes {
     cudaEvent_t fork, join, join2;
 };
 template <typename Real> int launch_energy(const DevNet<Real>& n, int want, int trial, const Lanes& L);
-// coop_grid > 0 (mixed engine, one replica): the gather, both finalizers, the
-// direction update and the reset run as one cooperative launch of that many
-// blocks (k_tail_coop) instead of launch_forces' gather and finalizer plus
-// launch_direction and launch_reset
-template <typename Real> int launch_forces(const DevNet<Real>& n, int want, const Lanes& L, int coop_grid = 0);
-// blocks of the cooperative iteration tail on `device` (all resident at once)
-int coop_tail_grid(int device);
-template <typename Real> int launch_direction(const DevNet<Real>& n, cudaStream_t s);
-template <typename Real> int launch_reset(const DevNet<Real>& n, cudaStream_t s);
+template <typename Real> int launch_forces(const DevNet<Real>& n, int want, const Lanes& L);
+// An empty kernel at the head of an unrolled graph: the first pass's lanes fork
+// from it.  As roots of a graph launched behind another one, the filament kernel
+// on the main lane starts ~25 us before the side lanes and holds every SM (a
+// pass of 82 us instead of 42 on 1M cylinders).
+int launch_graph_head(cudaStream_t s);
 // head of a body of the minimizer's conditional graph: sets the phase
 // conditions, counts the body and decides whether the loop continues
 template <typename Real> int launch_body_head(const DevNet<Real>& n, cudaStream_t s);
@@ -330,7 +332,7 @@ template <typename Real> int launch_backup_restore(const DevNet<Real>& n, cudaSt
 // 0 filament energy, 1 filament force, 2 bond/boundary energy, 3 bond/boundary force
 template <typename Real> int launch_part(const DevNet<Real>& n, int which, cudaStream_t s);
 // blocks of the mixed engine's persistent filament kernels on `device`
-// (which: 0 energy, 1 force, 2 direction), at most per_sm per SM (0: no cap)
+// (which: 0 energy, 1 force), at most per_sm per SM (0: no cap)
 int persistent_blocks(int device, int which, int per_sm);
 
 // Records the text mech_last_error returns on this thread; returns `code`.

@@ -24,11 +24,10 @@ import numpy as np
 # kernel ids, in the order of mech_internal.cuh's TraceKernel
 NAMES = {
     1: "fil_energy", 2: "fil_force", 3: "gather", 4: "fin_force", 5: "fin_energy", 6: "fil_energy_bulk",
-    7: "fil_force_bulk", 8: "direction_mx", 9: "bond", 10: "direction", 11: "fin_direction", 12: "reset",
-    13: "recover_maxabs", 14: "recover_move", 15: "backup", 16: "exvol_fb_force", 17: "exvol", 18: "exvol_ext",
+    7: "fil_force_bulk", 9: "bond", 13: "recover_maxabs", 14: "recover_move", 15: "backup", 16: "exvol_fb_force", 17: "exvol", 18: "exvol_ext",
     19: "exvol_tail", 20: "body_head", 21: "gather_mx",
     22: "fin_energy: loads", 23: "fin_energy: reduce", 24: "fin_energy: step", 25: "fin_force: loads",
-    26: "fin_force: reduce", 27: "fin_force: step", 28: "tail_coop",
+    26: "fin_force: reduce", 27: "fin_force: step",
 }
 SECTIONS = set(range(22, 28))
 
