@@ -88,6 +88,8 @@ __device__ __forceinline__ double record_energies(CGState& S, const double* e) {
 // phase it selects on: on this GPU every dependent round trip to L2 (partial
 // slots written by the other die's SMs) costs about a microsecond, and a
 // finalizer is a chain of them on the minimizer's critical path.
+constexpr int kFinSums = 16;   // sums of the energy finalizer: two trials' six fields and d . F, to a power of two
+
 template <typename Real>
 __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const RepTiles& rt, CGState& S, double* sh) {
     const int stride = sizeof(Real) == 4 ? n.ptiles[0] : 1;
@@ -104,7 +106,7 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
         // mixed: (hi, lo) pair slots summed compensated in single precision;
         // the doubles are formed in warp 0 only.  acc[0, 6): the (first) trial,
         // acc[6, 12): the second trial, acc[12]: d . F of a new direction.
-        FF acc[2 * MECH_NUM_FF + 1];
+        FF acc[kFinSums];
         // each sparse kind's first slot of this thread, loaded with the first filament slots
         float2 sp0[K_NUM_SPARSE], sp1[K_NUM_SPARSE];
 #pragma unroll
@@ -142,23 +144,12 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
         }
         MECH_TRACE_SECTION(n, TK_SEC_FE_LOAD, ts_load);
         MECH_TRACE_STAMP(ts_red);
-        block_reduce_ff<2 * MECH_NUM_FF + 1, 0>(acc, nullptr, reinterpret_cast<float*>(sh));
+        const FF sum = block_pair_sums<kFinSums>(acc, reinterpret_cast<float*>(sh));
         MECH_TRACE_SECTION(n, TK_SEC_FE_REDUCE, ts_red);
         if (threadIdx.x >= 32) return;
         // hi + lo in double, one pair per lane of warp 0: an FP64 warp
-        // instruction costs the same with 1 or 12 active lanes, so the
-        // conversions take 3 warp instructions instead of 36 in thread 0
-        const int lane = threadIdx.x;
-        float ph = 0.f, pl = 0.f;
-#pragma unroll
-        for (int k = 0; k < 2 * MECH_NUM_FF + 1; ++k) {
-            const float h = __shfl_sync(0xffffffffu, acc[k].h, 0), l = __shfl_sync(0xffffffffu, acc[k].l, 0);
-            if (lane == k) {
-                ph = h;
-                pl = l;
-            }
-        }
-        const double v = (double)ph + (double)pl;
+        // instruction costs the same with 1 or 13 active lanes
+        const double v = (double)sum.h + (double)sum.l;
 #pragma unroll
         for (int k = 0; k < MECH_NUM_FF; ++k) {
             e[k] = __shfl_sync(0xffffffffu, v, k);
@@ -168,7 +159,7 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
         if (threadIdx.x != 0) return;
     } else {
         // every thread issues its loads back to back, then sums in a fixed order
-        double acc[MECH_NUM_FF + 1] = {0, 0, 0, 0, 0, 0, 0};   // last: d . F of a new direction
+        double acc[8] = {};   // the six fields, d . F of a new direction
 #pragma unroll 8
         for (int k = threadIdx.x; k < nslot; k += blockDim.x) {
             const int i = run_slot(rt.fil_begin, stride, k);
@@ -183,13 +174,12 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
             for (int i = rt.sp_begin[k] + threadIdx.x; i < rt.sp_end[k]; i += blockDim.x)
                 acc[ffk[k]] += __ldcg(n.part_sp + i);
         }
+        const double v = block_sums<8>(acc, sh);
+        if (threadIdx.x >= 32) return;
 #pragma unroll
-        for (int k = 0; k <= MECH_NUM_FF; ++k) acc[k] = warp_sum(acc[k]);
-        const int ops[MECH_NUM_FF + 1] = {0, 0, 0, 0, 0, 0, 0};
-        block_combine<MECH_NUM_FF + 1>(acc, ops, sh);
+        for (int k = 0; k < MECH_NUM_FF; ++k) e[k] = __shfl_sync(0xffffffffu, v, k);
+        slope = __shfl_sync(0xffffffffu, v, MECH_NUM_FF);
         if (threadIdx.x != 0) return;
-        for (int k = 0; k < MECH_NUM_FF; ++k) e[k] = acc[k];
-        slope = acc[MECH_NUM_FF];
     }
     MECH_TRACE_STAMP(ts_tail);
     const double lam = S.lambda;   // the (first) trial's step, before the line search moves it
@@ -288,7 +278,7 @@ template <typename Real>
 __device__ void finalize_force(const DevNet<Real>& n, int r, const RepTiles& rt, CGState& S, double* sh) {
     // k_force_gather writes one slot per tile, k_force_gather_mx one per run of
     // a replica's tiles in a block
-    const int stride = sizeof(Real) == 4 ? kGatherTiles : 1;
+    const int stride = sizeof(Real) == 4 ? n.gtiles : 1;
     const int nslot = run_slots(rt.fil_begin, rt.fil_end, stride);
     double mx, ff, ffp;
     MECH_TRACE_STAMP(ts_load);

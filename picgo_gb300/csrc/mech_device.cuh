@@ -6,8 +6,14 @@
 
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stddef.h>
 
 #include "mech_internal.cuh"
+
+static_assert(offsetof(mech::CGState, active) == 4 && offsetof(mech::CGState, fbuf) == 12 &&
+                  offsetof(mech::CGState, dbuf) == 16 && offsetof(mech::CGState, dual) == 28 &&
+                  offsetof(mech::CGState, lambda) == 32 && offsetof(mech::CGState, beta) == 40,
+              "lane_state reads the head of CGState as three vectors");
 
 namespace mech {
 
@@ -82,12 +88,69 @@ __device__ __forceinline__ void block_combine(double (&w)[N], const int (&op)[N]
     }
 }
 
-// Deterministic sum of part[i * stride + off] for i in [b, e), whole block; result in thread 0.
-__device__ __forceinline__ double sum_slots(const double* part, int stride, int off, int b, int e, double* sh) {
-    double acc = 0.0;
-    for (int i = b + threadIdx.x; i < e; i += blockDim.x) acc += __ldcg(part + (size_t)i * stride + off);
-    return block_sum(acc, sh);
+// Sums of N values (a power of two) over each warp and then the block: the
+// first steps of the trees halve the number of values a lane carries, so N
+// trees take N + 3 additions (N = 4: 6) where one after another they take 5 N.
+// Thread t < N gets value t.  A value's tree has the shape of block_sum's
+// whatever its place among the N: same bits, and a tile's sums do not depend on
+// the tiles it shares a block with.  `sh` holds N * kBlock / 32 doubles.
+template <int N>
+__device__ __forceinline__ double block_sums(double (&v)[N], double* sh) {
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int idx = 0, o = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (l & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const double keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+        if (up) idx += h;
+    }
+#pragma unroll
+    for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    __syncthreads();
+    if ((l & (32 / N - 1)) == 0) sh[w * N + idx] = v[0];
+    __syncthreads();
+    double a[kBlock / 32] = {};
+    if (threadIdx.x < N) {
+#pragma unroll
+        for (int k = 0; k < kBlock / 32; ++k) a[k] = sh[k * N + threadIdx.x];
+#pragma unroll
+        for (int h = kBlock / 64; h >= 1; h >>= 1)
+#pragma unroll
+            for (int k = 0; k < h; ++k) a[k] += a[k + h];
+    }
+    return a[0];
 }
+// the same for maxima of N unsigned values
+template <int N>
+__device__ __forceinline__ unsigned long long block_maxima(unsigned long long (&v)[N], unsigned long long* sh) {
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int idx = 0, o = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (l & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const unsigned long long keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
+            v[k] = max(keep, __shfl_xor_sync(0xffffffffu, send, o));
+        }
+        if (up) idx += h;
+    }
+#pragma unroll
+    for (; o >= 1; o >>= 1) v[0] = max(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
+    __syncthreads();
+    if ((l & (32 / N - 1)) == 0) sh[w * N + idx] = v[0];
+    __syncthreads();
+    unsigned long long a = 0;
+    if (threadIdx.x < N)
+        for (int k = 0; k < kBlock / 32; ++k) a = max(a, sh[k * N + threadIdx.x]);
+    return a;
+}
+
+// Maximum of part[i * stride + off] for i in [b, e), whole block; result in thread 0.
 __device__ __forceinline__ double max_slots(const double* part, int stride, int off, int b, int e, double* sh) {
     double acc = 0.0;
     for (int i = b + threadIdx.x; i < e; i += blockDim.x) acc = fmax(acc, __ldcg(part + (size_t)i * stride + off));
@@ -275,14 +338,41 @@ struct Direction {
     Real* out;      // where the filament kernel stores a new direction
     Real beta;
 };
+// What an evaluation kernel needs of a replica's state, read by every thread
+// for itself (three broadcast loads issued together, no barrier).
 template <typename Real>
-__device__ __forceinline__ Direction<Real> direction_of(const DevNet<Real>& n, const CGState& S) {
+struct LaneState {
+    bool go;         // selected by the launch (replica_selected)
+    int xb, fb, dbuf, dIsF, dPending, dual;
+    double lambda;
+    Real lam, beta;
+};
+template <typename Real>
+__device__ __forceinline__ LaneState<Real> lane_state(const DevNet<Real>& n, int r, int want) {
+    const int4* q = reinterpret_cast<const int4*>(n.st + r);
+    const int4 a = q[0], b = q[1];
+    const double2 c = reinterpret_cast<const double2*>(q)[2];
+    LaneState<Real> s;
+    s.go = want < 0 ? a.y != 0 : a.x == want;
+    s.xb = a.z;
+    s.fb = a.w;
+    s.dbuf = b.x;
+    s.dIsF = b.y;
+    s.dPending = b.z;
+    s.dual = b.w;
+    s.lambda = c.x;
+    s.lam = (Real)c.x;
+    s.beta = (Real)c.y;
+    return s;
+}
+template <typename Real>
+__device__ __forceinline__ Direction<Real> direction_of(const DevNet<Real>& n, const LaneState<Real>& S) {
     Direction<Real> D;
-    const int fd = S.dPending ? S.fbuf ^ 1 : S.fbuf;   // the forces that are the direction
+    const int fd = S.dPending ? S.fb ^ 1 : S.fb;   // the forces that are the direction
     D.d = S.dIsF ? n.f[fd] : n.d[S.dbuf];
-    D.F = S.dPending ? n.f[S.fbuf] : nullptr;
+    D.F = S.dPending ? n.f[S.fb] : nullptr;
     D.out = n.d[S.dbuf ^ 1];
-    D.beta = (Real)S.beta;
+    D.beta = S.beta;
     return D;
 }
 __device__ __forceinline__ float new_direction(float F, float beta, float d) { return fmaf(beta, d, F); }
@@ -393,6 +483,55 @@ __device__ __forceinline__ void block_reduce_ff(FF (&a)[N], float* m, float* sh)
 template <int N, int M>
 __device__ __forceinline__ void block_reduce_pairs(FF (&a)[N], float (&m)[M], float* sh) {
     block_reduce_ff<N, M>(a, m, sh);
+}
+
+// Sums of N compensated pairs (a power of two, at most 32) over the block with
+// the trees of block_reduce_ff, packed as in block_sums: N pair additions per
+// warp where N trees take 5 N.  Lane t < N of warp 0 gets pair t.  `sh` holds
+// 2 N kBlock / 32 floats.
+__device__ __forceinline__ void add_pairs(FF& a, float h, float l) {
+    float t, te;
+    two_sum(a.h, h, t, te);
+    te = __fadd_rn(te, __fadd_rn(a.l, l));
+    fast_two_sum(t, te, a.h, a.l);
+}
+template <int N>
+__device__ __forceinline__ FF block_pair_sums(FF (&a)[N], float* sh) {
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int idx = 0, o = 16;
+#pragma unroll
+    for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (l & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            FF keep = up ? a[k + h] : a[k];
+            const FF send = up ? a[k] : a[k + h];
+            add_pairs(keep, __shfl_xor_sync(0xffffffffu, send.h, o), __shfl_xor_sync(0xffffffffu, send.l, o));
+            a[k] = keep;
+        }
+        if (up) idx += h;
+    }
+#pragma unroll
+    for (; o >= 1; o >>= 1)
+        add_pairs(a[0], __shfl_xor_sync(0xffffffffu, a[0].h, o), __shfl_xor_sync(0xffffffffu, a[0].l, o));
+    if ((l & (32 / N - 1)) == 0) {
+        sh[2 * (w * N + idx)] = a[0].h;
+        sh[2 * (w * N + idx) + 1] = a[0].l;
+    }
+    __syncthreads();
+    FF r[kBlock / 32];
+    if (threadIdx.x < N) {
+#pragma unroll
+        for (int k = 0; k < kBlock / 32; ++k) {
+            r[k].h = sh[2 * (k * N + threadIdx.x)];
+            r[k].l = sh[2 * (k * N + threadIdx.x) + 1];
+        }
+#pragma unroll
+        for (int h = kBlock / 64; h >= 1; h >>= 1)
+#pragma unroll
+            for (int k = 0; k < h; ++k) add_pairs(r[k], r[k + h].h, r[k + h].l);
+    }
+    return r[0];
 }
 
 // Mixed-engine partial slots: a compensated (hi, lo) float pair stored in the

@@ -113,7 +113,7 @@ __device__ void fb_energy_blocks(const DevNet<Real>& n, int blk, int nblk, doubl
         // positions of this evaluation: the entry records the trial lambda (0: plain evaluation)
         const double lam = __longlong_as_double(((const long long*)n.ev_fb_energy)[kExvolFallbackCap + k]);
         const bool tr = lam != 0.0;
-        const Direction<Real> dir = direction_of(n, S);
+        const Direction<Real> dir = direction_of(n, lane_state(n, n.ev_fb_list[2 * k], -1));
         double c1[3], c2[3], c3[3], c4[3];
         to_double(bead_at(n.x[S.xbuf], dir, bs.x, tr, (Real)lam), c1);
         to_double(bead_at(n.x[S.xbuf], dir, bs.y, tr, (Real)lam), c2);
@@ -501,27 +501,20 @@ template <typename Real>
 __global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, int trial, int force, int tile_off,
                                                     int unsplit) {
     MECH_TRACE_KERNEL(n, TK_EXVOL);
-    __shared__ int s_go, s_xb;
-    __shared__ double s_lam;
-    __shared__ Direction<Real> s_dir;
     __shared__ SplitShared s;
     const int sb = (int)blockIdx.x - 2 * unsplit;
-    const Tile t = n.stile[tile_off + (sb < 0 ? (int)blockIdx.x >> 1 : unsplit + (sb >> 3))];
+    int kind;
+    const Tile t = sparse_tile(n, tile_off + (sb < 0 ? (int)blockIdx.x >> 1 : unsplit + (sb >> 3)), &kind);
     const int begin = t.begin + (sb < 0 ? 128 * ((int)blockIdx.x & 1) : 32 * (sb & 7));
     if (begin >= t.end) return;
-    if (threadIdx.x == 0) {
-        const CGState& S = n.st[t.replica];
-        s_go = want < 0 ? (S.active != 0) : (S.phase == want);
-        s_xb = S.xbuf;
-        s_lam = S.lambda;
-        s_dir = direction_of(n, S);
-    }
-    __syncthreads();
-    if (!s_go) return;
-    const Real* X = n.x[s_xb];
+    const LaneState<Real> ls = lane_state(n, t.replica, want);
+    if (!ls.go) return;
+    const Direction<Real> dir = direction_of(n, ls);
+    const Real* X = n.x[ls.xb];
+    const double lam = ls.lambda;
     const bool tr = trial != 0;
     if (sb >= 0) {
-        exvol_split(n, t.replica, X, s_dir, tr, s_lam, force, begin, t.end, s);
+        exvol_split(n, t.replica, X, dir, tr, lam, force, begin, t.end, s);
         return;
     }
     const int i = begin + threadIdx.x;
@@ -529,14 +522,14 @@ __global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, in
     const int4 bs = n.ev_bead[i];
     const double kRep = (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i];
     double c1[3], c2[3], c3[3], c4[3];
-    to_double(bead_at(X, s_dir, bs.x, tr, (Real)s_lam), c1);
-    to_double(bead_at(X, s_dir, bs.y, tr, (Real)s_lam), c2);
-    to_double(bead_at(X, s_dir, bs.z, tr, (Real)s_lam), c3);
-    to_double(bead_at(X, s_dir, bs.w, tr, (Real)s_lam), c4);
+    to_double(bead_at(X, dir, bs.x, tr, (Real)lam), c1);
+    to_double(bead_at(X, dir, bs.y, tr, (Real)lam), c2);
+    to_double(bead_at(X, dir, bs.z, tr, (Real)lam), c3);
+    to_double(bead_at(X, dir, bs.w, tr, (Real)lam), c4);
     if (!force) {
         const double u = pair_energy_d(c1, c2, c3, c4, kRep);
         n.ev_energy[i] = u == u ? u : 0.0;
-        if (u != u) flag_fallback(n, t.replica, i, tr ? s_lam : 0.0);
+        if (u != u) flag_fallback(n, t.replica, i, tr ? lam : 0.0);
     } else {
         double out[4][3];
         const bool ok = pair_forces_d(c1, c2, c3, c4, kRep, out);
@@ -551,33 +544,23 @@ __global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, in
 template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int trial, int force, int tile_off) {
     MECH_TRACE_KERNEL(n, TK_EXVOL);
-    __shared__ int s_go, s_xb, s_dual;
-    __shared__ float s_lf;   // the step rounded once
-    __shared__ Direction<Real> s_dir;
-    const int ti = tile_off + blockIdx.x;
-    const Tile t = n.stile[ti];
+    int kind;
+    const Tile t = sparse_tile(n, tile_off + (int)blockIdx.x, &kind);
     const int r = t.replica;
-    if (threadIdx.x == 0) {
-        const CGState& S = n.st[r];
-        s_go = want < 0 ? (S.active != 0) : (S.phase == want);
-        s_xb = S.xbuf;
-        s_lf = (float)S.lambda;
-        s_dir = direction_of(n, S);
-        s_dual = S.dual;
-    }
-    __syncthreads();
-    if (!s_go) return;
-    const Real* X = n.x[s_xb];
+    const LaneState<Real> s = lane_state(n, r, want);
+    if (!s.go) return;
+    const Direction<Real> dir = direction_of(n, s);
+    const Real* X = n.x[s.xb];
     const bool tr = trial != 0;
     const int i = t.begin + threadIdx.x;
     const bool valid = i < t.end;
     float ef = 0.f;
     bool need64 = false, need64b = false;
     // a pass with a second trial also evaluates the energy at lambda / 2
-    const bool dual = !force && second_trial(trial, s_dual);
+    const bool dual = !force && second_trial(trial, s.dual);
     if (valid) {
         const int4 bs = n.ev_bead[i];
-        auto pos = [&](int b) -> Pos<float> { return bead_at(X, s_dir, b, tr, s_lf); };
+        auto pos = [&](int b) -> Pos<float> { return bead_at(X, dir, b, tr, s.lam); };
         const Pos<Real> p1 = pos(bs.x), p2 = pos(bs.y), p3 = pos(bs.z), p4 = pos(bs.w);
         if (!force) {
             // mixed engine: single precision unless the pair is ill-conditioned
@@ -585,9 +568,9 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
             ef = mixed_pair_energy(p1, p2, p3, p4, kRep, need64);
             store_pair(n.ev_energy + i, ef, 0.f);
             if (dual) {
-                const float lh = 0.5f * s_lf;
-                const float ef2 = mixed_pair_energy(bead_at(X, s_dir, bs.x, true, lh), bead_at(X, s_dir, bs.y, true, lh),
-                                                    bead_at(X, s_dir, bs.z, true, lh), bead_at(X, s_dir, bs.w, true, lh),
+                const float lh = 0.5f * s.lam;
+                const float ef2 = mixed_pair_energy(bead_at(X, dir, bs.x, true, lh), bead_at(X, dir, bs.y, true, lh),
+                                                    bead_at(X, dir, bs.z, true, lh), bead_at(X, dir, bs.w, true, lh),
                                                     kRep, need64b);
                 store_pair(n.ev_energy2 + i, ef2, 0.f);
             }
@@ -619,8 +602,8 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
                 if (!(fabsf(cop - 0.1f) >= 2e-3f)) {
                     need64 = true;
                 } else if (cop < 0.1f) {
-                    const float s = -0.01f / nn;
-                    const float dx = s * nx, dy = s * ny, dz = s * nz;   // c2 moves by +0.01 n / |n|
+                    const float push = -0.01f / nn;
+                    const float dx = push * nx, dy = push * ny, dz = push * nz;   // c2 moves by +0.01 n / |n|
                     v12[0] += dx; v12[1] += dy; v12[2] += dz;
                     v32[0] += dx; v32[1] += dy; v32[2] += dz;
                     v24[0] -= dx; v24[1] -= dy; v24[2] -= dz;
@@ -685,21 +668,22 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
         int r = 0, i = 0;
         bool second = false;   // the lambda / 2 trial of a two-trial pass
         double lam = 0.0;
+        LaneState<Real> ls{};
         if (valid) {
             r = n.ev_list[2 * k];
             i = n.ev_list[2 * k + 1];
             second = (i & kExtSecond) != 0;
             i &= ~kExtSecond;
-            lam = n.st[r].lambda;
+            ls = lane_state(n, r, -1);
+            lam = ls.lambda;
             if (second) lam *= 0.5;
         }
         // ---- positions: warp w converts bead w of every pair
         if (valid) {
-            const CGState& S = n.st[r];
             const int4 bs = n.ev_bead[i];
             const int bead = w == 0 ? bs.x : w == 1 ? bs.y : w == 2 ? bs.z : bs.w;
             double c[3];
-            to_double(bead_at(n.x[S.xbuf], direction_of(n, S), bead, trial != 0, (Real)lam), c);
+            to_double(bead_at(n.x[ls.xb], direction_of(n, ls), bead, trial != 0, (Real)lam), c);
             s_c[w][l][0] = c[0];
             s_c[w][l][1] = c[1];
             s_c[w][l][2] = c[2];
@@ -881,14 +865,15 @@ __global__ void __launch_bounds__(kBlock) k_exvol_energy_tail(DevNet<Real> n, in
         fb_energy_blocks(n, blockIdx.x, kFbEnergyBlocks, sh);
     } else {
         const int ti = tile_off + (int)blockIdx.x - kFbEnergyBlocks;
-        const Tile t = n.stile[ti];
-        const CGState& S = n.st[t.replica];
-        const bool go = want < 0 ? (S.active != 0) : (S.phase == want);
+        int kind;
+        const Tile t = sparse_tile(n, ti, &kind);
+        const LaneState<Real> s = lane_state(n, t.replica, want);
+        const bool go = s.go;
         if constexpr (sizeof(Real) == 4) {
             if (go) {   // block-uniform
                 // per-pair energies as (hi, lo) pairs, summed compensated in single precision
                 const int i = t.begin + threadIdx.x;
-                if (second_trial(trial, S.dual)) {   // both trials of the pass
+                if (second_trial(trial, s.dual)) {   // both trials of the pass
                     FF a[2];
                     if (i < t.end) {
                         add_pair(a[0], load_pair(n.ev_energy + i));

@@ -141,68 +141,6 @@ __global__ void __launch_bounds__(kBlock) k_body_head(DevNet<Real> n) {
 // ends, comparisons are made on the bits of the numbers, and the sums of a warp
 // share the additions of their trees.
 // ---------------------------------------------------------------------------
-// Sums of N values (a power of two) over each warp and then the block: the
-// first steps of the trees halve the number of values a lane carries, so N
-// trees take N + 3 additions (N = 4: 6) where one after another they take 5 N.
-// Thread t < N gets value t.  A value's tree has the shape of block_sum's
-// whatever its place among the N: same bits, and a tile's sums do not depend on
-// the tiles it shares a block with.  `sh` holds N * kBlock / 32 doubles.
-template <int N>
-__device__ __forceinline__ double block_sums(double (&v)[N], double* sh) {
-    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int idx = 0, o = 16;
-#pragma unroll
-    for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
-        const bool up = (l & o) != 0;
-#pragma unroll
-        for (int k = 0; k < h; ++k) {
-            const double keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
-            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-        if (up) idx += h;
-    }
-#pragma unroll
-    for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-    __syncthreads();
-    if ((l & (32 / N - 1)) == 0) sh[w * N + idx] = v[0];
-    __syncthreads();
-    double a[kBlock / 32] = {};
-    if (threadIdx.x < N) {
-#pragma unroll
-        for (int k = 0; k < kBlock / 32; ++k) a[k] = sh[k * N + threadIdx.x];
-#pragma unroll
-        for (int h = kBlock / 64; h >= 1; h >>= 1)
-#pragma unroll
-            for (int k = 0; k < h; ++k) a[k] += a[k + h];
-    }
-    return a[0];
-}
-// the same for maxima of N unsigned values
-template <int N>
-__device__ __forceinline__ unsigned long long block_maxima(unsigned long long (&v)[N], unsigned long long* sh) {
-    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int idx = 0, o = 16;
-#pragma unroll
-    for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
-        const bool up = (l & o) != 0;
-#pragma unroll
-        for (int k = 0; k < h; ++k) {
-            const unsigned long long keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
-            v[k] = max(keep, __shfl_xor_sync(0xffffffffu, send, o));
-        }
-        if (up) idx += h;
-    }
-#pragma unroll
-    for (; o >= 1; o >>= 1) v[0] = max(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
-    __syncthreads();
-    if ((l & (32 / N - 1)) == 0) sh[w * N + idx] = v[0];
-    __syncthreads();
-    unsigned long long a = 0;
-    if (threadIdx.x < N)
-        for (int k = 0; k < kBlock / 32; ++k) a = max(a, sh[k * N + threadIdx.x]);
-    return a;
-}
-
 __device__ __forceinline__ unsigned long long abs_bits(double x) {
     return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
 }
@@ -217,22 +155,6 @@ __device__ __forceinline__ double clamp_unit(double x) {
     return a > 0x3ff0000000000000ULL && a <= 0x7ff0000000000000ULL ? copysign(1.0, x) : x;
 }
 
-// What a block of the FP64 filament kernels needs of its tile's replica.
-struct FilTile {
-    int begin, end, go, xb, fb, backup;
-    double lam;
-    Direction<double> dir;
-};
-__device__ __forceinline__ void load_fil_tile(const DevNet<double>& n, int want, FilTile* s) {
-    if (threadIdx.x == 0) {
-        const Tile t = n.ftile[blockIdx.x];
-        const CGState& S = n.st[t.replica];
-        *s = FilTile{t.begin, t.end, replica_selected(S, want), S.xbuf, S.fbuf, S.backupPending, S.lambda,
-                     direction_of(n, S)};
-    }
-    __syncthreads();
-}
-
 // Stretching + bending energy of the tile's own cylinders and triples.  1M
 // beads: 86 us, against 121 us (66 FP64 instructions per bead) with each length
 // formed two or three times and a tree per sum.
@@ -243,13 +165,15 @@ __global__ void __launch_bounds__(kBlock) k_fil_energy(DevNet<double> n, int wan
     __shared__ double rs[4][kFilTile + 1];    // cylinders begin - 1 .. end - 1: vector, length
     __shared__ double dF[kFilTile];           // d . F of each bead (a new direction)
     __shared__ double sh[4 * kBlock / 32];
-    __shared__ FilTile t;
     const bool tr = trial != 0;
-    load_fil_tile(n, want, &t);
-    if (!t.go) return;
+    const Tile t = fil_tile(n, blockIdx.x);
+    const LaneState<double> s = lane_state(n, t.replica, want);
+    if (!s.go) return;
+    const Direction<double> dir = direction_of(n, s);
     const int T = t.end - t.begin;
-    const double* X = n.x[t.xb];
-    const bool pend = tr && t.dir.F;     // this pass forms the direction
+    const double* X = n.x[s.xb];
+    const bool pend = tr && dir.F;     // this pass forms the direction
+    const bool backup = pend && n.st[t.replica].backupPending;
     double e[4] = {0.0, 0.0, 0.0, 0.0};   // stretching, bending, d . F
     for (int i = threadIdx.x; i < T + 2; i += blockDim.x) {
         const int b = t.begin - 1 + i;
@@ -258,18 +182,18 @@ __global__ void __launch_bounds__(kBlock) k_fil_energy(DevNet<double> n, int wan
         if (tr) {
             const bool own = i >= 1 && i <= T;
             double d[3];
-            direction_at(t.dir, b, d);
+            direction_at(dir, b, d);
             if (pend && own) {
-                double* o = t.dir.out + 3 * (size_t)b;
-                const double* F = t.dir.F + 3 * (size_t)b;
+                double* o = dir.out + 3 * (size_t)b;
+                const double* F = dir.F + 3 * (size_t)b;
                 o[0] = d[0];
                 o[1] = d[1];
                 o[2] = d[2];
                 dF[i - 1] = bead_dot(d[0], d[1], d[2], F[0], F[1], F[2]);
-                if (t.backup) store_pos(n.xbest, b, p);
+                if (backup) store_pos(n.xbest, b, p);
             }
-            p = moved(p, d, t.lam);
-            if (own) store_pos(n.x[t.xb ^ 1], b, p);   // materialize the owned trial position
+            p = moved(p, d, s.lambda);
+            if (own) store_pos(n.x[s.xb ^ 1], b, p);   // materialize the owned trial position
         }
         xs[0][i] = p.x[0];
         xs[1][i] = p.x[1];
@@ -331,11 +255,11 @@ __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want
     __shared__ double rs[3][kFilTile + 3], Ls[kFilTile + 3];        // cylinders begin - 2 .. end: vector, L^2
     __shared__ double fs[3][kFilTile + 3];                          // their stretching forces on the second bead
     __shared__ double f1[3][kFilTile + 2], f2[3][kFilTile + 2];     // triples on begin - 1 .. end
-    __shared__ FilTile t;
-    load_fil_tile(n, want, &t);
-    if (!t.go) return;
+    const Tile t = fil_tile(n, blockIdx.x);
+    const LaneState<double> s = lane_state(n, t.replica, want);
+    if (!s.go) return;
     const int T = t.end - t.begin;
-    const double* X = n.x[t.xb];
+    const double* X = n.x[s.xb];
     for (int i = threadIdx.x; i < T + 4; i += blockDim.x) {
         const int b = t.begin - 2 + i;
         if (b < 0 || b >= n.nb) continue;
@@ -397,7 +321,7 @@ __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want
     __syncthreads();
     const int i = threadIdx.x;
     if (i < T) {
-        double* Fo = n.f[t.fb ^ 1] + 3 * (size_t)(t.begin + i);
+        double* Fo = n.f[s.fb ^ 1] + 3 * (size_t)(t.begin + i);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             double v = fs[q][i + 1];
@@ -421,6 +345,7 @@ __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want
 // is formed on the bits.  The mixed engine's
 // version is k_force_gather_mx below.
 // ---------------------------------------------------------------------------
+constexpr int kGatherAhead = 4;   // contributions of a bead loaded together
 template <typename Real>
 __device__ __forceinline__ void gather_force(const DevNet<Real>& n, int b, int fb, Real F[3], Real& ff, Real& ffp) {
     Real* Fo = n.f[fb ^ 1] + 3 * (size_t)b;
@@ -430,7 +355,20 @@ __device__ __forceinline__ void gather_force(const DevNet<Real>& n, int b, int f
     F[2] = Fo[2];
     const Real p0 = Fp[0], p1 = Fp[1], p2 = Fp[2];
     const int c0 = n.csr_off[b], c1 = n.csr_off[b + 1];
-    for (int c = c0; c < c1; ++c) {
+    // the first contributions loaded together: one after another, each costs a
+    // round trip to L2
+    Real g[kGatherAhead][3];
+#pragma unroll
+    for (int k = 0; k < kGatherAhead; ++k)
+        if (c0 + k < c1)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) g[k][q] = n.contrib[3 * (size_t)(c0 + k) + q];
+#pragma unroll
+    for (int k = 0; k < kGatherAhead; ++k)
+        if (c0 + k < c1)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) F[q] += g[k][q];
+    for (int c = c0 + kGatherAhead; c < c1; ++c) {
         F[0] += n.contrib[3 * (size_t)c];
         F[1] += n.contrib[3 * (size_t)c + 1];
         F[2] += n.contrib[3 * (size_t)c + 2];
@@ -456,103 +394,79 @@ __device__ __forceinline__ void gather_bead(const DevNet<double>& n, int b, int 
     mx = min(max(max(abs_bits(F[0]), abs_bits(F[1])), abs_bits(F[2])), 0x7ff0000000000000ULL);
 }
 
-// What a block of kGatherTiles tiles needs of them.
-struct GatherTiles {
-    int go[kGatherTiles], fb[kGatherTiles], rep[kGatherTiles];
-};
-__device__ __forceinline__ void load_gather_tiles(const DevNet<double>& n, int t0, int want, GatherTiles& g) {
-    if (threadIdx.x < kGatherTiles) {
-        const int ti = t0 + threadIdx.x;
-        int go = 0, fb = 0, rep = -1;
-        if (ti < n.n_ftiles) {
-            rep = n.ftile[ti].replica;
-            const CGState& S = n.st[rep];
-            go = replica_selected(S, want);
-            fb = S.fbuf;
-        }
-        g.go[threadIdx.x] = go;
-        g.fb[threadIdx.x] = fb;
-        g.rep[threadIdx.x] = rep;
-    }
-    __syncthreads();
-}
-
+// NT tiles per block (DevNet::gtiles)
+template <int NT>
 __global__ void __launch_bounds__(kBlock) k_force_gather(DevNet<double> n, int want) {
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_GATHER);
-    __shared__ double sh[2 * kGatherTiles * kBlock / 32];
-    __shared__ unsigned long long s_mx[kGatherTiles * kBlock / 32];
-    __shared__ GatherTiles g;
-    const int t0 = blockIdx.x * kGatherTiles;
-    load_gather_tiles(n, t0, want, g);
-    unsigned long long mx[kGatherTiles];
-    double v[2 * kGatherTiles];   // F.F of each tile, then F.Fprev
-    int any = 0;
+    __shared__ double sh[2 * NT * kBlock / 32];
+    __shared__ unsigned long long s_mx[NT * kBlock / 32];
+    const int t0 = blockIdx.x * NT;
+    unsigned long long mx[NT];
+    double v[2 * NT];   // F.F of each tile, then F.Fprev
+    unsigned go = 0;
 #pragma unroll
-    for (int j = 0; j < kGatherTiles; ++j) {
+    for (int j = 0; j < NT; ++j) {
         mx[j] = 0;
-        v[j] = v[kGatherTiles + j] = 0.0;
-        if (!g.go[j]) continue;
-        any = 1;
-        const Tile t = n.ftile[t0 + j];
+        v[j] = v[NT + j] = 0.0;
+        if (t0 + j >= n.n_ftiles) continue;
+        const Tile t = fil_tile(n, t0 + j);
+        const LaneState<double> s = lane_state(n, t.replica, want);
+        if (!s.go) continue;
+        go |= 1u << j;
         const int b = t.begin + threadIdx.x;
-        if (b < t.end) gather_bead(n, b, g.fb[j], mx[j], v[j], v[kGatherTiles + j]);
+        if (b < t.end) gather_bead(n, b, s.fb, mx[j], v[j], v[NT + j]);
     }
-    if (!any) return;   // block-uniform
-    const unsigned long long m = block_maxima<kGatherTiles>(mx, s_mx);
-    const double a = block_sums<2 * kGatherTiles>(v, sh);
-    if (threadIdx.x < 2 * kGatherTiles) {
-        const int j = threadIdx.x % kGatherTiles;
-        if (g.go[j]) {
+    if (!go) return;   // block-uniform
+    const unsigned long long m = block_maxima<NT>(mx, s_mx);
+    const double a = block_sums<2 * NT>(v, sh);
+    if (threadIdx.x < 2 * NT) {
+        const int j = threadIdx.x % NT;
+        if (go >> j & 1) {
             double* slot = n.part_fil + 4 * (size_t)(t0 + j);
-            if (threadIdx.x < kGatherTiles) slot[0] = __longlong_as_double((long long)m);
-            slot[1 + threadIdx.x / kGatherTiles] = a;
+            if (threadIdx.x < NT) slot[0] = __longlong_as_double((long long)m);
+            slot[1 + threadIdx.x / NT] = a;
         }
     }
 }
 
-// Mixed engine gather: 64 threads per tile, each taking 4 consecutive beads
-// whose force records (4 x 12 B) move as three 16-byte vectors, when the tile
-// starts on a multiple of 4 beads (always, unless a replica before it has a
-// bead count that is not; a partial group at the tile's end goes bead by
-// bead); otherwise 4 beads strided by 64.  The block's partials combine, in
-// warp order, the warps of each run of its tiles that belong to one replica,
-// into the slot of the run's first tile (run_slot with stride kGatherTiles),
-// so the force finalizer reads a quarter of the slots one per tile would take.
-struct GatherMxShared {
-    float sh[8][5];   // per warp: F.F (hi, lo), F.Fprev (hi, lo), max
-    int go[kGatherTiles], fb[kGatherTiles], rep[kGatherTiles];
-};
-
-// One gather unit (kGatherTiles consecutive tiles): the body of a
-// k_force_gather_mx block.
-__device__ void gather_mx_unit(const DevNet<float>& n, int want, int unit, GatherMxShared& g) {
+// Mixed engine gather: 64 threads per tile, n.gtiles tiles per block, each
+// thread taking 4 consecutive beads whose force records (4 x 12 B) move as three
+// 16-byte vectors and whose contributions, contiguous too, are loaded up to
+// kGatherAheadMx together, when the tile starts on a multiple of 4 beads (always,
+// unless a replica before it has a bead count that is not; a partial group at
+// the tile's end goes bead by bead); otherwise 4 beads strided by 64.  The
+// block's partials combine, in warp order, the warps of each run of its tiles
+// that belong to one replica, into the slot of the run's first tile (run_slot
+// with stride n.gtiles).
+constexpr int kGatherAheadMx = 8;
+__global__ void __launch_bounds__(kBlock) k_force_gather_mx(DevNet<float> n, int want) {
     static_assert(kFilTile == 256 && kBlock == 64 * kGatherTiles, "64 threads x 4 beads per tile");
-    float (&sh)[8][5] = g.sh;
-    int* s_go = g.go;
-    int* s_fb = g.fb;
-    int* s_rep = g.rep;
-    const int t0 = unit * kGatherTiles;
-    if (threadIdx.x < kGatherTiles) {
-        const int ti = t0 + threadIdx.x;
-        int go = 0, fb = 0, rep = -1;
-        if (ti < n.n_ftiles) {
-            rep = n.ftile[ti].replica;
-            const CGState& S = n.st[rep];
-            go = replica_selected(S, want);
-            fb = S.fbuf;
-        }
-        s_go[threadIdx.x] = go;
-        s_fb[threadIdx.x] = fb;
-        s_rep[threadIdx.x] = rep;
-    }
-    __syncthreads();
+    pdl_trigger();   // the next kernel of the main lane may be scheduled now
+    MECH_TRACE_KERNEL(n, TK_GATHER_MX);
+    __shared__ float sh[8][5];   // per warp: F.F (hi, lo), F.Fprev (hi, lo), max
+    __shared__ int s_go[kGatherTiles], s_rep[kGatherTiles];
+    const int nt = blockDim.x >> 6;   // tiles of this block
     const int j = threadIdx.x >> 6, tt = threadIdx.x & 63;
+    const int ti = blockIdx.x * nt + j;
+    Tile t{-1, 0, 0, 0};
+    bool go = false;
+    int fb = 0;
+    if (n.R == 1 && !lane_state(n, 0, want).go) return;
+    if (ti < n.n_ftiles) {
+        t = fil_tile(n, ti);
+        const LaneState<float> s = lane_state(n, t.replica, want);
+        go = s.go;
+        fb = s.fb;
+    }
+    if (tt == 0) {
+        s_go[j] = go;
+        s_rep[j] = t.replica;
+    }
+    const int t0 = blockIdx.x * nt;
     FF aff, affp;
     float mx = 0.f;
-    if (s_go[j]) {   // uniform over the tile's two warps
-        const Tile t = n.ftile[t0 + j];
-        const int fb = s_fb[j];
+    if (go) {   // uniform over the tile's two warps
         const int b0 = t.begin + 4 * tt;
         const bool vec_tile = (t.begin & 3) == 0;   // uniform over the tile
         if (vec_tile && b0 + 4 <= t.end) {
@@ -567,13 +481,30 @@ __device__ void gather_mx_unit(const DevNet<float>& n, int want, int unit, Gathe
             int off[5];
 #pragma unroll
             for (int q = 0; q < 5; ++q) off[q] = n.csr_off[b0 + q];
+            float g[kGatherAheadMx][3];
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                for (int c = off[k]; c < off[k + 1]; ++c) {
-                    F[3 * k] += n.contrib[3 * (size_t)c];
-                    F[3 * k + 1] += n.contrib[3 * (size_t)c + 1];
-                    F[3 * k + 2] += n.contrib[3 * (size_t)c + 2];
-                }
+            for (int m = 0; m < kGatherAheadMx; ++m)
+                if (off[0] + m < off[4])
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) g[m][q] = n.contrib[3 * (size_t)(off[0] + m) + q];
+#pragma unroll
+            for (int m = 0; m < kGatherAheadMx; ++m) {
+                const int c = off[0] + m;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (c >= off[k] && c < off[k + 1])
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) F[3 * k + q] += g[m][q];
+            }
+            if (off[4] - off[0] > kGatherAheadMx) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    for (int c = max(off[k], off[0] + kGatherAheadMx); c < off[k + 1]; ++c) {
+                        F[3 * k] += n.contrib[3 * (size_t)c];
+                        F[3 * k + 1] += n.contrib[3 * (size_t)c + 1];
+                        F[3 * k + 2] += n.contrib[3 * (size_t)c + 2];
+                    }
+            }
             reinterpret_cast<float4*>(Fo)[0] = make_float4(F[0], F[1], F[2], F[3]);
             reinterpret_cast<float4*>(Fo)[1] = make_float4(F[4], F[5], F[6], F[7]);
             reinterpret_cast<float4*>(Fo)[2] = make_float4(F[8], F[9], F[10], F[11]);
@@ -614,13 +545,13 @@ __device__ void gather_mx_unit(const DevNet<float>& n, int want, int unit, Gathe
     }
     __syncthreads();
     const int j0 = threadIdx.x;
-    if (j0 < kGatherTiles && s_go[j0] && (j0 == 0 || s_rep[j0 - 1] != s_rep[j0])) {
+    if (j0 < nt && s_go[j0] && (j0 == 0 || s_rep[j0 - 1] != s_rep[j0])) {
         // thread j0 starts a run: its tile and the following tiles of the same
         // replica, their warps' pairs added in order to compensated sums
         FF f1, f2;
         float m = 0.f;
-        for (int j = j0; j < kGatherTiles && s_rep[j] == s_rep[j0]; ++j)
-            for (int w = 2 * j; w < 2 * j + 2; ++w) {
+        for (int q = j0; q < nt && s_rep[q] == s_rep[j0]; ++q)
+            for (int w = 2 * q; w < 2 * q + 2; ++w) {
                 f1.add(sh[w][0]);
                 f1.add(sh[w][1]);
                 f2.add(sh[w][2]);
@@ -633,16 +564,9 @@ __device__ void gather_mx_unit(const DevNet<float>& n, int want, int unit, Gathe
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_force_gather_mx(DevNet<float> n, int want) {
-    pdl_trigger();   // the next kernel of the main lane may be scheduled now
-    MECH_TRACE_KERNEL(n, TK_GATHER_MX);
-    __shared__ GatherMxShared g;
-    gather_mx_unit(n, want, blockIdx.x, g);
-}
-
 // One block per replica: max |F|, the dots and the CG step logic after the gather.
 template <typename Real>
-__global__ void __launch_bounds__(kBlock) k_finalize_force(DevNet<Real> n, int want) {
+__global__ void __launch_bounds__(kBlock, 1) k_finalize_force(DevNet<Real> n, int want) {
     pdl_wait();      // the previous kernel of the main lane has finished
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_FIN_FORCE);
@@ -651,7 +575,7 @@ __global__ void __launch_bounds__(kBlock) k_finalize_force(DevNet<Real> n, int w
     const int r = blockIdx.x;
     CGState S;
     if (threadIdx.x == 0) S = n.st[r];   // issued together with the loads below
-    const RepTiles rt = n.rt[r];
+    const RepTiles rt = rep_tiles(n, r);
     if (replica_selected(n.st[r], want)) finalize_force(n, r, rt, S, sh);
     if (n.snap && threadIdx.x == 0) {   // what the host looks at after each graph
         if (S.phase == PH_DONE || S.phase >= PH_ERROR) n.snap[9 + r] = S.phase;
@@ -666,15 +590,15 @@ __global__ void __launch_bounds__(kBlock) k_finalize_force(DevNet<Real> n, int w
 // One block per replica: the energy reduction and the line-search step, after
 // every kernel of the evaluation has written its partial sums.
 template <typename Real>
-__global__ void __launch_bounds__(kBlock) k_finalize_energy(DevNet<Real> n, int want, int trial) {
+__global__ void __launch_bounds__(kBlock, 1) k_finalize_energy(DevNet<Real> n, int want, int trial) {
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_FIN_ENERGY);
-    __shared__ double sh[32 * (2 * MECH_NUM_FF + 1)];   // block_reduce_ff<13>: 32 * 26 floats
+    __shared__ double sh[kFinSums * kBlock / 32];   // block_pair_sums<16>: 16 pairs of floats per warp
     __shared__ int s_flag;
     const int r = blockIdx.x;
     CGState S;
     if (threadIdx.x == 0) S = n.st[r];   // issued together with the loads below
-    const RepTiles rt = n.rt[r];
+    const RepTiles rt = rep_tiles(n, r);
     if (replica_selected(n.st[r], want)) finalize_energy(n, r, trial, rt, S, sh);
     after_evaluation(n, kCondTrial, &s_flag);
 }
@@ -753,15 +677,18 @@ __device__ __forceinline__ StageRange stage_range(int tb, int te, int nb, int ha
 // tiles of it (its finalizer waits for every tile), so the copies stay valid.
 constexpr int kBulkMaxTiles = kFilBulkMaxTiles;
 
+__device__ __forceinline__ int4 descriptor(const Tile& t, const LaneState<float>& s, int backup) {
+    return make_int4(t.begin, t.end, t.replica,
+                     (s.go ? 1 : 0) | (s.xb << 1) | (s.fb << 3) | (s.dual ? 16 : 0) | (s.dPending << 5) |
+                         (s.dIsF << 6) | (s.dbuf << 7) | (backup << 8));
+}
 __device__ __forceinline__ void load_descriptors(const DevNet<float>& n, int t0, int nt, int want, int4* desc,
                                                  float2* step) {
     for (int k = threadIdx.x; k < nt; k += blockDim.x) {
-        const Tile t = n.ftile[t0 + k];
-        const CGState& S = n.st[t.replica];
-        desc[k] = make_int4(t.begin, t.end, t.replica,
-                            (replica_selected(S, want) ? 1 : 0) | (S.xbuf << 1) | (S.fbuf << 3) | (S.dual ? 16 : 0) |
-                                (S.dPending << 5) | (S.dIsF << 6) | (S.dbuf << 7) | (S.backupPending << 8));
-        step[k] = make_float2((float)S.lambda, (float)S.beta);
+        const Tile t = fil_tile(n, t0 + k);
+        const LaneState<float> s = lane_state(n, t.replica, want);
+        desc[k] = descriptor(t, s, n.st[t.replica].backupPending);
+        step[k] = make_float2(s.lam, s.beta);
     }
 }
 
@@ -805,6 +732,7 @@ __device__ void issue_energy_stage(const DevNet<float>& n, int4 t, bool tr, Ener
 // last tiles share a replica belongs to it alone.  The block then exits before
 // any barrier or descriptor setup.
 __device__ __forceinline__ bool idle_range(const DevNet<float>& n, int t0, int t1, int want, int* s_flag) {
+    if (n.R == 1) return t1 <= t0 || !lane_state(n, 0, want).go;   // the same in every thread
     if (threadIdx.x == 0) {
         int idle = t1 <= t0;
         if (!idle) {
@@ -1182,30 +1110,19 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
                                                      int ev_tiles) {
     MECH_TRACE_KERNEL(n, TK_BOND);
     __shared__ double sh[64];   // block_reduce_ff<2>: 32 * 4 floats
-    __shared__ int s_go, s_xb, s_dual;
-    __shared__ Real s_lam;                 // (mixed engine: the step rounded once)
-    __shared__ Direction<Real> s_dir;
     const int ti = blockIdx.x < n_lm_tiles ? blockIdx.x : blockIdx.x + ev_tiles;
-    const Tile t = n.stile[ti];
-    const int kind = n.stile_kind[ti];
-    const int r = t.replica;
-    if (threadIdx.x == 0) {
-        const CGState& S = n.st[r];
-        s_go = replica_selected(S, want);
-        s_xb = S.xbuf;
-        s_lam = (Real)S.lambda;
-        s_dir = direction_of(n, S);
-        s_dual = S.dual;
-    }
-    __syncthreads();
-    if (!s_go) return;
-    const Real* X = n.x[s_xb];
+    int kind;
+    const Tile t = sparse_tile(n, ti, &kind);
+    const LaneState<Real> s = lane_state(n, t.replica, want);
+    if (!s.go) return;
+    const Direction<Real> dir = direction_of(n, s);
+    const Real* X = n.x[s.xb];
     const bool tr = trial != 0;
     // a pass with a second trial also evaluates the energy at lambda / 2 (mixed engine)
-    const bool dual = sizeof(Real) == 4 && !force && second_trial(trial, s_dual);
-    auto pos = [&](int b) -> Pos<Real> { return bead_at(X, s_dir, b, tr, s_lam); };
-    const Real lh = (Real)0.5 * s_lam;
-    auto pos2 = [&](int b) -> Pos<Real> { return bead_at(X, s_dir, b, true, lh); };   // the second trial
+    const bool dual = sizeof(Real) == 4 && !force && second_trial(trial, s.dual);
+    auto pos = [&](int b) -> Pos<Real> { return bead_at(X, dir, b, tr, s.lam); };
+    const Real lh = (Real)0.5 * s.lam;
+    auto pos2 = [&](int b) -> Pos<Real> { return bead_at(X, dir, b, true, lh); };   // the second trial
     const int i = t.begin + threadIdx.x;
     Real e = 0, e2 = 0;
     if (i < t.end) {
@@ -1305,8 +1222,9 @@ __global__ void __launch_bounds__(kBlock) k_recover_maxabs(DevNet<Real> n) {
     const Tile t = n.ftile[blockIdx.x];
     const int r = t.replica;
     if (threadIdx.x == 0) {
-        s_go = n.st[r].phase == PH_RECOVER;
-        s_dir = direction_of(n, n.st[r]);
+        const LaneState<Real> s = lane_state(n, r, PH_RECOVER);
+        s_go = s.go;
+        s_dir = direction_of(n, s);
     }
     __syncthreads();
     if (!s_go) return;
@@ -1349,7 +1267,7 @@ __global__ void __launch_bounds__(kBlock) k_recover_move(DevNet<Real> n) {
         s_go = S.phase == PH_RECOVER_MOVE;
         s_xb = S.xbuf;
         s_step = (Real)S.lambda;
-        s_dir = direction_of(n, S);
+        s_dir = direction_of(n, lane_state(n, r, PH_RECOVER_MOVE));
     }
     __syncthreads();
     if (!s_go) return;
@@ -1382,6 +1300,14 @@ static int n_lm_tiles(const DevNet<Real>& n, int* ev_tiles, int* bb_tiles) {
     *ev_tiles = n.sp_tiles[K_EXVOL];
     *bb_tiles = n.sp_tiles[K_BOUNDARY];
     return n.sp_tiles[K_LINKER] + n.sp_tiles[K_MOTOR];
+}
+
+template <typename Real>
+static void launch_gather(const DevNet<Real>& n, int want, cudaStream_t s) {
+    const int grid = (n.n_ftiles + n.gtiles - 1) / n.gtiles;
+    if constexpr (sizeof(Real) == 4) k_force_gather_mx<<<grid, 64 * n.gtiles, 0, s>>>(n, want);
+    else if (n.gtiles == 1) k_force_gather<1><<<grid, kBlock, 0, s>>>(n, want);
+    else k_force_gather<kGatherTiles><<<grid, kBlock, 0, s>>>(n, want);
 }
 
 // The excluded-volume chain and the linker/motor/boundary kernel on side
@@ -1441,8 +1367,7 @@ int launch_forces(const DevNet<Real>& n, int want, const Lanes& L) {
     if (!n.fil_first[1]) fil();
     cudaStreamWaitEvent(L.main, L.join, 0);
     cudaStreamWaitEvent(L.main, L.join2, 0);
-    if constexpr (sizeof(Real) == 4) k_force_gather_mx<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, L.main>>>(n, want);
-    else k_force_gather<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, L.main>>>(n, want);
+    launch_gather(n, want, L.main);
     launch_k(n.pdl, k_finalize_force<Real>, n.R, kBlock, L.main, n, want);
     return launched + 3;
 }
@@ -1488,8 +1413,7 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
         case 1:
             if constexpr (sizeof(Real) == 4) k_fil_force_bulk<<<n.pgrid[1], kBlock, 0, s>>>(n, -1);
             else k_fil_force<<<n.n_ftiles, kBlock, 0, s>>>(n, -1);
-            if constexpr (sizeof(Real) == 4) k_force_gather_mx<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
-            else k_force_gather<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
+            launch_gather(n, -1, s);
             k_finalize_force<Real><<<n.R, kBlock, 0, s>>>(n, -1);
             return 3;
         case 2: if (lm + bb_t > 0) { k_bond_bnd<Real><<<lm + bb_t, kBlock, 0, s>>>(n, -1, 0, 0, lm, ev_t); return 1; } return 0;
@@ -1504,8 +1428,7 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
             else k_fil_force<<<n.n_ftiles, kBlock, 0, s>>>(n, -1);
             return 1;
         case 6:   // the sparse gather with the CG partials alone
-            if constexpr (sizeof(Real) == 4) k_force_gather_mx<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
-            else k_force_gather<<<(n.n_ftiles + kGatherTiles - 1) / kGatherTiles, kBlock, 0, s>>>(n, -1);
+            launch_gather(n, -1, s);
             return 1;
     }
     return 0;

@@ -207,6 +207,7 @@ DevNet<Real> make_devnet(MechContext* c) {
     n.bflag = c->bflag.as<uint8_t>();
     n.bpar = c->bpar.as<Real>();
     n.n_ftiles = c->compact ? c->n_ftiles_c : c->n_ftiles;
+    n.gtiles = n.n_ftiles < 152 * kGatherTiles ? 1 : kGatherTiles;
     n.ftile = (c->compact ? c->ftile_c : c->ftile).as<Tile>();
     for (int k = 0; k < 2; ++k) {
         const int per_sm = c->blocks_per_sm[k];

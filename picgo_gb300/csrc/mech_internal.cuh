@@ -62,9 +62,27 @@ enum Phase : int {
 };
 
 // Per-replica minimizer state, resident in device memory.
-struct CGState {
+struct __align__(16) CGState {
+    // what every evaluation kernel reads, in three 16-byte loads (LaneState)
+    int phase;
+    int active;            // replica participates in the current minimization / evaluation
+    int xbuf, fbuf;
+    // The search direction is d[dbuf], or (dIsF) the current forces themselves:
+    // a reset to steepest descent copies nothing.  dPending: the direction
+    // F + beta d of the search that begins is formed by its first line-search
+    // pass, every kernel for the beads it reads; the filament kernel stores it
+    // in d[dbuf ^ 1] with the d . F partials.
+    int dbuf, dIsF, dPending;
+    // Searches left whose passes also evaluate lambda / 2 (mixed engine).  A
+    // second trial costs 12 of 41 us of a pass on 1M cylinders and 1 us on
+    // 4,000; a rejected trial without it costs a block of idle launches (20-25
+    // us).  It is wanted in 3% of the searches near the start of a minimization
+    // and in up to half of them later, in runs: a rejected trial brings it for
+    // the rest of that search and the kDualSearches after it.
+    int dual;
+    double lambda;         // line-search step
+    double beta;
     // line search
-    double lambda;
     double E0;             // energy at the current coordinates (computeEnergy value)
     double Etrial;
     double reducedSlope;
@@ -73,7 +91,7 @@ struct CGState {
     double maxF;           // gradInfNorm
     double FdotF;          // F . F of the current forces
     double lastFdotF;
-    double newGrad, prevGrad, beta;
+    double newGrad, prevGrad;
     double prevEnergy;
     double energyRelChange;
     double newEnergy;
@@ -86,27 +104,11 @@ struct CGState {
     double eval[MECH_NUM_FF + 1];
     double before[MECH_NUM_FF + 1];   // energiesBefore of the current minimization
     int evalFailed;        // an FF reported failure in the last evaluation
-    int phase;
     int safeMode;
-    // Searches left whose passes also evaluate lambda / 2 (mixed engine).  A
-    // second trial costs 12 of 41 us of a pass on 1M cylinders and 1 us on
-    // 4,000; a rejected trial without it costs a block of idle launches (20-25
-    // us).  It is wanted in 3% of the searches near the start of a minimization
-    // and in up to half of them later, in runs: a rejected trial brings it for
-    // the rest of that search and the kDualSearches after it.
-    int dual;
     int searchTrials;      // trials of the current line search
-    int xbuf, fbuf;
-    // The search direction is d[dbuf], or (dIsF) the current forces themselves:
-    // a reset to steepest descent copies nothing.  dPending: the direction
-    // F + beta d of the search that begins is formed by its first line-search
-    // pass, every kernel for the beads it reads; the filament kernel stores it
-    // in d[dbuf ^ 1] with the d . F partials.
-    int dbuf, dIsF, dPending;
     int numIter, numEnergyCall, numForceCall, numEnergyEval, numTrials, numSafeMode, numRecover;
     int backupValid, backupPending;
     int errorFlags, status;
-    int active;            // replica participates in the current minimization
     int restore;           // copy the backup coordinates back (host request)
 };
 
@@ -190,6 +192,9 @@ struct DevNet {
     // partial sums
     double* part_fil;       // [n_ftiles * 4]
     double* part_df;        // [n_ftiles]: d . F of a pass that forms the direction
+    // filament tiles per block of the gather: kGatherTiles, or 1 where that
+    // leaves SMs without a block
+    int gtiles;
     double* part_sp;        // [n_stiles]
     // per replica
     CGState* st;
@@ -266,6 +271,58 @@ struct TraceGuard {
 #endif
 
 #ifdef __CUDACC__
+// Tile `ti` of the filament list / of the sparse list with its kind.  With one
+// replica both follow from the counts, which saves every kernel of an
+// iteration a dependent load (~0.7 us) before it can read anything else.
+template <typename Real>
+__device__ __forceinline__ Tile fil_tile(const DevNet<Real>& n, int ti) {
+    if (n.R == 1) {
+        const int b = ti * kFilTile;
+        return Tile{0, b, min(b + kFilTile, n.nb), 0};
+    }
+    return n.ftile[ti];
+}
+template <typename Real>
+__device__ __forceinline__ Tile sparse_tile(const DevNet<Real>& n, int ti, int* kind) {
+    if (n.R == 1) {
+        const int count[K_NUM_SPARSE] = {n.n_lk, n.n_mt, n.n_ev, n.n_bb};
+        int k = 0, first = 0, total = count[0];
+#pragma unroll
+        for (int q = 0, end = 0; q < K_NUM_SPARSE; ++q) {
+            if (ti >= end) {
+                k = q;
+                first = end;
+                total = count[q];
+            }
+            end += n.sp_tiles[q];
+        }
+        *kind = k;
+        const int b = (ti - first) * kSparseTile;
+        return Tile{0, b, min(b + kSparseTile, total), 0};
+    }
+    *kind = n.stile_kind[ti];
+    return n.stile[ti];
+}
+// Tile ranges of replica r.
+template <typename Real>
+__device__ __forceinline__ RepTiles rep_tiles(const DevNet<Real>& n, int r) {
+    if (n.R == 1) {
+        RepTiles t;
+        t.fil_begin = 0;
+        t.fil_end = n.n_ftiles;
+        int b = 0;
+#pragma unroll
+        for (int k = 0; k < K_NUM_SPARSE; ++k) {
+            t.sp_begin[k] = b;
+            b += n.sp_tiles[k];
+            t.sp_end[k] = b;
+        }
+        t.n_beads = n.nb;
+        return t;
+    }
+    return n.rt[r];
+}
+
 // Where the contribution of slot `slot` (= slot_base[kind] + interaction * beads + bead) is written.
 template <typename Real>
 __device__ __forceinline__ Real* slot_ptr(const DevNet<Real>& n, int slot) {
