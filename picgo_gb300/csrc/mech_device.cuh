@@ -642,6 +642,21 @@ __device__ __forceinline__ void load_par(const double* P, int j, double& ks, dou
     ks = a.x; l0 = a.y; kb = b.x; t0 = b.y;
 }
 
+// Comparisons of doubles on their bits, off the FP64 pipe.
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+    return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+}
+// areEqual(theta0, 0) on bits: the order of finite magnitudes is that of their
+// bits, and a NaN lies above every threshold
+__device__ __forceinline__ bool theta_is_zero(double t) {
+    return abs_bits(t) < (unsigned long long)__double_as_longlong(1e-6);
+}
+// x clamped to [-1, 1], a NaN kept
+__device__ __forceinline__ double clamp_unit(double x) {
+    const unsigned long long a = abs_bits(x);
+    return a > 0x3ff0000000000000ULL && a <= 0x7ff0000000000000ULL ? copysign(1.0, x) : x;
+}
+
 // ---------------------------------------------------------------------------
 // Filament stretching (FilamentStretchingHarmonic.cpp:185-275) and cosine
 // bending (FilamentBendingCosine.cpp:199-345) on difference vectors.
@@ -651,6 +666,14 @@ __device__ __forceinline__ Real stretch_energy(Real rx, Real ry, Real rz, Real k
     const Real L = sqrt(rx * rx + ry * ry + rz * rz);
     const Real dl = L - l0;
     return (Real)0.5 * k * dl * dl;
+}
+
+// FP64 bending energy of a triple from its cylinders' r1 . r2 and lengths.
+__device__ __forceinline__ double bend_energy_lengths(double l1l2, double L1, double L2, double k, double t0) {
+    const double x = clamp_unit(l1l2 / (L1 * L2));
+    if (theta_is_zero(t0)) return k * (1.0 - x);
+    const double sinA = fmax(sqrt(1.0 - x * x), 0.0);
+    return k * (1.0 - (x * cos(t0) + sinA * sin(t0)));
 }
 
 // Force on the second bead (the first gets the negation).

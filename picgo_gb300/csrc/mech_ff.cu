@@ -141,20 +141,6 @@ __global__ void __launch_bounds__(kBlock) k_body_head(DevNet<Real> n) {
 // ends, comparisons are made on the bits of the numbers, and the sums of a warp
 // share the additions of their trees.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long abs_bits(double x) {
-    return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
-}
-// areEqual(theta0, 0) on bits: the order of finite magnitudes is that of their
-// bits, and a NaN lies above every threshold
-__device__ __forceinline__ bool theta_is_zero(double t) {
-    return abs_bits(t) < (unsigned long long)__double_as_longlong(1e-6);
-}
-// x clamped to [-1, 1], a NaN kept
-__device__ __forceinline__ double clamp_unit(double x) {
-    const unsigned long long a = abs_bits(x);
-    return a > 0x3ff0000000000000ULL && a <= 0x7ff0000000000000ULL ? copysign(1.0, x) : x;
-}
-
 // Stretching + bending energy of the tile's own cylinders and triples.  1M
 // beads: 86 us, against 121 us (66 FP64 instructions per bead) with each length
 // formed two or three times and a tree per sum.
@@ -224,13 +210,7 @@ __global__ void __launch_bounds__(kBlock) k_fil_energy(DevNet<double> n, int wan
     __syncthreads();
     if ((fl & 3) == 3) {
         const double l1l2 = rs[0][i] * r2[0] + rs[1][i] * r2[1] + rs[2][i] * r2[2];
-        const double x = clamp_unit(l1l2 / (rs[3][i] * L2));
-        if (theta_is_zero(th)) {
-            e[1] = kb * (1.0 - x);
-        } else {
-            const double sinA = fmax(sqrt(1.0 - x * x), 0.0);
-            e[1] = kb * (1.0 - (x * cos(th) + sinA * sin(th)));
-        }
+        e[1] = bend_energy_lengths(l1l2, rs[3][i], L2, kb, th);
     }
     if (n.terms && (fl & 1)) {
         n.terms[j] = e[0];

@@ -33,13 +33,16 @@ constexpr int kStaticMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
-// Filament of cylinder c: the largest f with fcs[f] <= c (fcs ascending).
+// Filament of cylinder c: the largest f with fcs[f] <= c (fcs ascending).  All
+// lanes of a warp search together, 32 ranges a step: 20,000 filaments take three
+// dependent loads.
 __device__ __forceinline__ int filament_of(const int32_t* __restrict__ fcs, int nfil, int c) {
-    int lo = 0, hi = nfil - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(fcs + mid) <= c) lo = mid;
-        else hi = mid - 1;
+    int lo = 0, hi = nfil;   // fcs[lo] <= c < fcs[hi]
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) >> 5, probe = lo + ((int)(threadIdx.x & 31) + 1) * step;
+        const bool le = probe < hi && __ldg(fcs + probe) <= c;
+        lo += step * __popc(__ballot_sync(0xffffffffu, le));
+        hi = min(hi, lo + step);
     }
     return lo;
 }
@@ -47,35 +50,73 @@ __device__ __forceinline__ int filament_of(const int32_t* __restrict__ fcs, int 
 // One thread per cylinder: its stretching term and, unless it is the first
 // cylinder of its filament, the bending term of the triple it closes
 // (constants of the second cylinder).  Beads are filament-contiguous, so
-// cylinder c of filament f joins beads c + f and c + f + 1.
+// cylinder c of filament f joins beads c + f and c + f + 1.  Bound by the FP64
+// pipe: a cylinder's vector and length are formed once and serve its stretching
+// and the bending on both of its ends; the filament is searched for once per
+// block, and the starts of filaments inside the block are counted.
 __global__ void __launch_bounds__(kStaticBlock)
 k_fil_energy_static(const double* __restrict__ x, const int32_t* __restrict__ fcs, int nfil, int ncyl,
                     const double* __restrict__ ks, const double* __restrict__ l0, const double* __restrict__ kb,
                     const double* __restrict__ t0, unsigned char* scratch, double* out) {
-    __shared__ double sh[64];
-    __shared__ int s_last;
+    static_assert(kStaticBlock == kBlock, "block_sums");
+    __shared__ double sh[2 * kBlock / 32];
+    __shared__ double rs[4][kStaticBlock + 1];   // cylinders c0 - 1 ..: vector, length
+    __shared__ int s_last, s_f0, s_begin, s_starts[kStaticBlock / 32];
+    __shared__ unsigned char s_start[kStaticBlock];
     unsigned int* ticket = reinterpret_cast<unsigned int*>(scratch);
     double2* part = reinterpret_cast<double2*>(scratch + 256);
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    double es = 0.0, eb = 0.0;
-    if (c < ncyl) {
-        const int f = filament_of(fcs, nfil, c);
-        const size_t b = (size_t)c + (size_t)f;
-        const double* p0 = x + 3 * b;
-        const double* p1 = p0 + 3;
-        es = stretch_energy<double>(p1[0] - p0[0], p1[1] - p0[1], p1[2] - p0[2], ks[c], l0[c]);
-        if (c > __ldg(fcs + f)) {
-            const double* pm = p0 - 3;
-            const double r1[3] = {p0[0] - pm[0], p0[1] - pm[1], p0[2] - pm[2]};
-            const double r2[3] = {p1[0] - p0[0], p1[1] - p0[1], p1[2] - p0[2]};
-            eb = bend_energy<double>(r1, r2, kb[c], t0[c]);
+    const int i = threadIdx.x, c0 = blockIdx.x * blockDim.x, c = c0 + i, w = i >> 5, lane = i & 31;
+    s_start[i] = 0;
+    if (w == 0) {
+        const int f0 = filament_of(fcs, nfil, c0);
+        if (lane == 0) {
+            s_f0 = f0;
+            s_begin = __ldg(fcs + f0);
         }
     }
-    double w[2] = {warp_sum(es), warp_sum(eb)};
-    const int ops[2] = {0, 0};
-    block_combine<2>(w, ops, sh);
+    __syncthreads();
+    const int f0 = s_f0;
+    if (f0 + 1 + i < nfil) {   // the filaments after f0: at most one starts at each cylinder of the block
+        const int b = __ldg(fcs + f0 + 1 + i) - c0;
+        if (b > 0 && b < kStaticBlock) s_start[b] = 1;
+    }
+    if (i == 0 && s_begin == c0) s_start[0] = 2;   // f0 itself starts here
+    __syncthreads();
+    const int start = s_start[i];
+    const unsigned m = __ballot_sync(0xffffffffu, start == 1);
+    if (lane == 0) s_starts[w] = __popc(m);
+    __syncthreads();
+    int f = f0 + __popc(m & (0xffffffffu >> (31 - lane)));
+#pragma unroll
+    for (int k = 0; k < kStaticBlock / 32; ++k)
+        if (k < w) f += s_starts[k];
+    double e[2] = {0.0, 0.0}, r2[3] = {0, 0, 0}, L2 = 0.0;
+    const bool valid = c < ncyl;
+    if (valid) {
+        const double* p = x + 3 * ((size_t)c + (size_t)f);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) rs[q][i + 1] = r2[q] = p[3 + q] - p[q];
+        L2 = sqrt(r2[0] * r2[0] + r2[1] * r2[1] + r2[2] * r2[2]);
+        rs[3][i + 1] = L2;
+        const double dl = L2 - l0[c];
+        e[0] = 0.5 * ks[c] * dl * dl;
+    }
+    if (i == kStaticBlock - 32 && !s_start[0]) {   // the cylinder before the block, on the same filament
+        const double* p = x + 3 * ((size_t)c0 + (size_t)f0);
+        double r[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) rs[q][0] = r[q] = p[q] - p[q - 3];
+        rs[3][0] = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
+    }
+    __syncthreads();
+    if (valid && !start) {
+        const double l1l2 = rs[0][i] * r2[0] + rs[1][i] * r2[1] + rs[2][i] * r2[2];
+        e[1] = bend_energy_lengths(l1l2, rs[3][i], L2, kb[c], t0[c]);
+    }
+    const double a = block_sums<2>(e, sh);
+    const double b = __shfl_sync(0xffffffffu, a, 1);
     if (threadIdx.x == 0) {
-        part[blockIdx.x] = make_double2(w[0], w[1]);
+        part[blockIdx.x] = make_double2(a, b);
         __threadfence();
         s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
@@ -83,19 +124,15 @@ k_fil_energy_static(const double* __restrict__ x, const int32_t* __restrict__ fc
     if (!s_last) return;
     // last block: slots in a fixed order (thread t takes t, t + 256, ...), then the block tree
     __threadfence();
-    double a = 0.0, bsum = 0.0;
+    double t[2] = {0.0, 0.0};
     for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
         const double2 v = __ldcg(part + k);
-        a += v.x;
-        bsum += v.y;
+        t[0] += v.x;
+        t[1] += v.y;
     }
-    double t[2] = {warp_sum(a), warp_sum(bsum)};
-    block_combine<2>(t, ops, sh);
-    if (threadIdx.x == 0) {
-        out[0] = t[0];
-        out[1] = t[1];
-        *ticket = 0u;
-    }
+    const double s = block_sums<2>(t, sh);
+    if (threadIdx.x < 2) out[threadIdx.x] = s;
+    if (threadIdx.x == 0) *ticket = 0u;
 }
 
 // The scratch address belongs to the module loaded into one CUDA context: a
