@@ -1306,8 +1306,8 @@ int launch_energy(const DevNet<Real>& n, int want, int trial, const Lanes& L) {
     cudaStreamWaitEvent(L.side, L.fork, 0);
     cudaStreamWaitEvent(L.side2, L.fork, 0);
     auto fil = [&] {
-        if constexpr (sizeof(Real) == 4) launch_k(n.pdl, k_fil_energy_bulk, n.pgrid[0], kBlock, L.main, n, want, trial);
-        else launch_k(n.pdl, k_fil_energy, n.n_ftiles, kBlock, L.main, n, want, trial);
+        if constexpr (sizeof(Real) == 4) launch_k(n.pdl == 2, k_fil_energy_bulk, n.pgrid[0], kBlock, L.main, n, want, trial);
+        else launch_k(n.pdl == 2, k_fil_energy, n.n_ftiles, kBlock, L.main, n, want, trial);
     };
     if (n.fil_first[0]) fil();
     launched += launch_exvol_energy<Real>(n, want, trial, L.side, false);
@@ -1333,8 +1333,8 @@ int launch_forces(const DevNet<Real>& n, int want, const Lanes& L) {
     cudaStreamWaitEvent(L.side, L.fork, 0);
     cudaStreamWaitEvent(L.side2, L.fork, 0);
     auto fil = [&] {
-        if constexpr (sizeof(Real) == 4) launch_k(n.pdl, k_fil_force_bulk, n.pgrid[1], kBlock, L.main, n, want);
-        else launch_k(n.pdl, k_fil_force, n.n_ftiles, kBlock, L.main, n, want);
+        if constexpr (sizeof(Real) == 4) launch_k(n.pdl == 2, k_fil_force_bulk, n.pgrid[1], kBlock, L.main, n, want);
+        else launch_k(n.pdl == 2, k_fil_force, n.n_ftiles, kBlock, L.main, n, want);
     };
     if (n.fil_first[1]) fil();
     launched += launch_exvol_forces<Real>(n, want, L.side, false);

@@ -190,6 +190,7 @@ template <typename Real>
 DevNet<Real> make_devnet(MechContext* c) {
     DevNet<Real> n;
     std::memset(&n, 0, sizeof(n));   // padding too: the bytes are compared (iteration_graph)
+    n.pdl = 1;
     n.nb = c->nb;
     n.R = c->R;
     n.x[0] = c->x[0].as<Real>();
@@ -1101,7 +1102,7 @@ template <typename Real>
 static int iteration_graph(MechContext* c, int which) {
     auto& ig = c->iter[which];
     DevNet<Real> n = make_devnet<Real>(c);
-    n.pdl = c->graph_mode == MECH_GRAPH_UNROLLED_PDL ? 1 : 0;
+    if (c->graph_mode == MECH_GRAPH_UNROLLED_PDL) n.pdl = 2;
     n.snap = c->snap[0].word;
     std::vector<unsigned char> key(sizeof(n) + sizeof(int));
     std::memcpy(key.data(), &n, sizeof(n));
@@ -1182,6 +1183,7 @@ static int capture_conditional_graph(MechContext* c, cudaGraphExec_t* exec, Cond
     for (int k = 0; k < 2; ++k)
         if ((e = cudaGraphConditionalHandleCreate(&h[k], body, 0, 0)) != cudaSuccess) return fail(e, "phase handle");
     DevNet<Real> n = make_devnet<Real>(c);
+    n.pdl = 0;
     n.cond = GraphConds{h[0], h[1], h_loop, c->cond_counter.as<int>(), kBodiesPerLaunch, 1};
     // capture `fn` into `graph` after `dep` (none when null)
     auto capture_into = [&](cudaGraph_t graph, const cudaGraphNode_t* dep, auto&& fn) -> cudaError_t {

@@ -203,9 +203,11 @@ struct DevNet {
     int* gticket;           // whole-grid ticket
     unsigned* err;          // device error word
     GraphConds cond;
-    // programmatic dependent launch on the main lane (MECH_GRAPH_UNROLLED_PDL):
-    // the kernels that follow a reduction, and the reductions themselves, are
-    // scheduled while their predecessor runs and wait for it (griddepcontrol)
+    // programmatic dependent launch: the kernel is scheduled while its
+    // predecessor in the lane runs and waits for it (griddepcontrol).  1: the
+    // excluded-volume chain and the force reduction; 2: the filament kernels
+    // after a reduction too (MECH_GRAPH_UNROLLED_PDL); 0: none (loop bodies of
+    // conditional graphs).
     int pdl;
     // diagnostic (mech_energy_terms; null otherwise): the filament energy
     // kernels also store each bead's stretching [b] and bending [nb + b] term,
