@@ -1086,12 +1086,15 @@ static int eval_forces(MechContext* c, int replica, double* f_out = nullptr) {
 // run long enough for that one's construction (0.2 ms) to pay.
 static constexpr int kGraphBlocks[2] = {2, 8};
 static constexpr int kShortGraphs = 64;
-// Line-search launches per iteration block: FP64, two single-trial passes;
-// mixed, one two-trial pass (lambda and lambda / 2).
+// The line-search pass of an iteration block: in the mixed engine of lambda and,
+// where CGState::dual asks for it, lambda / 2; in FP64 of lambda alone.  A search
+// that rejects a trial goes on in the next block, after a force pass with nothing
+// to do (8 us; 4k cylinders).  An FP64 block of two passes spent 5 us on the
+// second one in the iterations whose first trial was accepted, nine tenths of
+// them: 62.5 us per iteration of a long run, 60.6 with one.
 template <typename Real>
 static int trial_launches(const DevNet<Real>& n, const Lanes& L) {
-    if constexpr (sizeof(Real) == 4) return launch_energy<Real>(n, PH_LS_TRIAL, kTrialDual, L);
-    return launch_energy<Real>(n, PH_LS_TRIAL, 1, L) + launch_energy<Real>(n, PH_LS_TRIAL, 1, L);
+    return launch_energy<Real>(n, PH_LS_TRIAL, sizeof(Real) == 4 ? kTrialDual : 1, L);
 }
 
 // The unrolled iteration graph of kGraphBlocks[which] blocks for the context's
