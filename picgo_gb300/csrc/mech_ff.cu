@@ -228,6 +228,14 @@ __global__ void __launch_bounds__(kBlock) k_fil_energy(DevNet<double> n, int wan
 // engine's minimizations amplify a changed rounding by up to ~1e8 over a hundred
 // iterations, so the forces keep every operation.  A triple reads its
 // cylinders' vectors and squared lengths instead of forming them again.
+// Bound by the FP64 pipe, where a warp with three active lanes costs as much as
+// a full one: a block of 256 beads has 259 cylinders and 258 triples, nine warps
+// of each.  A single network, whose beads may be cut anywhere (no sum crosses a
+// bead here), takes 253 a block: eight warps of each (1M beads: 214 -> 190 us).
+constexpr int kForceBeads = kFilTile - 3;
+inline int force_blocks(const DevNet<double>& n) {
+    return n.R == 1 ? (n.nb + kForceBeads - 1) / kForceBeads : n.n_ftiles;
+}
 __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want) {
     pdl_wait();      // the previous kernel of the main lane has finished
     MECH_TRACE_KERNEL(n, TK_FIL_FORCE);
@@ -235,7 +243,8 @@ __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want
     __shared__ double rs[3][kFilTile + 3], Ls[kFilTile + 3];        // cylinders begin - 2 .. end: vector, L^2
     __shared__ double fs[3][kFilTile + 3];                          // their stretching forces on the second bead
     __shared__ double f1[3][kFilTile + 2], f2[3][kFilTile + 2];     // triples on begin - 1 .. end
-    const Tile t = fil_tile(n, blockIdx.x);
+    const int own = (int)blockIdx.x * kForceBeads;
+    const Tile t = n.R == 1 ? Tile{0, own, min(own + kForceBeads, n.nb), 0} : fil_tile(n, blockIdx.x);
     const LaneState<double> s = lane_state(n, t.replica, want);
     if (!s.go) return;
     const int T = t.end - t.begin;
@@ -374,9 +383,11 @@ __device__ __forceinline__ void gather_bead(const DevNet<double>& n, int b, int 
     mx = min(max(max(abs_bits(F[0]), abs_bits(F[1])), abs_bits(F[2])), 0x7ff0000000000000ULL);
 }
 
-// NT tiles per block (DevNet::gtiles)
+// NT tiles per block (DevNet::gtiles).  Four blocks on an SM (64 registers) hold
+// 997 blocks of the 1M-bead network in two rounds; with three there were three,
+// the last of them a fifth full (iteration 712 -> 706 us).
 template <int NT>
-__global__ void __launch_bounds__(kBlock) k_force_gather(DevNet<double> n, int want) {
+__global__ void __launch_bounds__(kBlock, 4) k_force_gather(DevNet<double> n, int want) {
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_GATHER);
     __shared__ double sh[2 * NT * kBlock / 32];
@@ -1334,7 +1345,7 @@ int launch_forces(const DevNet<Real>& n, int want, const Lanes& L) {
     cudaStreamWaitEvent(L.side2, L.fork, 0);
     auto fil = [&] {
         if constexpr (sizeof(Real) == 4) launch_k(n.pdl == 2, k_fil_force_bulk, n.pgrid[1], kBlock, L.main, n, want);
-        else launch_k(n.pdl == 2, k_fil_force, n.n_ftiles, kBlock, L.main, n, want);
+        else launch_k(n.pdl == 2, k_fil_force, force_blocks(n), kBlock, L.main, n, want);
     };
     if (n.fil_first[1]) fil();
     launched += launch_exvol_forces<Real>(n, want, L.side, false);
@@ -1392,7 +1403,7 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
             return 1;
         case 1:
             if constexpr (sizeof(Real) == 4) k_fil_force_bulk<<<n.pgrid[1], kBlock, 0, s>>>(n, -1);
-            else k_fil_force<<<n.n_ftiles, kBlock, 0, s>>>(n, -1);
+            else k_fil_force<<<force_blocks(n), kBlock, 0, s>>>(n, -1);
             launch_gather(n, -1, s);
             k_finalize_force<Real><<<n.R, kBlock, 0, s>>>(n, -1);
             return 3;
@@ -1405,7 +1416,7 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
             return 1;
         case 5:   // filament forces alone
             if constexpr (sizeof(Real) == 4) k_fil_force_bulk<<<n.pgrid[1], kBlock, 0, s>>>(n, -1);
-            else k_fil_force<<<n.n_ftiles, kBlock, 0, s>>>(n, -1);
+            else k_fil_force<<<force_blocks(n), kBlock, 0, s>>>(n, -1);
             return 1;
         case 6:   // the sparse gather with the CG partials alone
             launch_gather(n, -1, s);
