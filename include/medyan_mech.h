@@ -250,9 +250,10 @@ int32_t mech_get_forces(MechContext* ctx, int32_t replica, double* f_out);
 
 /*
  * How mech_minimize drives the device.  MECH_GRAPH_UNROLLED (default): a graph
- * of 2, in longer runs 8, unrolled iteration blocks (line search: 2 single-trial passes, FP64,
- * or one pass, mixed; forces) relaunched by the host, every kernel reading its replica's phase and
- * exiting when it has nothing to do.  MECH_GRAPH_CONDITIONAL: one CUDA graph
+ * of 2, in longer runs 8, unrolled iteration blocks (one line-search pass, one
+ * force pass) relaunched by the host, every kernel reading its replica's phase
+ * and exiting when it has nothing to do; the kernels follow one another by
+ * programmatic dependent launch.  MECH_GRAPH_CONDITIONAL: one CUDA graph
  * whose device while loop runs, per body, only the phases some replica is in
  * (line-search pass, forces, direction, reset to steepest descent); the host is
  * involved only for recovery moves, errors and every 512 bodies.  Both run the
@@ -264,9 +265,8 @@ int32_t mech_get_forces(MechContext* ctx, int32_t replica, double* f_out);
  */
 #define MECH_GRAPH_CONDITIONAL 0
 #define MECH_GRAPH_UNROLLED 1
-/* the unrolled graph with programmatic dependent launch on its main lane: the
- * kernels around each single-block reduction are scheduled while their
- * predecessor runs and wait for it on the device (same results) */
+/* accepted and run as MECH_GRAPH_UNROLLED, whose kernels all use programmatic
+ * dependent launch now */
 #define MECH_GRAPH_UNROLLED_PDL 2
 /* accepted and run as MECH_GRAPH_UNROLLED: the mode's cooperative tail (gather,
  * reductions, direction update, reset in one launch) was slower than the

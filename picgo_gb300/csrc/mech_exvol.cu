@@ -152,6 +152,10 @@ __device__ __forceinline__ void release_next(const DevNet<Real>& n) {
     if (n.n_ftiles <= 4 * 152) pdl_trigger();
 }
 
+// Two blocks fit on an SM; a second wave of blocks that find nothing flagged
+// cost 0.7 us in every force evaluation.
+constexpr int kFbForceBlocks = 2 * 152;
+
 // numeric forces: partial moments of (entry, chunk), combined by the last chunk
 template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_exvol_fb_force(DevNet<Real> n, double* moments, int* tickets) {
@@ -515,6 +519,7 @@ __device__ void exvol_split(const DevNet<Real>& n, int r, const Real* X, const D
 template <typename Real>
 __global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, int trial, int force, int tile_off,
                                                     int unsplit) {
+    pdl_wait();      // the reduction before this evaluation has finished
     MECH_TRACE_KERNEL(n, TK_EXVOL);
     __shared__ SplitShared s;
     const int sb = (int)blockIdx.x - 2 * unsplit;
@@ -558,6 +563,7 @@ __global__ void __launch_bounds__(128) k_exvol_fp64(DevNet<Real> n, int want, in
 
 template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int trial, int force, int tile_off) {
+    pdl_wait();      // the reduction before this evaluation has finished
     MECH_TRACE_KERNEL(n, TK_EXVOL);
     int kind;
     const Tile t = sparse_tile(n, tile_off + (int)blockIdx.x, &kind);
@@ -939,46 +945,55 @@ static inline int ev_tiles_of(const DevNet<Real>& n, int* off) {
 // Inside an evaluation (standalone = false) the work-list counts are zero on
 // entry: the evaluation's reduction kernel zeroes them for the next one, which
 // keeps a memset off the head of the excluded-volume lane.  A standalone
-// launch zeroes them first and leaves them as they end.
+// launch zeroes them first and leaves them as they end.  `done`, unless null, is
+// recorded behind the chain.
 template <typename Real>
-int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t s, bool standalone) {
+int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t s, bool standalone, cudaEvent_t done) {
     int off = 0;
     const int nt = ev_tiles_of(n, &off);
-    if (nt == 0) return 0;
+    if (nt == 0) {
+        if (done) cudaEventRecord(done, s);
+        return 0;
+    }
     if (standalone) reset_counts(n, s);
     int k = 1;
     if constexpr (sizeof(Real) == 8) {
         const int split = exvol_split_tiles(nt);
-        k_exvol_fp64<Real><<<2 * (nt - split) + 8 * split, 128, 0, s>>>(n, want, trial, 0, off, nt - split);
+        launch_k(false, nullptr, k_exvol_fp64<Real>, 2 * (nt - split) + 8 * split, 128, s, n, want, trial, 0, off, nt - split);
     } else {
-        k_exvol<Real><<<nt, kBlock, 0, s>>>(n, want, trial, 0, off);
-        launch_k(n.pdl, k_exvol_ext<Real>, kExtBlocks, 128, s, n, trial, 0);
+        launch_k(false, nullptr, k_exvol<Real>, nt, kBlock, s, n, want, trial, 0, off);
+        launch_k(n.pdl, nullptr, k_exvol_ext<Real>, kExtBlocks, 128, s, n, trial, 0);
         ++k;
     }
-    launch_k(n.pdl, k_exvol_energy_tail<Real>, kFbEnergyBlocks + nt, kBlock, s, n, want, trial, off);
+    launch_k(n.pdl, n.pdl ? done : nullptr, k_exvol_energy_tail<Real>, kFbEnergyBlocks + nt, kBlock, s, n, want, trial, off);
+    if (done && !n.pdl) cudaEventRecord(done, s);
     return k + 1;
 }
 
 template <typename Real>
-int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool standalone) {
+int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool standalone, cudaEvent_t done) {
     int off = 0;
     const int nt = ev_tiles_of(n, &off);
-    if (nt == 0) return 0;
+    if (nt == 0) {
+        if (done) cudaEventRecord(done, s);
+        return 0;
+    }
     if (standalone) reset_counts(n, s);
     int k = 1;
     if constexpr (sizeof(Real) == 8) {
         const int split = exvol_split_tiles(nt);
-        k_exvol_fp64<Real><<<2 * (nt - split) + 8 * split, 128, 0, s>>>(n, want, 0, 1, off, nt - split);
+        launch_k(false, nullptr, k_exvol_fp64<Real>, 2 * (nt - split) + 8 * split, 128, s, n, want, 0, 1, off, nt - split);
     } else {
-        k_exvol<Real><<<nt, kBlock, 0, s>>>(n, want, 0, 1, off);
-        launch_k(n.pdl, k_exvol_ext<Real>, kExtBlocks, 128, s, n, 0, 1);
+        launch_k(false, nullptr, k_exvol<Real>, nt, kBlock, s, n, want, 0, 1, off);
+        launch_k(n.pdl, nullptr, k_exvol_ext<Real>, kExtBlocks, 128, s, n, 0, 1);
         ++k;
     }
-    launch_k(n.pdl, k_exvol_fb_force<Real>, 4 * 152, kBlock, s, n, n.fb_moments, n.fb_tickets);
+    launch_k(n.pdl, n.pdl ? done : nullptr, k_exvol_fb_force<Real>, kFbForceBlocks, kBlock, s, n, n.fb_moments, n.fb_tickets);
+    if (done && !n.pdl) cudaEventRecord(done, s);
     return k + 1;
 }
 
-template int launch_exvol_energy<MECH_EXVOL_REAL>(const DevNet<MECH_EXVOL_REAL>&, int, int, cudaStream_t, bool);
-template int launch_exvol_forces<MECH_EXVOL_REAL>(const DevNet<MECH_EXVOL_REAL>&, int, cudaStream_t, bool);
+template int launch_exvol_energy<MECH_EXVOL_REAL>(const DevNet<MECH_EXVOL_REAL>&, int, int, cudaStream_t, bool, cudaEvent_t);
+template int launch_exvol_forces<MECH_EXVOL_REAL>(const DevNet<MECH_EXVOL_REAL>&, int, cudaStream_t, bool, cudaEvent_t);
 
 }  // namespace mech

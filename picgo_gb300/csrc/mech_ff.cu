@@ -388,6 +388,7 @@ __device__ __forceinline__ void gather_bead(const DevNet<double>& n, int b, int 
 // the last of them a fifth full (iteration 712 -> 706 us).
 template <int NT>
 __global__ void __launch_bounds__(kBlock, 4) k_force_gather(DevNet<double> n, int want) {
+    pdl_wait();      // the force kernels have finished
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_GATHER);
     __shared__ double sh[2 * NT * kBlock / 32];
@@ -432,6 +433,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_gather(DevNet<double> n, in
 // with stride n.gtiles).
 constexpr int kGatherAheadMx = 8;
 __global__ void __launch_bounds__(kBlock) k_force_gather_mx(DevNet<float> n, int want) {
+    pdl_wait();      // the force kernels have finished
     static_assert(kFilTile == 256 && kBlock == 64 * kGatherTiles, "64 threads x 4 beads per tile");
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_GATHER_MX);
@@ -582,6 +584,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_finalize_force(DevNet<Real> n, in
 // every kernel of the evaluation has written its partial sums.
 template <typename Real>
 __global__ void __launch_bounds__(kBlock, 1) k_finalize_energy(DevNet<Real> n, int want, int trial) {
+    pdl_wait();      // every kernel of the evaluation has finished
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_FIN_ENERGY);
     __shared__ double sh[kFinSums * kBlock / 32];   // block_pair_sums<16>: 16 pairs of floats per warp
@@ -1099,6 +1102,7 @@ __global__ void __launch_bounds__(kBlock) k_fil_force_bulk(DevNet<float> n, int 
 template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, int trial, int force, int n_lm_tiles,
                                                      int ev_tiles) {
+    pdl_wait();      // the reduction before this evaluation has finished
     MECH_TRACE_KERNEL(n, TK_BOND);
     __shared__ double sh[64];   // block_reduce_ff<2>: 32 * 4 floats
     const int ti = blockIdx.x < n_lm_tiles ? blockIdx.x : blockIdx.x + ev_tiles;
@@ -1294,73 +1298,76 @@ static int n_lm_tiles(const DevNet<Real>& n, int* ev_tiles, int* bb_tiles) {
 }
 
 template <typename Real>
-static void launch_gather(const DevNet<Real>& n, int want, cudaStream_t s) {
+static void launch_gather(const DevNet<Real>& n, int want, cudaStream_t s, bool pdl) {
     const int grid = (n.n_ftiles + n.gtiles - 1) / n.gtiles;
-    if constexpr (sizeof(Real) == 4) k_force_gather_mx<<<grid, 64 * n.gtiles, 0, s>>>(n, want);
-    else if (n.gtiles == 1) k_force_gather<1><<<grid, kBlock, 0, s>>>(n, want);
-    else k_force_gather<kGatherTiles><<<grid, kBlock, 0, s>>>(n, want);
+    if constexpr (sizeof(Real) == 4) launch_k(pdl, nullptr, k_force_gather_mx, grid, 64 * n.gtiles, s, n, want);
+    else if (n.gtiles == 1) launch_k(pdl, nullptr, k_force_gather<1>, grid, kBlock, s, n, want);
+    else launch_k(pdl, nullptr, k_force_gather<kGatherTiles>, grid, kBlock, s, n, want);
 }
 
-// The excluded-volume chain and the linker/motor/boundary kernel on side
-// lanes, the filament kernel on the main lane, then (after the joins) the
-// reduction on the main lane.
+// The three lanes of an evaluation: the excluded-volume chain and the
+// linker/motor/boundary kernel on side lanes, the filament kernel (`fil`) on the
+// main lane, which then waits for the others.
 // The filament kernel of an evaluation is launched before the side lanes when
 // its residency is capped (n.fil_first[k]): its blocks then start streaming at
 // once and the excluded-volume and linker kernels fill the room the cap leaves;
 // uncapped, it fills every SM and is launched after them.
-template <typename Real>
-int launch_energy(const DevNet<Real>& n, int want, int trial, const Lanes& L) {
+// With n.pdl the lanes fork and join by programmatic events, so that a kernel's
+// blocks are on the SMs when the ones it waits for end.  Per iteration, with
+// plain events / programmatic: 60k cylinders 56.2 / 54.4 us, 4k 57.9 / 56.5,
+// 32 replicas 95.5 / 93.7, 1M 127.0 / 127.2; FP64 4k 61.0 / 59.5, 1M 684 / 682.
+// All three lanes have to start together: where the filament kernel comes first
+// it takes the SMs and the excluded-volume chain, which is the longer lane, ends
+// later (60k: 62 us).  So the side lanes' kernels, which follow the fork's event
+// alone, are not serialized with the previous ones of their streams, and an
+// evaluation that does not fork from a reduction (L.forked) has a plain edge to
+// its filament kernel, as to the others.
+template <typename Real, typename Fil>
+static int launch_lanes(const DevNet<Real>& n, int want, int trial, bool force, const Lanes& L, Fil&& fil) {
     int ev_t = 0, bb_t = 0;
     const int lm = n_lm_tiles(n, &ev_t, &bb_t);
-    int launched = 0;
-    cudaEventRecord(L.fork, L.main);
+    if (!L.forked) cudaEventRecord(L.fork, L.main);
     cudaStreamWaitEvent(L.side, L.fork, 0);
     cudaStreamWaitEvent(L.side2, L.fork, 0);
-    auto fil = [&] {
-        if constexpr (sizeof(Real) == 4) launch_k(n.pdl == 2, k_fil_energy_bulk, n.pgrid[0], kBlock, L.main, n, want, trial);
-        else launch_k(n.pdl == 2, k_fil_energy, n.n_ftiles, kBlock, L.main, n, want, trial);
-    };
-    if (n.fil_first[0]) fil();
-    launched += launch_exvol_energy<Real>(n, want, trial, L.side, false);
-    cudaEventRecord(L.join, L.side);
+    if (n.fil_first[force]) fil();
+    int launched = 1;
+    launched += force ? launch_exvol_forces<Real>(n, want, L.side, false, L.join)
+                      : launch_exvol_energy<Real>(n, want, trial, L.side, false, L.join);
     if (lm + bb_t > 0) {
-        k_bond_bnd<Real><<<lm + bb_t, kBlock, 0, L.side2>>>(n, want, trial, 0, lm, ev_t);
+        launch_k(false, n.pdl ? L.join2 : nullptr, k_bond_bnd<Real>, lm + bb_t, kBlock, L.side2, n, want, trial,
+                 force ? 1 : 0, lm, ev_t);
         ++launched;
     }
-    cudaEventRecord(L.join2, L.side2);
-    if (!n.fil_first[0]) fil();
+    if (!n.pdl || lm + bb_t == 0) cudaEventRecord(L.join2, L.side2);
+    if (!n.fil_first[force]) fil();
     cudaStreamWaitEvent(L.main, L.join, 0);
     cudaStreamWaitEvent(L.main, L.join2, 0);
-    k_finalize_energy<Real><<<n.R, kBlock, 0, L.main>>>(n, want, trial);
-    return launched + 2;
+    return launched;
+}
+
+// An evaluation's reduction follows its lanes on the main lane; with n.pdl it
+// records the event that a following evaluation forks from (Lanes::forked).
+template <typename Real>
+int launch_energy(const DevNet<Real>& n, int want, int trial, const Lanes& L) {
+    const int k = launch_lanes(n, want, trial, false, L, [&] {
+        if constexpr (sizeof(Real) == 4)
+            launch_k(L.forked, nullptr, k_fil_energy_bulk, n.pgrid[0], kBlock, L.main, n, want, trial);
+        else launch_k(L.forked, nullptr, k_fil_energy, n.n_ftiles, kBlock, L.main, n, want, trial);
+    });
+    launch_k(n.pdl, n.pdl ? L.fork : nullptr, k_finalize_energy<Real>, n.R, kBlock, L.main, n, want, trial);
+    return k + 1;
 }
 
 template <typename Real>
 int launch_forces(const DevNet<Real>& n, int want, const Lanes& L) {
-    int ev_t = 0, bb_t = 0;
-    const int lm = n_lm_tiles(n, &ev_t, &bb_t);
-    int launched = 0;
-    cudaEventRecord(L.fork, L.main);
-    cudaStreamWaitEvent(L.side, L.fork, 0);
-    cudaStreamWaitEvent(L.side2, L.fork, 0);
-    auto fil = [&] {
-        if constexpr (sizeof(Real) == 4) launch_k(n.pdl == 2, k_fil_force_bulk, n.pgrid[1], kBlock, L.main, n, want);
-        else launch_k(n.pdl == 2, k_fil_force, force_blocks(n), kBlock, L.main, n, want);
-    };
-    if (n.fil_first[1]) fil();
-    launched += launch_exvol_forces<Real>(n, want, L.side, false);
-    cudaEventRecord(L.join, L.side);
-    if (lm + bb_t > 0) {
-        k_bond_bnd<Real><<<lm + bb_t, kBlock, 0, L.side2>>>(n, want, 0, 1, lm, ev_t);
-        ++launched;
-    }
-    cudaEventRecord(L.join2, L.side2);
-    if (!n.fil_first[1]) fil();
-    cudaStreamWaitEvent(L.main, L.join, 0);
-    cudaStreamWaitEvent(L.main, L.join2, 0);
-    launch_gather(n, want, L.main);
-    launch_k(n.pdl, k_finalize_force<Real>, n.R, kBlock, L.main, n, want);
-    return launched + 3;
+    const int k = launch_lanes(n, want, 0, true, L, [&] {
+        if constexpr (sizeof(Real) == 4)
+            launch_k(L.forked, nullptr, k_fil_force_bulk, n.pgrid[1], kBlock, L.main, n, want);
+        else launch_k(L.forked, nullptr, k_fil_force, force_blocks(n), kBlock, L.main, n, want);
+    });
+    launch_gather(n, want, L.main, n.pdl);
+    launch_k(n.pdl, n.pdl ? L.fork : nullptr, k_finalize_force<Real>, n.R, kBlock, L.main, n, want);
+    return k + 2;
 }
 
 int launch_graph_head(cudaStream_t s) {
@@ -1404,7 +1411,7 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
         case 1:
             if constexpr (sizeof(Real) == 4) k_fil_force_bulk<<<n.pgrid[1], kBlock, 0, s>>>(n, -1);
             else k_fil_force<<<force_blocks(n), kBlock, 0, s>>>(n, -1);
-            launch_gather(n, -1, s);
+            launch_gather(n, -1, s, false);
             k_finalize_force<Real><<<n.R, kBlock, 0, s>>>(n, -1);
             return 3;
         case 2: if (lm + bb_t > 0) { k_bond_bnd<Real><<<lm + bb_t, kBlock, 0, s>>>(n, -1, 0, 0, lm, ev_t); return 1; } return 0;
@@ -1419,7 +1426,7 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
             else k_fil_force<<<force_blocks(n), kBlock, 0, s>>>(n, -1);
             return 1;
         case 6:   // the sparse gather with the CG partials alone
-            launch_gather(n, -1, s);
+            launch_gather(n, -1, s, false);
             return 1;
     }
     return 0;

@@ -1105,7 +1105,6 @@ template <typename Real>
 static int iteration_graph(MechContext* c, int which) {
     auto& ig = c->iter[which];
     DevNet<Real> n = make_devnet<Real>(c);
-    if (c->graph_mode == MECH_GRAPH_UNROLLED_PDL) n.pdl = 2;
     n.snap = c->snap[0].word;
     std::vector<unsigned char> key(sizeof(n) + sizeof(int));
     std::memcpy(key.data(), &n, sizeof(n));
@@ -1115,9 +1114,11 @@ static int iteration_graph(MechContext* c, int which) {
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     int k = launch_graph_head(c->stream);
+    Lanes L = c->lanes();
     for (int b = 0; b < kGraphBlocks[which]; ++b) {
-        k += trial_launches<Real>(n, c->lanes());
-        k += launch_forces<Real>(n, PH_FORCE, c->lanes());
+        k += trial_launches<Real>(n, L);
+        L.forked = true;
+        k += launch_forces<Real>(n, PH_FORCE, L);
     }
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (e != cudaSuccess) return set_err(MECH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -1808,7 +1809,7 @@ int32_t mech_set_graph_mode(MechContext* ctx, int32_t mode) {
     if (mode != MECH_GRAPH_CONDITIONAL && mode != MECH_GRAPH_UNROLLED && mode != MECH_GRAPH_UNROLLED_PDL &&
         mode != MECH_GRAPH_UNROLLED_COOP)
         return set_err(MECH_ERR_ARG, "bad graph mode");
-    ctx->graph_mode = mode == MECH_GRAPH_UNROLLED_COOP ? MECH_GRAPH_UNROLLED : mode;
+    ctx->graph_mode = mode == MECH_GRAPH_CONDITIONAL ? mode : MECH_GRAPH_UNROLLED;
     return MECH_OK;
 }
 

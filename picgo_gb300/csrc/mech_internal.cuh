@@ -203,11 +203,9 @@ struct DevNet {
     int* gticket;           // whole-grid ticket
     unsigned* err;          // device error word
     GraphConds cond;
-    // programmatic dependent launch: the kernel is scheduled while its
-    // predecessor in the lane runs and waits for it (griddepcontrol).  1: the
-    // excluded-volume chain and the force reduction; 2: the filament kernels
-    // after a reduction too (MECH_GRAPH_UNROLLED_PDL); 0: none (loop bodies of
-    // conditional graphs).
+    // programmatic dependent launch: the kernels of an evaluation are scheduled
+    // while the kernels before them run and wait for those (griddepcontrol);
+    // off in the loop bodies of conditional graphs
     int pdl;
     // diagnostic (mech_energy_terms; null otherwise): the filament energy
     // kernels also store each bead's stretching [b] and bending [nb + b] term,
@@ -332,27 +330,34 @@ __device__ __forceinline__ Real* slot_ptr(const DevNet<Real>& n, int slot) {
 }
 #endif
 
-// Launch of `kernel` on stream `s`, with programmatic stream serialization when
-// `pdl` is set: the kernel may then start while the previous kernel of the
-// stream is still running (once that kernel's blocks have called pdl_trigger()),
-// and calls pdl_wait() before it reads anything the previous kernel wrote.
+// Launch of `kernel` on stream `s`.  With `pdl` it may be scheduled while the
+// kernels it depends on (the previous one of its stream, and those behind the
+// events its stream waits for) are still running, and calls pdl_wait() before
+// it reads anything they wrote.  With `done`, the event is recorded behind the
+// launch such that kernels waiting for it may be scheduled early in the same
+// way (from the kernel's pdl_trigger() on, or from its end without one).
 template <typename... KArgs, typename... Args>
-inline void launch_k(bool pdl, void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t s,
-                     Args... args) {
-    if (!pdl) {
-        kernel<<<grid, block, 0, s>>>(args...);
-        return;
-    }
+inline void launch_k(bool pdl, cudaEvent_t done, void (*kernel)(KArgs...), unsigned grid, unsigned block,
+                     cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned na = 0;
+    if (pdl) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (done) {
+        attr[na].id = cudaLaunchAttributeProgrammaticEvent;
+        attr[na].val.programmaticEvent.event = done;
+        attr[na].val.programmaticEvent.flags = 0;
+        attr[na++].val.programmaticEvent.triggerAtBlockStart = 0;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = na;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 #ifdef __CUDACC__
@@ -374,6 +379,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 struct Lanes {
     cudaStream_t main, side, side2;
     cudaEvent_t fork, join, join2;
+    // the reduction before this evaluation has recorded `fork` (programmatic launch)
+    bool forked = false;
 };
 template <typename Real> int launch_energy(const DevNet<Real>& n, int want, int trial, const Lanes& L);
 template <typename Real> int launch_forces(const DevNet<Real>& n, int want, const Lanes& L);
@@ -400,8 +407,9 @@ int set_error_text(int code, const std::string& msg);
 // (standalone: zero the work-list counts first; inside an evaluation they are
 // zero on entry, reset by the evaluation's reduction kernel)
 template <typename Real> int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t s,
-                                                 bool standalone);
-template <typename Real> int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool standalone);
+                                                 bool standalone, cudaEvent_t done = nullptr);
+template <typename Real> int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool standalone,
+                                                 cudaEvent_t done = nullptr);
 
 // ---- Hessian-vector products and solves (mech_hvp.cu, FP64 engine) --------
 // hv = (H + shift I) v at the positions in x[0], v and hv in internal bead

@@ -213,9 +213,8 @@ class Engine:
 
     def set_graph_mode(self, mode: str) -> None:
         """'unrolled' (default): relaunched graphs of 2 (longer runs: 8) unrolled iteration blocks;
-        'unrolled_pdl': the same with programmatic dependent launch around the reductions;
         'conditional': one graph whose device while loop runs only the phases in use;
-        'unrolled_coop': accepted, the same as 'unrolled'.  Same results."""
+        'unrolled_pdl', 'unrolled_coop': accepted, the same as 'unrolled'.  Same results."""
         check(self._L.mech_set_graph_mode(self._ctx, {"conditional": 0, "unrolled": 1, "unrolled_pdl": 2,
                                                      "unrolled_coop": 3}[mode]))
 
