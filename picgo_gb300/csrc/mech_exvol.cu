@@ -253,31 +253,60 @@ __device__ __forceinline__ void flag_fallback(const DevNet<Real>& n, int r, int 
 constexpr float kMixedTauEnergy = 0.005f;  // extended pass below this normalized triple product (energy)
 constexpr float kMixedTauForce = 0.02f;    // (forces, whose formula loses more to cancellation)
 
-// Warp-aggregated append of (replica, pair) to the extended-pass pair list.
+// Warp-aggregated append of an entry (a, b) to a list of 2 n_ev entries.
 template <typename Real>
-__device__ __forceinline__ void append_fp64(const DevNet<Real>& n, bool need, int r, int pr) {
+__device__ __forceinline__ void append_entry(const DevNet<Real>& n, int* list, int* count, bool need, int a, int b) {
     const unsigned m = __ballot_sync(0xffffffffu, need);
     if (!m) return;
     const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
     int base = 0;
-    if (lane == leader) base = atomicAdd(n.ev_list_count, __popc(m));
+    if (lane == leader) base = atomicAdd(count, __popc(m));
     base = __shfl_sync(0xffffffffu, base, leader);
     if (need) {
         const int k = base + __popc(m & ((1u << lane) - 1u));
         if (k < 2 * n.n_ev) {   // room for both trials of a two-trial pass
-            n.ev_list[2 * k] = r;
-            n.ev_list[2 * k + 1] = pr;
+            list[2 * k] = a;
+            list[2 * k + 1] = b;
         } else {
             atomicOr(n.err, 4u);
         }
     }
 }
+// (replica, pair) to the extended-pass pair list
+template <typename Real>
+__device__ __forceinline__ void append_fp64(const DevNet<Real>& n, bool need, int r, int pr) {
+    append_entry(n, n.ev_list, n.ev_list_count, need, r, pr);
+}
+
+// How the mixed engine forms a pair's forces.  The reference moves c2 0.01 nm
+// along the unit normal of (c1, c2, c3) when it judges the pair coplanar
+// (|n . v3| < 0.1 with n = (c2-c1) x (c3-c1), v3 = c4 - c1; :610-626).  Pairs
+// whose test single precision cannot decide, and ill-conditioned ones (q), go
+// to the extended pass; the others are moved here (with q >= kMixedTauForce the
+// move leaves them well conditioned).
+struct ForceCase {
+    bool ill;             // to the extended pass
+    float nx, ny, nz;     // -n
+    float nn, cop;        // |n|, the reference's test
+};
+__device__ __forceinline__ ForceCase force_case(const float* v12, const float* v31, const float* v14, float q) {
+    ForceCase c;
+    c.nx = v12[1] * v31[2] - v12[2] * v31[1];
+    c.ny = v12[2] * v31[0] - v12[0] * v31[2];
+    c.nz = v12[0] * v31[1] - v12[1] * v31[0];
+    c.nn = sqrtf(c.nx * c.nx + c.ny * c.ny + c.nz * c.nz);
+    c.cop = fabsf(c.nx * v14[0] + c.ny * v14[1] + c.nz * v14[2]) / (c.nn * sqrtf(dot3(v14, v14)));
+    c.ill = !(q >= kMixedTauForce) || !(fabsf(c.cop - 0.1f) >= 2e-3f);
+    return c;
+}
 
 // Mixed engine: the energy of one pair in single precision, or need64 when the
 // pair is ill-conditioned (normalized triple product under kMixedTauEnergy) or
-// the formula gives no number; such pairs go to the extended pass.
+// the formula gives no number; such pairs go to the extended pass.  With `list`
+// also whether the pair's forces would.
 __device__ __forceinline__ float mixed_pair_energy(const Pos<float>& p1, const Pos<float>& p2, const Pos<float>& p3,
-                                                   const Pos<float>& p4, float kRep, bool& need64) {
+                                                   const Pos<float>& p4, float kRep, bool& need64, bool list,
+                                                   bool& ill) {
     float v12[3], v34[3], v31[3], v14[3], v32[3], v24[3];
     pdiff(p2, p1, v12);
     pdiff(p4, p3, v34);
@@ -289,6 +318,7 @@ __device__ __forceinline__ float mixed_pair_energy(const Pos<float>& p1, const P
                 cz = v12[0] * v34[1] - v12[1] * v34[0];
     const float trip = fabsf(cx * v31[0] + cy * v31[1] + cz * v31[2]);
     const float q = trip / (sqrtf(dot3(v12, v12)) * sqrtf(dot3(v34, v34)) * sqrtf(dot3(v31, v31)));
+    if (list) ill = force_case(v12, v31, v14, q).ill;
     need64 = !(q >= kMixedTauEnergy);
     if (need64) return 0.f;
     PairInv<float> pi;
@@ -576,9 +606,11 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
     const int i = t.begin + threadIdx.x;
     const bool valid = i < t.end;
     float ef = 0.f;
-    bool need64 = false, need64b = false;
+    bool need64 = false, need64b = false, ill = false, illb = false;
     // a pass with a second trial also evaluates the energy at lambda / 2
     const bool dual = !force && second_trial(trial, s.dual);
+    // position buffers of the trials
+    const int buf = (s.xb + 1) % 3, bufb = (s.xb + 2) % 3;
     if (valid) {
         const int4 bs = n.ev_bead[i];
         auto pos = [&](int b) -> Pos<float> { return bead_at(X, dir, b, tr, s.lam); };
@@ -586,16 +618,17 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
         if (!force) {
             // mixed engine: single precision unless the pair is ill-conditioned
             const float kRep = n.ev_k[i] * n.ev_la[i] * n.ev_lb[i];
-            ef = mixed_pair_energy(p1, p2, p3, p4, kRep, need64);
+            ef = mixed_pair_energy(p1, p2, p3, p4, kRep, need64, n.prelist, ill);
             store_pair(n.ev_energy + i, ef, 0.f);
             if (dual) {
                 const float lh = 0.5f * s.lam;
                 const float ef2 = mixed_pair_energy(bead_at(X, dir, bs.x, true, lh), bead_at(X, dir, bs.y, true, lh),
                                                     bead_at(X, dir, bs.z, true, lh), bead_at(X, dir, bs.w, true, lh),
-                                                    kRep, need64b);
+                                                    kRep, need64b, n.prelist, illb);
                 store_pair(n.ev_energy2 + i, ef2, 0.f);
             }
-        } else {
+            if (n.prelist) n.ev_mark[i] = (uint8_t)((ill << buf) | (illb << bufb));
+        } else if (!n.prelist || !(n.ev_mark[i] >> s.xb & 1)) {
             // mixed engine, forces: single precision unless the pair is ill-conditioned
             const float kRep = n.ev_k[i] * n.ev_la[i] * n.ev_lb[i];
             float v12[3], v34[3], v31[3], v14[3], v32[3], v24[3];
@@ -609,26 +642,14 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
                         cz = v12[0] * v34[1] - v12[1] * v34[0];
             const float trip = fabsf(cx * v31[0] + cy * v31[1] + cz * v31[2]);
             const float q = trip / (sqrtf(dot3(v12, v12)) * sqrtf(dot3(v34, v34)) * sqrtf(dot3(v31, v31)));
-            need64 = !(q >= (force ? kMixedTauForce : kMixedTauEnergy));
-            if (force && !need64) {
-                // the reference moves c2 0.01 nm along the unit normal of (c1, c2, c3)
-                // when it judges the pair coplanar (|n . v3| < 0.1 with
-                // n = (c2-c1) x (c3-c1), v3 = c4 - c1; :610-626).  Pairs whose test
-                // single precision cannot decide go to the extended pass; the others are moved
-                // here (with q >= kMixedTauForce the move leaves them well conditioned).
-                const float nx = v12[1] * v31[2] - v12[2] * v31[1], ny = v12[2] * v31[0] - v12[0] * v31[2],
-                            nz = v12[0] * v31[1] - v12[1] * v31[0];   // = -n
-                const float nn = sqrtf(nx * nx + ny * ny + nz * nz);
-                const float cop = fabsf(nx * v14[0] + ny * v14[1] + nz * v14[2]) / (nn * sqrtf(dot3(v14, v14)));
-                if (!(fabsf(cop - 0.1f) >= 2e-3f)) {
-                    need64 = true;
-                } else if (cop < 0.1f) {
-                    const float push = -0.01f / nn;
-                    const float dx = push * nx, dy = push * ny, dz = push * nz;   // c2 moves by +0.01 n / |n|
-                    v12[0] += dx; v12[1] += dy; v12[2] += dz;
-                    v32[0] += dx; v32[1] += dy; v32[2] += dz;
-                    v24[0] -= dx; v24[1] -= dy; v24[2] -= dz;
-                }
+            const ForceCase fc = force_case(v12, v31, v14, q);
+            need64 = n.prelist ? false : fc.ill;
+            if (!need64 && fc.cop < 0.1f) {
+                const float push = -0.01f / fc.nn;
+                const float dx = push * fc.nx, dy = push * fc.ny, dz = push * fc.nz;   // c2 moves by +0.01 n / |n|
+                v12[0] += dx; v12[1] += dy; v12[2] += dz;
+                v32[0] += dx; v32[1] += dy; v32[2] += dz;
+                v24[0] -= dx; v24[1] -= dy; v24[2] -= dz;
             }
             if (!need64) {
                 PairInv<float> pi;
@@ -647,6 +668,10 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
     }
     append_fp64(n, need64, r, i);
     if (dual) append_fp64(n, need64b, r, i | kExtSecond);   // block-uniform
+    if (n.prelist && !force) {
+        append_entry(n, n.ev_flist, n.ev_flist_count, ill, r | buf << kListBuffer, i);
+        if (dual) append_entry(n, n.ev_flist, n.ev_flist_count, illb, r | bufb << kListBuffer, i);
+    }
     release_next(n);
 }
 
@@ -674,7 +699,7 @@ struct ExtTerm {
 };
 
 template <typename Real>
-__global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, int force) {
+__global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, int force, int listed) {
     pdl_wait();      // the listing pass has finished
     MECH_TRACE_KERNEL(n, TK_EXVOL_EXT);
     __shared__ double s_c[4][32][3];       // bead positions
@@ -682,22 +707,30 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
     __shared__ ExtTerm s_t[4][32];
     __shared__ double s_G[6][32];
     __shared__ int s_bad[32];
-    const int cnt = min(*n.ev_list_count, 2 * n.n_ev);
+    const int* list = listed ? n.ev_flist : n.ev_list;
+    const int cnt = min(listed ? *n.ev_flist_count : *n.ev_list_count, 2 * n.n_ev);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int ngroups = (cnt + 31) >> 5;
     for (int g = blockIdx.x; g < ngroups; g += gridDim.x) {
         const int k = 32 * g + l;
-        const bool valid = k < cnt;
+        bool valid = k < cnt;
         int r = 0, i = 0;
         bool second = false;   // the lambda / 2 trial of a two-trial pass
         double lam = 0.0;
         LaneState<Real> ls{};
         if (valid) {
-            r = n.ev_list[2 * k];
-            i = n.ev_list[2 * k + 1];
-            second = (i & kExtSecond) != 0;
-            i &= ~kExtSecond;
-            ls = lane_state(n, r, -1);
+            r = list[2 * k];
+            i = list[2 * k + 1];
+            if (listed) {   // of the accepted trial
+                const int buf = r >> kListBuffer;
+                r &= (1 << kListBuffer) - 1;
+                ls = lane_state(n, r, PH_FORCE);
+                valid = ls.go && ls.xb == buf;
+            } else {
+                second = (i & kExtSecond) != 0;
+                i &= ~kExtSecond;
+                ls = lane_state(n, r, -1);
+            }
             lam = ls.lambda;
             if (second) lam *= 0.5;
         }
@@ -743,12 +776,14 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
                     }
                 }
             }
-            a = dot3(v12, v12);
-            b = dot3(v34, v34);
-            c = dot3(v31, v31);
-            d = dot3(v12, v34);
-            e = dot3(v12, v31);
-            F = dot3(v34, v31);
+            if (force) {
+                a = dot3(v12, v12);
+                b = dot3(v34, v34);
+                c = dot3(v31, v31);
+                d = dot3(v12, v34);
+                e = dot3(v12, v31);
+                F = dot3(v34, v31);
+            }
             x21[0] = v34[1] * v12[2] - v34[2] * v12[1];
             x21[1] = v34[2] * v12[0] - v34[0] * v12[2];
             x21[2] = v34[0] * v12[1] - v34[1] * v12[0];
@@ -945,12 +980,14 @@ static inline int ev_tiles_of(const DevNet<Real>& n, int* off) {
 // Inside an evaluation (standalone = false) the work-list counts are zero on
 // entry: the evaluation's reduction kernel zeroes them for the next one, which
 // keeps a memset off the head of the excluded-volume lane.  A standalone
-// launch zeroes them first and leaves them as they end.  `done`, unless null, is
-// recorded behind the chain.
+// launch zeroes them first and leaves them as they end.  `L`, unless null, are
+// the evaluation's lanes: `s` is the side lane, and L->join is recorded behind
+// the chain.
 template <typename Real>
-int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t s, bool standalone, cudaEvent_t done) {
+int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t s, bool standalone, const Lanes* L) {
     int off = 0;
     const int nt = ev_tiles_of(n, &off);
+    const cudaEvent_t done = L ? L->join : nullptr;
     if (nt == 0) {
         if (done) cudaEventRecord(done, s);
         return 0;
@@ -962,7 +999,7 @@ int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t
         launch_k(false, nullptr, k_exvol_fp64<Real>, 2 * (nt - split) + 8 * split, 128, s, n, want, trial, 0, off, nt - split);
     } else {
         launch_k(false, nullptr, k_exvol<Real>, nt, kBlock, s, n, want, trial, 0, off);
-        launch_k(n.pdl, nullptr, k_exvol_ext<Real>, kExtBlocks, 128, s, n, trial, 0);
+        launch_k(n.pdl, nullptr, k_exvol_ext<Real>, kExtBlocks, 128, s, n, trial, 0, 0);
         ++k;
     }
     launch_k(n.pdl, n.pdl ? done : nullptr, k_exvol_energy_tail<Real>, kFbEnergyBlocks + nt, kBlock, s, n, want, trial, off);
@@ -971,9 +1008,10 @@ int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t
 }
 
 template <typename Real>
-int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool standalone, cudaEvent_t done) {
+int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool standalone, const Lanes* L) {
     int off = 0;
     const int nt = ev_tiles_of(n, &off);
+    const cudaEvent_t done = L ? L->join : nullptr;
     if (nt == 0) {
         if (done) cudaEventRecord(done, s);
         return 0;
@@ -985,15 +1023,21 @@ int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool st
         launch_k(false, nullptr, k_exvol_fp64<Real>, 2 * (nt - split) + 8 * split, 128, s, n, want, 0, 1, off, nt - split);
     } else {
         launch_k(false, nullptr, k_exvol<Real>, nt, kBlock, s, n, want, 0, 1, off);
-        launch_k(n.pdl, nullptr, k_exvol_ext<Real>, kExtBlocks, 128, s, n, 0, 1);
+        if (n.prelist) {
+            cudaStreamWaitEvent(L->side3, L->fork, 0);
+            launch_k(false, L->join3, k_exvol_ext<Real>, kExtBlocks, 128, L->side3, n, 0, 1, 1);
+            ++k;
+        }
+        launch_k(n.pdl, nullptr, k_exvol_ext<Real>, kExtBlocks, 128, s, n, 0, 1, 0);
         ++k;
+        if (n.prelist) cudaStreamWaitEvent(s, L->join3, 0);
     }
     launch_k(n.pdl, n.pdl ? done : nullptr, k_exvol_fb_force<Real>, kFbForceBlocks, kBlock, s, n, n.fb_moments, n.fb_tickets);
     if (done && !n.pdl) cudaEventRecord(done, s);
     return k + 1;
 }
 
-template int launch_exvol_energy<MECH_EXVOL_REAL>(const DevNet<MECH_EXVOL_REAL>&, int, int, cudaStream_t, bool, cudaEvent_t);
-template int launch_exvol_forces<MECH_EXVOL_REAL>(const DevNet<MECH_EXVOL_REAL>&, int, cudaStream_t, bool, cudaEvent_t);
+template int launch_exvol_energy<MECH_EXVOL_REAL>(const DevNet<MECH_EXVOL_REAL>&, int, int, cudaStream_t, bool, const Lanes*);
+template int launch_exvol_forces<MECH_EXVOL_REAL>(const DevNet<MECH_EXVOL_REAL>&, int, cudaStream_t, bool, const Lanes*);
 
 }  // namespace mech

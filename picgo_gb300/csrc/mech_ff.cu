@@ -119,6 +119,7 @@ __device__ void after_evaluation(const DevNet<Real>& n, int phase_slot, int* s_f
     if (threadIdx.x == 0) {
         if (n.ev_list_count) *n.ev_list_count = 0;
         if (n.ev_fb_count) *n.ev_fb_count = 0;
+        if (n.prelist && phase_slot == kCondForce) *n.ev_flist_count = 0;
     }
     if (n.cond.on) set_conditions(n, false, phase_slot);
 }
@@ -1331,8 +1332,8 @@ static int launch_lanes(const DevNet<Real>& n, int want, int trial, bool force, 
     cudaStreamWaitEvent(L.side2, L.fork, 0);
     if (n.fil_first[force]) fil();
     int launched = 1;
-    launched += force ? launch_exvol_forces<Real>(n, want, L.side, false, L.join)
-                      : launch_exvol_energy<Real>(n, want, trial, L.side, false, L.join);
+    launched += force ? launch_exvol_forces<Real>(n, want, L.side, false, &L)
+                      : launch_exvol_energy<Real>(n, want, trial, L.side, false, &L);
     if (lm + bb_t > 0) {
         launch_k(false, n.pdl ? L.join2 : nullptr, k_bond_bnd<Real>, lm + bb_t, kBlock, L.side2, n, want, trial,
                  force ? 1 : 0, lm, ev_t);

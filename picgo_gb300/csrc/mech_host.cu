@@ -65,9 +65,9 @@ struct MechContext {
     int device = 0;
     int precision = MECH_PREC_FP64;
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr, side2 = nullptr;      // lanes of the sparse force fields
-    cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
-    Lanes lanes() const { return Lanes{stream, side, side2, fork, join, join2}; }
+    cudaStream_t side = nullptr, side2 = nullptr, side3 = nullptr;   // lanes of the sparse force fields
+    cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr, join3 = nullptr;
+    Lanes lanes() const { return Lanes{stream, side, side2, side3, fork, join, join2, join3}; }
     int R = 0;
     int nb = 0, ncyl = 0, nlk = 0, nmt = 0, nplanes = 0;
     long long nev = 0, nbb = 0, nbcyl = 0;
@@ -82,7 +82,7 @@ struct MechContext {
     // boundary
     DeviceBuffer planes, planes_f, plane_k, plane_slen, bb_k, bb_slen;
     // excluded volume
-    DeviceBuffer ev_bead, ev_k, ev_la, ev_lb, ev_list, ev_list_count, ev_energy, ev_energy2;
+    DeviceBuffer ev_bead, ev_k, ev_la, ev_lb, ev_list, ev_list_count, ev_energy, ev_energy2, ev_mark, ev_flist;
     // tiles, partials, state
     DeviceBuffer ftile, stile, stile_kind, rt, part_fil, part_df, part_sp, part_sp2, st, ticket, gticket, cond_counter;
     int graph_mode = MECH_GRAPH_UNROLLED;
@@ -171,8 +171,10 @@ struct MechContext {
         if (fork) cudaEventDestroy(fork);
         if (join) cudaEventDestroy(join);
         if (join2) cudaEventDestroy(join2);
+        if (join3) cudaEventDestroy(join3);
         if (side) cudaStreamDestroy(side);
         if (side2) cudaStreamDestroy(side2);
+        if (side3) cudaStreamDestroy(side3);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -203,6 +205,9 @@ DevNet<Real> make_devnet(MechContext* c) {
     n.xbest = c->xbest.as<Real>();
     n.ev_list = c->ev_list.as<int>();
     n.ev_list_count = c->ev_list_count.as<int>();
+    n.ev_mark = c->ev_mark.as<uint8_t>();
+    n.ev_flist = c->ev_flist.as<int>();
+    n.ev_flist_count = c->ev_list_count.as<int>() + 1;
     n.ev_energy = c->ev_energy.as<double>();
     n.ev_energy2 = c->ev_energy2.as<double>();
     n.bflag = c->bflag.as<uint8_t>();
@@ -941,6 +946,10 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
     CU(c->ev_lb.ensure(rs * std::max<long long>(P, 1)));
     // the extended-pass list holds up to two entries per pair (both trials of a two-trial pass)
     CU(c->ev_list.ensure(sizeof(int) * 4 * std::max<long long>(P, 1)));
+    if (c->precision == MECH_PREC_MIXED) {
+        CU(c->ev_mark.ensure(std::max<long long>(P, 1)));
+        CU(c->ev_flist.ensure(sizeof(int) * 4 * std::max<long long>(P, 1)));
+    }
     CU(c->ev_energy.ensure(sizeof(double) * std::max<long long>(P, 1)));
     CU(c->ev_energy2.ensure(sizeof(double) * std::max<long long>(P, 1)));
     CU(c->ev_list_count.ensure(sizeof(int) * 4));
@@ -1106,6 +1115,7 @@ static int iteration_graph(MechContext* c, int which) {
     auto& ig = c->iter[which];
     DevNet<Real> n = make_devnet<Real>(c);
     n.snap = c->snap[0].word;
+    n.prelist = c->precision == MECH_PREC_MIXED && n.n_ev > 0 ? 1 : 0;
     std::vector<unsigned char> key(sizeof(n) + sizeof(int));
     std::memcpy(key.data(), &n, sizeof(n));
     std::memcpy(key.data() + sizeof(n), &c->graph_mode, sizeof(int));
@@ -1490,9 +1500,11 @@ int32_t mech_ctx_create(int32_t precision, int32_t device, MechContext** out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, prio_greatest);
     if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&c->side2, cudaStreamNonBlocking, prio_greatest);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&c->side3, cudaStreamNonBlocking, prio_greatest);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join2, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join3, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         delete c;
         return set_err(MECH_ERR_CUDA, cudaGetErrorString(e));
@@ -1506,6 +1518,7 @@ int32_t mech_ctx_destroy(MechContext* ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->side);
     cudaStreamSynchronize(ctx->side2);
+    cudaStreamSynchronize(ctx->side3);
     cudaStreamSynchronize(ctx->stream);
     delete ctx;
     return MECH_OK;

@@ -43,6 +43,7 @@ constexpr int kFbChunks = 64;       // work split of one numeric force fallback
 constexpr int kTrialDual = 2;
 constexpr int kTrialBoth = 3;   // (profiling) as kTrialDual with a second trial for every replica
 // the ext-pass list marks entries of the second trial with this bit of the pair index
+constexpr int kListBuffer = 28;   // bits of the replica in an entry of ev_flist
 constexpr int kExtSecond = 1 << 30;
 
 enum Kind : int { K_LINKER = 0, K_MOTOR = 1, K_EXVOL = 2, K_BOUNDARY = 3, K_NUM_SPARSE = 4 };
@@ -186,6 +187,16 @@ struct DevNet {
     int* fb_tickets;        // [cap]
     // mixed precision: pairs evaluated in FP64 (compacted list) and per-pair energies
     int* ev_list; int* ev_list_count; double* ev_energy;
+    // iteration graphs of the mixed engine (prelist): a line-search pass decides
+    // at its trial positions which pairs' forces go to the extended pass, so
+    // that in the force pass that follows it, at the accepted trial, this pass
+    // runs beside the single-precision one (12 us of 54 per iteration of 60k
+    // cylinders, whose force pass waited 5 us for the list first; 54.4 -> 47.4,
+    // 32 replicas 93.7 -> 86, 1M cylinders in a long run 127.2 -> 121.3).  Per
+    // pair one bit per position buffer, and the list of
+    // (replica | buffer << kListBuffer, pair)
+    int prelist;
+    uint8_t* ev_mark; int* ev_flist; int* ev_flist_count;
     // mixed-precision line-search passes at lambda and lambda / 2: the second
     // trial's per-pair excluded-volume energies and sparse tile partials
     double* ev_energy2; double* part_sp2;
@@ -377,8 +388,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // `main`; `fork` starts them, `join` / `join2` end them, then the reduction
 // runs on `main`.
 struct Lanes {
-    cudaStream_t main, side, side2;
-    cudaEvent_t fork, join, join2;
+    cudaStream_t main, side, side2, side3;
+    cudaEvent_t fork, join, join2, join3;
     // the reduction before this evaluation has recorded `fork` (programmatic launch)
     bool forked = false;
 };
@@ -407,9 +418,9 @@ int set_error_text(int code, const std::string& msg);
 // (standalone: zero the work-list counts first; inside an evaluation they are
 // zero on entry, reset by the evaluation's reduction kernel)
 template <typename Real> int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t s,
-                                                 bool standalone, cudaEvent_t done = nullptr);
+                                                 bool standalone, const Lanes* L = nullptr);
 template <typename Real> int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool standalone,
-                                                 cudaEvent_t done = nullptr);
+                                                 const Lanes* L = nullptr);
 
 // ---- Hessian-vector products and solves (mech_hvp.cu, FP64 engine) --------
 // hv = (H + shift I) v at the positions in x[0], v and hv in internal bead
