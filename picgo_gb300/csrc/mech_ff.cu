@@ -231,12 +231,8 @@ __global__ void __launch_bounds__(kBlock) k_fil_energy(DevNet<double> n, int wan
 // cylinders' vectors and squared lengths instead of forming them again.
 // Bound by the FP64 pipe, where a warp with three active lanes costs as much as
 // a full one: a block of 256 beads has 259 cylinders and 258 triples, nine warps
-// of each.  A single network, whose beads may be cut anywhere (no sum crosses a
-// bead here), takes 253 a block: eight warps of each (1M beads: 214 -> 190 us).
-constexpr int kForceBeads = kFilTile - 3;
-inline int force_blocks(const DevNet<double>& n) {
-    return n.R == 1 ? (n.nb + kForceBeads - 1) / kForceBeads : n.n_ftiles;
-}
+// of each; no sum crosses a bead here, and a block takes 253 beads
+// (kForceBeads), eight warps of each (1M beads: 214 -> 190 us).
 __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want) {
     pdl_wait();      // the previous kernel of the main lane has finished
     MECH_TRACE_KERNEL(n, TK_FIL_FORCE);
@@ -244,8 +240,7 @@ __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want
     __shared__ double rs[3][kFilTile + 3], Ls[kFilTile + 3];        // cylinders begin - 2 .. end: vector, L^2
     __shared__ double fs[3][kFilTile + 3];                          // their stretching forces on the second bead
     __shared__ double f1[3][kFilTile + 2], f2[3][kFilTile + 2];     // triples on begin - 1 .. end
-    const int own = (int)blockIdx.x * kForceBeads;
-    const Tile t = n.R == 1 ? Tile{0, own, min(own + kForceBeads, n.nb), 0} : fil_tile(n, blockIdx.x);
+    const Tile t = force_tile(n, blockIdx.x);
     const LaneState<double> s = lane_state(n, t.replica, want);
     if (!s.go) return;
     const int T = t.end - t.begin;
@@ -677,10 +672,10 @@ __device__ __forceinline__ int4 descriptor(const Tile& t, const LaneState<float>
                      (s.go ? 1 : 0) | (s.xb << 1) | (s.fb << 3) | (s.dual ? 16 : 0) | (s.dPending << 5) |
                          (s.dIsF << 6) | (s.dbuf << 7) | (backup << 8));
 }
-__device__ __forceinline__ void load_descriptors(const DevNet<float>& n, int t0, int nt, int want, int4* desc,
-                                                 float2* step) {
+__device__ __forceinline__ void load_descriptors(const DevNet<float>& n, bool force, int t0, int nt, int want,
+                                                 int4* desc, float2* step) {
     for (int k = threadIdx.x; k < nt; k += blockDim.x) {
-        const Tile t = fil_tile(n, t0 + k);
+        const Tile t = force ? force_tile(n, t0 + k) : fil_tile(n, t0 + k);
         const LaneState<float> s = lane_state(n, t.replica, want);
         desc[k] = descriptor(t, s, n.st[t.replica].backupPending);
         step[k] = make_float2(s.lam, s.beta);
@@ -726,12 +721,13 @@ __device__ void issue_energy_stage(const DevNet<float>& n, int4 t, bool tr, Ener
 // range [t0, t1): tiles are ordered by replica, so a range whose first and
 // last tiles share a replica belongs to it alone.  The block then exits before
 // any barrier or descriptor setup.
-__device__ __forceinline__ bool idle_range(const DevNet<float>& n, int t0, int t1, int want, int* s_flag) {
+__device__ __forceinline__ bool idle_range(const DevNet<float>& n, const Tile* tiles, int t0, int t1, int want,
+                                           int* s_flag) {
     if (n.R == 1) return t1 <= t0 || !lane_state(n, 0, want).go;   // the same in every thread
     if (threadIdx.x == 0) {
         int idle = t1 <= t0;
         if (!idle) {
-            const int ra = n.ftile[t0].replica, rb = n.ftile[t1 - 1].replica;
+            const int ra = tiles[t0].replica, rb = tiles[t1 - 1].replica;
             idle = ra == rb && !replica_selected(n.st[ra], want);
         }
         *s_flag = idle;
@@ -753,7 +749,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
     const int t0 = blockIdx.x * n.ptiles[0], t1 = min(t0 + n.ptiles[0], n.n_ftiles);
     const int nt = t1 - t0;
     const bool tr = trial != 0;
-    if (idle_range(n, t0, t1, want, &s_abort)) return;
+    if (idle_range(n, n.ftile, t0, t1, want, &s_abort)) return;
     if (threadIdx.x == 0) {
         for (int k = 0; k < kBulkStages; ++k) mbar_init(&bar[k], 1);
         mbar_init_fence();
@@ -763,7 +759,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
         if (threadIdx.x == 0) atomicOr(n.err, 16u);
         return;
     }
-    load_descriptors(n, t0, nt, want, s_desc, s_step);
+    load_descriptors(n, false, t0, nt, want, s_desc, s_step);
     __syncthreads();
     // producer state (thread 0): next tile to consider, copies issued
     int pi = 0, issued = 0;
@@ -987,7 +983,10 @@ __device__ void issue_force_stage(const DevNet<float>& n, int4 t, ForceStage* st
 // (two-bead halo), the constants and flags of its beads and their neighbours
 // arrive by cp.async.bulk like k_fil_energy_bulk; every bead's filament force
 // is written to the force buffer, where k_force_gather adds the bead's sparse
-// contributions and forms the CG partials.
+// contributions and forms the CG partials.  A tile is 254 beads (kForceBeads):
+// with 256 the block's first warp ran the term phase a second time for the two
+// slots beyond, and the other seven waited for it (iteration of the 1M-cylinder
+// network 121.1 -> 119.6 us, of 32 replicas 85.5 -> 84.4 us).
 __global__ void __launch_bounds__(kBlock) k_fil_force_bulk(DevNet<float> n, int want) {
     pdl_wait();      // the previous kernel of the main lane has finished
     MECH_TRACE_KERNEL(n, TK_FIL_FORCE_BULK);
@@ -999,9 +998,9 @@ __global__ void __launch_bounds__(kBlock) k_fil_force_bulk(DevNet<float> n, int 
     // per tile: stretching force of each cylinder (q, q + 1) and the two bending
     // terms of each triple centred on q, for q = tile begin - 1 .. tile end
     __shared__ float s_st[kFilTile + 2][3], s_a1[kFilTile + 2][3], s_a2[kFilTile + 2][3];
-    const int t0 = blockIdx.x * n.ptiles[1], t1 = min(t0 + n.ptiles[1], n.n_ftiles);
+    const int t0 = blockIdx.x * n.ptiles[1], t1 = min(t0 + n.ptiles[1], n.n_force_tiles);
     const int nt = t1 - t0;
-    if (idle_range(n, t0, t1, want, &s_abort)) return;
+    if (idle_range(n, n.ftile_force, t0, t1, want, &s_abort)) return;
     if (threadIdx.x == 0) {
         for (int k = 0; k < kBulkStages; ++k) mbar_init(&bar[k], 1);
         mbar_init_fence();
@@ -1011,7 +1010,7 @@ __global__ void __launch_bounds__(kBlock) k_fil_force_bulk(DevNet<float> n, int 
         if (threadIdx.x == 0) atomicOr(n.err, 16u);
         return;
     }
-    load_descriptors(n, t0, nt, want, s_desc, s_step);
+    load_descriptors(n, true, t0, nt, want, s_desc, s_step);
     __syncthreads();
     int pi = 0, issued = 0;
     if (threadIdx.x == 0) {
@@ -1364,7 +1363,7 @@ int launch_forces(const DevNet<Real>& n, int want, const Lanes& L) {
     const int k = launch_lanes(n, want, 0, true, L, [&] {
         if constexpr (sizeof(Real) == 4)
             launch_k(L.forked, nullptr, k_fil_force_bulk, n.pgrid[1], kBlock, L.main, n, want);
-        else launch_k(L.forked, nullptr, k_fil_force, force_blocks(n), kBlock, L.main, n, want);
+        else launch_k(L.forked, nullptr, k_fil_force, n.n_force_tiles, kBlock, L.main, n, want);
     });
     launch_gather(n, want, L.main, n.pdl);
     launch_k(n.pdl, n.pdl ? L.fork : nullptr, k_finalize_force<Real>, n.R, kBlock, L.main, n, want);
@@ -1411,7 +1410,7 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
             return 1;
         case 1:
             if constexpr (sizeof(Real) == 4) k_fil_force_bulk<<<n.pgrid[1], kBlock, 0, s>>>(n, -1);
-            else k_fil_force<<<force_blocks(n), kBlock, 0, s>>>(n, -1);
+            else k_fil_force<<<n.n_force_tiles, kBlock, 0, s>>>(n, -1);
             launch_gather(n, -1, s, false);
             k_finalize_force<Real><<<n.R, kBlock, 0, s>>>(n, -1);
             return 3;
@@ -1424,7 +1423,7 @@ int launch_part(const DevNet<Real>& n, int which, cudaStream_t s) {
             return 1;
         case 5:   // filament forces alone
             if constexpr (sizeof(Real) == 4) k_fil_force_bulk<<<n.pgrid[1], kBlock, 0, s>>>(n, -1);
-            else k_fil_force<<<force_blocks(n), kBlock, 0, s>>>(n, -1);
+            else k_fil_force<<<n.n_force_tiles, kBlock, 0, s>>>(n, -1);
             return 1;
         case 6:   // the sparse gather with the CG partials alone
             launch_gather(n, -1, s, false);

@@ -96,7 +96,7 @@ struct MechContext {
     // Hessian-vector products, adjoint and Newton solves (FP64 engine)
     DeviceBuffer hv_a, hv_b, cg_x, cg_r, cg_p, cg_Ap, cg_scal, cg_part, cg_ticket, hess_fil, hess_lm, hess_ev, hess_bb;
     DeviceBuffer lf_ends, lf_types, lf_ms, lf_nm, lf_out;   // load forces
-    int n_ftiles = 0, n_stiles = 0;
+    int n_ftiles = 0, n_force_tiles = 0, n_stiles = 0;
     int sp_tiles[K_NUM_SPARSE] = {0, 0, 0, 0};
     // host copies of the full tile lists, and the compacted view that a
     // batched minimization switches to once most replicas have finished
@@ -104,7 +104,7 @@ struct MechContext {
     std::vector<int> h_skind;
     DeviceBuffer ftile_c, stile_c, stile_kind_c, rt_c;
     bool compact = false;
-    int n_ftiles_c = 0, n_stiles_c = 0;
+    int n_ftiles_c = 0, n_force_tiles_c = 0, n_stiles_c = 0;
     // tuning (mech_autotune): tiles per block of the mixed filament energy and
     // force kernels, and a multiplier on the default neighbor-list bin edge
     int tile_cap[2] = {kFilBulkMaxTiles, kFilBulkMaxTiles};
@@ -215,19 +215,22 @@ DevNet<Real> make_devnet(MechContext* c) {
     n.n_ftiles = c->compact ? c->n_ftiles_c : c->n_ftiles;
     n.gtiles = n.n_ftiles < 152 * kGatherTiles ? 1 : kGatherTiles;
     n.ftile = (c->compact ? c->ftile_c : c->ftile).as<Tile>();
+    n.n_force_tiles = c->compact ? c->n_force_tiles_c : c->n_force_tiles;
+    n.ftile_force = n.ftile + n.n_ftiles;   // behind them in the same buffer
     for (int k = 0; k < 2; ++k) {
         const int per_sm = c->blocks_per_sm[k];
         n.fil_first[k] = (c->precision == MECH_PREC_MIXED && per_sm > 0) ? 1 : 0;
         const int resident = persistent_blocks(c->device, k, per_sm);
-        n.pgrid[k] = std::max(1, std::min(n.n_ftiles, resident));
-        n.ptiles[k] = (n.n_ftiles + n.pgrid[k] - 1) / n.pgrid[k];
+        const int tiles = k == 0 ? n.n_ftiles : n.n_force_tiles;
+        n.pgrid[k] = std::max(1, std::min(tiles, resident));
+        n.ptiles[k] = (tiles + n.pgrid[k] - 1) / n.pgrid[k];
         // the bulk-staged energy/force kernels keep a block's tile descriptors in
         // shared memory (at most kFilBulkMaxTiles); a tuned smaller run length adds
         // waves, unless a residency cap is set, which the grid then keeps to
         n.ptiles[k] = std::max(1, std::min(n.ptiles[k], c->tile_cap[k]));
-        if (per_sm > 0) n.ptiles[k] = std::max(n.ptiles[k], (n.n_ftiles + resident - 1) / resident);
+        if (per_sm > 0) n.ptiles[k] = std::max(n.ptiles[k], (tiles + resident - 1) / resident);
         n.ptiles[k] = std::min(n.ptiles[k], kFilBulkMaxTiles);
-        n.pgrid[k] = (n.n_ftiles + n.ptiles[k] - 1) / n.ptiles[k];
+        n.pgrid[k] = (tiles + n.ptiles[k] - 1) / n.ptiles[k];
     }
     n.n_lk = c->nlk;
     n.n_mt = c->nmt;
@@ -511,6 +514,14 @@ const int* perm_of(MechContext* c, int r) { return c->perm_all.as<int>() + c->re
 // round bead ranges outward to 16-byte multiples and may read into it
 static constexpr size_t kBulkPad = 256;
 
+// The force kernel's tiles of replica r, behind the filament tiles (make_devnet).
+static void add_force_tiles(const MechContext* c, int r, std::vector<Tile>& ft) {
+    const ReplicaHost& h = c->reps[r];
+    const int step = c->precision == MECH_PREC_FP64 ? kForceBeads<double> : kForceBeads<float>;
+    for (int b = 0; b < h.nb; b += step)
+        ft.push_back(Tile{r, h.bead_begin + b, h.bead_begin + std::min(h.nb, b + step), 0});
+}
+
 static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
     if (R <= 0 || !nets) return set_err(MECH_ERR_ARG, "no networks");
     c->reps.assign(R, ReplicaHost());
@@ -728,9 +739,11 @@ static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
     c->n_ftiles = (int)ft.size();
     c->h_ftiles = ft;
     c->compact = false;
-    if ((rc = upload(c->ftile, ft, s))) return rc;
     CU(c->part_fil.ensure(sizeof(double) * 4 * ft.size()));
     CU(c->part_df.ensure(sizeof(double) * ft.size()));
+    for (int r = 0; r < R; ++r) add_force_tiles(c, r, ft);
+    c->n_force_tiles = (int)ft.size() - c->n_ftiles;
+    if ((rc = upload(c->ftile, ft, s))) return rc;
     // states
     CU(c->st.ensure(sizeof(CGState) * R + 16));
     CU(cudaMemsetAsync(c->st.p, 0, sizeof(CGState) * R + 16, s));
@@ -1254,6 +1267,10 @@ static int compact_tiles(MechContext* c, const std::vector<char>& active) {
         rt[r].fil_end = (int)ft.size();
         rt[r].n_beads = full.n_beads;
     }
+    c->n_ftiles_c = (int)ft.size();
+    for (int r = 0; r < c->R; ++r)
+        if (active[r]) add_force_tiles(c, r, ft);
+    c->n_force_tiles_c = (int)ft.size() - c->n_ftiles_c;
     for (int k = 0; k < K_NUM_SPARSE; ++k) {
         const int t0 = (int)st.size();
         for (int r = 0; r < c->R; ++r) {
@@ -1270,7 +1287,6 @@ static int compact_tiles(MechContext* c, const std::vector<char>& active) {
     if ((rc = upload(c->ftile_c, ft, c->stream)) || (rc = upload(c->stile_c, st, c->stream)) ||
         (rc = upload(c->stile_kind_c, kind, c->stream)) || (rc = upload(c->rt_c, rt, c->stream)))
         return rc;
-    c->n_ftiles_c = (int)ft.size();
     c->n_stiles_c = (int)st.size();
     c->compact = true;
     return MECH_OK;

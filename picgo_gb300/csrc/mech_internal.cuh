@@ -30,6 +30,7 @@
 namespace mech {
 
 constexpr int kFilTile = 256;     // beads per filament tile (one block)
+template <typename Real> constexpr int kForceBeads = sizeof(Real) == 8 ? kFilTile - 3 : kFilTile - 2;   // of the force kernel (force_tile)
 constexpr int kGatherTiles = 4;   // filament tiles per block of the force gather kernels
 constexpr int kSparseTile = 256;  // interactions per sparse tile (one block)
 constexpr int kFilBulkMaxTiles = 64;   // filament tiles per block of the bulk-staged mixed kernels
@@ -158,6 +159,7 @@ struct DevNet {
     // block `ptiles` consecutive tiles on a grid of `pgrid` blocks
     int n_ftiles;
     const Tile* ftile;
+    int n_force_tiles; const Tile* ftile_force;   // the same for the force kernel (force_tile)
     int pgrid[2], ptiles[2];   // [0] energy, [1] force kernels
     int fil_first[2];          // energy / force: filament kernel launched before the side lanes (capped residency)
     // sparse interactions (internal bead indices)
@@ -292,6 +294,17 @@ __device__ __forceinline__ Tile fil_tile(const DevNet<Real>& n, int ti) {
         return Tile{0, b, min(b + kFilTile, n.nb), 0};
     }
     return n.ftile[ti];
+}
+// Tile `ti` of the filament force kernel, which forms no sum over a tile: its
+// tiles are cut so that the cylinders (FP64) or term slots (mixed) that they
+// touch beyond their own beads fill a block's threads once.
+template <typename Real>
+__device__ __forceinline__ Tile force_tile(const DevNet<Real>& n, int ti) {
+    if (n.R == 1) {
+        const int b = ti * kForceBeads<Real>;
+        return Tile{0, b, min(b + kForceBeads<Real>, n.nb), 0};
+    }
+    return n.ftile_force[ti];
 }
 template <typename Real>
 __device__ __forceinline__ Tile sparse_tile(const DevNet<Real>& n, int ti, int* kind) {
