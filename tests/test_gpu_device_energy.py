@@ -51,3 +51,31 @@ def test_device_energy_at_block_edges(name, theta0):
                                                        C.c_void_p(torch.cuda.current_stream().cuda_stream)))
     want, scale = reference(fcs, x, ks, l0, kb, t0)
     assert np.all(np.abs(out.cpu().numpy() - want) <= 1e-12 * scale), (out, want)
+
+
+SHARES = {
+    "filaments without cylinders": [0, 0, 3, 0, 5, 0, 0, 40, 1, 0, 31, 0, 0, 0, 64, 0],
+    "more of them than a read": [7] + [0] * 70 + [90, 0, 2],
+    "a chunk": [32], "over a chunk": [33], "a chunk and a start": [32, 32, 1],
+    "one share each": [17] * 9156, "two chunks in some": [40] * 3900, "long shares": [997] * 500, "one filament": [300001],
+}
+
+
+@pytest.mark.parametrize("name", SHARES)
+def test_device_energy_at_share_edges(name):
+    """The same where a warp's share of the 32-cylinder chunks begins, ends and passes from one chunk to the next."""
+    torch = pytest.importorskip("torch")
+    fcs = np.concatenate([[0], np.cumsum(SHARES[name])]).astype(np.int32)
+    n, nfil = int(fcs[-1]), len(fcs) - 1
+    rng = np.random.default_rng(n)
+    x = np.cumsum(rng.normal(0, 60, (n + nfil, 3)) + [40, 0, 0], axis=0) % 5000.0
+    ks, l0, kb = rng.uniform(50, 150, n), rng.uniform(80, 130, n), rng.uniform(300, 900, n)
+    t0 = np.zeros(n)
+    dev = [torch.from_numpy(a).cuda() for a in (fcs, x, ks, l0, kb, t0)]
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())   # noqa: E731
+    for _ in range(2):
+        _lib.check(_lib.load().mech_filament_energy_device(nfil, n, *[p(t) for t in dev], p(out),
+                                                           C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    want, scale = reference(fcs, x, ks, l0, kb, t0)
+    assert np.all(np.abs(out.cpu().numpy() - want) <= 1e-11 * scale), (out, want)
