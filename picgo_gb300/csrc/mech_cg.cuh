@@ -286,13 +286,13 @@ __device__ void finalize_force(const DevNet<Real>& n, int r, const RepTiles& rt,
         // mixed slots hold float maxima and (hi, lo) pairs; sum them compensated
         // in single precision and form the doubles in thread 0 only
         FF a[2];
-        float m[1] = {0.f};
+        float m = 0.f;
 #pragma unroll 4
         for (int k = threadIdx.x; k < nslot; k += blockDim.x) {
             const float* p = reinterpret_cast<const float*>(n.part_fil + 4 * (size_t)run_slot(rt.fil_begin, stride, k));
             const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
             const float w = __ldcg(p + 4);
-            m[0] = fmaxf(m[0], v.x);
+            m = fmaxf(m, v.x);
             a[0].add(v.y);
             a[0].add(v.z);
             a[1].add(v.w);
@@ -300,29 +300,40 @@ __device__ void finalize_force(const DevNet<Real>& n, int r, const RepTiles& rt,
         }
         MECH_TRACE_SECTION(n, TK_SEC_FF_LOAD, ts_load);
         MECH_TRACE_STAMP(ts_red);
-        block_reduce_pairs<2, 1>(a, m, reinterpret_cast<float*>(sh));
+        // the maxima, none negative, are ordered like their bits
+        unsigned* s_mx = reinterpret_cast<unsigned*>(sh + 32);
+        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+        if ((threadIdx.x & 31) == 0) s_mx[threadIdx.x >> 5] = wm;
+        const FF s = block_pair_sums<2>(a, reinterpret_cast<float*>(sh));   // its barrier publishes s_mx
+        const double sum = (double)s.h + (double)s.l;
+        ff = sum;
+        ffp = __shfl_sync(0xffffffffu, sum, 1);
         MECH_TRACE_SECTION(n, TK_SEC_FF_REDUCE, ts_red);
         if (threadIdx.x != 0) return;
-        mx = (double)m[0];
-        ff = (double)a[0].h + (double)a[0].l;
-        ffp = (double)a[1].h + (double)a[1].l;
+        unsigned bm = 0;
+#pragma unroll
+        for (int k = 0; k < kBlock / 32; ++k) bm = max(bm, s_mx[k]);
+        mx = (double)__uint_as_float(bm);
     } else {
-        double a_mx = 0.0, a_ff = 0.0, a_ffp = 0.0;
+        unsigned long long a_mx = 0;
+        double a_ff = 0.0, a_ffp = 0.0;
 #pragma unroll 8
         for (int k = threadIdx.x; k < nslot; k += blockDim.x) {
             const int i = run_slot(rt.fil_begin, stride, k);
             const double2 v = __ldcg(reinterpret_cast<const double2*>(n.part_fil + 4 * (size_t)i));
             const double w = __ldcg(n.part_fil + 4 * (size_t)i + 2);
-            a_mx = fmax(a_mx, v.x);
+            a_mx = max(a_mx, (unsigned long long)__double_as_longlong(v.x));
             a_ff += v.y;
             a_ffp += w;
         }
-        double red[3] = {warp_max(a_mx), warp_sum(a_ff), warp_sum(a_ffp)};
-        const int ops[3] = {1, 0, 0};
-        block_combine<3>(red, ops, sh);
-        mx = red[0];
-        ff = red[1];
-        ffp = red[2];
+        // the maxima, none negative, are ordered like their bits, off the FP64 pipe
+        unsigned long long m[1] = {a_mx};
+        const unsigned long long bm = block_maxima<1>(m, reinterpret_cast<unsigned long long*>(sh));
+        double v[2] = {a_ff, a_ffp};
+        const double s = block_sums<2>(v, sh + 32);
+        mx = __longlong_as_double((long long)bm);
+        ff = s;
+        ffp = __shfl_sync(0xffffffffu, s, 1);
         if (threadIdx.x != 0) return;
     }
     MECH_TRACE_STAMP(ts_tail);

@@ -66,28 +66,6 @@ __device__ __forceinline__ double block_max(double v, double* sh) {
     return r;
 }
 
-// Combine per-warp results (valid in lane 0 of each warp) over the block in a
-// fixed order; results valid in thread 0.  op[k]: 0 sum, 1 max.
-// `sh` holds at least 32 * N doubles.
-template <int N>
-__device__ __forceinline__ void block_combine(double (&w)[N], const int (&op)[N], double* sh) {
-    const int wi = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    __syncthreads();
-    if (l == 0) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) sh[k * 32 + wi] = w[k];
-    }
-    __syncthreads();
-    if (wi == 0) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            double r = l < nw ? sh[k * 32 + l] : (op[k] ? -1.0 / 0.0 : 0.0);
-            r = op[k] ? warp_max(r) : warp_sum(r);
-            w[k] = r;
-        }
-    }
-}
-
 // Sums of N values (a power of two) over each warp and then the block: the
 // first steps of the trees halve the number of values a lane carries, so N
 // trees take N + 3 additions (N = 4: 6) where one after another they take 5 N.
@@ -430,65 +408,12 @@ struct FF {
         fast_two_sum(s, lo, h, l);
     }
 };
-// warp sum of (h, l) pairs in place, result in lane 0
-__device__ __forceinline__ void warp_reduce_pair(float& s, float& e) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float s2 = __shfl_down_sync(0xffffffffu, s, o), e2 = __shfl_down_sync(0xffffffffu, e, o);
-        float t, te;
-        two_sum(s, s2, t, te);
-        te = __fadd_rn(te, __fadd_rn(e, e2));
-        fast_two_sum(t, te, s, e);
-    }
-}
-__device__ __forceinline__ float warp_max_f(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_down_sync(0xffffffffu, v, o));
-    return v;
-}
-// Block reduction with no double arithmetic: N compensated pairs and M maxima
-// of non-negative floats (`m` may be null when M is 0), in a fixed order;
-// results valid in thread 0.  A warp's FP64 instruction holds its sub-
-// partition's FP64 pipe for ~78 cycles on this part, so a per-tile double tree
-// costs more than the tile's loads.  `sh` holds 32 * (2N + M) floats.
-template <int N, int M>
-__device__ __forceinline__ void block_reduce_ff(FF (&a)[N], float* m, float* sh) {
-    const int wi = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < N; ++k) warp_reduce_pair(a[k].h, a[k].l);
-#pragma unroll
-    for (int k = 0; k < M; ++k) m[k] = warp_max_f(m[k]);
-    __syncthreads();
-    if (l == 0) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            sh[(2 * k) * 32 + wi] = a[k].h;
-            sh[(2 * k + 1) * 32 + wi] = a[k].l;
-        }
-#pragma unroll
-        for (int k = 0; k < M; ++k) sh[(2 * N + k) * 32 + wi] = m[k];
-    }
-    __syncthreads();
-    if (wi == 0) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            a[k].h = l < nw ? sh[(2 * k) * 32 + l] : 0.f;
-            a[k].l = l < nw ? sh[(2 * k + 1) * 32 + l] : 0.f;
-            warp_reduce_pair(a[k].h, a[k].l);
-        }
-#pragma unroll
-        for (int k = 0; k < M; ++k) m[k] = warp_max_f(l < nw ? sh[(2 * N + k) * 32 + l] : 0.f);
-    }
-}
-template <int N, int M>
-__device__ __forceinline__ void block_reduce_pairs(FF (&a)[N], float (&m)[M], float* sh) {
-    block_reduce_ff<N, M>(a, m, sh);
-}
-
-// Sums of N compensated pairs (a power of two, at most 32) over the block with
-// the trees of block_reduce_ff, packed as in block_sums: N pair additions per
-// warp where N trees take 5 N.  Lane t < N of warp 0 gets pair t.  `sh` holds
-// 2 N kBlock / 32 floats.
+// Sums of N compensated pairs (a power of two, at most 32) over a warp: the trees
+// packed as in block_sums, N pair additions (and a few) where N trees take 5 N.
+// Every lane gets the sum, in a[0], of the pair whose number is returned: lane
+// 32 k / N that of one of the N.  No double arithmetic: a warp's FP64 instruction
+// holds its sub-partition's FP64 pipe for ~78 cycles on this part, so a per-tile
+// double tree costs more than the tile's loads.
 __device__ __forceinline__ void add_pairs(FF& a, float h, float l) {
     float t, te;
     two_sum(a.h, h, t, te);
@@ -496,8 +421,8 @@ __device__ __forceinline__ void add_pairs(FF& a, float h, float l) {
     fast_two_sum(t, te, a.h, a.l);
 }
 template <int N>
-__device__ __forceinline__ FF block_pair_sums(FF (&a)[N], float* sh) {
-    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+__device__ __forceinline__ int warp_pair_sums(FF (&a)[N]) {
+    const int l = threadIdx.x & 31;
     int idx = 0, o = 16;
 #pragma unroll
     for (int h = N / 2; h >= 1; h >>= 1, o >>= 1) {
@@ -514,6 +439,14 @@ __device__ __forceinline__ FF block_pair_sums(FF (&a)[N], float* sh) {
 #pragma unroll
     for (; o >= 1; o >>= 1)
         add_pairs(a[0], __shfl_xor_sync(0xffffffffu, a[0].h, o), __shfl_xor_sync(0xffffffffu, a[0].l, o));
+    return idx;
+}
+// The same over the block: lane t < N of warp 0 gets pair t.  `sh` holds
+// 2 N kBlock / 32 floats.
+template <int N>
+__device__ __forceinline__ FF block_pair_sums(FF (&a)[N], float* sh) {
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int idx = warp_pair_sums<N>(a);
     if ((l & (32 / N - 1)) == 0) {
         sh[2 * (w * N + idx)] = a[0].h;
         sh[2 * (w * N + idx) + 1] = a[0].l;
@@ -569,48 +502,8 @@ __device__ __forceinline__ Pos<float> split(const double x[3]) {
 }
 
 // ---------------------------------------------------------------------------
-// Reductions of per-thread values of the engine's precision.  FP64: plain
-// double tree.  Mixed: float pairs (hi, lo) summed with error-free
-// transformations within each warp, then double across warps and tiles.
+// Maximum of per-thread values of the engine's precision, in thread 0.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double warp_sum_ff(float v) {
-    float s = v, e = 0.f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float s2 = __shfl_down_sync(0xffffffffu, s, o), e2 = __shfl_down_sync(0xffffffffu, e, o);
-        float t, te;
-        two_sum(s, s2, t, te);
-        te = __fadd_rn(te, __fadd_rn(e, e2));
-        fast_two_sum(t, te, s, e);
-    }
-    double r = 0.0;
-    if ((threadIdx.x & 31) == 0) r = (double)s + (double)e;
-    return r;
-}
-__device__ __forceinline__ double warp_sum_r(double v) { return warp_sum(v); }
-__device__ __forceinline__ double warp_sum_r(float v) { return warp_sum_ff(v); }
-__device__ __forceinline__ double warp_max_r(double v) { return warp_max(v); }
-__device__ __forceinline__ double warp_max_r(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_down_sync(0xffffffffu, v, o));
-    double r = 0.0;
-    if ((threadIdx.x & 31) == 0) r = (double)v;
-    return r;
-}
-__device__ __forceinline__ double block_sum_r(double v, double* sh) { return block_sum(v, sh); }
-__device__ __forceinline__ double block_sum_r(float v, double* sh) {
-    const double w = warp_sum_ff(v);
-    const int wi = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) sh[wi] = w;
-    __syncthreads();
-    double r = 0.0;
-    if (wi == 0) {
-        r = (l < (blockDim.x >> 5)) ? sh[l] : 0.0;
-        r = warp_sum(r);
-    }
-    return r;
-}
 __device__ __forceinline__ double block_max_r(double v, double* sh) { return block_max(v, sh); }
 __device__ __forceinline__ double block_max_r(float v, double* sh) {
 #pragma unroll

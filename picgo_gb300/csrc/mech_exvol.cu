@@ -920,7 +920,7 @@ template <typename Real>
 __global__ void __launch_bounds__(kBlock) k_exvol_energy_tail(DevNet<Real> n, int want, int trial, int tile_off) {
     pdl_wait();      // the per-pair energies are complete
     MECH_TRACE_KERNEL(n, TK_EXVOL_TAIL);
-    __shared__ double sh[64];   // block_reduce_ff<2>: 32 * 4 floats
+    __shared__ double sh[32];   // block_pair_sums<2>: 32 floats
     if ((int)blockIdx.x < kFbEnergyBlocks) {
         fb_energy_blocks(n, blockIdx.x, kFbEnergyBlocks, sh);
     } else {
@@ -939,16 +939,13 @@ __global__ void __launch_bounds__(kBlock) k_exvol_energy_tail(DevNet<Real> n, in
                         add_pair(a[0], load_pair(n.ev_energy + i));
                         add_pair(a[1], load_pair(n.ev_energy2 + i));
                     }
-                    block_reduce_ff<2, 0>(a, nullptr, reinterpret_cast<float*>(sh));
-                    if (threadIdx.x == 0) {
-                        store_pair(n.part_sp + ti, a[0].h, a[0].l);
-                        store_pair(n.part_sp2 + ti, a[1].h, a[1].l);
-                    }
+                    const FF se = block_pair_sums<2>(a, reinterpret_cast<float*>(sh));
+                    if (threadIdx.x < 2) store_pair((threadIdx.x ? n.part_sp2 : n.part_sp) + ti, se.h, se.l);
                 } else {
                     FF a[1];
                     if (i < t.end) add_pair(a[0], load_pair(n.ev_energy + i));
-                    block_reduce_ff<1, 0>(a, nullptr, reinterpret_cast<float*>(sh));
-                    if (threadIdx.x == 0) store_pair(n.part_sp + ti, a[0].h, a[0].l);
+                    const FF se = block_pair_sums<1>(a, reinterpret_cast<float*>(sh));
+                    if (threadIdx.x == 0) store_pair(n.part_sp + ti, se.h, se.l);
                 }
             }
         } else if (go) {

@@ -521,16 +521,14 @@ __global__ void __launch_bounds__(kBlock) k_force_gather_mx(DevNet<float> n, int
             }
         }
     }
-    warp_reduce_pair(aff.h, aff.l);
-    warp_reduce_pair(affp.h, affp.l);
-    mx = warp_max_f(mx);
+    FF sums[2] = {aff, affp};
+    const int which = warp_pair_sums<2>(sums);   // lane 0: F.F, lane 16: F.Fprev
+    const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));   // none negative: ordered like the bits
     const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-        sh[w][0] = aff.h;
-        sh[w][1] = aff.l;
-        sh[w][2] = affp.h;
-        sh[w][3] = affp.l;
-        sh[w][4] = mx;
+    if ((threadIdx.x & 15) == 0) {
+        sh[w][2 * which] = sums[0].h;
+        sh[w][2 * which + 1] = sums[0].l;
+        sh[w][4] = __uint_as_float(wm);
     }
     __syncthreads();
     const int j0 = threadIdx.x;
@@ -607,13 +605,16 @@ __global__ void __launch_bounds__(kBlock, 1) k_finalize_energy(DevNet<Real> n, i
 // first tile; the reduction kernel that follows the evaluation reads them.
 // a: stretching, bending, d . F and, with a second trial, its stretching and bending.
 template <int N>
-__device__ __forceinline__ void write_run(const DevNet<float>& n, int first, FF (&a)[N], double* sh) {
-    block_reduce_ff<N, 0>(a, nullptr, reinterpret_cast<float*>(sh));
-    if (threadIdx.x == 0) {
+__device__ __forceinline__ void write_run(const DevNet<float>& n, int first, const FF (&a)[N], float* sh) {
+    constexpr int P = N <= 4 ? 4 : 8;   // the packed trees take a power of two
+    FF v[P];
 #pragma unroll
-        for (int k = 0; k < N; ++k)
-            store_pair(k == 2 ? n.part_df + first : n.part_fil + 4 * (size_t)first + (k < 2 ? k : k - 1), a[k].h, a[k].l);
-    }
+    for (int k = 0; k < N; ++k) v[k] = a[k];
+    const FF s = block_pair_sums<P>(v, sh);
+    const int k = threadIdx.x;
+    if (k < N)
+        store_pair(k == 2 ? n.part_df + first : n.part_fil + 4 * (size_t)first + (k < 2 ? k : k - 1), s.h, s.l);
+    __syncthreads();   // `sh` may be used again
 }
 
 // ---------------------------------------------------------------------------
@@ -743,7 +744,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
     __shared__ __align__(8) uint64_t bar[kBulkStages];
     __shared__ int4 s_desc[kBulkMaxTiles];
     __shared__ float2 s_step[kBulkMaxTiles];
-    __shared__ double sh[32 * 5];   // block_reduce_ff<5>: 32 * 10 floats
+    __shared__ float sh[2 * 8 * kBlock / 32];   // block_pair_sums<8>
     __shared__ __align__(16) float s_mv[6 * kBulkXBeads];   // the staged beads moved to a trial
     __shared__ int s_abort;
     const int t0 = blockIdx.x * n.ptiles[0], t1 = min(t0 + n.ptiles[0], n.n_ftiles);
@@ -1104,7 +1105,7 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
                                                      int ev_tiles) {
     pdl_wait();      // the reduction before this evaluation has finished
     MECH_TRACE_KERNEL(n, TK_BOND);
-    __shared__ double sh[64];   // block_reduce_ff<2>: 32 * 4 floats
+    __shared__ double sh[32];   // block_pair_sums<2>: 32 floats
     const int ti = blockIdx.x < n_lm_tiles ? blockIdx.x : blockIdx.x + ev_tiles;
     int kind;
     const Tile t = sparse_tile(n, ti, &kind);
@@ -1189,19 +1190,16 @@ __global__ void __launch_bounds__(kBlock) k_bond_bnd(DevNet<Real> n, int want, i
                 FF a[2];
                 a[0].h = e;
                 a[1].h = e2;
-                block_reduce_ff<2, 0>(a, nullptr, reinterpret_cast<float*>(sh));
-                if (threadIdx.x == 0) {
-                    store_pair(n.part_sp + ti, a[0].h, a[0].l);
-                    store_pair(n.part_sp2 + ti, a[1].h, a[1].l);
-                }
+                const FF se = block_pair_sums<2>(a, reinterpret_cast<float*>(sh));
+                if (threadIdx.x < 2) store_pair((threadIdx.x ? n.part_sp2 : n.part_sp) + ti, se.h, se.l);
             } else {
                 FF a[1];
                 a[0].h = e;
-                block_reduce_ff<1, 0>(a, nullptr, reinterpret_cast<float*>(sh));
-                if (threadIdx.x == 0) store_pair(n.part_sp + ti, a[0].h, a[0].l);
+                const FF se = block_pair_sums<1>(a, reinterpret_cast<float*>(sh));
+                if (threadIdx.x == 0) store_pair(n.part_sp + ti, se.h, se.l);
             }
         } else {
-            const double se = block_sum_r(e, sh);
+            const double se = block_sum(e, sh);
             if (threadIdx.x == 0) n.part_sp[ti] = se;
         }
     }
