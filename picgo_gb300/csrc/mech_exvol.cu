@@ -357,44 +357,26 @@ inline int exvol_split_tiles(int nt) {
 struct SplitTerm {
     double tC, tX, te, ta;    // partials of the term (forces)
     double S;                 // N / Y * ATG
+    double q[3];              // the quotients by Y that G takes (forces)
 };
+enum SplitDot { SD_a, SD_b, SD_c, SD_d, SD_e, SD_F, SD_g, SD_h, SD_I, SD_D2, SD_E2, SD_JJ, SD_N };
 struct SplitShared {
     double c[4][3][32];       // bead positions; c2 moved off the plane for forces
-    double N[4][32];          // CC, GG, DD (HH = CC + GG - DD)
+    double d[SD_N][32];       // the products of pair_inv (cross = false)
+    double N[3][32];          // CC, GG, DD (HH = CC + GG - DD)
     SplitTerm t[4][32];
-    double Y[4][32];
     double G[6][32];          // G00, G01, G02, G11, G12, G22
+    double J[6][32];          // the same of J
+    double pref[32], m[32];   // kRep / (2 JJ), -S / JJ
     int bad[32];
 };
 
-// The invariants that every warp forms (pair_inv, cross = false).
-struct SplitInv {
-    double v12[3], v34[3], v31[3];
-    double a, b, c, d, e, F, JJ;
-};
-__device__ __forceinline__ void split_invariants(const SplitShared& s, int l, SplitInv& p) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        p.v12[k] = s.c[1][k][l] - s.c[0][k][l];
-        p.v34[k] = s.c[3][k][l] - s.c[2][k][l];
-        p.v31[k] = s.c[0][k][l] - s.c[2][k][l];
-    }
-    p.a = dot3(p.v12, p.v12);
-    p.b = dot3(p.v34, p.v34);
-    p.c = dot3(p.v31, p.v31);
-    p.d = dot3(p.v12, p.v34);
-    p.e = dot3(p.v12, p.v31);
-    p.F = dot3(p.v34, p.v31);
-    const double* v12 = p.v12;
-    const double* v34 = p.v34;
-    const double* v31 = p.v31;
-    const double x21[3] = {v34[1] * v12[2] - v34[2] * v12[1], v34[2] * v12[0] - v34[0] * v12[2],
-                           v34[0] * v12[1] - v34[1] * v12[0]};
-    const double trip = -(x21[0] * v31[0] + x21[1] * v31[1] + x21[2] * v31[2]);
-    p.JJ = -trip * trip;
-}
-
-// 32 pairs [i0, min(i0 + 32, end)) of replica r in a block of four warps.
+// 32 pairs [i0, min(i0 + 32, end)) of replica r in a block of four warps.  The
+// pass takes as long as the longest warp's FP64 instructions, so what more than
+// one warp needs is formed by one of them, in steps of about equal length, and
+// for forces what does not hang on c2 while one warp decides on its move (78
+// pairs, in an iteration: energy 12.2 -> 10.8 us, forces 20.4 -> 18.1 us, against
+// every warp forming the products, J and the factors for itself).
 template <typename Real>
 __device__ void exvol_split(const DevNet<Real>& n, int r, const Real* X, const Direction<Real>& dir, bool tr, double lam,
                             int force, int i0, int end, SplitShared& s) {
@@ -410,55 +392,115 @@ __device__ void exvol_split(const DevNet<Real>& n, int r, const Real* X, const D
     }
     if (w == 0) s.bad[l] = 0;
     __syncthreads();
-    if (force) {   // the reference's move of c2, decided and applied by one warp
-        if (w == 1 && valid) {
-            double c[4][3], m[3];
+    auto diff = [&](int a, int b, double v[3]) {   // bead a - bead b
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+        for (int k = 0; k < 3; ++k) v[k] = s.c[a][k][l] - s.c[b][k][l];
+    };
+    double v12[3], v34[3], v31[3];
+    if (force) {
+        if (valid) {
+            if (w == 1) {   // the reference's move of c2, decided and applied
+                double c[4][3], m[3];
 #pragma unroll
-                for (int k = 0; k < 3; ++k) c[a][k] = s.c[a][k][l];
-            if (nearly_coplanar(c[0], c[1], c[2], c[3])) {
-                push_c2(c[0], c[1], c[2], m);
+                for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int k = 0; k < 3; ++k) s.c[1][k][l] = m[k];
+                    for (int k = 0; k < 3; ++k) c[a][k] = s.c[a][k][l];
+                if (nearly_coplanar(c[0], c[1], c[2], c[3])) {
+                    push_c2(c[0], c[1], c[2], m);
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) s.c[1][k][l] = m[k];
+                }
+            } else if (w == 0) {
+                diff(0, 2, v31);
+                s.d[SD_c][l] = dot3(v31, v31);
+            } else if (w == 2) {
+                diff(3, 2, v34);
+                diff(0, 2, v31);
+                s.d[SD_b][l] = dot3(v34, v34);
+                s.d[SD_F][l] = dot3(v34, v31);
+            } else {
+                double v14[3];
+                diff(3, 0, v14);
+                diff(3, 2, v34);
+                s.d[SD_D2][l] = dot3(v14, v14);
+                s.d[SD_I][l] = dot3(v34, v14);
             }
         }
         __syncthreads();
     }
-    SplitInv p;
-    double Y = 1, N = 0, ATG = 0, al = 0, be = 0;
     if (valid) {
-        split_invariants(s, l, p);
-        // term w: Y, N and the two abscissae (A, E, B, F of the reference)
-        double u = p.a, v = p.c, x = p.e;   // Y = sqrt((sqrt(u v) + x) (sqrt(u v) - x))
-        al = p.a + p.e;
-        be = p.e;
         if (w == 0) {
-            N = p.d * p.e - p.a * p.F;
+            diff(1, 0, v12);
+            diff(3, 2, v34);
+            diff(0, 2, v31);
+            s.d[SD_a][l] = dot3(v12, v12);
+            const double x21[3] = {v34[1] * v12[2] - v34[2] * v12[1], v34[2] * v12[0] - v34[0] * v12[2],
+                                   v34[0] * v12[1] - v34[1] * v12[0]};
+            const double trip = -(x21[0] * v31[0] + x21[1] * v31[1] + x21[2] * v31[2]);
+            s.d[SD_JJ][l] = -trip * trip;
         } else if (w == 1) {
             double v14[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) v14[k] = s.c[3][k][l] - s.c[0][k][l];
-            v = dot3(v14, v14);
-            x = dot3(p.v12, v14);
-            N = p.d * x - p.a * dot3(p.v34, v14);
-            al = p.a + p.e - p.d;
-            be = p.e - p.d;
+            diff(1, 0, v12);
+            diff(3, 0, v14);
+            s.d[SD_g][l] = dot3(v12, v14);
+            if (!force) {
+                diff(3, 2, v34);
+                s.d[SD_D2][l] = dot3(v14, v14);
+                s.d[SD_I][l] = dot3(v34, v14);
+            }
         } else if (w == 2) {
-            u = p.b;
-            x = p.F;
-            N = p.b * p.e - p.d * p.F;
-            al = p.F;
-            be = p.F - p.b;
+            diff(1, 0, v12);
+            diff(3, 2, v34);
+            diff(0, 2, v31);
+            s.d[SD_d][l] = dot3(v12, v34);
+            s.d[SD_e][l] = dot3(v12, v31);
+            if (!force) s.d[SD_c][l] = dot3(v31, v31);
         } else {
             double v32[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) v32[k] = s.c[1][k][l] - s.c[2][k][l];
-            u = p.b;
-            v = dot3(v32, v32);
-            x = dot3(p.v34, v32);
-            al = p.d + p.F;
-            be = p.d + p.F - p.b;
+            diff(1, 2, v32);
+            diff(3, 2, v34);
+            s.d[SD_E2][l] = dot3(v32, v32);
+            s.d[SD_h][l] = dot3(v34, v32);
+            if (!force) {
+                diff(0, 2, v31);
+                s.d[SD_b][l] = dot3(v34, v34);
+                s.d[SD_F][l] = dot3(v34, v31);
+            }
+        }
+    }
+    __syncthreads();
+    double a = 0, b = 0, c = 0, d = 0, e = 0, F = 0, Y = 1, N = 0, ATG = 0, al = 0, be = 0;
+    if (valid) {
+        a = s.d[SD_a][l];
+        b = s.d[SD_b][l];
+        c = s.d[SD_c][l];
+        d = s.d[SD_d][l];
+        e = s.d[SD_e][l];
+        F = s.d[SD_F][l];
+        // term w: Y, N and the two abscissae (A, E, B, F of the reference)
+        double u = a, v = c, x = e;   // Y = sqrt((sqrt(u v) + x) (sqrt(u v) - x))
+        al = a + e;
+        be = e;
+        if (w == 0) {
+            N = d * e - a * F;
+        } else if (w == 1) {
+            v = s.d[SD_D2][l];
+            x = s.d[SD_g][l];
+            N = d * x - a * s.d[SD_I][l];
+            al = a + e - d;
+            be = e - d;
+        } else if (w == 2) {
+            u = b;
+            x = F;
+            N = b * e - d * F;
+            al = F;
+            be = F - b;
+        } else {
+            u = b;
+            v = s.d[SD_E2][l];
+            x = s.d[SD_h][l];
+            al = d + F;
+            be = d + F - b;
         }
         const double uv = sqrt(u * v);
         Y = sqrt(fmax(0.0, (uv + x) * (uv - x)));
@@ -470,71 +512,80 @@ __device__ void exvol_split(const DevNet<Real>& n, int r, const Real* X, const D
         if (w == 3) N = s.N[0][l] + s.N[1][l] - s.N[2][l];
         SplitTerm t;
         t.S = N / Y * ATG;
-        t.tC = t.tX = t.te = t.ta = 0.0;
+        t.tC = t.tX = t.te = t.ta = t.q[0] = t.q[1] = t.q[2] = 0.0;
         if (force) {
             const double T1 = Y * Y / (Y * Y + al * al), T2 = Y * Y / (Y * Y + be * be);
             t.tC = ATG / Y;
             t.tX = -(ATG * N) / (Y * Y) + (-T1 * al + T2 * be) * N / (Y * Y * Y);
             t.te = (T1 - T2) * N / (Y * Y);
             t.ta = T1 * N / (Y * Y);
+            t.q[0] = (w == 0 ? c : w == 1 ? b + c - 2 * F : b) / Y;
+            t.q[1] = (w == 0 ? -e : w == 1 ? e - d : w == 2 ? c : -(d + F)) / Y;
+            t.q[2] = (w == 0 || w == 1 ? a : w == 2 ? -F : a + c + 2 * e) / Y;
         }
         s.t[w][l] = t;
-        s.Y[w][l] = Y;
     }
     __syncthreads();
-    const double kRep = valid ? (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i] : 0.0;
     if (!force) {
         if (w == 0 && valid) {
-            const double U = 0.5 * kRep / p.JJ * (s.t[0][l].S + s.t[1][l].S + s.t[2][l].S + s.t[3][l].S);
+            const double kRep = (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i];
+            const double U = 0.5 * kRep / s.d[SD_JJ][l] * (s.t[0][l].S + s.t[1][l].S + s.t[2][l].S + s.t[3][l].S);
             const bool ok = !(bad_value(U) || U < -1.0);
             n.ev_energy[i] = ok ? U : 0.0;
             if (!ok) flag_fallback(n, r, i, tr ? lam : 0.0);
         }
         return;
     }
-    if (valid) {   // entries of G, split over the warps
+    if (valid) {   // entries of G and J and the factors, split over the warps
         const SplitTerm A = s.t[0][l], E = s.t[1][l], B = s.t[2][l], T = s.t[3][l];
-        const double AA = s.Y[0][l], EE = s.Y[1][l], BB = s.Y[2][l], FF = s.Y[3][l];
-        const double a = p.a, b = p.b, c = p.c, d = p.d, e = p.e, F = p.F;
         if (w == 0) {
-            s.G[0][l] = A.tC * (-2 * F) + A.tX * (c / AA) + A.ta * 2 + E.tC * (2 * (F - b)) + E.tX * ((b + c - 2 * F) / EE) +
-                        E.ta * 2 + T.tC * (-2 * b) + T.tX * (b / FF);
-            s.G[5][l] = A.tX * (a / AA) + E.tX * (a / EE) + B.tX * (b / BB) + T.tX * (b / FF);
+            s.G[0][l] = A.tC * (-2 * F) + A.tX * A.q[0] + A.ta * 2 + E.tC * (2 * (F - b)) + E.tX * E.q[0] + E.ta * 2 +
+                        T.tC * (-2 * b) + T.tX * T.q[0];
+            s.G[5][l] = A.tX * A.q[2] + E.tX * E.q[2] + B.tX * B.q[0] + T.tX * T.q[0];
+            s.J[5][l] = 2 * (d * d - a * b);
         } else if (w == 1) {
-            s.G[1][l] = A.tC * e + E.tC * (2 * d - e) + E.tX * ((e - d) / EE) + E.te * (-1) + B.tC * (-F) +
-                        T.tC * (2 * d + F) + T.tX * (-(d + F) / FF) + T.te;
-            s.G[2][l] = A.tC * d + A.tX * (-e / AA) + A.te + E.tC * (-d) + E.tX * (-(e - d) / EE) + E.te + B.tC * b +
-                        T.tC * (-b) + T.tX * (b / FF);
+            s.G[1][l] = A.tC * e + E.tC * (2 * d - e) + E.tX * E.q[1] + E.te * (-1) + B.tC * (-F) + T.tC * (2 * d + F) +
+                        T.tX * T.q[1] + T.te;
+            s.G[2][l] = A.tC * d + A.tX * A.q[1] + A.te + E.tC * (-d) + E.tX * (-E.q[1]) + E.te + B.tC * b + T.tC * (-b) +
+                        T.tX * T.q[0];
         } else if (w == 2) {
-            s.G[3][l] = E.tC * (-2 * a) + E.tX * (a / EE) + B.tC * (2 * e) + B.tX * (c / BB) + B.te * (-2) + B.ta * 2 +
-                        T.tC * (-2 * (a + e)) + T.tX * ((a + c + 2 * e) / FF) + T.te * (-2) + T.ta * 2;
+            s.G[3][l] = E.tC * (-2 * a) + E.tX * E.q[2] + B.tC * (2 * e) + B.tX * B.q[1] + B.te * (-2) + B.ta * 2 +
+                        T.tC * (-2 * (a + e)) + T.tX * T.q[2] + T.te * (-2) + T.ta * 2;
+            s.J[3][l] = 2 * (-a * c + e * e);
+            s.J[4][l] = 2 * (-d * e + a * F);
+            s.J[0][l] = 2 * (-b * c + F * F);
         } else {
-            s.G[4][l] = A.tC * (-a) + E.tC * a + E.tX * (-a / EE) + B.tC * (-d) + B.tX * (-F / BB) + B.te + T.tC * d +
-                        T.tX * (-(d + F) / FF) + T.te;
+            s.G[4][l] = A.tC * (-a) + E.tC * a + E.tX * (-E.q[2]) + B.tC * (-d) + B.tX * B.q[2] + B.te + T.tC * d +
+                        T.tX * T.q[1] + T.te;
+            s.J[1][l] = 2 * (c * d - e * F);
+            s.J[2][l] = 2 * (b * e - d * F);
+            const double kRep = (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i];
+            const double invJJ = 1.0 / s.d[SD_JJ][l];
+            const double S = A.S + E.S + B.S + T.S;
+            s.pref[l] = kRep * invJJ / 2.0;
+            s.m[l] = -invJJ * S;
         }
     }
     __syncthreads();
     if (valid) {   // warp w: the force on bead w
-        const double a = p.a, b = p.b, c = p.c, d = p.d, e = p.e, F = p.F;
         const double G[3][3] = {{s.G[0][l], s.G[1][l], s.G[2][l]}, {s.G[1][l], s.G[3][l], s.G[4][l]}, {s.G[2][l], s.G[4][l], s.G[5][l]}};
-        const double J00 = 2 * (-b * c + F * F), J01 = 2 * (c * d - e * F), J02 = 2 * (b * e - d * F),
-                     J11 = 2 * (-a * c + e * e), J12 = 2 * (-d * e + a * F), J22 = 2 * (d * d - a * b);
-        const double J[3][3] = {{J00, J01, J02}, {J01, J11, J12}, {J02, J12, J22}};
-        const double invJJ = 1.0 / p.JJ;
-        const double S = s.t[0][l].S + s.t[1][l].S + s.t[2][l].S + s.t[3][l].S;
-        const double pref = kRep * invJJ / 2.0;
+        const double J[3][3] = {{s.J[0][l], s.J[1][l], s.J[2][l]}, {s.J[1][l], s.J[3][l], s.J[4][l]}, {s.J[2][l], s.J[4][l], s.J[5][l]}};
+        const double pref = s.pref[l], m = s.m[l];
+        diff(1, 0, v12);
+        diff(3, 2, v34);
+        diff(0, 2, v31);
         double dv[3];
 #pragma unroll
         for (int y = 0; y < 3; ++y) {
             const double Jw = w == 0 ? J[2][y] - J[0][y] : w == 1 ? J[0][y] : w == 2 ? -J[2][y] - J[1][y] : J[1][y];
             const double Gw = w == 0 ? G[2][y] - G[0][y] : w == 1 ? G[0][y] : w == 2 ? -G[2][y] - G[1][y] : G[1][y];
-            dv[y] = pref * (-invJJ * S * Jw + Gw);
+            dv[y] = pref * (m * Jw + Gw);
         }
         Real* dst = slot_ptr(n, n.slot_base[K_EXVOL] + 4 * i + w);
         bool bad = false;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const double o = -(dv[0] * p.v12[k] + dv[1] * p.v34[k] + dv[2] * p.v31[k]);
+            const double o = -(dv[0] * v12[k] + dv[1] * v34[k] + dv[2] * v31[k]);
             if (bad_value(o)) bad = true;
             dst[k] = (Real)o;
         }
@@ -683,10 +734,11 @@ __global__ void __launch_bounds__(kBlock) k_exvol(DevNet<Real> n, int want, int 
 // operations in one warp took ~35 us.  Here lane l of every warp takes pair
 // 32 g + l of the block's group g, and warp w evaluates the w-th of the four
 // arctangent terms of the integral (A, E, B, F below: cross product, norm,
-// numerator, arctangent and, for forces, its partial derivatives); the shared
-// invariants are formed by every warp, the six entries of the G matrix are
-// split over the warps, and warp w forms the force on bead w.  Partial results
-// pass through shared memory.  The cancellation-free forms of pair_inv
+// numerator, arctangent and, for forces, its partial derivatives); the vectors
+// are formed by every warp, the scalar products, the entries of the G and J
+// matrices and the common factors each by one of them (forces 13.0 -> 11.9 us in
+// an iteration of 60k cylinders, against every warp forming all but G), and warp
+// w forms the force on bead w.  Partial results pass through shared memory.  The cancellation-free forms of pair_inv
 // (cross = true) and forces_from<true> are followed term by term, with the
 // reference's coplanar move of c2 (:610-626, forces only, decided without
 // divisions: (n . v3)^2 < 0.01 |n|^2 |v3|^2).
@@ -706,6 +758,10 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
     __shared__ double s_N[3][32];          // CC, GG, DD for the F term's HH
     __shared__ ExtTerm s_t[4][32];
     __shared__ double s_G[6][32];
+    __shared__ double s_dot[6][32];        // a, b, c, d, e, F
+    __shared__ double s_J[6][32];          // J00, J01, J02, J11, J12, J22
+    __shared__ double s_JJ[32], s_k[32];   // JJ; kRep, then (forces) kRep / (2 JJ)
+    __shared__ double s_m[32];             // -S / JJ
     __shared__ int s_bad[32];
     const int* list = listed ? n.ev_flist : n.ev_list;
     const int cnt = min(listed ? *n.ev_flist_count : *n.ev_list_count, 2 * n.n_ev);
@@ -747,7 +803,7 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
         if (w == 0) s_bad[l] = 0;
         __syncthreads();
         double v12[3], v34[3], v31[3], v14[3], v32[3], v24[3];
-        double a = 0, b = 0, c = 0, d = 0, e = 0, F = 0, JJ = 1, kRep = 0;
+        double a = 0, b = 0, c = 0, d = 0, e = 0, F = 0;
         double x21[3] = {0, 0, 0};
         if (valid) {
 #pragma unroll
@@ -776,20 +832,27 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
                     }
                 }
             }
-            if (force) {
-                a = dot3(v12, v12);
-                b = dot3(v34, v34);
-                c = dot3(v31, v31);
-                d = dot3(v12, v34);
-                e = dot3(v12, v31);
-                F = dot3(v34, v31);
-            }
             x21[0] = v34[1] * v12[2] - v34[2] * v12[1];
             x21[1] = v34[2] * v12[0] - v34[0] * v12[2];
             x21[2] = v34[0] * v12[1] - v34[1] * v12[0];
-            const double trip = -(x21[0] * v31[0] + x21[1] * v31[1] + x21[2] * v31[2]);
-            JJ = -trip * trip;
-            kRep = (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i];
+            // what every warp needs later, each formed by one of them
+            if (w == 3) {
+                const double trip = -(x21[0] * v31[0] + x21[1] * v31[1] + x21[2] * v31[2]);
+                s_JJ[l] = -trip * trip;
+                s_k[l] = (double)n.ev_k[i] * (double)n.ev_la[i] * (double)n.ev_lb[i];
+            }
+            if (force) {
+                if (w == 0) {
+                    s_dot[0][l] = dot3(v12, v12);
+                    s_dot[1][l] = dot3(v34, v34);
+                } else if (w == 1) {
+                    s_dot[2][l] = dot3(v31, v31);
+                    s_dot[3][l] = dot3(v12, v34);
+                } else if (w == 2) {
+                    s_dot[4][l] = dot3(v12, v31);
+                    s_dot[5][l] = dot3(v34, v31);
+                }
+            }
         }
         // ---- term w: cross product, norm, numerator
         double xu[3] = {0, 0, 0}, Y = 1, N = 0;
@@ -825,6 +888,12 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
             t.rY = 1.0 / Y;
             t.S = N * t.rY * t.ATG;
             if (force) {
+                a = s_dot[0][l];
+                b = s_dot[1][l];
+                c = s_dot[2][l];
+                d = s_dot[3][l];
+                e = s_dot[4][l];
+                F = s_dot[5][l];
                 const double al = w == 0 ? a + e : w == 1 ? a + e - d : w == 2 ? F : d + F;
                 const double be = al - (w < 2 ? a : b);
                 const double Y2 = Y * Y;
@@ -843,7 +912,7 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
         if (!force) {
             if (w == 0 && valid) {
                 const double Ssum = s_t[0][l].S + s_t[1][l].S + s_t[2][l].S + s_t[3][l].S;
-                const double U = 0.5 * kRep / JJ * Ssum;
+                const double U = 0.5 * s_k[l] / s_JJ[l] * Ssum;
                 double* dst = (second ? n.ev_energy2 : n.ev_energy) + i;
                 if (!(fabs(U) < 1.0 / 0.0) || U < -1.0) {
                     flag_fallback(n, r, i, trial != 0 ? lam : 0.0);
@@ -856,7 +925,8 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
             __syncthreads();   // shared arrays are reused by the next group
             continue;
         }
-        // ---- G entries, split over the warps (0: G00, G12; 1: G01, G22; 2: G02; 3: G11)
+        // ---- entries of G and J and the factors, split over the warps
+        // (0: G00, G12; 1: G01, G22, J11, J12, J22; 2: G02, factors; 3: G11, J00, J01, J02)
         if (valid) {
             const ExtTerm A = s_t[0][l], E = s_t[1][l], B = s_t[2][l], FT = s_t[3][l];
             if (w == 0) {
@@ -868,12 +938,22 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
                 s_G[1][l] = A.tN * e + E.tN * (2 * d - e) + E.tXr * (e - d) - E.tlo + B.tN * (-F) + FT.tN * (2 * d + F) +
                             FT.tXr * (-(d + F)) + FT.tlo;
                 s_G[5][l] = A.tXr * a + E.tXr * a + B.tXr * b + FT.tXr * b;
+                s_J[3][l] = 2 * (-a * c + e * e);
+                s_J[4][l] = 2 * (-d * e + a * F);
+                s_J[5][l] = 2 * (d * d - a * b);
             } else if (w == 2) {
+                const double invJJ = 1.0 / s_JJ[l];
+                const double Ssum = A.S + E.S + B.S + FT.S;
+                s_k[l] = s_k[l] * invJJ / 2.0;
+                s_m[l] = -invJJ * Ssum;
                 s_G[2][l] = A.tN * d + A.tXr * (-e) + A.tlo + E.tN * (-d) + E.tXr * (-(e - d)) + E.tlo + B.tN * b +
                             FT.tN * (-b) + FT.tXr * b;
             } else {
                 s_G[3][l] = E.tN * (-2 * a) + E.tXr * a + B.tN * (2 * e) + B.tXr * c + B.tlo * (-2) + B.thi * 2 +
                             FT.tN * (-2 * (a + e)) + FT.tXr * (a + c + 2 * e) + FT.tlo * (-2) + FT.thi * 2;
+                s_J[0][l] = 2 * (-b * c + F * F);
+                s_J[1][l] = 2 * (c * d - e * F);
+                s_J[2][l] = 2 * (b * e - d * F);
             }
         }
         __syncthreads();
@@ -882,12 +962,10 @@ __global__ void __launch_bounds__(128) k_exvol_ext(DevNet<Real> n, int trial, in
             const double G[3][3] = {{s_G[0][l], s_G[1][l], s_G[2][l]},
                                     {s_G[1][l], s_G[3][l], s_G[4][l]},
                                     {s_G[2][l], s_G[4][l], s_G[5][l]}};
-            const double J[3][3] = {{2 * (-b * c + F * F), 2 * (c * d - e * F), 2 * (b * e - d * F)},
-                                    {2 * (c * d - e * F), 2 * (-a * c + e * e), 2 * (-d * e + a * F)},
-                                    {2 * (b * e - d * F), 2 * (-d * e + a * F), 2 * (d * d - a * b)}};
-            const double invJJ = 1.0 / JJ;
-            const double Ssum = s_t[0][l].S + s_t[1][l].S + s_t[2][l].S + s_t[3][l].S;
-            const double pref = kRep * invJJ / 2.0, m = -invJJ * Ssum;
+            const double J[3][3] = {{s_J[0][l], s_J[1][l], s_J[2][l]},
+                                    {s_J[1][l], s_J[3][l], s_J[4][l]},
+                                    {s_J[2][l], s_J[4][l], s_J[5][l]}};
+            const double pref = s_k[l], m = s_m[l];
             double dv[3];
 #pragma unroll
             for (int y = 0; y < 3; ++y) {
