@@ -330,37 +330,36 @@ __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want
 // is formed on the bits.  The mixed engine's
 // version is k_force_gather_mx below.
 // ---------------------------------------------------------------------------
-constexpr int kGatherAhead = 4;   // contributions of a bead loaded together
+constexpr int kGatherAhead = 4;   // contributions loaded together
+// `acc` plus `count` contributions, 3 numbers apart from `g` on, in order.  The
+// first are loaded together: one after another, each costs a round trip to L2.
+template <typename Real, int N>
+__device__ __forceinline__ void add_contributions(const Real* g, int count, Real (&acc)[N]) {
+    Real v[kGatherAhead][N];
+#pragma unroll
+    for (int k = 0; k < kGatherAhead; ++k)
+        if (k < count)
+#pragma unroll
+            for (int q = 0; q < N; ++q) v[k][q] = g[3 * k + q];
+#pragma unroll
+    for (int k = 0; k < kGatherAhead; ++k)
+        if (k < count)
+#pragma unroll
+            for (int q = 0; q < N; ++q) acc[q] += v[k][q];
+    for (int k = kGatherAhead; k < count; ++k)
+#pragma unroll
+        for (int q = 0; q < N; ++q) acc[q] += g[3 * (size_t)k + q];
+}
 template <typename Real>
 __device__ __forceinline__ void gather_force(const DevNet<Real>& n, int b, int fb, Real F[3], Real& ff, Real& ffp) {
     Real* Fo = n.f[fb ^ 1] + 3 * (size_t)b;
     const Real* Fp = n.f[fb] + 3 * (size_t)b;
-    F[0] = Fo[0];
-    F[1] = Fo[1];
-    F[2] = Fo[2];
+    Real acc[3] = {Fo[0], Fo[1], Fo[2]};
     const Real p0 = Fp[0], p1 = Fp[1], p2 = Fp[2];
     const int c0 = n.csr_off[b], c1 = n.csr_off[b + 1];
-    // the first contributions loaded together: one after another, each costs a
-    // round trip to L2
-    Real g[kGatherAhead][3];
+    add_contributions<Real, 3>(n.contrib + 3 * (size_t)c0, c1 - c0, acc);
 #pragma unroll
-    for (int k = 0; k < kGatherAhead; ++k)
-        if (c0 + k < c1)
-#pragma unroll
-            for (int q = 0; q < 3; ++q) g[k][q] = n.contrib[3 * (size_t)(c0 + k) + q];
-#pragma unroll
-    for (int k = 0; k < kGatherAhead; ++k)
-        if (c0 + k < c1)
-#pragma unroll
-            for (int q = 0; q < 3; ++q) F[q] += g[k][q];
-    for (int c = c0 + kGatherAhead; c < c1; ++c) {
-        F[0] += n.contrib[3 * (size_t)c];
-        F[1] += n.contrib[3 * (size_t)c + 1];
-        F[2] += n.contrib[3 * (size_t)c + 2];
-    }
-    Fo[0] = F[0];
-    Fo[1] = F[1];
-    Fo[2] = F[2];
+    for (int q = 0; q < 3; ++q) Fo[q] = F[q] = acc[q];
     ff = bead_dot(F[0], F[1], F[2], F[0], F[1], F[2]);
     ffp = bead_dot_prev(F, p0, p1, p2);
 }
@@ -372,11 +371,67 @@ __device__ __forceinline__ void gather_bead(const DevNet<float>& n, int b, int f
     mx = fin ? fmaxf(fmaxf(fabsf(F[0]), fabsf(F[1])), fabsf(F[2])) : INFINITY;
 }
 // the same on bits: infinity and NaN have the largest, cut to infinity's
-__device__ __forceinline__ void gather_bead(const DevNet<double>& n, int b, int fb, unsigned long long& mx, double& ff,
-                                            double& ffp) {
-    double F[3];
-    gather_force(n, b, fb, F, ff, ffp);
-    mx = min(max(max(abs_bits(F[0]), abs_bits(F[1])), abs_bits(F[2])), 0x7ff0000000000000ULL);
+__device__ __forceinline__ unsigned long long max_bits(const double F[3]) {
+    return min(max(max(abs_bits(F[0]), abs_bits(F[1])), abs_bits(F[2])), 0x7ff0000000000000ULL);
+}
+// FP64, the beads of a warp together: an addition costs the warp the same for
+// one lane as for 32, and few beads have contributions, so the components of
+// those that have some are spread over the lanes (a third of the additions of a
+// warp that adds three for every contribution of its busiest bead).  The gather
+// of 1M beads 52.5 -> 40 us; not in a small network, where a block has an SM for
+// itself and the detour through shared memory is 0.3 us of latency.
+struct GatherWarp {
+    double F[96];      // components of the beads with contributions
+    int2 range[32];    // their first contribution and count
+};
+__device__ __forceinline__ void gather_warp(const DevNet<double>& n, int b, bool own, int fb, GatherWarp& s,
+                                            unsigned long long& mx, double& ff, double& ffp) {
+    const int lane = threadIdx.x & 31;
+    double* Fo = n.f[fb ^ 1] + 3 * (size_t)b;
+    const double* Fp = n.f[fb] + 3 * (size_t)b;
+    double F[3] = {0, 0, 0}, p0 = 0, p1 = 0, p2 = 0;
+    int c0 = 0, count = 0;
+    if (own) {
+        c0 = n.csr_off[b];
+        count = n.csr_off[b + 1] - c0;
+        F[0] = Fo[0];
+        F[1] = Fo[1];
+        F[2] = Fo[2];
+        p0 = Fp[0];
+        p1 = Fp[1];
+        p2 = Fp[2];
+    }
+    const unsigned some = __ballot_sync(0xffffffffu, count > 0);
+    if (some) {
+        const int rank = __popc(some & ((1u << lane) - 1u)), items = 3 * __popc(some);
+        if (count > 0) {
+            s.range[rank] = make_int2(c0, count);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) s.F[3 * rank + q] = F[q];
+        }
+        __syncwarp();
+        for (int t = lane; t < items; t += 32) {
+            const int e = t / 3;
+            const int2 r = s.range[e];
+            double acc[1] = {s.F[t]};
+            add_contributions<double, 1>(n.contrib + 3 * (size_t)r.x + (t - 3 * e), r.y, acc);
+            s.F[t] = acc[0];
+        }
+        __syncwarp();
+        if (count > 0) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) F[q] = s.F[3 * rank + q];
+        }
+        __syncwarp();   // the next tile's beads use the same arrays
+    }
+    if (own) {
+        Fo[0] = F[0];
+        Fo[1] = F[1];
+        Fo[2] = F[2];
+        ff = bead_dot(F[0], F[1], F[2], F[0], F[1], F[2]);
+        ffp = bead_dot_prev(F, p0, p1, p2);
+        mx = max_bits(F);
+    }
 }
 
 // NT tiles per block (DevNet::gtiles).  Four blocks on an SM (64 registers) hold
@@ -389,6 +444,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_gather(DevNet<double> n, in
     MECH_TRACE_KERNEL(n, TK_GATHER);
     __shared__ double sh[2 * NT * kBlock / 32];
     __shared__ unsigned long long s_mx[NT * kBlock / 32];
+    __shared__ GatherWarp s_warp[NT > 1 ? kBlock / 32 : 1];
     const int t0 = blockIdx.x * NT;
     unsigned long long mx[NT];
     double v[2 * NT];   // F.F of each tile, then F.Fprev
@@ -403,7 +459,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_gather(DevNet<double> n, in
         if (!s.go) continue;
         go |= 1u << j;
         const int b = t.begin + threadIdx.x;
-        if (b < t.end) gather_bead(n, b, s.fb, mx[j], v[j], v[NT + j]);
+        if constexpr (NT > 1) {
+            gather_warp(n, b, b < t.end, s.fb, s_warp[threadIdx.x >> 5], mx[j], v[j], v[NT + j]);
+        } else if (b < t.end) {
+            double F[3];
+            gather_force(n, b, s.fb, F, v[0], v[1]);
+            mx[0] = max_bits(F);
+        }
     }
     if (!go) return;   // block-uniform
     const unsigned long long m = block_maxima<NT>(mx, s_mx);
