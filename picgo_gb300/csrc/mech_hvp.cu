@@ -81,7 +81,11 @@ __device__ bool pair_forces_dual(const Dual* c1, const Dual* c2in, const Dual* c
     return forces_from<true>(p, v12, v34, v31, Dual(kRep), out);
 }
 
-__global__ void __launch_bounds__(kHvpBlock) k_hvp_sparse(DevNet<double> n, const double* __restrict__ V, int jac) {
+// A warp of pairs takes ~1,500 FP64 instructions, ~50 us of its sub-partition's
+// pipe: blocks of two warps spread them over the SMs (60,000 cylinders, 45 warps
+// of pairs: 119 us with eight warps a block, 77 with two).
+constexpr int kHvpSparseBlock = 64;
+__global__ void __launch_bounds__(kHvpSparseBlock) k_hvp_sparse(DevNet<double> n, const double* __restrict__ V, int jac) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const double* X = n.x[0];
     const int nlm = n.n_lk + n.n_mt;
@@ -143,61 +147,86 @@ __global__ void __launch_bounds__(kHvpBlock) k_hvp_sparse(DevNet<double> n, cons
     }
 }
 
-// Owner side: the filament terms touching bead b on duals, plus the bead's
-// gathered sparse contributions; hv = -dF + shift v.
+// Owner side: the filament terms touching each bead on duals, plus the bead's
+// gathered sparse contributions; hv = -dF + shift v.  Bound by the FP64 pipe, so
+// every cylinder's and triple's terms are formed once and read by the beads they
+// act on, and a block takes the beads whose cylinders, three more, fill its warps
+// (60,000 cylinders: 41 us; 85 with each bead forming its two and three).
+constexpr int kHvpFilBeads = kHvpBlock - 3;
 __global__ void __launch_bounds__(kHvpBlock) k_hvp_fil(DevNet<double> n, const double* __restrict__ V, double shift,
                                                       double* __restrict__ HV) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= n.nb) return;
+    __shared__ double s_p[6][kHvpBlock + 1];                       // beads first - 2 .. : value and direction
+    __shared__ double s_r[6][kHvpBlock];                           // cylinders first - 2 .. : vector
+    __shared__ double s_S[3][kHvpBlock];                           // d(force) of their stretching on the second bead
+    __shared__ double s_1[3][kHvpBlock], s_2[3][kHvpBlock];        // d of the triples' terms, on first - 1 ..
+    const int first = blockIdx.x * kHvpFilBeads, T = min(kHvpFilBeads, n.nb - first);
     const double* X = n.x[0];
-    const int f0 = n.bflag[b];
-    const int fm = (f0 & 2) ? n.bflag[b - 1] : 0;
-    const int fp = (f0 & 1) ? n.bflag[b + 1] : 0;
-    Dual p0[3], pm1[3], pp1[3], pm2[3], pp2[3];
-    dual_bead(X, V, b, p0);
-    if (f0 & 2) dual_bead(X, V, b - 1, pm1);
-    if (f0 & 1) dual_bead(X, V, b + 1, pp1);
-    if (fm & 2) dual_bead(X, V, b - 2, pm2);
-    if (fp & 1) dual_bead(X, V, b + 2, pp2);
-    Dual F[3];
-    Dual rm[3], rp[3];
+    for (int i = threadIdx.x; i < T + 4; i += blockDim.x) {
+        const int b = first - 2 + i;
+        if (b < 0 || b >= n.nb) continue;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            s_p[q][i] = X[3 * (size_t)b + q];
+            s_p[3 + q][i] = V[3 * (size_t)b + q];
+        }
+    }
+    __syncthreads();
+    const int i = threadIdx.x;
+    Dual r2[3];
+    double ks = 0, l0 = 0, kb = 0, th = 0;
+    {
+        const int c = first - 2 + i;
+        double S[3] = {0, 0, 0};
+        if (i < T + 3 && c >= 0 && c < n.nb && (n.bflag[c] & 1)) {
+            load_par(n.bpar, c, ks, l0, kb, th);
+            Dual F[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                r2[q] = Dual(s_p[q][i + 1], s_p[3 + q][i + 1]) - Dual(s_p[q][i], s_p[3 + q][i]);
+                s_r[q][i] = r2[q].v;
+                s_r[3 + q][i] = r2[q].d;
+            }
+            stretch_force<Dual>(r2[0], r2[1], r2[2], Dual(ks), Dual(l0), F);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) S[q] = F[q].d;
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) s_S[q][i] = S[q];
+    }
+    __syncthreads();
+    {   // thread i: the triple on bead first - 2 + i, at whose second cylinder it is already
+        const int c = first - 2 + i;
+        double A[3] = {0, 0, 0}, B[3] = {0, 0, 0};
+        if (i >= 1 && i < T + 3 && c >= 0 && c < n.nb && (n.bflag[c] & 3) == 3) {
+            Dual r1[3], a1[3], a2[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) r1[q] = Dual(s_r[q][i - 1], s_r[3 + q][i - 1]);
+            bend_force<Dual>(r1, r2, Dual(kb), Dual(th), a1, a2);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                A[q] = a1[q].d;
+                B[q] = a2[q].d;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            s_1[q][i] = A[q];
+            s_2[q][i] = B[q];
+        }
+    }
+    __syncthreads();
+    if (i >= T) return;
+    const int b = first + i;   // bead b's own cylinder and triple are at i + 2
+    double h[3];
+#pragma unroll
     for (int q = 0; q < 3; ++q) {
-        rm[q] = p0[q] - pm1[q];
-        rp[q] = pp1[q] - p0[q];
+        double F = s_S[q][i + 1];
+        F -= s_S[q][i + 2];
+        F += s_2[q][i + 1];
+        F += s_1[q][i + 2] - s_2[q][i + 2];
+        F -= s_1[q][i + 3];
+        h[q] = -F;
     }
-    double ksm = 0, l0m = 0, kbm = 0, thm = 0, ks = 0, l0 = 0, kb = 0, th = 0;
-    if (f0 & 2) load_par(n.bpar, b - 1, ksm, l0m, kbm, thm);
-    if (f0 & 1) load_par(n.bpar, b, ks, l0, kb, th);
-    if (f0 & 2) {
-        Dual S1[3];
-        stretch_force<Dual>(rm[0], rm[1], rm[2], Dual(ksm), Dual(l0m), S1);
-        for (int q = 0; q < 3; ++q) F[q] += S1[q];
-    }
-    if (f0 & 1) {
-        Dual S2[3];
-        stretch_force<Dual>(rp[0], rp[1], rp[2], Dual(ks), Dual(l0), S2);
-        for (int q = 0; q < 3; ++q) F[q] -= S2[q];
-    }
-    if ((f0 & 2) && (fm & 2)) {
-        Dual r1[3], a1[3], a2[3];
-        for (int q = 0; q < 3; ++q) r1[q] = pm1[q] - pm2[q];
-        bend_force<Dual>(r1, rm, Dual(kbm), Dual(thm), a1, a2);
-        for (int q = 0; q < 3; ++q) F[q] += a2[q];
-    }
-    if ((f0 & 3) == 3) {
-        Dual a1[3], a2[3];
-        bend_force<Dual>(rm, rp, Dual(kb), Dual(th), a1, a2);
-        for (int q = 0; q < 3; ++q) F[q] += a1[q] - a2[q];
-    }
-    if ((f0 & 1) && (fp & 1)) {
-        double ksp, l0p, kbp, thp;
-        load_par(n.bpar, b + 1, ksp, l0p, kbp, thp);
-        Dual r2[3], a1[3], a2[3];
-        for (int q = 0; q < 3; ++q) r2[q] = pp2[q] - pp1[q];
-        bend_force<Dual>(rp, r2, Dual(kbp), Dual(thp), a1, a2);
-        for (int q = 0; q < 3; ++q) F[q] -= a1[q];
-    }
-    double h[3] = {-F[0].d, -F[1].d, -F[2].d};
     const int c0 = n.csr_off[b], c1 = n.csr_off[b + 1];
     for (int c = c0; c < c1; ++c) {
         h[0] += n.contrib[3 * (size_t)c];
@@ -209,7 +238,7 @@ __global__ void __launch_bounds__(kHvpBlock) k_hvp_fil(DevNet<double> n, const d
 
 // ---- The Hessian of a solve, held as blocks ------------------------------------
 // A solve applies one H to many vectors, and an application by duals costs
-// 119 + 85 us on 60,000 cylinders (FP64 pipe: ~1,500 instructions per excluded-
+// 77 + 41 us on 60,000 cylinders (FP64 pipe: ~1,500 instructions per excluded-
 // volume pair and ~250 per bead, most of them the same for every vector).  So a
 // solve first evaluates the duals along the unit vectors of each interaction's
 // difference vectors and keeps the derivatives:
@@ -610,10 +639,10 @@ int launch_hvp(const DevNet<double>& n, const double* v, double* hv, double shif
     const int ns = n.n_lk + n.n_mt + n.n_ev + n.n_bb;
     int k = 0;
     if (ns > 0) {
-        k_hvp_sparse<<<(ns + kHvpBlock - 1) / kHvpBlock, kHvpBlock, 0, s>>>(n, v, jacobian ? 1 : 0);
+        k_hvp_sparse<<<(ns + kHvpSparseBlock - 1) / kHvpSparseBlock, kHvpSparseBlock, 0, s>>>(n, v, jacobian ? 1 : 0);
         ++k;
     }
-    k_hvp_fil<<<(n.nb + kHvpBlock - 1) / kHvpBlock, kHvpBlock, 0, s>>>(n, v, shift, hv);
+    k_hvp_fil<<<(n.nb + kHvpFilBeads - 1) / kHvpFilBeads, kHvpBlock, 0, s>>>(n, v, shift, hv);
     return k + 1;
 }
 
