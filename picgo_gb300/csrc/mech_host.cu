@@ -1330,10 +1330,12 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
     };
     if ((rc = build_graph())) return rc;
     long long graphs = 0;
+    // more line-search passes than any search within the call limits makes: the
+    // first kShortGraphs graphs have kGraphBlocks[0] passes, the others kGraphBlocks[1]
     long long max_graphs = 0;
     for (int r = 0; r < c->R; ++r)
         max_graphs = std::max<long long>(
-            max_graphs, 4LL * std::max(p->force_call_limit, 3 * c->reps[r].nb) / kGraphBlocks[0] + 1000);
+            max_graphs, 4LL * std::max(p->force_call_limit, 3 * c->reps[r].nb) / kGraphBlocks[0] + 2200);
     int status = MECH_OK;
     // The next graph is launched before the host reads the snapshot of the
     // previous one, so the device does not idle while the host checks the
