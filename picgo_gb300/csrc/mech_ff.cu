@@ -684,12 +684,17 @@ __device__ __forceinline__ void write_run(const DevNet<float>& n, int first, con
 // tiles with run-start partial slots (see write_run), where each selected
 // tile's positions (with a one-bead halo),
 // constants, flags and (for a trial) search direction arrive in shared memory
-// by cp.async.bulk on a three-stage mbarrier ring, so a block keeps several
-// ~14 KB transfers in flight instead of per-thread dependent loads.  Ranges
+// by cp.async.bulk on an mbarrier ring, so a block keeps several
+// ~14-18 KB transfers in flight instead of per-thread dependent loads.  Ranges
 // are rounded outward to the 16-byte copy granularity; the bead arrays are
 // allocated with the padding that rounding needs.
 // ---------------------------------------------------------------------------
-constexpr int kBulkStages = 3;
+constexpr int kBulkStages = 3;                // forces
+// Energy: with the forces of a new direction staged too, three stages would
+// leave room for three blocks on an SM instead of four.  Staged forces and
+// stores in whole vectors: a two-trial pass that forms the direction 46.9 -> 41.7
+// us on 1M beads, an iteration of the 1M-cylinder network 117.3 -> 115.5 us.
+constexpr int kEnergyStages = 2;
 constexpr int kBulkXBeads = kFilTile + 4;    // tile + 1-bead halo, even-aligned ends
 constexpr int kBulkDBeads = kFilTile + 8;    // tile + halo, 4-bead aligned ends
 constexpr int kBulkFlags = kFilTile + 32;    // tile + halo, 16-byte aligned ends
@@ -699,6 +704,7 @@ struct __align__(16) EnergyStage {
     float x[6 * kBulkXBeads];      // float-float positions, beads [xs, xe)
     float4 par[kFilTile];          // k_str, l0, k_bend, theta0, beads [tb, te)
     float d[3 * kBulkDBeads];      // search direction, beads [ds, de)
+    float f[3 * kBulkDBeads];      // forces of a new direction, the same beads
     uint8_t flag[kBulkFlags];      // bead flags, beads [fs, fe)
 };
 
@@ -757,14 +763,15 @@ __device__ __forceinline__ const float* staged_direction(const DevNet<float>& n,
 __device__ void issue_energy_stage(const DevNet<float>& n, int4 t, bool tr, EnergyStage* st, uint64_t* bar) {
     const float* X = n.x[(t.w >> 1) & 3];
     const StageRange rg = stage_range(t.x, t.y, n.nb, 1);
-    const void* src[4] = {X + 6 * (size_t)rg.xs, n.bpar + 4 * (size_t)t.x, staged_direction(n, t.w) + 3 * (size_t)rg.ds,
-                          n.bflag + rg.fs};
-    void* dst[4] = {st->x, st->par, st->d, st->flag};
-    const unsigned bytes[4] = {24u * (unsigned)(rg.xe - rg.xs), 16u * (unsigned)(t.y - t.x),
-                               tr ? 12u * (unsigned)(rg.de - rg.ds) : 0u, (unsigned)(rg.fe - rg.fs)};
+    const unsigned vec = 12u * (unsigned)(rg.de - rg.ds);
+    const void* src[5] = {X + 6 * (size_t)rg.xs, n.bpar + 4 * (size_t)t.x, n.bflag + rg.fs,
+                          staged_direction(n, t.w) + 3 * (size_t)rg.ds, n.f[(t.w >> 3) & 1] + 3 * (size_t)rg.ds};
+    void* dst[5] = {st->x, st->par, st->flag, st->d, st->f};
+    const unsigned bytes[5] = {24u * (unsigned)(rg.xe - rg.xs), 16u * (unsigned)(t.y - t.x), (unsigned)(rg.fe - rg.fs),
+                               tr ? vec : 0u, tr && (t.w & 32) ? vec : 0u};
     unsigned total = 0;
     bool ok = true;
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 5; ++k) {
         if (!bytes[k]) continue;
         if (!aligned16(src[k], bytes[k]) || !aligned16(dst[k], bytes[k])) ok = false;
         total += bytes[k];
@@ -776,7 +783,7 @@ __device__ void issue_energy_stage(const DevNet<float>& n, int4 t, bool tr, Ener
         return;
     }
     mbar_arrive_expect_tx(bar, total);
-    for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < 5; ++k)
         if (bytes[k]) bulk_copy_g2s(dst[k], src[k], bytes[k], bar);
 }
 
@@ -799,22 +806,44 @@ __device__ __forceinline__ bool idle_range(const DevNet<float>& n, const Tile* t
     return *s_flag != 0;
 }
 
+// `count` floats from shared to consecutive global memory, by the whole block,
+// in the widest vectors that both allow (16 bytes in a single network, 8 or 4
+// where a replica before has a bead count that is not a multiple of 4; a record
+// of 12 or 24 bytes per thread takes three store instructions that each touch
+// all its sectors).
+template <typename Vec>
+__device__ __forceinline__ void store_vectors(float* dst, const float* src, int count) {
+    constexpr int W = sizeof(Vec) / sizeof(float);
+    const int whole = count / W;
+    for (int k = threadIdx.x; k < whole; k += blockDim.x)
+        reinterpret_cast<Vec*>(dst)[k] = reinterpret_cast<const Vec*>(src)[k];
+    const int k = whole * W + threadIdx.x;
+    if (k < count) dst[k] = src[k];
+}
+__device__ __forceinline__ void store_records(float* dst, const float* src, int count) {
+    const unsigned off = (unsigned)(reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src));
+    if ((off & 15u) == 0) store_vectors<float4>(dst, src, count);
+    else if ((off & 7u) == 0) store_vectors<float2>(dst, src, count);
+    else store_vectors<float>(dst, src, count);
+}
+
 __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, int want, int trial) {
     pdl_wait();      // the previous kernel of the main lane has finished
     MECH_TRACE_KERNEL(n, TK_FIL_ENERGY_BULK);
-    __shared__ EnergyStage stage[kBulkStages];
-    __shared__ __align__(8) uint64_t bar[kBulkStages];
+    __shared__ EnergyStage stage[kEnergyStages];
+    __shared__ __align__(8) uint64_t bar[kEnergyStages];
     __shared__ int4 s_desc[kBulkMaxTiles];
     __shared__ float2 s_step[kBulkMaxTiles];
     __shared__ float sh[2 * 8 * kBlock / 32];   // block_pair_sums<8>
     __shared__ __align__(16) float s_mv[6 * kBulkXBeads];   // the staged beads moved to a trial
+    __shared__ __align__(16) float s_d[3 * kFilTile];       // the tile's new direction
     __shared__ int s_abort;
     const int t0 = blockIdx.x * n.ptiles[0], t1 = min(t0 + n.ptiles[0], n.n_ftiles);
     const int nt = t1 - t0;
     const bool tr = trial != 0;
     if (idle_range(n, n.ftile, t0, t1, want, &s_abort)) return;
     if (threadIdx.x == 0) {
-        for (int k = 0; k < kBulkStages; ++k) mbar_init(&bar[k], 1);
+        for (int k = 0; k < kEnergyStages; ++k) mbar_init(&bar[k], 1);
         mbar_init_fence();
         s_abort = 0;
     }
@@ -827,9 +856,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
     // producer state (thread 0): next tile to consider, copies issued
     int pi = 0, issued = 0;
     if (threadIdx.x == 0) {
-        for (; pi < nt && issued < kBulkStages; ++pi)
+        for (; pi < nt && issued < kEnergyStages; ++pi)
             if (s_desc[pi].w & 1) {
-                issue_energy_stage(n, s_desc[pi], tr, &stage[issued % kBulkStages], &bar[issued % kBulkStages]);
+                issue_energy_stage(n, s_desc[pi], tr, &stage[issued % kEnergyStages], &bar[issued % kEnergyStages]);
                 ++issued;
             }
     }
@@ -872,21 +901,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
         }
         if (!go) continue;
         ++cnt;
-        const int sidx = j % kBulkStages;
+        const int sidx = j % kEnergyStages;
         const int b = t.x + threadIdx.x;
         const StageRange rg = stage_range(t.x, t.y, n.nb, 1);
         const bool own = b < t.y;
-        // the forces of a new direction are read directly (a fourth staged
-        // array would cost a resident block), ahead of the wait for the stage
-        const float* Fn = n.f[(t.w >> 3) & 1];
-        float Fq[3] = {0.f, 0.f, 0.f};
-        if (pend && rg.xs + (int)threadIdx.x < min(rg.xe, n.nb)) {
-            const float* F = Fn + 3 * (size_t)(rg.xs + threadIdx.x);
-            Fq[0] = F[0];
-            Fq[1] = F[1];
-            Fq[2] = F[2];
-        }
-        if (!mbar_wait_bounded(&bar[sidx], (unsigned)((j / kBulkStages) & 1), kBulkWaitLimit)) {
+        if (!mbar_wait_bounded(&bar[sidx], (unsigned)((j / kEnergyStages) & 1), kBulkWaitLimit)) {
             atomicOr(n.err, 32u);
             s_abort = 1;
         }
@@ -909,20 +928,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
                 const float lch = ch ? 0.5f * lf : lf;
                 for (int q = threadIdx.x; q < rg.xe - rg.xs; q += blockDim.x) {
                     const Pos<float> p = load_pos(S.x, q);
-                    const float* ds = S.d + 3 * (q + rg.xs - rg.ds);
-                    float d[3] = {ds[0], ds[1], ds[2]};
+                    const int bq = rg.xs + q, dq = 3 * (bq - rg.ds);
+                    float d[3] = {S.d[dq], S.d[dq + 1], S.d[dq + 2]};
                     if (pend) {
-                        const int bq = rg.xs + q;
-                        float F[3] = {Fq[0], Fq[1], Fq[2]};
-                        if (q >= kBlock && bq < n.nb) {   // the few beads past one per thread
-                            F[0] = Fn[3 * (size_t)bq];
-                            F[1] = Fn[3 * (size_t)bq + 1];
-                            F[2] = Fn[3 * (size_t)bq + 2];
-                        }
+                        const float F[3] = {S.f[dq], S.f[dq + 1], S.f[dq + 2]};
 #pragma unroll
                         for (int m = 0; m < 3; ++m) d[m] = new_direction(F[m], beta, d[m]);
                         if (!ch && bq >= t.x && bq < t.y) {   // the tile's own bead: the direction, d . F, the backup
-                            float* o = n.d[((t.w >> 7) & 1) ^ 1] + 3 * (size_t)bq;
+                            float* o = s_d + 3 * (bq - t.x);
                             o[0] = d[0];
                             o[1] = d[1];
                             o[2] = d[2];
@@ -934,10 +947,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
                 }
                 __syncthreads();
                 P = s_mv;
+                // materialize the owned trial positions and the new direction
+                store_records(n.x[(xb + 1 + ch) % 3] + 6 * (size_t)t.x, s_mv + 6 * (t.x - rg.xs), 6 * (t.y - t.x));
+                if (pend && !ch)
+                    store_records(n.d[((t.w >> 7) & 1) ^ 1] + 3 * (size_t)t.x, s_d, 3 * (t.y - t.x));
             }
             if (own) {
                 const Pos<float> p0 = load_pos(P, b - rg.xs);
-                if (tr) store_pos(n.x[(xb + 1 + ch) % 3], b, p0);   // materialize the owned trial position
                 if (fl & 1) {
                     const Pos<float> pp = load_pos(P, b + 1 - rg.xs);
                     float r2[3];
@@ -968,7 +984,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
         if (threadIdx.x == 0) {
             for (; pi < nt; ++pi)
                 if (s_desc[pi].w & 1) {
-                    issue_energy_stage(n, s_desc[pi], tr, &stage[issued % kBulkStages], &bar[issued % kBulkStages]);
+                    issue_energy_stage(n, s_desc[pi], tr, &stage[issued % kEnergyStages], &bar[issued % kEnergyStages]);
                     ++issued;
                     ++pi;
                     break;
@@ -979,7 +995,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
         // drain: copies still in flight must land before the block's shared memory is released
         if (threadIdx.x == 0)
             for (int q = max(j - 1, 0); q < issued; ++q)
-                mbar_wait_bounded(&bar[q % kBulkStages], (unsigned)((q / kBulkStages) & 1), kBulkWaitLimit);
+                mbar_wait_bounded(&bar[q % kEnergyStages], (unsigned)((q / kEnergyStages) & 1), kBulkWaitLimit);
         return;
     }
     if (cnt) flush();
