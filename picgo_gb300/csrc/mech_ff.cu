@@ -109,18 +109,25 @@ __device__ void set_conditions(const DevNet<Real>& n, bool head, int phase_slot)
     }
 }
 
-// After an evaluation's per-replica reduction: the last block zeroes the
-// excluded-volume work-list counts for the next evaluation (every block has
-// read them by then), then sets the graph conditions when there are any.
+// Zero the excluded-volume work-list counts for the next evaluation, once every
+// kernel that reads them has ended (one thread).
+template <typename Real>
+__device__ __forceinline__ void zero_counts(const DevNet<Real>& n, bool force) {
+    if (n.ev_list_count) *n.ev_list_count = 0;
+    if (n.ev_fb_count) *n.ev_fb_count = 0;
+    if (n.prelist && force) *n.ev_flist_count = 0;
+}
+// After an energy's per-replica reduction, which reads the fallback list: the last
+// block zeroes the counts (a force evaluation's gather, behind the last reader,
+// has done that: with 32 replicas the ticket took 1 us).  Then, after both, it
+// sets the graph conditions when there are any.
 template <typename Real>
 __device__ void after_evaluation(const DevNet<Real>& n, int phase_slot, int* s_flag) {
+    const bool force = phase_slot == kCondForce;
+    if (force && !n.cond.on) return;
     if (gridDim.x == 1) __syncthreads();   // one replica: this block is the last, no ticket needed
     else if (!last_tile(n.gticket, 0, gridDim.x, s_flag)) return;
-    if (threadIdx.x == 0) {
-        if (n.ev_list_count) *n.ev_list_count = 0;
-        if (n.ev_fb_count) *n.ev_fb_count = 0;
-        if (n.prelist && phase_slot == kCondForce) *n.ev_flist_count = 0;
-    }
+    if (threadIdx.x == 0 && !force) zero_counts(n, false);
     if (n.cond.on) set_conditions(n, false, phase_slot);
 }
 
@@ -442,6 +449,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_force_gather(DevNet<double> n, in
     pdl_wait();      // the force kernels have finished
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_GATHER);
+    if (blockIdx.x == 0 && threadIdx.x == 0) zero_counts(n, true);   // their readers have finished
     __shared__ double sh[2 * NT * kBlock / 32];
     __shared__ unsigned long long s_mx[NT * kBlock / 32];
     __shared__ GatherWarp s_warp[NT > 1 ? kBlock / 32 : 1];
@@ -495,6 +503,7 @@ __global__ void __launch_bounds__(kBlock) k_force_gather_mx(DevNet<float> n, int
     static_assert(kFilTile == 256 && kBlock == 64 * kGatherTiles, "64 threads x 4 beads per tile");
     pdl_trigger();   // the next kernel of the main lane may be scheduled now
     MECH_TRACE_KERNEL(n, TK_GATHER_MX);
+    if (blockIdx.x == 0 && threadIdx.x == 0) zero_counts(n, true);   // their readers have finished
     __shared__ float sh[8][5];   // per warp: F.F (hi, lo), F.Fprev (hi, lo), max
     __shared__ int s_go[kGatherTiles], s_rep[kGatherTiles];
     const int nt = blockDim.x >> 6;   // tiles of this block
