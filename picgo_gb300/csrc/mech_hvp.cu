@@ -477,7 +477,8 @@ __global__ void __launch_bounds__(kHvpBlock) k_hess_apply_sparse(DevNet<double> 
 constexpr int kCgBlocks = 304;
 
 // scal: [0], [1] r.r of the even and odd iterations, [2] alpha, [3] b.b,
-// [4] curvature flag, [5] beta
+// [4] kCgRunning, or why the iterate is frozen, [5] beta
+constexpr double kCgRunning = 0.0, kCgCurvature = 1.0, kCgConverged = 2.0;
 // Sum over the grid's blocks; `finish` gets it in one thread of the last block.
 template <typename F>
 __device__ __forceinline__ void grid_dot(double v, double* part, unsigned* ticket, double* sh, F&& finish) {
@@ -515,14 +516,22 @@ __global__ void __launch_bounds__(kHvpBlock) k_cg_start(const double* __restrict
     grid_dot(v, part, ticket, sh, [&](double bb) { scal[0] = scal[3] = bb; });
 }
 
+// The CG step alpha = r.r / p.Ap from p.Ap.  No positive curvature freezes the
+// iterate (alpha = 0): the truncated solution is what the caller gets, as
+// non-positive curvature, or, where the residual is within the tolerance already,
+// as the solution.  The host looks every kCheck iterations, and by then a residual
+// in few of H's eigenvectors can have underflowed to 0, with p.Ap = 0.
+__device__ __forceinline__ void cg_alpha(double pAp, double* scal, int odd, double tol2) {
+    if (scal[4] == kCgRunning && !(pAp > 0.0)) scal[4] = scal[odd] <= tol2 ? kCgConverged : kCgCurvature;
+    scal[2] = scal[4] != kCgRunning ? 0.0 : scal[odd] / pAp;
+}
+
 // hv = H v + shift v at the beads (the filaments' blocks and the gathered sparse
-// contributions), v . hv, and the CG step alpha = r.r / v.hv.  scal[4] latches
-// non-positive curvature: the iterate is frozen there (alpha = 0; the truncated
-// solution is what the caller gets).
+// contributions), v . hv, and the CG step.
 __global__ void __launch_bounds__(kHvpBlock) k_hess_apply_fil(DevNet<double> n, const double* __restrict__ V,
                                                              const double* __restrict__ A, double shift,
                                                              double* __restrict__ HV, double* scal, int odd,
-                                                             double* part, unsigned* ticket) {
+                                                             double tol2, double* part, unsigned* ticket) {
     __shared__ double sh[32];
     __shared__ double su[kHvpBlock + 3][3];   // u of cylinders first - 2 .. first + kHvpBlock
     __shared__ double sg[kHvpBlock + 1][3];   // G of cylinders first - 1 .. first + kHvpBlock - 1
@@ -571,11 +580,7 @@ __global__ void __launch_bounds__(kHvpBlock) k_hess_apply_fil(DevNet<double> n, 
             v += vq * h[q];
         }
     }
-    grid_dot(v, part, ticket, sh, [&](double pAp) {
-        const bool stop = scal[4] != 0.0 || !(pAp > 0.0);
-        if (stop) scal[4] = 1.0;
-        scal[2] = stop ? 0.0 : scal[odd] / pAp;
-    });
+    grid_dot(v, part, ticket, sh, [&](double pAp) { cg_alpha(pAp, scal, odd, tol2); });
 }
 
 // x += alpha p, r -= alpha Ap; the new r . r and beta
@@ -593,7 +598,7 @@ __global__ void __launch_bounds__(kHvpBlock) k_cg_step(double* __restrict__ x, d
         v += ri * ri;
     }
     grid_dot(v, part, ticket, sh, [&](double rr) {
-        scal[5] = rr / scal[odd];
+        scal[5] = scal[odd] > 0.0 ? rr / scal[odd] : 0.0;
         scal[odd ^ 1] = rr;
     });
 }
@@ -696,7 +701,7 @@ cudaError_t hvp_cg_solve(const DevNet<double>& n, const double* b, double* x, co
             k_hess_apply_sparse<<<sp_blocks, B, 0, s>>>(n, w.p, w.blocks, lm_blocks, ev_blocks);
             ++per_iter;
         }
-        k_hess_apply_fil<<<(n.nb + B - 1) / B, B, 0, s>>>(n, w.p, w.blocks.fil, shift, w.Ap, w.scal, odd, w.part, w.ticket);
+        k_hess_apply_fil<<<(n.nb + B - 1) / B, B, 0, s>>>(n, w.p, w.blocks.fil, shift, w.Ap, w.scal, odd, tol2, w.part, w.ticket);
         k_cg_step<<<G, B, 0, s>>>(x, w.r, w.p, w.Ap, N, w.scal, odd, w.part, w.ticket);
         k_cg_dir<<<G, B, 0, s>>>(w.p, w.r, N, w.scal);
     };
@@ -726,7 +731,7 @@ cudaError_t hvp_cg_solve(const DevNet<double>& n, const double* b, double* x, co
         const double rr = h[it & 1];
         res->iterations = it;
         res->rel_residual = sqrt(rr / bb);
-        if (h[4] != 0.0) {   // non-positive curvature met: the iterate stopped there
+        if (h[4] == kCgCurvature) {   // non-positive curvature met: the iterate stopped there
             res->negative_curvature = 1;
             break;
         }
