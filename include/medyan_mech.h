@@ -162,7 +162,9 @@ int32_t mech_ctx_destroy(MechContext* ctx);
 /*
  * Load networks: serializeDof + ForceFieldManager::vectorizeAllForceFields
  * (Structure/DofSerializer.hpp:64-187, Mechanics/ForceField/ForceFieldManager.cpp:35-93).
- * Rebuilds the neighbor lists at the given coordinates.
+ * Rebuilds the neighbor lists at the given coordinates.  A call that fails on
+ * its networks leaves the context without one: other calls then return
+ * MECH_ERR_STATE until networks are loaded.
  */
 int32_t mech_set_networks(MechContext* ctx, int32_t n_replicas, const MechNetwork* nets);
 

@@ -524,6 +524,9 @@ static void add_force_tiles(const MechContext* c, int r, std::vector<Tile>& ft) 
 
 static int set_networks(MechContext* c, int R, const MechNetwork* nets) {
     if (R <= 0 || !nets) return set_err(MECH_ERR_ARG, "no networks");
+    // From here on the context's description is replaced, its buffers further
+    // down: a call that ends in between leaves it without a network.
+    c->have_net = c->have_lists = c->h_fresh = false;
     c->reps.assign(R, ReplicaHost());
     c->R = R;
     int nb = 0, ncyl = 0, nlk = 0, nmt = 0, npl = 0;
