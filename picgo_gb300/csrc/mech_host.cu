@@ -903,6 +903,7 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
         R1.pad = 0;
     }
     if (ncells > 2000000000LL) return set_err(MECH_ERR_CAPACITY, "bin grid too large");
+    c->have_lists = false;   // counts and buffers change one by one from here: all of them, or the next call builds again
     int rc;
     if ((rc = upload(c->nl_rep, rep, s))) return rc;
     NLInput in{};

@@ -25,12 +25,21 @@
 
 namespace mech {
 
+#ifdef MECH_ALLOC_LIMIT
+// builds for tests of what follows a failed allocation: larger ones fail
+extern "C" size_t mech_alloc_limit = MECH_ALLOC_LIMIT;
+#endif
+
 cudaError_t DeviceBuffer::ensure(size_t nbytes) {
     if (nbytes <= bytes && p) return cudaSuccess;
     release();
+#ifdef MECH_ALLOC_LIMIT
+    if (nbytes > mech_alloc_limit) return cudaErrorMemoryAllocation;
+#endif
     size_t want = nbytes < 256 ? 256 : nbytes;
     cudaError_t e = cudaMalloc(&p, want);
     if (e != cudaSuccess) {
+        cudaGetLastError();   // returned here, and not found again by the next call's launches
         p = nullptr;
         bytes = 0;
         return e;

@@ -1,0 +1,82 @@
+"""Device allocations that fail, by a build of the library whose device buffers refuse more than a limit that the test
+sets (no memory is filled): a call that fails on one leaves its context usable, and nothing runs on lists that are new
+in part."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from picgo_gb300 import Engine, _lib, build, make_network
+
+pytestmark = pytest.mark.gpu
+
+ERR_CUDA = -3
+NO_LIMIT = 1 << 62
+
+
+@pytest.fixture(scope="module")
+def limited_library(tmp_path_factory):
+    """The library with mech_nl.cu (which allocates) compiled for a limit, and its other objects as they are."""
+    d = tmp_path_factory.mktemp("limited")
+    nl, out = str(d / "mech_nl.o"), str(d / build.LIBNAME)
+    subprocess.run([build.nvcc(), *build.ARCH, *build.COMMON, f"-DMECH_ALLOC_LIMIT={NO_LIMIT}ull", "-c",
+                    os.path.join(build.CSRC, "mech_nl.cu"), "-o", nl], check=True)
+    objs = [nl if o == "mech_nl.o" else os.path.join(build.OUTDIR, o) for _, o, _ in build.UNITS]
+    subprocess.run([build.nvcc(), *build.ARCH, "-shared", "-o", out, *objs, "-Xcompiler", "-fPIC"], check=True)
+    return out
+
+
+@pytest.fixture
+def limit(limited_library, monkeypatch):
+    """Contexts made in the test use that library; the fixture sets the limit in bytes."""
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(build, "lib_path", lambda: limited_library)
+    value = C.c_size_t.in_dll(_lib.load(), "mech_alloc_limit")
+
+    def set_limit(n):
+        value.value = n
+    set_limit(NO_LIMIT)
+    yield set_limit
+    set_limit(NO_LIMIT)
+
+
+def chain_net(n_filaments=200):
+    return make_network("c1", n_filaments=n_filaments, n_linkers=0, seed=4)
+
+
+def crowded(net):
+    """The same filaments, all of them within the pair cutoff of one another."""
+    x = net.coord.reshape(net.n_filaments, -1, 3)
+    rng = np.random.default_rng(1)
+    return (x[:1] + rng.normal(0, 2.0, (net.n_filaments, 1, 3))).reshape(-1, 3)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_lists_after_a_rebuild_that_fails(precision, limit):
+    net = chain_net()
+    with Engine(precision) as eng:
+        eng.set_network(net)
+        want, pairs, f = eng.energies(), eng.pairs().copy(), eng.forces()
+        n_full = 0
+        with Engine(precision) as other:
+            other.set_network(net)
+            other.set_coords(crowded(net))
+            n_full = other.rebuild()["n_exvol_pairs"]
+        assert n_full > 50 * net.n_cyl
+        limit(16 * n_full // 2)          # the pair list fits (8 bytes a pair), the beads of the pairs (16) do not
+        eng.set_coords(crowded(net))
+        for call in (lambda: eng.rebuild(), lambda: eng.energies(), lambda: eng.forces(), lambda: eng.minimize()):
+            with pytest.raises(_lib.MechError) as e:
+                call()
+            assert e.value.code == ERR_CUDA
+        with pytest.raises(_lib.MechError):
+            eng.pairs()
+        eng.set_coords(net.coord)        # what fitted fits again, by the lists that the evaluation builds
+        got = eng.energies()
+        assert np.array_equal(got[0], want[0]) and got[1:] == want[1:]
+        assert np.array_equal(eng.pairs(), pairs) and np.array_equal(eng.forces(), f)
+        limit(NO_LIMIT)
+        eng.set_coords(crowded(net))
+        assert eng.rebuild()["n_exvol_pairs"] == n_full
