@@ -1495,6 +1495,13 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
 // ===========================================================================
 // C ABI
 // ===========================================================================
+// What a call returns that fails with copies from or to the caller's memory
+// possibly in flight (pinned memory is read and written in stream order).
+static int drained(MechContext* ctx, int rc) {
+    if (rc) cudaStreamSynchronize(ctx->stream);
+    return rc;
+}
+
 extern "C" {
 
 int32_t mech_abi_version(void) { return MECH_ABI_VERSION; }
@@ -1550,7 +1557,7 @@ int32_t mech_set_networks(MechContext* ctx, int32_t n_replicas, const MechNetwor
     if (!ctx) return set_err(MECH_ERR_ARG, "null context");
     CU(cudaSetDevice(ctx->device));
     const int rc = set_networks(ctx, n_replicas, nets);
-    if (rc) return rc;
+    if (rc) return drained(ctx, rc);
     return rebuild(ctx, 0.0, nullptr);
 }
 
@@ -1588,7 +1595,7 @@ int32_t mech_set_coords(MechContext* ctx, int32_t r, const double* coord) {
     int rc = check_replica(ctx, r);
     if (rc) return rc;
     if (!coord) return set_err(MECH_ERR_ARG, "null coord");
-    if ((rc = put_coords(ctx, r, coord))) return rc;
+    if ((rc = put_coords(ctx, r, coord))) return drained(ctx, rc);
     CU(cudaStreamSynchronize(ctx->stream));
     return MECH_OK;
 }
@@ -1765,11 +1772,11 @@ int32_t mech_energy_terms(MechContext* ctx, int32_t r, double* stretch, double* 
 int32_t mech_energy(MechContext* ctx, int32_t r, const double* coord, double* per_ff, double* total, double* energy) {
     int rc = check_replica(ctx, r);
     if (rc) return rc;
-    if (coord && (rc = put_coords(ctx, r, coord))) return rc;
+    if (coord && (rc = put_coords(ctx, r, coord))) return drained(ctx, rc);
     CU(cudaSetDevice(ctx->device));
-    if (!ctx->have_lists && (rc = rebuild(ctx, 0.0, nullptr))) return rc;
+    if (!ctx->have_lists && (rc = rebuild(ctx, 0.0, nullptr))) return drained(ctx, rc);
     rc = ctx->precision == MECH_PREC_FP64 ? eval_energy<double>(ctx, r) : eval_energy<float>(ctx, r);
-    if (rc) return rc;
+    if (rc) return drained(ctx, rc);
     if (*ctx->h_err & (2u | 4u | 16u | 32u)) return err_status(*ctx->h_err);
     const CGState& S = ctx->h_st[r];
     if (per_ff)
@@ -1782,11 +1789,11 @@ int32_t mech_energy(MechContext* ctx, int32_t r, const double* coord, double* pe
 int32_t mech_forces(MechContext* ctx, int32_t r, const double* coord, double* f_out) {
     int rc = check_replica(ctx, r);
     if (rc) return rc;
-    if (coord && (rc = put_coords(ctx, r, coord))) return rc;
+    if (coord && (rc = put_coords(ctx, r, coord))) return drained(ctx, rc);
     CU(cudaSetDevice(ctx->device));
-    if (!ctx->have_lists && (rc = rebuild(ctx, 0.0, nullptr))) return rc;
+    if (!ctx->have_lists && (rc = rebuild(ctx, 0.0, nullptr))) return drained(ctx, rc);
     rc = ctx->precision == MECH_PREC_FP64 ? eval_forces<double>(ctx, r, f_out) : eval_forces<float>(ctx, r, f_out);
-    if (rc) return rc;
+    if (rc) return drained(ctx, rc);
     return *ctx->h_err ? err_status(*ctx->h_err) : MECH_OK;
 }
 

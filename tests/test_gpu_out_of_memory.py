@@ -80,3 +80,26 @@ def test_lists_after_a_rebuild_that_fails(precision, limit):
         limit(NO_LIMIT)
         eng.set_coords(crowded(net))
         assert eng.rebuild()["n_exvol_pairs"] == n_full
+
+
+@pytest.mark.parametrize("forces", [False, True])
+def test_coordinates_of_a_failed_evaluation_have_been_read(forces, limit):
+    """An evaluation that fails before its first wait (no room for the lists) has read the caller's pinned coordinates
+    when it returns: they can be overwritten at once."""
+    torch = pytest.importorskip("torch")
+    net = make_network("c1", n_filaments=10000, n_cyl_per_filament=50, box=10000.0, n_linkers=0, seed=4)
+    moved = net.coord + 1.0
+    with Engine("mixed") as eng:
+        limit(28 * net.n_beads)          # positions (24 bytes a bead) fit, the neighbors kept from the count (32) do not
+        with pytest.raises(_lib.MechError):
+            eng.set_network(net)
+        eng.nbeads, eng.nlinkers, eng.nmotors = [net.n_beads], [0], [0]
+        pinned = torch.empty((net.n_beads, 3), dtype=torch.float64, pin_memory=True)
+        pinned.copy_(torch.from_numpy(moved))
+        x = pinned.numpy()
+        with pytest.raises(_lib.MechError) as e:
+            eng.forces(x) if forces else eng.energies(x)
+        x[:] = -1e6
+        assert e.value.code == ERR_CUDA
+        # positions are held to 48 bits
+        assert np.abs(eng.coords() - moved).max() <= 1e-10
