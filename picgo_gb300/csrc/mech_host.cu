@@ -2110,12 +2110,17 @@ static int hvp_buffers(MechContext* c, HvpCgWork* w) {
     CU(c->cg_scal.ensure(sizeof(double) * 8));
     CU(c->cg_part.ensure(sizeof(double) * std::max<size_t>(512, (size_t)c->nb / 256 + 1)));
     CU(c->cg_ticket.ensure(sizeof(unsigned) * 4));
-    CU(c->hess_fil.ensure(12 * v));
-    CU(c->hess_lm.ensure(sizeof(double) * 5 * (size_t)std::max(c->nlk + c->nmt, 1)));
-    CU(c->hess_ev.ensure(sizeof(double) * 81 * (size_t)std::max<long long>(c->nev, 1)));
-    CU(c->hess_bb.ensure(sizeof(double) * (size_t)std::max<long long>(c->nbb, 1)));
+    cudaError_t e = c->hess_fil.ensure(12 * v);
+    if (e == cudaSuccess) e = c->hess_lm.ensure(sizeof(double) * 5 * (size_t)std::max(c->nlk + c->nmt, 1));
+    if (e == cudaSuccess) e = c->hess_ev.ensure(sizeof(double) * 81 * (size_t)std::max<long long>(c->nev, 1));
+    if (e == cudaSuccess) e = c->hess_bb.ensure(sizeof(double) * (size_t)std::max<long long>(c->nbb, 1));
     w->blocks = HvpBlocks{c->hess_fil.as<double>(), c->hess_lm.as<double>(), c->hess_ev.as<double>(),
                           c->hess_bb.as<double>()};
+    if (e != cudaSuccess) {   // no room for the blocks: a solve needs none
+        if (e != cudaErrorMemoryAllocation) return set_err(MECH_ERR_CUDA, cudaGetErrorString(e));
+        for (DeviceBuffer* b : {&c->hess_fil, &c->hess_lm, &c->hess_ev, &c->hess_bb}) b->release();
+        w->blocks = HvpBlocks{};
+    }
     w->r = c->cg_r.as<double>();
     w->p = c->cg_p.as<double>();
     w->Ap = c->cg_Ap.as<double>();

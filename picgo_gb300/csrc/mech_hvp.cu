@@ -253,7 +253,8 @@ __global__ void __launch_bounds__(kHvpBlock) k_hvp_fil(DevNet<double> n, const d
 // An application is then ~45 FP64 instructions per bead and ~60 per 8 pairs, and
 // reads the blocks once, coalesced (the 216 bytes per cylinder bound it from
 // about 100,000 cylinders on, when they leave L2).  Setting them up costs about
-// two applications by duals.
+// two applications by duals.  They take 288 bytes per bead and 648 per pair; where
+// that cannot be had a solve applies the duals in every iteration.
 __device__ __forceinline__ Dual unit(double v, bool on) { return Dual(v, on ? 1.0 : 0.0); }
 
 __global__ void __launch_bounds__(kHvpBlock) k_hess_fil(DevNet<double> n, double* __restrict__ A) {
@@ -583,6 +584,17 @@ __global__ void __launch_bounds__(kHvpBlock) k_hess_apply_fil(DevNet<double> n, 
     grid_dot(v, part, ticket, sh, [&](double pAp) { cg_alpha(pAp, scal, odd, tol2); });
 }
 
+// the CG step of a product formed by duals: v . hv
+__global__ void __launch_bounds__(kHvpBlock) k_cg_alpha(const double* __restrict__ v, const double* __restrict__ hv,
+                                                        long long n, double* scal, int odd, double tol2, double* part,
+                                                        unsigned* ticket) {
+    __shared__ double sh[32];
+    double a = 0.0;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        a += v[i] * hv[i];
+    grid_dot(a, part, ticket, sh, [&](double pAp) { cg_alpha(pAp, scal, odd, tol2); });
+}
+
 // x += alpha p, r -= alpha Ap; the new r . r and beta
 __global__ void __launch_bounds__(kHvpBlock) k_cg_step(double* __restrict__ x, double* __restrict__ r,
                                                        const double* __restrict__ p, const double* __restrict__ Ap,
@@ -688,7 +700,8 @@ cudaError_t hvp_cg_solve(const DevNet<double>& n, const double* b, double* x, co
         return cudaSuccess;
     }
     const double tol2 = rel_tol * rel_tol * bb;
-    res->launches = assemble_hessian(n, w.blocks, s);
+    const bool blocks = w.blocks.fil != nullptr;
+    if (blocks) res->launches = assemble_hessian(n, w.blocks, s);
     // kCheck iterations per CUDA graph launch; the host reads the residual between launches
     constexpr int kCheck = 16;   // even: a graph starts on an even iteration
     const int lm_blocks = (n.n_lk + n.n_mt + B - 1) / B, ev_blocks = (int)((4LL * n.n_ev + B - 1) / B),
@@ -697,11 +710,16 @@ cudaError_t hvp_cg_solve(const DevNet<double>& n, const double* b, double* x, co
     auto iteration = [&](int it) {
         const int odd = it & 1;
         per_iter = 3;
-        if (sp_blocks > 0) {
-            k_hess_apply_sparse<<<sp_blocks, B, 0, s>>>(n, w.p, w.blocks, lm_blocks, ev_blocks);
-            ++per_iter;
+        if (!blocks) {
+            per_iter += launch_hvp(n, w.p, w.Ap, shift, false, s);
+            k_cg_alpha<<<G, B, 0, s>>>(w.p, w.Ap, N, w.scal, odd, tol2, w.part, w.ticket);
+        } else {
+            if (sp_blocks > 0) {
+                k_hess_apply_sparse<<<sp_blocks, B, 0, s>>>(n, w.p, w.blocks, lm_blocks, ev_blocks);
+                ++per_iter;
+            }
+            k_hess_apply_fil<<<(n.nb + B - 1) / B, B, 0, s>>>(n, w.p, w.blocks.fil, shift, w.Ap, w.scal, odd, tol2, w.part, w.ticket);
         }
-        k_hess_apply_fil<<<(n.nb + B - 1) / B, B, 0, s>>>(n, w.p, w.blocks.fil, shift, w.Ap, w.scal, odd, tol2, w.part, w.ticket);
         k_cg_step<<<G, B, 0, s>>>(x, w.r, w.p, w.Ap, N, w.scal, odd, w.part, w.ticket);
         k_cg_dir<<<G, B, 0, s>>>(w.p, w.r, N, w.scal);
     };

@@ -440,7 +440,7 @@ template <typename Real> int launch_exvol_forces(const DevNet<Real>& n, int want
 // order; H is the energy's Hessian, or with `jacobian` minus the Jacobian of
 // the force routine (which moves nearly coplanar excluded-volume pairs)
 int launch_hvp(const DevNet<double>& n, const double* v, double* hv, double shift, bool jacobian, cudaStream_t s);
-// blocks of the Hessian that a solve applies (mech_hvp.cu)
+// blocks of the Hessian that a solve applies (mech_hvp.cu); null: it applies products by duals
 struct HvpBlocks {
     double* fil;   // [36 * nb]
     double* lm;    // [5 * (linkers + motors)]

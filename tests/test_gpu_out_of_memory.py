@@ -8,7 +8,7 @@ import subprocess
 import numpy as np
 import pytest
 
-from picgo_gb300 import Engine, _lib, build, make_network
+from picgo_gb300 import Engine, _lib, build, jitter, make_network
 
 pytestmark = pytest.mark.gpu
 
@@ -103,3 +103,33 @@ def test_coordinates_of_a_failed_evaluation_have_been_read(forces, limit):
         assert e.value.code == ERR_CUDA
         # positions are held to 48 bits
         assert np.abs(eng.coords() - moved).max() <= 1e-10
+
+
+@pytest.mark.parametrize("what", ["filaments", "pairs"])
+def test_solves_without_room_for_the_hessian(what, limit):
+    """A solve that finds no room for the Hessian's blocks applies it by duals: the same Hessian, rounded differently.
+    The eigenvalues of this network's (central differences of the oracle's forces) plus the shift lie between 160 and
+    1,900, so a relative residual of 1e-12 leaves the solutions within 1e-10 of their size; 1e-8 of the gradients."""
+    cfg = dict(n_filaments=17, n_cyl_per_filament=14, box=700.0, n_linkers=34, linker_k=(4.0, 12.0),
+               linker_l0=(20.0, 40.0), n_motors=17, shape="chain")
+    net = jitter(make_network(cfg, seed=1), 0.2, seed=2)
+    net.cyl_kexvol = 1e-4 * net.cyl_kexvol
+    net.exvol_cutoff = 100.0
+    g = np.random.default_rng(3).normal(size=net.coord.shape)
+    kw = dict(rel_tol=1e-12, max_iter=2000, shift=200.0)
+    with Engine("fp64") as eng:
+        eng.set_network(net)
+        n = eng.rebuild()["n_exvol_pairs"]
+        assert 648 * n > 400 * net.n_beads
+        want = eng.adjoint(g, 0.5, **kw)
+    with Engine("fp64") as eng:
+        eng.set_network(net)
+        limit({"filaments": 100, "pairs": 300}[what] * net.n_beads)
+        got = eng.adjoint(g, 0.5, **kw)
+        flat = eng.adjoint(np.ones_like(g), 0.5, rel_tol=1e-10, max_iter=200, shift=200.0)
+        limit(NO_LIMIT)
+        after = eng.adjoint(g, 0.5, **kw)
+    assert want[2]["converged"] and got[2]["converged"] and flat[2]["converged"] and after[2]["converged"]
+    assert got[2]["launches"] != want[2]["launches"] and after[2]["launches"] == want[2]["launches"]
+    for a, b, c in zip(want[:2], got[:2], after[:2]):
+        assert np.abs(a - b).max() <= 1e-8 * np.abs(a).max() and np.array_equal(a, c)
