@@ -430,10 +430,9 @@ int32_t mech_newton_refine(MechContext* ctx, int32_t max_steps, double force_tol
  * scratch is a fixed 131,328-byte device array inside the library.
  *
  * Inputs (device pointers, current device): fil_cyl_start[n_filaments+1]
- * strictly ascending cylinder ranges from 0 to n_cylinders: every filament
- * holds at least one cylinder, as every MEDYAN filament does (not checked:
- * the arrays are on the device; an empty filament shifts the beads of every
- * later filament and gives wrong energies); coord[3 * (n_cylinders + n_filaments)] with the
+ * ascending cylinder ranges from 0 to n_cylinders (not checked: the arrays are
+ * on the device; every MEDYAN filament holds at least one cylinder, and one
+ * without any takes up one bead); coord[3 * (n_cylinders + n_filaments)] with the
  * beads filament by filament, minus end first (cylinder c of filament f joins
  * beads c + f and c + f + 1); per-cylinder k_stretch, eq_length, k_bend,
  * eq_theta (the bending triple ending in cylinder c uses c's constants).

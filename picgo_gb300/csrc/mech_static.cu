@@ -102,11 +102,13 @@ k_fil_energy_static(const double* __restrict__ x, const int32_t* __restrict__ fc
         const int c0 = 32 * k, c = c0 + lane, g = fp + 1 + lane;
         const int s = g < nfil ? __ldg(fcs + g) - c0 : 32;   // the next filaments' first cylinders, ascending from 0
         const unsigned starts = __reduce_or_sync(kAll, s < 32 ? 1u << s : 0u);
+        // a start equal to the next one read, or (32 starts in the chunk) to the one behind them
         const int before = __shfl_up_sync(kAll, s, 1);
+        const bool twice = s < 32 && ((lane > 0 && s == before) || (lane == 31 && __ldg(fcs + g + 1) - c0 == s));
         const bool valid = c < ncyl;
         int f;
         bool first;
-        if (!__any_sync(kAll, lane > 0 && s < 32 && s == before)) {
+        if (!__any_sync(kAll, twice)) {
             f = fp + __popc(starts & (kAll >> (31 - lane)));
             first = starts >> lane & 1;
             fp += __popc(starts);
