@@ -882,7 +882,8 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
         R1.rmax2 = (double)(float)(h.rmax * h.rmax);
         R1.rmin2 = 0.0;
         const double box = std::max(h.box[0], std::max(h.box[1], h.box[2]));
-        // float-midpoint prefilter slack (coordinates up to a few boxes from the origin; 2 ulp per midpoint)
+        // float-midpoint prefilter slack (coordinates up to a few boxes from the
+        // origin, beyond which every pair takes the exact test; 2 ulp per midpoint)
         const double M = 4.0 * box + 1e4;
         const double delta = (2.0 * M + h.rmax) * 1.2e-7;
         const double slack = 2.0 * h.rmax * std::sqrt(3.0) * delta + 3.0 * delta * delta + 4e-7 * h.rmax * h.rmax + 1e-2;
@@ -900,7 +901,7 @@ static int rebuild(MechContext* c, double cell_req, MechListInfo* info) {
         R1.cyl_begin = h.cyl_begin;
         R1.plane_begin = h.plane_begin;
         R1.bnd_cutoff_f = (float)h.bcut;
-        R1.pad = 0;
+        R1.reach = (float)M;
     }
     if (ncells > 2000000000LL) return set_err(MECH_ERR_CAPACITY, "bin grid too large");
     c->have_lists = false;   // counts and buffers change one by one from here: all of them, or the next call builds again

@@ -247,6 +247,8 @@ __device__ __forceinline__ void nl_visit(const NLInput& in, const int* cell_star
     const int4 g = R.dims;
     const int ix = cell_axis(fc.x, R.inv, g.x), iy = cell_axis(fc.y, R.inv, g.y), iz = cell_axis(fc.z, R.inv, g.z);
     const int z0 = max(iz - 1, 0), z1 = min(iz + 1, g.z - 1) + 1;
+    const bool far = !(fmaxf(fmaxf(fabsf(fc.x), fabsf(fc.y)), fabsf(fc.z)) <= R.reach);
+    const float pre = far ? INFINITY : R.pre, sure = far ? -INFINITY : R.sure;
     int s0[9], s1[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
@@ -265,7 +267,7 @@ __device__ __forceinline__ void nl_visit(const NLInput& in, const int* cell_star
             const float4 fn = sorted[s];
             const float ex = fn.x - fc.x, ey = fn.y - fc.y, ez = fn.z - fc.z;
             const float f2 = ex * ex + ey * ey + ez * ez;
-            if (f2 > R.pre) continue;
+            if (f2 > pre) continue;
             const int n = __float_as_int(fn.w);
             if (n == c) continue;
             if (!have) {   // the cylinder's own data, for the few that have a candidate
@@ -276,7 +278,7 @@ __device__ __forceinline__ void nl_visit(const NLInput& in, const int* cell_star
             }
             if (idc <= in.cyl_id[n]) continue;
             if (filc == in.cyl_fil[n] && abs(posc - in.cyl_pos[n]) <= 2) continue;
-            if (!(f2 < R.sure)) {   // within the rounding of the cutoff: the reference's test on the exact midpoints
+            if (!(f2 < sure)) {   // within the rounding of the cutoff: the reference's test on the exact midpoints
                 double mc[3], mn[3], d2 = 0.0;
                 exact_mid(in.x, in.mixed, in.cyl_b1[c], mc);
                 exact_mid(in.x, in.mixed, in.cyl_b1[n], mn);

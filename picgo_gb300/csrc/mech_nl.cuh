@@ -13,7 +13,7 @@ struct NLReplica {
     double rmax2, rmin2;       // squared cutoffs rounded to float, held as double
     double bnd_cutoff;
     float bnd_cutoff_f;
-    int pad;
+    float reach;               // pre and sure hold up to this magnitude of a midpoint coordinate
     long long bnd_begin;       // first (plane, cylinder) entry
     int ncyl, cyl_begin, plane_begin;
 };
