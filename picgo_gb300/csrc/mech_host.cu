@@ -96,6 +96,7 @@ struct MechContext {
     // Hessian-vector products, adjoint and Newton solves (FP64 engine)
     DeviceBuffer hv_a, hv_b, cg_x, cg_r, cg_p, cg_Ap, cg_scal, cg_part, cg_ticket, hess_fil, hess_lm, hess_ev, hess_bb;
     DeviceBuffer lf_ends, lf_types, lf_ms, lf_nm, lf_out;   // load forces
+    DeviceBuffer et_terms, et_out;                          // energy terms
     int n_ftiles = 0, n_force_tiles = 0, n_stiles = 0;
     int sp_tiles[K_NUM_SPARSE] = {0, 0, 0, 0};
     // host copies of the full tile lists, and the compacted view that a
@@ -1741,7 +1742,9 @@ int32_t mech_energy_terms(MechContext* ctx, int32_t r, double* stretch, double* 
     if ((rc = select_replicas(ctx, r))) return rc;
     ctx->h_fresh = false;
     const ReplicaHost& h = ctx->reps[r];
-    DeviceBuffer terms, out;
+    // kept: allocating and freeing them took 20 to 120 us of 66 to 170 (60,000
+    // cylinders), by what else the context holds
+    DeviceBuffer &terms = ctx->et_terms, &out = ctx->et_out;
     const size_t rs = real_size(ctx);
     CU(terms.ensure(rs * 2 * (size_t)ctx->nb));
     CU(out.ensure(sizeof(double) * 2 * (size_t)h.ncyl));

@@ -8,7 +8,7 @@ import subprocess
 import numpy as np
 import pytest
 
-from picgo_gb300 import Engine, _lib, build, jitter, make_network
+from picgo_gb300 import Engine, _lib, build, cg_params, jitter, make_network
 
 pytestmark = pytest.mark.gpu
 
@@ -133,3 +133,26 @@ def test_solves_without_room_for_the_hessian(what, limit):
     assert got[2]["launches"] != want[2]["launches"] and after[2]["launches"] == want[2]["launches"]
     for a, b, c in zip(want[:2], got[:2], after[:2]):
         assert np.abs(a - b).max() <= 1e-8 * np.abs(a).max() and np.array_equal(a, c)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_repeated_calls_allocate_nothing(precision, limit):
+    net = jitter(make_network("c1", n_filaments=60, n_cyl_per_filament=12, box=1500.0, n_linkers=80, n_motors=40, seed=3),
+                 0.3, seed=7)
+    p = cg_params(energy_rel_tol=0.0, energy_call_limit=300)
+    v = np.random.default_rng(1).normal(size=net.coord.shape)
+    with Engine(precision) as eng:
+        calls = [lambda: eng.set_network(net), lambda: eng.energies(net.coord)[0], lambda: eng.forces(),
+                 lambda: eng.energy_terms(), lambda: eng.load_forces(), lambda: eng.rebuild()["n_exvol_pairs"],
+                 lambda: list(eng.minimize(p)[0]["energies_after"]), lambda: eng.coords(), lambda: eng.stretch_forces(),
+                 lambda: eng.set_coords(net.coord)]
+        if precision == "fp64":
+            calls += [lambda: eng.hvp(v), lambda: eng.adjoint(v, max_iter=32, shift=1e4)[0]]
+        first = [call() for call in calls]
+        limit(0)
+        for call, want in zip(calls, first):
+            got = call()
+            if isinstance(want, tuple):
+                assert all(np.array_equal(a, b) for a, b in zip(want, got))
+            else:
+                assert want is None or np.array_equal(want, got)
