@@ -2102,8 +2102,20 @@ static int hvp_vectors(MechContext* c) {
     return MECH_OK;
 }
 
+// Whether a solve of at most `max_iter` iterations earns the Hessian's blocks.
+// Setting them up evaluates every pair's duals nine times, an iteration without
+// them once, in rounds of a pair per lane of every FP64 pipe (~55 us each); the
+// rest of such an iteration takes half a round more than one with blocks.  60,000
+// cylinders with 34,715 pairs: one iteration 1,340 us with blocks and 519 without,
+// six 1,602 and 1,465, eight 1,698 and 1,847; with 1,380 pairs blocks from the first.
+static bool hessian_blocks_pay(int max_iter, long long pairs) {
+    constexpr long long kRound = 152 * 4 * 32;
+    auto rounds = [](long long n) { return std::max(1LL, (n + kRound - 1) / kRound); };
+    return max_iter * (2 * rounds(pairs) + 1) >= 2 * rounds(9 * pairs);
+}
+
 // the solver's vectors (3 * nb doubles each), scalars and Hessian blocks
-static int hvp_buffers(MechContext* c, HvpCgWork* w) {
+static int hvp_buffers(MechContext* c, int max_iter, HvpCgWork* w) {
     int rc;
     if ((rc = hvp_vectors(c))) return rc;
     const size_t v = sizeof(double) * 3 * (size_t)std::max(c->nb, 1);
@@ -2114,16 +2126,19 @@ static int hvp_buffers(MechContext* c, HvpCgWork* w) {
     CU(c->cg_scal.ensure(sizeof(double) * 8));
     CU(c->cg_part.ensure(sizeof(double) * std::max<size_t>(512, (size_t)c->nb / 256 + 1)));
     CU(c->cg_ticket.ensure(sizeof(unsigned) * 4));
-    cudaError_t e = c->hess_fil.ensure(12 * v);
-    if (e == cudaSuccess) e = c->hess_lm.ensure(sizeof(double) * 5 * (size_t)std::max(c->nlk + c->nmt, 1));
-    if (e == cudaSuccess) e = c->hess_ev.ensure(sizeof(double) * 81 * (size_t)std::max<long long>(c->nev, 1));
-    if (e == cudaSuccess) e = c->hess_bb.ensure(sizeof(double) * (size_t)std::max<long long>(c->nbb, 1));
-    w->blocks = HvpBlocks{c->hess_fil.as<double>(), c->hess_lm.as<double>(), c->hess_ev.as<double>(),
-                          c->hess_bb.as<double>()};
-    if (e != cudaSuccess) {   // no room for the blocks: a solve needs none
-        if (e != cudaErrorMemoryAllocation) return set_err(MECH_ERR_CUDA, cudaGetErrorString(e));
-        for (DeviceBuffer* b : {&c->hess_fil, &c->hess_lm, &c->hess_ev, &c->hess_bb}) b->release();
-        w->blocks = HvpBlocks{};
+    if (hessian_blocks_pay(max_iter, c->nev)) {
+        cudaError_t e = c->hess_fil.ensure(12 * v);
+        if (e == cudaSuccess) e = c->hess_lm.ensure(sizeof(double) * 5 * (size_t)std::max(c->nlk + c->nmt, 1));
+        if (e == cudaSuccess) e = c->hess_ev.ensure(sizeof(double) * 81 * (size_t)std::max<long long>(c->nev, 1));
+        if (e == cudaSuccess) e = c->hess_bb.ensure(sizeof(double) * (size_t)std::max<long long>(c->nbb, 1));
+        if (e == cudaSuccess) {
+            w->blocks = HvpBlocks{c->hess_fil.as<double>(), c->hess_lm.as<double>(), c->hess_ev.as<double>(),
+                                  c->hess_bb.as<double>()};
+        } else if (e == cudaErrorMemoryAllocation) {   // no room: a solve needs none
+            for (DeviceBuffer* b : {&c->hess_fil, &c->hess_lm, &c->hess_ev, &c->hess_bb}) b->release();
+        } else {
+            return set_err(MECH_ERR_CUDA, cudaGetErrorString(e));
+        }
     }
     w->r = c->cg_r.as<double>();
     w->p = c->cg_p.as<double>();
@@ -2229,7 +2244,7 @@ int32_t mech_adjoint(MechContext* ctx, int32_t r, const double* dL_dx, double dL
     CU(cudaSetDevice(ctx->device));
     if ((rc = hvp_ready(ctx))) return rc;
     HvpCgWork w{};
-    if ((rc = hvp_buffers(ctx, &w))) return rc;
+    if ((rc = hvp_buffers(ctx, sp->max_iter, &w))) return rc;
     if ((rc = put_replica_vec(ctx, r, dL_dx, ctx->hv_a))) return rc;
     if ((rc = clear_error(ctx))) return rc;
     ctx->h_fresh = false;
@@ -2263,7 +2278,7 @@ int32_t mech_newton_refine(MechContext* ctx, int32_t max_steps, double force_tol
     int rc;
     if ((rc = hvp_ready(ctx))) return rc;
     HvpCgWork w{};
-    if ((rc = hvp_buffers(ctx, &w))) return rc;
+    if ((rc = hvp_buffers(ctx, sp->max_iter, &w))) return rc;
     cudaStream_t s = ctx->stream;
     const long long N = 3LL * ctx->nb;
     HvpCgResult total{};
