@@ -257,13 +257,13 @@ int32_t mech_get_forces(MechContext* ctx, int32_t replica, double* f_out);
  * and exiting when it has nothing to do; the kernels follow one another by
  * programmatic dependent launch.  MECH_GRAPH_CONDITIONAL: one CUDA graph
  * whose device while loop runs, per body, only the phases some replica is in
- * (line-search pass, forces, direction, reset to steepest descent); the host is
- * involved only for recovery moves, errors and every 512 bodies.  Both run the
- * same active kernels in the same order and give bitwise the same results; on
- * GB300 with driver 580 the conditional bodies cost more than the idle
- * launches they replace (1M-cylinder minimization: 242 vs 199 us per
- * iteration).  No reference counterpart (the reference minimizer is a host
- * loop).
+ * (line-search pass, forces); the host is involved only for recovery moves,
+ * errors and every 512 bodies.  Both run the same active kernels in the same
+ * order and give bitwise the same results; on GB300 with driver 580 the
+ * conditional bodies cost more than the idle launches they replace (200 energy
+ * calls of a minimization with 1M cylinders: 13.9 ms, unrolled 10.7; 9,000 with
+ * 4,000 cylinders: 211 and 142 ms).  No reference counterpart (the reference
+ * minimizer is a host loop).
  */
 #define MECH_GRAPH_CONDITIONAL 0
 #define MECH_GRAPH_UNROLLED 1
@@ -319,13 +319,13 @@ typedef struct MechProfile {
     int64_t n_beads, n_exvol_pairs, n_boundary, n_linkers, n_motors, n_slots;
     int64_t n_exvol_ext_energy;    /* mixed engine: pairs its last energy pass sent to the extended-precision pass */
     int64_t n_exvol_ext_force;     /* and its last force pass */
-    double ms_iteration_idle;      /* one minimizer iteration block (two line-search trials, forces,
-                                      direction, reset) with no replica selected:
-                                      the cost of the launches that find nothing to do */
-    double ms_trial_energy_eval;   /* one line-search trial: energy at x + lambda d, trial positions written */
+    double ms_iteration_idle;      /* one minimizer iteration block (a line-search pass, forces) with no
+                                      replica selected: the cost of the launches that find nothing to do */
+    double ms_trial_energy_eval;   /* the first line-search pass of a search: the direction formed and written,
+                                      energy at x + lambda d (mixed: and at x + lambda / 2 d), positions written */
     int64_t n_exvol_fallback_energy;   /* pairs the last energy pass sent to the Simpson fallback */
     int64_t n_exvol_fallback_force;    /* and the last force pass */
-    double ms_fil_energy_trial;    /* filament energy of a trial (x + lambda d formed and written) */
+    double ms_fil_energy_trial;    /* filament energy of such a pass */
     double ms_fil_force_kernel;    /* filament forces alone (without the gather and reduction) */
     double ms_force_gather;        /* sparse gather with the CG partials alone */
 } MechProfile;
@@ -427,7 +427,7 @@ int32_t mech_newton_refine(MechContext* ctx, int32_t max_steps, double force_tol
  * For callers that must not allocate device memory at this point: cudaMalloc
  * and cudaFree can synchronize the whole device, and some hosts hand every
  * byte of HBM to their own pool up front.  The call needs no context; its
- * scratch is a fixed 131,328-byte device array inside the library.
+ * scratch is a fixed 5,120-byte device array inside the library.
  *
  * Inputs (device pointers, current device): fil_cyl_start[n_filaments+1]
  * ascending cylinder ranges from 0 to n_cylinders (not checked: the arrays are
@@ -439,7 +439,8 @@ int32_t mech_newton_refine(MechContext* ctx, int32_t max_steps, double force_tol
  * Output: energies[2] = {stretching, bending}, written on `stream` (a
  * cudaStream_t; NULL = legacy default stream); synchronize before reading.
  *
- * Limits: n_cylinders <= 2,097,152, else MECH_ERR_CAPACITY and nothing runs.
+ * Limits: n_cylinders <= 2,097,152 (of the interface, not of the scratch), else
+ * MECH_ERR_CAPACITY and nothing runs.
  * The first call in each CUDA context of a device looks up the scratch
  * address (again after a cudaDeviceReset or any other re-creation of the
  * context, since the array can move): make that call before any stream

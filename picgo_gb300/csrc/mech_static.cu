@@ -8,12 +8,12 @@
 // call makes no cudaMalloc/cudaFree (which can synchronize the whole device)
 // and needs no context.
 //
-// Scratch layout (kScratchBytes):
+// Scratch layout (kStaticScratchBytes):
 //   [0, 256)                      completion ticket (one unsigned int); must be
 //                                 zero when the kernel starts: the entry point
 //                                 clears it on the caller's stream before each
 //                                 launch and the last block leaves it at zero
-//   [256, 256 + 16 * kMaxBlocks)  per-block (stretching, bending) partial sums
+//   [256, 256 + 16 * kStaticGrid) per-block (stretching, bending) partial sums
 // Calls that overlap in time (different streams or host threads, same
 // device) share this scratch and race; the caller orders them.
 #include <cuda_runtime.h>
@@ -32,8 +32,10 @@ constexpr int kStaticBlock = 256;
 // and more of them only shorten the shares (1M cylinders with 1, 2, 3, 4, 8
 // blocks: 84.8, 75.8, 77.9, 80.7, 88.2 us).
 constexpr int kStaticGrid = 2 * 152;
-constexpr int kStaticMaxBlocks = 8192;   // partial-sum slots: up to 2,097,152 cylinders
-constexpr size_t kStaticScratchBytes = 256 + 16 * (size_t)kStaticMaxBlocks;   // 131,328 bytes
+// A limit of the interface, named for the scratch of a slot per 256 cylinders that
+// it once was: the shares of a fixed grid need no more for more cylinders.
+constexpr long long kStaticMaxCylinders = 2097152;
+constexpr size_t kStaticScratchBytes = 256 + 16 * (size_t)kStaticGrid;   // 5,120 bytes
 constexpr int kStaticMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
@@ -222,11 +224,11 @@ extern "C" int32_t mech_filament_energy_device(int32_t n_filaments, int32_t n_cy
         !eq_theta || !energies)
         return set_error_text(MECH_ERR_ARG, "mech_filament_energy_device: null pointer or bad count");
     const long long blocks = ((long long)n_cylinders + kStaticBlock - 1) / kStaticBlock;
-    if (blocks > kStaticMaxBlocks)
+    if (n_cylinders > kStaticMaxCylinders)
         return set_error_text(MECH_ERR_CAPACITY,
                               "mech_filament_energy_device: n_cylinders " + std::to_string(n_cylinders) +
-                                  " exceeds the fixed scratch limit of " +
-                                  std::to_string((long long)kStaticMaxBlocks * kStaticBlock) + " cylinders");
+                                  " exceeds the fixed scratch limit of " + std::to_string(kStaticMaxCylinders) +
+                                  " cylinders");
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
         cudaGetLastError();
