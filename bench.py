@@ -220,13 +220,13 @@ def run_ours(args, rank, world, dist):
     rs = 4 if args.precision == "mixed" else 8
     nb = prof["n_beads"]
     # Algorithmic bytes per launch (each input read once, each output written once).  The
-    # dominant kernel of a minimization is the filament energy of a line-search pass: it
-    # reads positions (24 B), flags (1 B), the four per-bead constants and the direction,
-    # and writes the trial positions (24 B per trial: the mixed engine evaluates lambda and
-    # lambda / 2 in one pass, FP64 one trial).
+    # dominant kernel of a minimization is the filament energy of a search's first line-search
+    # pass: it reads positions (24 B), flags (1 B), the four per-bead constants, the forces and
+    # the last direction, and writes the new direction and the trial positions (24 B per trial:
+    # the mixed engine evaluates lambda and lambda / 2 in one pass, FP64 one trial).
     trial_writes = 48 if args.precision == "mixed" else 24
     kernels = {
-        "fil_energy_trial": (prof["ms_fil_energy_trial"], nb * (24 + 1 + 4 * rs + 3 * rs + trial_writes)),
+        "fil_energy_trial": (prof["ms_fil_energy_trial"], nb * (24 + 1 + 4 * rs + 9 * rs + trial_writes)),
         "fil_force": (prof["ms_fil_force_kernel"], nb * (24 + 1 + 4 * rs + 3 * rs)),
         "force_gather": (prof["ms_force_gather"],
                          nb * (3 * rs * 3 + 4) + prof["n_slots"] * 3 * rs),

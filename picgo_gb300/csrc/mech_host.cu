@@ -115,10 +115,11 @@ struct MechContext {
     // defaults to 2: its blocks stream from the start of the evaluation while
     // the excluded-volume chain (FP32 pass, extended-precision pass, fallbacks)
     // and the linker kernel keep room on every SM.  Force evaluation on the
-    // 1M-cylinder network, graph replays at fixed states: 77 us at 2 blocks,
-    // 95 at 3, 125 uncapped (the kernel alone: 28.7, 22.6, 20.5 us).  A cap on
-    // the energy kernel only delays the excluded-volume chain (trial pass 78 us
-    // uncapped, 90 at 2, 107 at 3).
+    // 1M-cylinder network, graph replays: 57 us at 2 blocks, 63 at 1, 60 at 3 and
+    // 4, 72 uncapped (the kernel alone: 22.6, 34.9, 18.5); an iteration 101 us at
+    // 2, 102 to 104 above, 114 at 1.  A cap on the energy kernel only delays the
+    // excluded-volume chain (trial pass 69 us uncapped, 81 at 3, 79 at 2, 113 at
+    // 1; the iteration 101, 107, 125, 169).
     int blocks_per_sm[2] = {0, 2};
     double cell_scale = 1.0;
     int sp_tiles_c[K_NUM_SPARSE] = {0, 0, 0, 0};
@@ -1336,8 +1337,9 @@ static int minimize_impl(MechContext* c, const MechCGParams* p, MechResult* res)
     };
     if ((rc = build_graph())) return rc;
     long long graphs = 0;
-    // more line-search passes than any search within the call limits makes: the
-    // first kShortGraphs graphs have kGraphBlocks[0] passes, the others kGraphBlocks[1]
+    // a safety limit on the line-search passes, 16 for every force call allowed and
+    // 17,000 more: the first kShortGraphs graphs have kGraphBlocks[0] passes, the
+    // others kGraphBlocks[1]
     long long max_graphs = 0;
     for (int r = 0; r < c->R; ++r)
         max_graphs = std::max<long long>(
@@ -1879,7 +1881,14 @@ static int profile_impl(MechContext* c, int iters, MechProfile* o) {
     int rc;
     if (!c->have_lists && (rc = rebuild(c, 0.0, nullptr))) return rc;
     if ((rc = select_replicas(c, -1))) return rc;
+    // the line-search passes form their direction, as the first one of a search does
+    const std::vector<CGState> saved(c->h_st, c->h_st + c->R);
     c->h_fresh = false;
+    for (int r = 0; r < c->R; ++r) {
+        c->h_st[r].dPending = 1;
+        c->h_st[r].dIsF = c->h_st[r].backupPending = 0;
+    }
+    if ((rc = push_states(c))) return rc;
     const DevNet<Real> n = make_devnet<Real>(c);
     cudaStream_t s = c->stream;
     cudaEvent_t e0, e1;
@@ -1939,7 +1948,6 @@ static int profile_impl(MechContext* c, int iters, MechProfile* o) {
     // a line-search trial: positions x + lambda d formed and materialized on the fly
     o->ms_trial_energy_eval = timeit([&] { launch_energy<Real>(n, -1, sizeof(Real) == 4 ? kTrialBoth : 1, c->lanes()); });
     // every replica finished: each launch of an iteration block reads its phase and exits
-    const std::vector<CGState> saved(c->h_st, c->h_st + c->R);
     for (int r = 0; r < c->R; ++r) c->h_st[r].phase = PH_DONE;
     if ((rc = push_states(c))) return rc;
     o->ms_iteration_idle = timeit([&] {
