@@ -1,9 +1,7 @@
 // The per-replica reductions and CG step logic of the device-resident
 // minimizer (CGMethod.hpp:238-373 and :826-1743, ForceFieldManager.cpp:96-290;
-// paths relative to medyan-5.4.0/src), shared by the translation units whose
-// kernels end an evaluation: the separate finalizer kernels (one block per
-// replica) and, for a single replica, the last block of the kernel that
-// writes an evaluation's final partial sums.
+// paths relative to medyan-5.4.0/src), run by the finalizer kernels, one block
+// per replica, behind an evaluation's last partial sums.
 #pragma once
 
 #include "mech_device.cuh"

@@ -333,7 +333,7 @@ __device__ __forceinline__ float mixed_pair_energy(const Pos<float>& p1, const P
 
 // ---------------------------------------------------------------------------
 // FP64 engine: the reference's formulas for every pair, bound by the FP64 pipe
-// (a warp's FP64 instruction holds its SM sub-partition's pipe for ~70 cycles
+// (a warp's FP64 instruction holds its SM sub-partition's pipe for ~78 cycles
 // whatever the number of active lanes).  A pair per lane takes ~800 FP64
 // instructions for the energy and ~1,650 for the forces in one warp, so a few
 // pairs take as long as 608 warps of them (28 and 59 us).  Split over the four
@@ -1053,8 +1053,8 @@ static inline int ev_tiles_of(const DevNet<Real>& n, int* off) {
 }
 
 // Inside an evaluation (standalone = false) the work-list counts are zero on
-// entry: the evaluation's reduction kernel zeroes them for the next one, which
-// keeps a memset off the head of the excluded-volume lane.  A standalone
+// entry: the energy's reduction, or the force gather, has zeroed them behind
+// their last reader, which keeps a memset off the head of the excluded-volume lane.  A standalone
 // launch zeroes them first and leaves them as they end.  `L`, unless null, are
 // the evaluation's lanes: `s` is the side lane, and L->join is recorded behind
 // the chain.

@@ -8,11 +8,11 @@
 //   CGMethod.hpp:238-373 and :826-1743, CGMethod.cpp:317-360,
 //   MController.h:273-339 (recovery move).
 //
-// Filament forces are computed owner-side: a block loads its 256 beads plus a
-// two-bead halo into shared memory, evaluates every cylinder and bending
-// triple touching its beads once, and each bead sums its own terms in a fixed
-// order (the filament's, then the sparse force fields' through the CSR gather),
-// so no floating-point atomics are used.
+// Filament forces are computed owner-side: a block loads a tile's beads (254 in
+// mixed precision, 253 in FP64: kForceBeads) plus a two-bead halo into shared
+// memory, evaluates every cylinder and bending triple touching them once, and
+// each bead sums its own terms in a fixed order (the filament's, then the sparse
+// force fields' through the CSR gather), so no floating-point atomics are used.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kBlock) k_body_head(DevNet<Real> n) {
 
 // ---------------------------------------------------------------------------
 // FP64 engine: filament energy and forces.  Bound by the FP64 pipe (a warp's
-// FP64 instruction holds its sub-partition's pipe for ~70 cycles), so what
+// FP64 instruction holds its sub-partition's pipe for ~78 cycles), so what
 // counts is FP64 instructions per bead: every cylinder's vector, length and
 // reciprocal length is formed once and read by the bending terms on both of its
 // ends, comparisons are made on the bits of the numbers, and the sums of a warp
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kBlock) k_fil_force(DevNet<double> n, int want
 // reduced by k_finalize_force (a per-tile completion ticket on one address per
 // replica would serialize thousands of atomics).  Each block takes
 // kGatherTiles consecutive tiles and issues the loads of all of them before
-// the reduction.  FP64 engine: FP64-pipe bound (53 us on 1M beads, 94 us with a
+// the reduction.  FP64 engine: FP64-pipe bound (43 us on 1M beads, 94 us with a
 // tree per sum, and the maximum and the finiteness tests in FP64); the maximum
 // is formed on the bits.  The mixed engine's
 // version is k_force_gather_mx below.
@@ -1012,11 +1012,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_fil_energy_bulk(DevNet<float> n, 
 
 
 // ---------------------------------------------------------------------------
-// Mixed engine, bulk-staged filament forces: the same walk, with each
-// selected tile's positions (two-bead halo), constants and flags of
-// the neighbouring beads, previous forces and CSR offsets staged by
-// cp.async.bulk like k_fil_energy_bulk; the bead's gathered contributions are
-// contiguous in memory and read directly.
+// Mixed engine, bulk-staged filament forces: the same walk (k_fil_force_bulk).
 // ---------------------------------------------------------------------------
 constexpr int kBulkFXBeads = kFilTile + 8;    // tile + 2-bead halo, even-aligned ends
 constexpr int kBulkFPar = kFilTile + 4;       // constants of beads tb - 1 .. te

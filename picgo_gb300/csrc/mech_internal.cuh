@@ -429,7 +429,7 @@ int persistent_blocks(int device, int which, int per_sm);
 int set_error_text(int code, const std::string& msg);
 // excluded-volume kernels (mech_exvol.cu, one object per precision)
 // (standalone: zero the work-list counts first; inside an evaluation they are
-// zero on entry, reset by the evaluation's reduction kernel)
+// zero on entry, reset behind their last reader)
 template <typename Real> int launch_exvol_energy(const DevNet<Real>& n, int want, int trial, cudaStream_t s,
                                                  bool standalone, const Lanes* L = nullptr);
 template <typename Real> int launch_exvol_forces(const DevNet<Real>& n, int want, cudaStream_t s, bool standalone,
