@@ -280,15 +280,17 @@ __device__ void finalize_energy(const DevNet<Real>& n, int r, int trial, const R
 // Whether the direction F + beta F_prev, of a search that follows one along F_prev,
 // has lost conjugacy for certain: its slope F.F + beta F.F_prev is negative by more
 // than the pass that forms the direction can round it.  That pass adds rounded
-// products, whose magnitudes' sum is at most |F|^2 + beta |F| |F_prev|: ten roundings
-// of single precision at the most with compensated sums, and in FP64 as many as its
+// products, whose magnitudes' sum is at most |F|^2 + beta |F| |F_prev|, and that at
+// most |F|^2 + beta (|F|^2 + |F_prev|^2) / 2 (no roots in thread 0): ten roundings of
+// single precision at the most with compensated sums, and in FP64 as many as its
 // longest chain of additions has (60 with 1M beads).  The bound is 40 and 4,500 of
 // them.  Squares near underflow and an overflowing beta are left to the pass.
+// A call: inlined, the iterations that never get here took 0.1 us longer.
 template <typename Real>
-__device__ __forceinline__ bool conjugacy_lost(double ff, double ffp, double ff_prev, double beta) {
+__device__ __noinline__ bool conjugacy_lost(double ff, double ffp, double ff_prev, double beta) {
     constexpr double kRound = sizeof(Real) == 4 ? 2.4e-6 : 1e-12;
     return ff > 1e-30 && ff_prev > 1e-30 && beta < 1e30 &&
-           ff + beta * ffp < -kRound * (ff + beta * sqrt(ff) * sqrt(ff_prev));
+           ff + beta * ffp < -kRound * (ff + 0.5 * beta * (ff + ff_prev));
 }
 
 // CG bookkeeping after the forces (CGMethod.hpp:1540-1580): max |F|, beta.
@@ -327,7 +329,7 @@ __device__ __forceinline__ void force_step(CGState& S, double mx, double ff, dou
         // which starts the search over along F where it finds conjugacy lost.  A
         // search along F is followed by such a loss in most iterations of a long
         // run (20,517 of 21,105 with 4,000 cylinders), and there d . F is known
-        // already: no pass is spent on it (75.1 -> 47.9 us per iteration, FP64 92.5 -> 72.3).
+        // already: no pass is spent on it (75.1 -> 47 us per iteration, FP64 92.5 -> 71.6).
         // A pending backup is written by the pass that forms the direction.
         if (S.dIsF && !S.backupPending && conjugacy_lost<Real>(ff, ffp, ff_prev, beta)) {
             S.slope = ff;
